@@ -7,7 +7,7 @@
 // (the sum that sequential::BruteForce folds, particular/src/sequential.rs:189-193,
 // and that the wgpu shader tiles, particular/src/gpu/bruteforce_shared.wgsl:16-28).
 //
-// Three kernels:
+// Kernels:
 //  * bf_fast  : the throughput path. CTAs own an i-block of THREADS*K targets (K
 //               targets per thread) and a j-slice; source tiles of TILE bodies, in
 //               structure-of-arrays form (bf_to_soa), are staged in shared memory by
@@ -17,8 +17,8 @@
 //               FP32 inside a tile and compensated (two-sum) across tiles. j-slices
 //               (grid.y) keep all SMs busy at small N; their partials are combined by
 //               bf_fixup in a fixed order, so the result is deterministic.
-//  * bf_exact : one thread per target, sequential j order, IEEE sqrt/div and no
-//               contraction: bit-identical to sequential::BruteForce.
+//  * bf_ordered, bf_exact : IEEE sqrt/div, no contraction, sums in sequential j order:
+//               bit-identical to sequential::BruteForce (bf_ordered for f64 bodies too).
 //  * bf_f64   : the same formula in double, the error judge.
 #include "pt_common.cuh"
 #include "pt_f32x2.cuh"
@@ -324,56 +324,130 @@ __global__ void bf_f64_fixup(const double *__restrict__ part, int n_aff, int sli
     out[k] = acc;
 }
 
-// glam DVec3 bodies (impl_acceleration_cpu_scalar!(DVec3, f64) at
-// particular/src/gravity/impls/glam.rs:234 over gravity/impls/mod.rs:150-166, folded
-// as sequential.rs:189-193): the exact kernel in double. Every operation is an
-// explicitly rounded IEEE op and j runs in order, so the result is the reference's
-// bit for bit. Bodies are double[4] (x, y, z, mu); a tile of 256 sources is staged
-// in shared memory per step.
-__global__ void __launch_bounds__(THREADS)
-    bf_dvec3(const double *__restrict__ aff, int n_aff, const double *__restrict__ src, int n_src, double soft2,
-             int checked, double *__restrict__ out) {
-    __shared__ __align__(16) double tile[TILE][4];
-    const int i = blockIdx.x * THREADS + threadIdx.x;
-    double xi = 0.0, yi = 0.0, zi = 0.0;
-    if (i < n_aff) {
-        xi = aff[4 * size_t(i) + 0];
-        yi = aff[4 * size_t(i) + 1];
-        zi = aff[4 * size_t(i) + 2];
+// The exact per-pair terms, every operation an explicitly rounded IEEE op in the
+// reference's order: f32 (gravity/impls/mod.rs:156-165), with glam Vec3A's operand order
+// when VEC3A, and f64 for glam DVec3 bodies (impl_acceleration_cpu_scalar!(DVec3, f64) at
+// particular/src/gravity/impls/glam.rs:234).
+template <bool VEC3A>
+__device__ __forceinline__ void exact_term(float4 p, float xi, float yi, float zi, float soft2, int checked, float &ax,
+                                           float &ay, float &az) {
+    const float dx = __fsub_rn(p.x, xi), dy = __fsub_rn(p.y, yi), dz = __fsub_rn(p.z, zi);
+    const float n = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+    if (checked && n == 0.0f) {
+        ax = dx;
+        ay = dy;
+        az = dz;
+        return;
     }
-    double sx = 0.0, sy = 0.0, sz = 0.0;
-    for (int j0 = 0; j0 < n_src; j0 += TILE) {
-        const int cnt = min(TILE, n_src - j0);
-        __syncthreads();
-        for (int k = threadIdx.x; k < 4 * cnt; k += THREADS) (&tile[0][0])[k] = src[4 * size_t(j0) + k];
-        __syncthreads();
-#pragma unroll 1
-        for (int jj = 0; jj < cnt; ++jj) {
-            const double dx = __dsub_rn(tile[jj][0], xi);
-            const double dy = __dsub_rn(tile[jj][1], yi);
-            const double dz = __dsub_rn(tile[jj][2], zi);
-            const double n = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-            double ax, ay, az;
-            if (checked && n == 0.0) {
-                ax = dx;
-                ay = dy;
-                az = dz;
-            } else {
-                const double ns = __dadd_rn(n, soft2);
-                const double s = __ddiv_rn(tile[jj][3], __dmul_rn(ns, __dsqrt_rn(ns)));
-                ax = __dmul_rn(dx, s);
-                ay = __dmul_rn(dy, s);
-                az = __dmul_rn(dz, s);
+    const float ns = __fadd_rn(n, soft2);
+    const float den = __fmul_rn(ns, __fsqrt_rn(ns));
+    if (VEC3A) {
+        ax = __fdiv_rn(__fmul_rn(dx, p.w), den);
+        ay = __fdiv_rn(__fmul_rn(dy, p.w), den);
+        az = __fdiv_rn(__fmul_rn(dz, p.w), den);
+    } else {
+        const float s = __fdiv_rn(p.w, den);
+        ax = __fmul_rn(dx, s);
+        ay = __fmul_rn(dy, s);
+        az = __fmul_rn(dz, s);
+    }
+}
+
+struct Row64 {
+    double x, y, z, w;
+};
+
+template <bool VEC3A>
+__device__ __forceinline__ void exact_term(Row64 p, double xi, double yi, double zi, double soft2, int checked,
+                                           double &ax, double &ay, double &az) {
+    const double dx = __dsub_rn(p.x, xi), dy = __dsub_rn(p.y, yi), dz = __dsub_rn(p.z, zi);
+    const double n = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+    if (checked && n == 0.0) {
+        ax = dx;
+        ay = dy;
+        az = dz;
+        return;
+    }
+    const double ns = __dadd_rn(n, soft2);
+    const double s = __ddiv_rn(p.w, __dmul_rn(ns, __dsqrt_rn(ns)));
+    ax = __dmul_rn(dx, s);
+    ay = __dmul_rn(dy, s);
+    az = __dmul_rn(dz, s);
+}
+
+__device__ __forceinline__ float4 ord_load(const float *p, int j) { return __ldg(reinterpret_cast<const float4 *>(p) + j); }
+__device__ __forceinline__ Row64 ord_load(const double *p, int j) {  // rows are 8-byte aligned only
+    const double *q = p + 4 * size_t(j);
+    return Row64{__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3)};
+}
+__device__ __forceinline__ float ord_add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double ord_add(double a, double b) { return __dadd_rn(a, b); }
+
+// Targets per block, warps that form terms (one more adds them up), sources per round.
+// Swept over 4-32 targets, 4-16 warps and 32-128 sources: these are fastest or within 3 %
+// at N = 4999, 10007 and 32768 (f32: 80 / 239 / 2210 us; 32 targets: 189 / 389 / 2641) and
+// at N = 1000 and 6007 (f64: 95 / 2404 us; 32 targets: 315 / 3692).
+constexpr int ORD_TG = 8;
+constexpr int ORD_WARPS = 8;
+constexpr int ORD_J = 64;
+constexpr int ORD_THREADS = 32 * (ORD_WARPS + 1);
+static_assert(32 % ORD_TG == 0 && 3 * ORD_TG <= 32, "one warp adds the terms");
+
+// The reference's sum with its order kept and its terms formed in parallel. A target's
+// terms do not depend on each other, only their additions do: ORD_WARPS warps form the
+// terms of ORD_J sources for ORD_TG targets into one half of a shared buffer, while the
+// last warp, a thread per target and component, adds the previous round's terms in
+// ascending j from the other half. Results are the reference's bit for bit.
+// A thread per target that does both waits on its own divide and square root for every
+// source (10 % of the issue slots at N = 10007, 13 % of the FP64 pipe at N = 6007): f32
+// N = 1024 / 10007 / 32768 took 119 / 1126 / 3882 us and take 14 / 239 / 2210; f64 N =
+// 1000 / 6007 took 1247 / 7485 and take 95 / 2404, where the FP64 pipe is the bound (about
+// 40 of its lane-operations a pair).
+template <class T, bool VEC3A>
+__global__ void __launch_bounds__(ORD_THREADS)
+    bf_ordered(const T *__restrict__ aff, int n_aff, const T *__restrict__ src, int n_src, T soft2, int checked,
+               T *__restrict__ out) {
+    constexpr int TG = ORD_TG;
+    __shared__ T buf[2 * ORD_J * 3 * TG];
+    constexpr int SUB = 32 / TG;  // sources a warp takes at once
+    constexpr int STEP = ORD_WARPS * SUB;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int i0 = blockIdx.x * TG;
+    const int rounds = (n_src + ORD_J - 1) / ORD_J;
+    if (warp < ORD_WARPS) {
+        const int tg = lane % TG, sub = lane / TG;
+        const int i = min(i0 + tg, n_aff - 1);
+        const T xi = aff[4 * size_t(i)], yi = aff[4 * size_t(i) + 1], zi = aff[4 * size_t(i) + 2];
+        for (int r = 0; r <= rounds; ++r) {
+            if (r < rounds) {
+                T *b = buf + (r & 1) * (ORD_J * 3 * TG);
+#pragma unroll 2
+                for (int e = warp * SUB + sub; e < ORD_J; e += STEP) {
+                    const int j = r * ORD_J + e;
+                    if (j >= n_src) break;
+                    T ax, ay, az;
+                    exact_term<VEC3A>(ord_load(src, j), xi, yi, zi, soft2, checked, ax, ay, az);
+                    b[(e * 3 + 0) * TG + tg] = ax;
+                    b[(e * 3 + 1) * TG + tg] = ay;
+                    b[(e * 3 + 2) * TG + tg] = az;
+                }
             }
-            sx = __dadd_rn(sx, ax);
-            sy = __dadd_rn(sy, ay);
-            sz = __dadd_rn(sz, az);
+            __syncthreads();  // round r formed, round r - 1 added
         }
-    }
-    if (i < n_aff) {
-        out[3 * size_t(i) + 0] = sx;
-        out[3 * size_t(i) + 1] = sy;
-        out[3 * size_t(i) + 2] = sz;
+    } else {
+        const int k = threadIdx.x - 32 * ORD_WARPS;  // component k / TG of target k % TG
+        T s = T(0);
+        for (int r = 0; r <= rounds; ++r) {
+            if (r > 0 && k < 3 * TG) {
+                const T *b = buf + ((r - 1) & 1) * (ORD_J * 3 * TG) + k;
+                const int cnt = min(ORD_J, n_src - (r - 1) * ORD_J);
+#pragma unroll 8
+                for (int e = 0; e < cnt; ++e) s = ord_add(s, b[e * 3 * TG]);
+            }
+            __syncthreads();
+        }
+        const int i = i0 + k % TG;
+        if (k < 3 * TG && i < n_aff) out[3 * size_t(i) + k / TG] = s;
     }
 }
 
@@ -448,6 +522,20 @@ static Plan plan(const pt_ctx *ctx, int n_aff, int n_src, bool guard, int force_
     return p;
 }
 
+// Below this many targets the terms and the sum run in different warps (bf_ordered); from
+// here on a thread per target fills the chip and saves the trip through shared memory
+// (N = 50000: 4916 us ordered, 6233 a thread per target; N = 65535: 8238 and 9007; N =
+// 131071: 35452 and 25940).
+constexpr int ORD_MAX_AFF = 65536;
+
+template <class T, bool VEC3A>
+static int launch_ordered(pt_ctx *ctx, const T *aff, int n_aff, const T *src, int n_src, T soft2, int checked,
+                          T *out) {
+    bf_ordered<T, VEC3A><<<(n_aff + ORD_TG - 1) / ORD_TG, ORD_THREADS, 0, ctx->stream>>>(aff, n_aff, src, n_src, soft2,
+                                                                                        checked, out);
+    return check_launch(ctx, "bf_ordered");
+}
+
 struct Forced {
     int k = 0, s = 0;
 };
@@ -472,6 +560,11 @@ int bf_launch_f32(pt_ctx *ctx, const float4 *aff, int n_aff, const float4 *src, 
     }
     const float soft2 = softening * softening;
     if (flags & PT_BF_EXACT) {
+        if (n_aff < ORD_MAX_AFF) {
+            const float *a = reinterpret_cast<const float *>(aff), *b = reinterpret_cast<const float *>(src);
+            return flags & PT_BF_VEC3A ? launch_ordered<float, true>(ctx, a, n_aff, b, n_src, soft2, checked, out)
+                                       : launch_ordered<float, false>(ctx, a, n_aff, b, n_src, soft2, checked, out);
+        }
         dim3 grid((n_aff + THREADS - 1) / THREADS);
         if (flags & PT_BF_VEC3A) bf_exact<true><<<grid, THREADS, 0, st>>>(aff, n_aff, src, n_src, soft2, checked, out);
         else bf_exact<false><<<grid, THREADS, 0, st>>>(aff, n_aff, src, n_src, soft2, checked, out);
@@ -540,9 +633,7 @@ int bf_launch_dvec3(pt_ctx *ctx, const double *aff, int n_aff, const double *src
         return PT_OK;
     }
     mark(ctx, 1);
-    bf_dvec3<<<(n_aff + THREADS - 1) / THREADS, THREADS, 0, ctx->stream>>>(aff, n_aff, src, n_src,
-                                                                          softening * softening, checked, out);
-    PT_TRY(check_launch(ctx, "bf_dvec3"));
+    PT_TRY((launch_ordered<double, false>(ctx, aff, n_aff, src, n_src, softening * softening, checked, out)));
     mark(ctx, 2);
     return PT_OK;
 }
