@@ -8,13 +8,12 @@
 // and that the wgpu shader tiles, particular/src/gpu/bruteforce_shared.wgsl:16-28).
 //
 // Kernels:
-//  * bf_fast  : the throughput path. CTAs own an i-block of THREADS*K targets (K
-//               targets per thread) and a j-slice; source tiles of TILE bodies, in
-//               structure-of-arrays form (bf_to_soa), are staged in shared memory by
-//               cp.async through a STAGES-deep ring; every thread reads them as warp
-//               broadcasts and evaluates two pairs per packed f32x2 instruction
-//               (12 FMA-pipe lanes-ops and one MUFU rsqrt per pair). Sums are plain
-//               FP32 inside a tile and compensated (two-sum) across tiles. j-slices
+//  * bf_fast, bf_fast_ring : the throughput path. CTAs own an i-block of THREADS*K targets
+//               (K targets per thread) and a j-slice; source tiles of TILE bodies, in
+//               structure-of-arrays form, are staged in shared memory; every thread reads
+//               them as warp broadcasts and evaluates two pairs per packed f32x2
+//               instruction (12 FMA-pipe lane-ops and one MUFU rsqrt per pair). Sums are
+//               plain FP32 inside a tile and compensated (two-sum) across tiles. j-slices
 //               (grid.y) keep all SMs busy at small N; their partials are combined by
 //               bf_fixup in a fixed order, so the result is deterministic.
 //  * bf_ordered, bf_exact : IEEE sqrt/div, no contraction, sums in sequential j order:
@@ -24,6 +23,7 @@
 #include "pt_f32x2.cuh"
 
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 #include <cmath>
 
@@ -78,12 +78,253 @@ __device__ __forceinline__ void for_each_tile(float4 (*tiles)[TILE], const float
     cp_async_wait<0>();
 }
 
-// Sources in structure-of-arrays form (x[], y[], z[], mu[], each padded to a
-// multiple of TILE) so that one LDS.128 yields two packed source pairs.
+// A slice's last, shorter tile is added in plain FP32 runs of TAIL_RUN sources (padded to
+// whole runs). Where it is the slice's only tile every source is compensated: there is no
+// whole tile whose rounding would hide that of the runs.
+constexpr int TAIL_RUN = 8;
+
+// A tile of sources in structure-of-arrays form, so that one LDS.128 yields two packed
+// source pairs.
 struct SoaTile {
     float c[4][TILE];
 };
 
+// This thread's sources of tile t of [j0, j_end), past the end massless ones far away: they
+// add exactly 0 (r^2 overflows, 1 / r is 0).
+template <int TH>
+__device__ __forceinline__ void fetch_tile(float4 (&pre)[TILE / TH], const float4 *__restrict__ src, int j0, int j_end,
+                                           int t) {
+#pragma unroll
+    for (int c = 0; c < TILE / TH; ++c) {
+        const int j = j0 + t * TILE + c * TH + threadIdx.x;
+        pre[c] = j < j_end ? __ldg(src + j) : make_float4(1e30f, 1e30f, 1e30f, 0.f);
+    }
+}
+
+template <int TH>
+__device__ __forceinline__ void stage_tile(SoaTile &T, const float4 (&pre)[TILE / TH]) {
+#pragma unroll
+    for (int c = 0; c < TILE / TH; ++c) {
+        const int e = c * TH + threadIdx.x;
+        T.c[0][e] = pre[c].x;
+        T.c[1][e] = pre[c].y;
+        T.c[2][e] = pre[c].z;
+        T.c[3][e] = pre[c].w;
+    }
+}
+
+// bf_fast's inner loop is bound by the FMA pipe (12 lane-ops a pair: 82 % of its cycles at
+// N = 65536, the rest lost to operand reads and the two-sum folds). What else a call paid
+// for, and no longer does: the launch that laid the sources out, the coincidence test's
+// selects on every pair, and a scalar loop over the sources of a last, shorter tile
+// (1000003 targets x 3001 sources: unsoftened 1424 -> 1109 us, softened 1251 -> 1114; N =
+// 4999 45 -> 39 us).
+
+// Four sources against a thread's K targets, in packed lo/hi partials.
+template <int K, bool GUARD>
+__device__ __forceinline__ void quad(float4 x, float4 y, float4 z, float4 m, const f2 (&xi)[K], const f2 (&yi)[K],
+                                     const f2 (&zi)[K], f2 e2, f2 (&ax)[K], f2 (&ay)[K], f2 (&az)[K]) {
+    const f2 xa = pk2(x.x, x.y), xb = pk2(x.z, x.w);
+    const f2 ya = pk2(y.x, y.y), yb = pk2(y.z, y.w);
+    const f2 za = pk2(z.x, z.y), zb = pk2(z.z, z.w);
+    const f2 ma = pk2(m.x, m.y), mb = pk2(m.z, m.w);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        interact2<GUARD>(xa, ya, za, ma, xi[k], yi[k], zi[k], ax[k], ay[k], az[k], e2);
+        interact2<GUARD>(xb, yb, zb, mb, xi[k], yi[k], zi[k], ax[k], ay[k], az[k], e2);
+    }
+}
+
+template <int K, bool GUARD>
+__device__ __forceinline__ void tile_quad(const SoaTile &T, int q, const f2 (&xi)[K], const f2 (&yi)[K],
+                                          const f2 (&zi)[K], f2 e2, f2 (&ax)[K], f2 (&ay)[K], f2 (&az)[K]) {
+    quad<K, GUARD>(reinterpret_cast<const float4 *>(T.c[0])[q], reinterpret_cast<const float4 *>(T.c[1])[q],
+                   reinterpret_cast<const float4 *>(T.c[2])[q], reinterpret_cast<const float4 *>(T.c[3])[q], xi, yi, zi,
+                   e2, ax, ay, az);
+}
+
+// Adds a run's partials (quads [q0, q1) of the tile) to the targets' compensated sums and
+// zeroes them.
+// GUARD (checked, eps == 0): runs are evaluated without the test for coincidence, which
+// costs two selects per pair. A coincident pair then always makes the run's sum NaN
+// (0 times an infinite s, or 0 times NaN), so only a run whose sum is not finite is done
+// again with the test, by the threads that met it: one run per target that is its own
+// source. A sum that is not finite for another reason comes out the same again.
+template <int K, bool GUARD>
+__device__ __forceinline__ void fold_run(const SoaTile &T, int q0, int q1, const f2 (&xi)[K], const f2 (&yi)[K],
+                                         const f2 (&zi)[K], f2 e2, f2 (&ax)[K], f2 (&ay)[K], f2 (&az)[K],
+                                         float (&sx)[K], float (&sy)[K], float (&sz)[K], float (&cx)[K],
+                                         float (&cy)[K], float (&cz)[K]) {
+    const f2 zero2 = pk2(0.f, 0.f);
+    float tx[K], ty[K], tz[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        float l, h;
+        upk2(ax[k], l, h);
+        tx[k] = l + h;
+        upk2(ay[k], l, h);
+        ty[k] = l + h;
+        upk2(az[k], l, h);
+        tz[k] = l + h;
+    }
+    if (GUARD) {
+        bool redo = false;
+#pragma unroll
+        for (int k = 0; k < K; ++k) redo |= !(fabsf(tx[k]) + fabsf(ty[k]) + fabsf(tz[k]) <= FLT_MAX);
+        if (redo) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) ax[k] = ay[k] = az[k] = zero2;
+#pragma unroll 1
+            for (int q = q0; q < q1; ++q) tile_quad<K, true>(T, q, xi, yi, zi, e2, ax, ay, az);
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                float l, h;
+                upk2(ax[k], l, h);
+                tx[k] = l + h;
+                upk2(ay[k], l, h);
+                ty[k] = l + h;
+                upk2(az[k], l, h);
+                tz[k] = l + h;
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        two_sum_acc(sx[k], cx[k], tx[k]);
+        two_sum_acc(sy[k], cy[k], ty[k]);
+        two_sum_acc(sz[k], cz[k], tz[k]);
+        ax[k] = ay[k] = az[k] = zero2;
+    }
+}
+
+// Two-sum of packed sums: s + c tracks each half's running sum and its rounding errors.
+__device__ __forceinline__ void two_sum_acc2(f2 &s, f2 &c, f2 t) {
+    const f2 sn = add2(s, t);
+    const f2 bp = sub2(sn, s);
+    c = add2(c, add2(sub2(s, sub2(sn, bp)), sub2(t, bp)));
+    s = sn;
+}
+
+// The first cnt sources of a tile, each added with its rounding error kept: pairs of them
+// in packed sums, whose halves then enter the targets' sums.
+template <int K, bool GUARD>
+__device__ __forceinline__ void each_pair(const SoaTile &T, int cnt, const f2 (&xi)[K], const f2 (&yi)[K],
+                                          const f2 (&zi)[K], f2 e2, float (&sx)[K], float (&sy)[K], float (&sz)[K],
+                                          float (&cx)[K], float (&cy)[K], float (&cz)[K]) {
+    const f2 zero2 = pk2(0.f, 0.f);
+    f2 s[K][3], c[K][3];
+#pragma unroll
+    for (int k = 0; k < K; ++k) s[k][0] = s[k][1] = s[k][2] = c[k][0] = c[k][1] = c[k][2] = zero2;
+#pragma unroll 1
+    for (int e = 0; e < cnt; e += 2) {
+        const f2 x = *reinterpret_cast<const f2 *>(&T.c[0][e]), y = *reinterpret_cast<const f2 *>(&T.c[1][e]);
+        const f2 z = *reinterpret_cast<const f2 *>(&T.c[2][e]), m = *reinterpret_cast<const f2 *>(&T.c[3][e]);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            f2 ax = zero2, ay = zero2, az = zero2;
+            interact2<GUARD>(x, y, z, m, xi[k], yi[k], zi[k], ax, ay, az, e2);
+            two_sum_acc2(s[k][0], c[k][0], ax);
+            two_sum_acc2(s[k][1], c[k][1], ay);
+            two_sum_acc2(s[k][2], c[k][2], az);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        float *sum[3] = {&sx[k], &sy[k], &sz[k]}, *err[3] = {&cx[k], &cy[k], &cz[k]};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            float l, h, cl, ch;
+            upk2(s[k][a], l, h);
+            upk2(c[k][a], cl, ch);
+            two_sum_acc(*sum[a], *err[a], l);
+            two_sum_acc(*sum[a], *err[a], h);
+            *err[a] += cl + ch;
+        }
+    }
+}
+
+// Sources are read as rows and transposed on their way into shared memory, one tile ahead:
+// the next tile's rows are in registers while this tile is evaluated.
+// part (when non-null): [gridDim.y][2][n_aff] float4 = per-slice (sum, compensation).
+template <int K, bool GUARD>
+__global__ void __launch_bounds__(THREADS, K == 1 ? 8 : 1)
+    bf_fast(const float4 *__restrict__ aff, int n_aff, const float4 *__restrict__ src, int n_src, float eps2,
+            int slice_len, float4 *__restrict__ part, float *__restrict__ out) {
+    __shared__ __align__(16) SoaTile tiles[2];
+    const int i0 = blockIdx.x * (THREADS * K);
+    const int j0 = blockIdx.y * slice_len;
+    const int j_end = min(n_src, j0 + slice_len);
+    const int ntiles = (j_end - j0 + TILE - 1) / TILE;
+    float4 pre[TILE / THREADS];
+    fetch_tile<THREADS>(pre, src, j0, j_end, 0);
+
+    float sx[K], sy[K], sz[K], cx[K], cy[K], cz[K];
+    f2 xi2[K], yi2[K], zi2[K], ax[K], ay[K], az[K];
+    const f2 e2 = pk2(eps2, eps2);
+    const f2 zero2 = pk2(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int i = i0 + k * THREADS + threadIdx.x;
+        const float4 p = (i < n_aff) ? aff[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        xi2[k] = pk2(p.x, p.x);
+        yi2[k] = pk2(p.y, p.y);
+        zi2[k] = pk2(p.z, p.z);
+        ax[k] = ay[k] = az[k] = zero2;
+        sx[k] = sy[k] = sz[k] = 0.f;
+        cx[k] = cy[k] = cz[k] = 0.f;
+    }
+
+    const int whole = (j_end - j0) / TILE;
+    for (int t = 0; t < whole; ++t) {  // a whole tile is one plain FP32 run
+        SoaTile &T = tiles[t & 1];
+        stage_tile<THREADS>(T, pre);
+        __syncthreads();  // tile t visible; every thread is done with tile t - 1's other buffer
+        if (t + 1 < ntiles) fetch_tile<THREADS>(pre, src, j0, j_end, t + 1);
+        const float4 *X = reinterpret_cast<const float4 *>(T.c[0]);
+        const float4 *Y = reinterpret_cast<const float4 *>(T.c[1]);
+        const float4 *Z = reinterpret_cast<const float4 *>(T.c[2]);
+        const float4 *M = reinterpret_cast<const float4 *>(T.c[3]);
+#pragma unroll 2
+        for (int q = 0; q < TILE / 4; ++q) quad<K, false>(X[q], Y[q], Z[q], M[q], xi2, yi2, zi2, e2, ax, ay, az);
+        fold_run<K, GUARD>(T, 0, TILE / 4, xi2, yi2, zi2, e2, ax, ay, az, sx, sy, sz, cx, cy, cz);
+    }
+    if (whole < ntiles) {  // the last, shorter tile
+        SoaTile &T = tiles[whole & 1];
+        stage_tile<THREADS>(T, pre);
+        __syncthreads();
+        const int cnt = j_end - (j0 + whole * TILE);
+        if (whole == 0) {
+            each_pair<K, GUARD>(T, cnt, xi2, yi2, zi2, e2, sx, sy, sz, cx, cy, cz);
+        } else {
+#pragma unroll 1
+            for (int q = 0; 4 * q < cnt; q += TAIL_RUN / 4) {
+#pragma unroll
+                for (int r = 0; r < TAIL_RUN / 4; ++r)
+                    tile_quad<K, false>(T, q + r, xi2, yi2, zi2, e2, ax, ay, az);
+                fold_run<K, GUARD>(T, q, q + TAIL_RUN / 4, xi2, yi2, zi2, e2, ax, ay, az, sx, sy, sz, cx, cy, cz);
+            }
+        }
+    }
+
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int i = i0 + k * THREADS + threadIdx.x;
+        if (i >= n_aff) continue;
+        if (part) {
+            float4 *ps = part + size_t(blockIdx.y) * 2 * size_t(n_aff);
+            ps[i] = make_float4(sx[k], sy[k], sz[k], 0.f);
+            ps[size_t(n_aff) + i] = make_float4(cx[k], cy[k], cz[k], 0.f);
+        } else {
+            out[3 * size_t(i) + 0] = sx[k] + cx[k];
+            out[3 * size_t(i) + 1] = sy[k] + cy[k];
+            out[3 * size_t(i) + 2] = sz[k] + cz[k];
+        }
+    }
+}
+
+// The same sum for many sources without the coincidence test: sources converted once per
+// call (bf_to_soa) to x[], y[], z[], mu[] (each padded to a multiple of TILE), tiles staged
+// by cp.async through a STAGES-deep ring.
 __device__ __forceinline__ void load_tile_soa(SoaTile &stage, const float *__restrict__ soa, int n_pad, int j0,
                                               int j_end, int t) {
     const int base = j0 + t * TILE;
@@ -96,10 +337,9 @@ __device__ __forceinline__ void load_tile_soa(SoaTile &stage, const float *__res
     }
 }
 
-// part (when non-null): [gridDim.y][2][n_aff] float4 = per-slice (sum, compensation).
-template <int K, bool GUARD>
+template <int K>
 __global__ void __launch_bounds__(THREADS)
-    bf_fast(const float4 *__restrict__ aff, int n_aff, const float *__restrict__ soa, int n_src, int n_pad,
+    bf_fast_ring(const float4 *__restrict__ aff, int n_aff, const float *__restrict__ soa, int n_src, int n_pad,
             float eps2, int slice_len, float4 *__restrict__ part, float *__restrict__ out) {
     __shared__ __align__(16) SoaTile tiles[STAGES];
     const int i0 = blockIdx.x * (THREADS * K);
@@ -153,8 +393,8 @@ __global__ void __launch_bounds__(THREADS)
                 const f2 ma = pk2(m.x, m.y), mb = pk2(m.z, m.w);
 #pragma unroll
                 for (int k = 0; k < K; ++k) {
-                    interact2<GUARD>(xa, ya, za, ma, xi2[k], yi2[k], zi2[k], ax[k], ay[k], az[k], e2);
-                    interact2<GUARD>(xb, yb, zb, mb, xi2[k], yi2[k], zi2[k], ax[k], ay[k], az[k], e2);
+                    interact2<false>(xa, ya, za, ma, xi2[k], yi2[k], zi2[k], ax[k], ay[k], az[k], e2);
+                    interact2<false>(xb, yb, zb, mb, xi2[k], yi2[k], zi2[k], ax[k], ay[k], az[k], e2);
                 }
             }
 #pragma unroll
@@ -175,7 +415,7 @@ __global__ void __launch_bounds__(THREADS)
 #pragma unroll
                 for (int k = 0; k < K; ++k) {
                     float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-                    interact1<GUARD>(xj, yj, zj, mj, xi[k], yi[k], zi[k], a0, a1, a2, eps2);
+                    interact1<false>(xj, yj, zj, mj, xi[k], yi[k], zi[k], a0, a1, a2, eps2);
                     two_sum_acc(sx[k], cx[k], a0);
                     two_sum_acc(sy[k], cy[k], a1);
                     two_sum_acc(sz[k], cz[k], a2);
@@ -451,7 +691,7 @@ __global__ void __launch_bounds__(ORD_THREADS)
     }
 }
 
-using FastKernel = void (*)(const float4 *, int, const float *, int, int, float, int, float4 *, float *);
+using FastKernel = void (*)(const float4 *, int, const float4 *, int, float, int, float4 *, float *);
 
 template <int K>
 FastKernel pick(bool guard) {
@@ -466,6 +706,24 @@ FastKernel fast_kernel(int K, bool guard) {
     }
 }
 
+using RingKernel = void (*)(const float4 *, int, const float *, int, int, float, int, float4 *, float *);
+
+RingKernel ring_kernel(int K) {
+    switch (K) {
+        case 1: return bf_fast_ring<1>;
+        case 2: return bf_fast_ring<2>;
+        default: return bf_fast_ring<4>;
+    }
+}
+
+// Unguarded sums over this many sources and more take bf_fast_ring: it needs a launch to
+// lay the sources out, and its inner loop holds 9 blocks per SM where bf_fast's holds 8
+// (K = 1; N = 24001: 254 us against 263, N = 65000: 1593 against 1668, N = 131072: 6273
+// against 6510; at N = 16384 the launch costs more than the loop gains, 137 against 129).
+constexpr int RING_MIN_SRC = 20480;
+
+static bool use_ring(bool guard, int n_src) { return !guard && n_src >= RING_MIN_SRC; }
+
 struct Plan {
     int K = 4;
     int slices = 1;
@@ -473,15 +731,17 @@ struct Plan {
     int n_ib = 0;
 };
 
-// Occupancy of the fast kernels, cached per (K, guard).
-static int occupancy(int K, bool guard) {
-    static int cache[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+// Occupancy of the fast kernels, cached per (K, kernel): 0 = bf_fast, 1 = bf_fast guarded,
+// 2 = bf_fast_ring.
+static int occupancy(int K, int which) {
+    static int cache[3][3] = {};
     const int kk = K == 1 ? 0 : (K == 2 ? 1 : 2);
-    int &o = cache[kk][guard ? 1 : 0];
+    int &o = cache[kk][which];
     if (o == 0) {
         int v = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, fast_kernel(K, guard), THREADS, 0) != cudaSuccess || v < 1)
-            v = 1;
+        const void *f = which == 2 ? reinterpret_cast<const void *>(ring_kernel(K))
+                                   : reinterpret_cast<const void *>(fast_kernel(K, which == 1));
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, f, THREADS, 0) != cudaSuccess || v < 1) v = 1;
         o = v;
     }
     return o;
@@ -496,7 +756,7 @@ static Plan plan(const pt_ctx *ctx, int n_aff, int n_src, bool guard, int force_
     p.K = force_k ? force_k : (n_aff >= (1 << 18) ? 2 : 1);
     p.n_ib = (n_aff + THREADS * p.K - 1) / (THREADS * p.K);
     const int tiles = (n_src + TILE - 1) / TILE;
-    const long long slots = (long long)std::max(1, ctx->sm_count) * occupancy(p.K, guard);
+    const long long slots = (long long)std::max(1, ctx->sm_count) * occupancy(p.K, guard ? 1 : use_ring(guard, n_src) ? 2 : 0);
     int best_s = 1;
     double best_cost = 1e300;
     const int max_s = std::max(1, std::min(tiles, 256));
@@ -577,15 +837,20 @@ int bf_launch_f32(pt_ctx *ctx, const float4 *aff, int n_aff, const float4 *src, 
         PT_TRY(ensure(ctx, BUF_PART, sizeof(float4) * 2 * size_t(n_aff) * size_t(p.slices)));
         part = static_cast<float4 *>(ctx->bufs[BUF_PART].ptr);
     }
-    const int n_pad = (n_src + TILE - 1) / TILE * TILE;
-    PT_TRY(ensure(ctx, BUF_SOA, sizeof(float) * 4 * size_t(n_pad)));
-    float *soa = static_cast<float *>(ctx->bufs[BUF_SOA].ptr);
-    mark(ctx, 0);
-    bf_to_soa<<<(n_pad + 255) / 256, 256, 0, st>>>(src, n_src, n_pad, soa);
-    PT_TRY(check_launch(ctx, "bf_to_soa"));
-    mark(ctx, 1);
     dim3 grid(p.n_ib, p.slices);
-    fast_kernel(p.K, guard)<<<grid, THREADS, 0, st>>>(aff, n_aff, soa, n_src, n_pad, soft2, p.slice_len, part, out);
+    mark(ctx, 0);
+    if (use_ring(guard, n_src)) {
+        const int n_pad = (n_src + TILE - 1) / TILE * TILE;
+        PT_TRY(ensure(ctx, BUF_SOA, sizeof(float) * 4 * size_t(n_pad)));
+        float *soa = static_cast<float *>(ctx->bufs[BUF_SOA].ptr);
+        bf_to_soa<<<(n_pad + 255) / 256, 256, 0, st>>>(src, n_src, n_pad, soa);
+        PT_TRY(check_launch(ctx, "bf_to_soa"));
+        mark(ctx, 1);
+        ring_kernel(p.K)<<<grid, THREADS, 0, st>>>(aff, n_aff, soa, n_src, n_pad, soft2, p.slice_len, part, out);
+    } else {
+        mark(ctx, 1);
+        fast_kernel(p.K, guard)<<<grid, THREADS, 0, st>>>(aff, n_aff, src, n_src, soft2, p.slice_len, part, out);
+    }
     PT_TRY(check_launch(ctx, "bf_fast"));
     if (part) {
         bf_fixup<<<(n_aff + 255) / 256, 256, 0, st>>>(part, n_aff, p.slices, out);
@@ -854,14 +1119,18 @@ extern "C" int pt_bf_accel_f32_noalloc(const float *d_aff, size_t n_aff, const f
             p.slices = (ns + p.slice_len - 1) / p.slice_len;
         }
     }
-    const int n_pad = (ns + TILE - 1) / TILE * TILE;
-    float *soa = reinterpret_cast<float *>(scratch);
     float4 *part = p.slices > 1 ? reinterpret_cast<float4 *>(scratch + NOALLOC_SOA_BYTES) : nullptr;
-    bf_to_soa<<<(n_pad + 255) / 256, 256, 0, st>>>(reinterpret_cast<const float4 *>(d_src), ns, n_pad, soa);
-    PT_CUDA(cudaGetLastError());
     dim3 grid(p.n_ib, p.slices);
-    fast_kernel(p.K, guard)<<<grid, THREADS, 0, st>>>(reinterpret_cast<const float4 *>(d_aff), na, soa, ns, n_pad,
-                                                      soft2, p.slice_len, part, d_out);
+    const float4 *aff = reinterpret_cast<const float4 *>(d_aff), *src = reinterpret_cast<const float4 *>(d_src);
+    if (use_ring(guard, ns)) {
+        const int n_pad = (ns + TILE - 1) / TILE * TILE;
+        float *soa = reinterpret_cast<float *>(scratch);
+        bf_to_soa<<<(n_pad + 255) / 256, 256, 0, st>>>(src, ns, n_pad, soa);
+        PT_CUDA(cudaGetLastError());
+        ring_kernel(p.K)<<<grid, THREADS, 0, st>>>(aff, na, soa, ns, n_pad, soft2, p.slice_len, part, d_out);
+    } else {
+        fast_kernel(p.K, guard)<<<grid, THREADS, 0, st>>>(aff, na, src, ns, soft2, p.slice_len, part, d_out);
+    }
     PT_CUDA(cudaGetLastError());
     if (part) {
         bf_fixup<<<(na + 255) / 256, 256, 0, st>>>(part, na, p.slices, d_out);

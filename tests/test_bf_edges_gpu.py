@@ -35,3 +35,27 @@ def test_f64_sums_are_the_sequential_ones(res, oracle, n_aff, n_src):
     got = cuda.BruteForce(res, AccelerationSoftened(0.01), dvec3=True).compute(Between(aff, src))
     want = oracle.bf_dvec3(aff, src, 0.01, True)
     assert np.array_equal(got.view(np.uint64), want.view(np.uint64))
+
+
+# tiles of 256 sources, the last one in runs of 8, or each source compensated
+# where it is the only one; sources laid out beforehand from 20480 on
+# when no pair has to be tested for coincidence
+@pytest.mark.parametrize("n_src", [1, 2, 7, 15, 16, 17, 255, 256, 257, 271, 272, 273, 513, 20479, 20480])
+@pytest.mark.parametrize("soft", [0.0, 0.05])
+def test_fast_sums_at_tile_edges(res, oracle, n_src, soft):
+    src = bodies(n_src, n_src)
+    src[n_src // 2, 3] = 0.0  # a massless source
+    aff = bodies(333, 9)
+    k = min(n_src, 200)
+    aff[:k] = src[n_src - k:]  # targets that are sources, the last ones among them
+    it = AccelerationSoftened(soft) if soft else Acceleration.checked()
+    got = cuda.BruteForce(res, it).compute(Between(aff, src))
+    want = oracle.bf_f64(aff, src, soft, True)
+    # per pair 3 rsqrt factors (2^-22 each) and the differences; a run adds at most 128
+    # terms into each packed half: 1e-5 of the sum of the terms' magnitudes
+    d = src[None, :, :3].astype(np.float64) - aff[:, None, :3].astype(np.float64)
+    r2 = (d * d).sum(-1)
+    eps = float(np.float32(soft))
+    scale = (src[None, :, 3] * np.sqrt(r2) / np.where(r2 > 0, r2 + eps * eps, 1.0) ** 1.5).sum(1)
+    assert np.isfinite(got).all()
+    assert (np.abs(got - want).max(1) <= 1e-5 * scale + 1e-30).all()
