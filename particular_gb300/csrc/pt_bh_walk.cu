@@ -1479,22 +1479,35 @@ __global__ void __launch_bounds__(32 * MW_WARPS)
 
 // ---- the reference rule over DVec3 bodies (f64 method) -------------------------
 // As bh_walk_masked with one body per lane, in double: node data, widths and the
-// per-pair kernel (impl_acceleration_cpu_scalar!(DVec3, f64): d * (m / (n_s sqrt
-// n_s)), IEEE-rounded in the reference's order) are f64; accepted sets per body
-// are the reference's. Monopole only, as the reference.
-constexpr int W64_WARPS = 4;
+// per-pair kernel (impl_acceleration_cpu_scalar!(DVec3, f64): d * (m / (n_s sqrt n_s)))
+// are f64; accepted sets per body are the reference's. Monopole only, as the reference.
 constexpr int W64_STACK = 384;
+
+// m / (n_s sqrt(n_s)) without the FP64 square root and divide, which cost more than the rest
+// of the pair on a pipe that does two lane-operations a cycle: an FP32 reciprocal root y of
+// n_s, then the binomial series of n_s^(-3/2) = y^3 (1 - e)^(-3/2) about e = 1 - n_s y^2,
+// y^3 (1 + 3/2 e + 15/8 e^2). y has 24 bits, so y^2 is exact; |e| < 7e-7, so the series'
+// remainder is below 2^-60. The rounding errors left are those of the four operations that
+// the square root, product, divide form has too: against 80-bit values over 2e6 random pairs
+// 0.734 units of 2^-53 rms, where sqrt and divide give 0.735.
+__device__ __forceinline__ double inv_cube64(double ns, double m) {
+    if (!(ns > 1e-36 && ns < 1e36)) return __ddiv_rn(m, __dmul_rn(ns, __dsqrt_rn(ns)));  // outside FP32's range
+    const double y = double(rsqrt_ftz(float(ns)));
+    const double y2 = y * y;
+    const double e = fma(-ns, y2, 1.0);
+    const double my3 = m * (y2 * y);
+    return fma(my3, e * fma(1.875, e, 1.5), my3);
+}
 
 __device__ __forceinline__ void pair64(double px, double py, double pz, double cx, double cy, double cz, double m,
                                        double eps2, double &ax, double &ay, double &az) {
-    const double dx = __dsub_rn(cx, px), dy = __dsub_rn(cy, py), dz = __dsub_rn(cz, pz);
-    const double n = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+    const double dx = cx - px, dy = cy - py, dz = cz - pz;
+    const double n = fma(dx, dx, fma(dy, dy, dz * dz));
     if (n == 0.0) return;  // checked: d itself, which is zero
-    const double ns = __dadd_rn(n, eps2);
-    const double s = __ddiv_rn(m, __dmul_rn(ns, __dsqrt_rn(ns)));
-    ax = __dadd_rn(ax, __dmul_rn(dx, s));
-    ay = __dadd_rn(ay, __dmul_rn(dy, s));
-    az = __dadd_rn(az, __dmul_rn(dz, s));
+    const double s = inv_cube64(n + eps2, m);
+    ax = fma(dx, s, ax);
+    ay = fma(dy, s, ay);
+    az = fma(dz, s, az);
 }
 
 struct List64 {
@@ -1503,33 +1516,71 @@ struct List64 {
     unsigned mask[CAP];
 };
 
+// Transposes a 32 x 32 bit matrix held as one row per lane: afterwards bit r of lane c is
+// what bit c of lane r was.
+__device__ __forceinline__ unsigned transpose32(unsigned x) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1) {
+        const unsigned m = 0xffffffffu / ((1u << j) + 1u);  // the columns c with (c & j) == 0
+        const unsigned y = __shfl_xor_sync(0xffffffffu, x, j);
+        x = lane & j ? (x & ~m) | ((y & ~m) >> j) : (x & m) | ((y & m) << j);
+    }
+    return x;
+}
+
+// Each lane evaluates its own body's accepted entries of the list, in list order. The pair
+// costs some 40 lane-operations of an FP64 pipe that does two a cycle, so a lane whose body
+// does not accept an entry goes on to its own next entry instead of waiting for the lanes
+// whose bodies do: the list takes as many rounds as the body with the most accepted entries
+// has, not as many as it holds. (Entry by entry with the mask's lanes on, N = 50021 at theta
+// 0.5 took 11.9 ms through the host API, and 8.3 ms like this.) With LPB lanes to a body,
+// lane % LPB takes the entries e with e % LPB equal to it.
+template <int LPB>
 __device__ __forceinline__ void eval_list64(const List64 &Lst, int cnt, double px, double py, double pz, double eps2,
                                             double &ax, double &ay, double &az) {
     const int lane = threadIdx.x & 31;
+    constexpr int WORDS = List64::CAP / 32;
+    constexpr unsigned share = LPB == 1 ? 0xffffffffu : LPB == 2 ? 0x55555555u : 0x11111111u;
     __syncwarp();
-    for (int e = 0; e < cnt; ++e)
-        if ((Lst.mask[e] >> lane) & 1u) pair64(px, py, pz, Lst.f[0][e], Lst.f[1][e], Lst.f[2][e], Lst.f[3][e], eps2, ax, ay, az);
+    unsigned w[WORDS];  // bit e of word k: this lane's body accepts entry 32 k + e
+#pragma unroll
+    for (int k = 0; k < WORDS; ++k)
+        w[k] = transpose32(32 * k + lane < cnt ? Lst.mask[32 * k + lane] : 0u) & (share << (lane % LPB));
+    for (;;) {
+        int e = -1;
+#pragma unroll
+        for (int k = 0; k < WORDS; ++k)
+            if (e < 0 && w[k]) {
+                e = 32 * k + __ffs(w[k]) - 1;
+                w[k] &= w[k] - 1;
+            }
+        if (__all_sync(0xffffffffu, e < 0)) break;
+        if (e >= 0) pair64(px, py, pz, Lst.f[0][e], Lst.f[1][e], Lst.f[2][e], Lst.f[3][e], eps2, ax, ay, az);
+    }
     __syncwarp();
 }
 
-__global__ void __launch_bounds__(32 * W64_WARPS)
+// One warp per CTA, so that a finished warp's slot is refilled at once. LPB lanes share a
+// body (32 / LPB bodies per warp): they vote alike and split its accepted entries.
+template <int LPB>
+__global__ void __launch_bounds__(32)
     bh_walk64(const double4_32a *__restrict__ tbody, const uint32_t *__restrict__ tidx, int n_aff,
               const double4_32a *__restrict__ nodeA, const int4 *__restrict__ nodeB,
               const double4_32a *__restrict__ nodeG, const double4_32a *__restrict__ sbody,
               const int *__restrict__ counters, double th2, double eps2, double *__restrict__ out,
               unsigned long long *__restrict__ stats, int *__restrict__ err) {
-    __shared__ int4 s_stack[W64_WARPS][W64_STACK];
-    __shared__ List64 s_list[W64_WARPS];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int group = blockIdx.x * W64_WARPS + warp;
-    if (group * 32 >= n_aff) return;
-    const int t = group * 32 + lane;
+    __shared__ int4 stack[W64_STACK];
+    __shared__ List64 Lst;
+    const int lane = threadIdx.x;
+    const int group = blockIdx.x;
+    constexpr int BODIES = 32 / LPB;
+    if (group * BODIES >= n_aff) return;
+    const int t = group * BODIES + lane / LPB;
     const bool valid = t < n_aff;
-    const double4_32a p = tbody[valid ? t : group * 32];
+    const double4_32a p = tbody[valid ? t : group * BODIES];
     const unsigned lt = (1u << lane) - 1u;
     const unsigned valid_mask = __ballot_sync(0xffffffffu, valid);
-    int4 *stack = s_stack[warp];
-    List64 &Lst = s_list[warp];
     const int T = counters[1];
     double mn0 = p.x, mn1 = p.y, mn2 = p.z, mx0 = p.x, mx1 = p.y, mx2 = p.z;
 #pragma unroll
@@ -1628,7 +1679,7 @@ __global__ void __launch_bounds__(32 * W64_WARPS)
         const unsigned ms = __ballot_sync(0xffffffffu, single);
         const int ns = __popc(ms);
         if (Nl + ns > List64::CAP) {
-            eval_list64(Lst, Nl, p.x, p.y, p.z, eps2, ax, ay, az);
+            eval_list64<LPB>(Lst, Nl, p.x, p.y, p.z, eps2, ax, ay, az);
             Nl = 0;
         }
         if (single) {
@@ -1649,7 +1700,7 @@ __global__ void __launch_bounds__(32 * W64_WARPS)
             for (int base = 0; base < c; base += 32) {
                 const int n = min(32, c - base);
                 if (Nl + n > List64::CAP) {
-                    eval_list64(Lst, Nl, p.x, p.y, p.z, eps2, ax, ay, az);
+                    eval_list64<LPB>(Lst, Nl, p.x, p.y, p.z, eps2, ax, ay, az);
                     Nl = 0;
                 }
                 if (lane < n) {
@@ -1665,25 +1716,31 @@ __global__ void __launch_bounds__(32 * W64_WARPS)
         }
         __syncwarp();
     }
-    eval_list64(Lst, Nl, p.x, p.y, p.z, eps2, ax, ay, az);
+    eval_list64<LPB>(Lst, Nl, p.x, p.y, p.z, eps2, ax, ay, az);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         acc_pairs += __shfl_xor_sync(0xffffffffu, acc_pairs, o);
         visit_pairs += __shfl_xor_sync(0xffffffffu, visit_pairs, o);
     }
+#pragma unroll
+    for (int o = 1; o < LPB; o <<= 1) {  // the body's lanes
+        ax += __shfl_xor_sync(0xffffffffu, ax, o);
+        ay += __shfl_xor_sync(0xffffffffu, ay, o);
+        az += __shfl_xor_sync(0xffffffffu, az, o);
+    }
     if (failed) {  // no stackless fallback in f64: the bodies are NaN and the call fails
         ax = ay = az = __longlong_as_double(0x7ff8000000000000ll);
         if (lane == 0) atomicOr(err, 1);
     }
-    if (valid) {
+    if (valid && lane % LPB == 0) {
         const uint32_t o = tidx[t];
         out[3 * size_t(o) + 0] = ax;
         out[3 * size_t(o) + 1] = ay;
         out[3 * size_t(o) + 2] = az;
     }
     if (stats && lane == 0) {
-        atomicAdd(stats + 0, acc_pairs);
-        atomicAdd(stats + 1, visit_pairs);
+        atomicAdd(stats + 0, acc_pairs / LPB);
+        atomicAdd(stats + 1, visit_pairs / LPB);
         atomicAdd(stats + 2, 1ull);
     }
 }
@@ -1742,6 +1799,16 @@ int run(pt_ctx *ctx, const float4 *d_aff, int n_aff, const float4 *d_src, int n_
     return walk(ctx, S, tbody, tidx, n_aff, theta, softening, flags, d_out);
 }
 
+// Lanes that share a body in bh_walk64: as many as keep every warp resident at once (20 per
+// SM by registers). One warp of a small call is bound by its own FP64 latency, so more
+// warps, each with fewer list entries per lane, win until the chip is full (N = 5000 at
+// theta 0.6, host API, 1 / 2 / 4 lanes: 1995 / 1438 / 1207 us; N = 20000 2836 / 2327 / 2298);
+// beyond that they only repeat the traversal (N = 50021 at theta 0.9: 2458 / 2641 / 2934).
+static int lanes_per_body64(const pt_ctx *ctx, int n_aff) {
+    const long long slots = 20ll * std::max(1, ctx->sm_count) * 32;
+    return 4ll * n_aff <= slots ? 4 : 2ll * n_aff <= slots ? 2 : 1;
+}
+
 // The f64 method: build over DVec3 bodies, walk with the reference rule in double.
 int run64(pt_ctx *ctx, const double4_32a *d_aff, int n_aff, const double4_32a *d_src, int n_src,
                  double theta, double softening, double *d_out) {
@@ -1765,7 +1832,9 @@ int run64(pt_ctx *ctx, const double4_32a *d_aff, int n_aff, const double4_32a *d
     PT_CUDA(cudaMemsetAsync(stats, 0, 9 * sizeof(unsigned long long), st));
     PT_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
     mark(ctx, 1);
-    bh_walk64<<<(n_aff + 32 * W64_WARPS - 1) / (32 * W64_WARPS), 32 * W64_WARPS, 0, st>>>(
+    const int lpb = lanes_per_body64(ctx, n_aff);
+    auto kern = lpb == 4 ? bh_walk64<4> : lpb == 2 ? bh_walk64<2> : bh_walk64<1>;
+    kern<<<(n_aff + 32 / lpb - 1) / (32 / lpb), 32, 0, st>>>(
         tbody, tidx, n_aff, as<double4_32a>(S.nodeA64), as<int4>(S.nodeB), as<double4_32a>(S.nodeG64),
         as<double4_32a>(S.sbody64), as<int>(S.counters), theta * theta, softening * softening, d_out, stats, err);
     PT_TRY(check_launch(ctx, "bh_walk64"));
