@@ -112,9 +112,9 @@ void pt_bh_state_free(pt_ctx *ctx) {
     auto *S = static_cast<bh::State *>(ctx->bh);
     if (!S) return;
     prim_free(ctx, S->prims);
-    DevBuf *all[] = {&S->box_part, &S->box,    &S->keys,   &S->idx,    &S->sbody,   &S->flags,  &S->uscan,
+    DevBuf *all[] = {&S->box_part, &S->box,    &S->keys,   &S->idx,    &S->sbody,
                      &S->ukey,     &S->ufirst, &S->bfirst, &S->blast,  &S->bdelta,  &S->bparent, &S->lparent,
-                     &S->top,      &S->oparent, &S->loparent, &S->cnt, &S->pscan,   &S->pre,    &S->nkid, &S->kid, &S->cslot, &S->lslot, &S->levels, &S->by_level,
+                     &S->top,      &S->oparent, &S->loparent, &S->starts, &S->pscan, &S->pre, &S->kmask, &S->kid, &S->slot, &S->nspan, &S->spans,
                      &S->nodeA,  &S->nodeB,  &S->nodeQ,  &S->nodeG, &S->nodeR, &S->mom,     &S->tkeys,  &S->tidx,
                      &S->tbody,    &S->counters, &S->out,  &S->aff_h,  &S->src_h, &S->lrec, &S->lgroup,
                      &S->lnext,    &S->lpart,  &S->lhead, &S->lcentre, &S->lused, &S->sbody64, &S->nodeA64,

@@ -59,9 +59,9 @@ struct State {
     PrimScratch prims;
     DevBuf box_part, box;
     DevBuf keys, idx, sbody;
-    DevBuf flags, uscan, ukey, ufirst;
+    DevBuf ukey, ufirst;
     DevBuf bfirst, blast, bdelta, bparent, lparent, top, oparent, loparent;
-    DevBuf cnt, pscan, pre, nkid, kid, cslot, lslot, levels, by_level;
+    DevBuf starts, pscan, pre, kmask, kid, slot, nspan, spans;
     DevBuf nodeA, nodeB, nodeQ, nodeG, nodeR, mom;
     DevBuf sbody64, nodeA64, nodeG64, tbody64;  // the f64 (DVec3) method's bodies and nodes
     DevBuf tkeys, tidx, tbody;

@@ -18,13 +18,13 @@
 //     reference tree disappear: accepting a chain cell or its only child adds the
 //     same (COM, M), so the result is unchanged.
 //  6. cells are laid out in depth-first preorder with skip pointers (index after
-//     the subtree), leaves interleaved; every cell gets a list of its children and
-//     the cells are bucketed by octree level.
-//  7. moments (mass, centre of mass, second moment -> traceless quadrupole): the
-//     leaves, then one launch per octree level, deepest first, a thread per cell
-//     combining its children (parallel-axis theorem), in compensated FP32 for f32
-//     trees and FP64 for DVec3 trees.
+//     the subtree), leaves interleaved.
+//  7. moments (mass, centre of mass, second moment -> traceless quadrupole) bottom-up
+//     (parallel-axis theorem), in compensated FP32 for f32 trees and FP64 for DVec3 trees:
+//     the cells inside a chunk of 512 units by the block that lays the chunk out, from
+//     shared memory, the few larger ones block of chunks by block of chunks.
 #include "pt_bh.cuh"
+#include "pt_scan.cuh"
 
 #include <type_traits>
 
@@ -149,28 +149,28 @@ __global__ void gather_bodies(const V4 *__restrict__ src, const uint32_t *__rest
 }
 
 // ---- 4. unique keys -> leaf units ------------------------------------------
-__global__ void unit_flags(const uint64_t *__restrict__ keys, int n, uint32_t *__restrict__ flags) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) flags[k] = (k == 0 || keys[k] != keys[k - 1]) ? 1u : 0u;
-}
-
+// A scan over the sorted bodies of "the first body of its key" numbers the units.
+struct UnitHead {
+    const uint64_t *keys;
+    __device__ uint32_t operator()(int k) const { return (k == 0 || keys[k] != keys[k - 1]) ? 1u : 0u; }
+};
 // counters[0] = M (units)
-__global__ void unit_fill(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ flags,
-                          const uint32_t *__restrict__ uscan, int n, uint64_t *__restrict__ ukey,
-                          uint32_t *__restrict__ ufirst, int *__restrict__ counters) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    if (flags[k]) {
-        const uint32_t u = uscan[k];
+struct UnitFill {
+    const uint64_t *keys;
+    int n;
+    uint64_t *ukey;
+    uint32_t *ufirst;
+    int *counters;
+    __device__ void operator()(int k, uint32_t head, uint32_t u) const {
+        if (!head) return;
         ukey[u] = keys[k];
         ufirst[u] = uint32_t(k);
     }
-    if (k == 0) {
-        const uint32_t M = uscan[n];
+    __device__ void total(uint32_t M) const {
         ufirst[M] = uint32_t(n);
         counters[0] = int(M);
     }
-}
+};
 
 // ---- 5. Karras binary radix tree ---------------------------------------------
 __device__ __forceinline__ int kdelta(const uint64_t *__restrict__ k, int M, int i, int j) {
@@ -178,14 +178,54 @@ __device__ __forceinline__ int kdelta(const uint64_t *__restrict__ k, int M, int
     return __clzll(k[i] ^ k[j]) - 1;  // bit 63 is always 0: prefix length of the 63-bit keys
 }
 
-__global__ void karras(const uint64_t *__restrict__ ukey, const int *__restrict__ counters, int *__restrict__ bfirst,
-                       int *__restrict__ blast, int *__restrict__ bdelta, int *__restrict__ bparent,
-                       int *__restrict__ lparent) {
+// The moments are combined block by block of units (section 7): chunks of CHUNK units first,
+// then, stage by stage, blocks of SPAN_FAN of the blocks before. A cell's stage is the first
+// whose blocks hold its whole range.
+constexpr int CHUNK_SHIFT = 9;
+constexpr int CHUNK = 1 << CHUNK_SHIFT;
+constexpr int FAN_SHIFT = 6;
+// A cell of stage s >= 1 holds one of its block's 63 inner boundaries between blocks of the
+// stage before, and a boundary has one such cell per level at most.
+constexpr int SPAN_CAP = ((1 << FAN_SHIFT) - 1) * LEVELS;
+
+__host__ __device__ constexpr int stage_shift(int stage) { return CHUNK_SHIFT + FAN_SHIFT * stage; }
+__host__ __device__ inline int stage_blocks(int n, int stage) { return int(((long long)n + (1ll << stage_shift(stage)) - 1) >> stage_shift(stage)); }
+// Blocks of the stages 1 .. stage - 1 come first in the arrays of the blocks' cells.
+__host__ __device__ inline int stage_first(int n, int stage) {
+    int f = 0;
+    for (int s = 1; s < stage; ++s) f += stage_blocks(n, s);
+    return f;
+}
+// Stages after the chunks' until one block holds all n units.
+inline int stages(int n) {
+    int s = 0;
+    while (stage_blocks(n, s) > 1) ++s;
+    return s;
+}
+__device__ __forceinline__ int stage_of(int first, int last) {
+    int s = 0;
+    while (((long long)first >> stage_shift(s)) != ((long long)last >> stage_shift(s))) ++s;
+    return s;
+}
+
+// Binary node i: its range, its split's children's parents, and whether it is an octree
+// cell: the root, or a node whose common-prefix level (delta / 3) exceeds its parent's. The
+// parent's prefix is the longer of those that the range shares with its neighbours, so no
+// second pass over the parents is needed. top[i] = 1 + stage for a cell, else 0. Thread i
+// also clears what the next pass counts.
+__global__ void karras(const uint64_t *__restrict__ ukey, const int *__restrict__ counters, int n,
+                       int *__restrict__ bfirst, int *__restrict__ blast, int *__restrict__ bdelta,
+                       int *__restrict__ bparent, int *__restrict__ lparent, uint8_t *__restrict__ top,
+                       uint32_t *__restrict__ starts, uint32_t *__restrict__ kmask, int *__restrict__ nspan,
+                       int span_blocks) {
     const int M = counters[0];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i <= n) starts[i] = 0u;
+    if (i < span_blocks) nspan[i] = 0;
     if (i >= M - 1) return;
-    const int d = (kdelta(ukey, M, i, i + 1) - kdelta(ukey, M, i, i - 1)) >= 0 ? 1 : -1;
-    const int dmin = kdelta(ukey, M, i, i - d);
+    const int dn = kdelta(ukey, M, i, i + 1), dp = kdelta(ukey, M, i, i - 1);
+    const int d = dn >= dp ? 1 : -1;
+    const int dmin = min(dn, dp);
     int lmax = 2;
     while (kdelta(ukey, M, i, i + lmax * d) > dmin) lmax <<= 1;
     int l = 0;
@@ -206,16 +246,14 @@ __global__ void karras(const uint64_t *__restrict__ ukey, const int *__restrict_
     if (first == gamma) lparent[gamma] = i; else bparent[gamma] = i;
     if (last == gamma + 1) lparent[gamma + 1] = i; else bparent[gamma + 1] = i;
     if (i == 0) bparent[0] = -1;
-}
-
-// A binary node is an octree cell iff it is the root or its common-prefix level
-// (delta / 3) exceeds its parent's.
-__global__ void octree_top(const int *__restrict__ counters, const int *__restrict__ bdelta,
-                           const int *__restrict__ bparent, uint8_t *__restrict__ top) {
-    const int M = counters[0];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= M - 1) return;
-    top[i] = (i == 0 || bdelta[bparent[i]] / 3 < bdelta[i] / 3) ? 1 : 0;
+    const int dparent = max(dmin, kdelta(ukey, M, j, j + d));
+    uint8_t c = 0;
+    if (i == 0 || dparent / 3 < dnode / 3) {
+        const int stage = stage_of(first, last);
+        if (stage > 0) kmask[i] = 0u;
+        c = uint8_t(1 + stage);
+    }
+    top[i] = c;
 }
 
 __device__ __forceinline__ int climb(int p, const uint8_t *__restrict__ top, const int *__restrict__ bparent) {
@@ -223,57 +261,53 @@ __device__ __forceinline__ int climb(int p, const uint8_t *__restrict__ top, con
     return p;
 }
 
-// Octree parents, child counts (nkid, zeroed before) with each child's slot in its
-// parent's child list, the count of cells starting at each unit, and the count of
-// cells per octree level (levels[L], zeroed before).
-__global__ void octree_links(const int *__restrict__ counters, const int *__restrict__ bfirst,
+// The octant digit of a key at an octree level.
+__device__ __forceinline__ int digit_at(uint64_t key, int level) {
+    return int((key >> (3 * (LEVELS - 1 - level))) & 7u);
+}
+
+// Octree parents and the levels of the cells starting at each unit (a bit each); a cell that
+// spans chunks enters its block's list, and its children that come from earlier stages the
+// digits of its child list.
+__global__ void octree_links(const int *__restrict__ counters, int n, const int *__restrict__ bfirst,
                              const int *__restrict__ bparent, const int *__restrict__ lparent,
                              const uint8_t *__restrict__ top, const int *__restrict__ bdelta,
-                             int *__restrict__ oparent, int *__restrict__ loparent, uint32_t *__restrict__ cnt,
-                             int *__restrict__ nkid, uint8_t *__restrict__ cslot, uint8_t *__restrict__ lslot,
-                             int *__restrict__ levels) {
-    __shared__ int h[LEVELS];
-    if (threadIdx.x < LEVELS) h[threadIdx.x] = 0;
-    __syncthreads();
+                             const uint64_t *__restrict__ ukey, int *__restrict__ oparent, int *__restrict__ loparent,
+                             uint32_t *__restrict__ starts, uint32_t *__restrict__ kmask, int *__restrict__ nspan,
+                             int *__restrict__ spans) {
     const int M = counters[0];
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < M - 1 && top[k]) {
         const int op = (k == 0) ? -1 : climb(bparent[k], top, bparent);
+        const int b = bfirst[k];
         oparent[k] = op;
-        if (op >= 0) cslot[k] = uint8_t(atomicAdd(&nkid[op], 1));  // < 8: one child per octant
-        atomicAdd(&cnt[bfirst[k]], 1u);
-        atomicAdd(&h[bdelta[k] / 3], 1);
+        atomicOr(&starts[b], 1u << (bdelta[k] / 3));
+        if (op >= 0 && top[op] > top[k]) atomicOr(&kmask[op], 1u << digit_at(ukey[b], bdelta[op] / 3));
+        const int stage = top[k] - 1;
+        if (stage > 0) {
+            const int blk = stage_first(n, stage) + int((long long)b >> stage_shift(stage));
+            spans[size_t(blk) * SPAN_CAP + atomicAdd(&nspan[blk], 1)] = k;
+        }
     }
     if (k < M) {
         const int op = (M == 1) ? -1 : climb(lparent[k], top, bparent);
         loparent[k] = op;
-        if (op >= 0) lslot[k] = uint8_t(atomicAdd(&nkid[op], 1));
+        if (op >= 0 && top[op] > 1) atomicOr(&kmask[op], 1u << digit_at(ukey[k], bdelta[op] / 3));
     }
-    __syncthreads();
-    if (threadIdx.x < LEVELS && h[threadIdx.x]) atomicAdd(&levels[threadIdx.x], h[threadIdx.x]);
 }
 
-// levels[0 .. LEVELS) = cells per level, levels[LEVELS + 1 + L] = offset of level L in
-// by_level, levels[2 LEVELS + 2 + L] = its fill cursor.
-__global__ void level_offsets(int *__restrict__ levels) {
-    if (threadIdx.x != 0) return;
-    int acc = 0;
-    for (int L = 0; L < LEVELS; ++L) {
-        levels[LEVELS + 1 + L] = acc;
-        levels[2 * LEVELS + 2 + L] = acc;
-        acc += levels[L];
-    }
-    levels[2 * LEVELS + 1] = acc;
-}
+// The number of cells that start at each unit.
+struct CellStarts {
+    const uint32_t *starts;
+    __device__ uint32_t operator()(int b) const { return uint32_t(__popc(starts[b])); }
+};
 
 // ---- 7. moments ------------------------------------------------------------
-// Leaves first (in the layout pass, one thread per leaf unit), then the cells one
-// octree level per launch, deepest first, one thread per cell: every cell's children are complete
-// when it is combined, and it reads them from its child list, all loads at once.
-// The order of every sum is fixed by the tree. (A single bottom-up launch in which
-// the last child to arrive combined its parent was slower, 2.04 against 1.81 ms of
-// build at N = 4M: its climbing lanes wait on L2 with 4 of 32 lanes active.)
-// Children's records are read once, through L2 (ld.global.cg).
+// The leaves, then the cells, each after all its children, the children always summed in
+// preorder, so the order of every sum is fixed by the tree. A block of threads combines the
+// cells of one stage that lie in its block of units, deepest level first, from records in
+// shared memory: the chunks' in the layout pass, the few that span chunks stage by stage
+// (cells_span). Records that cross between stages are read through L2 (ld.global.cg).
 __device__ __forceinline__ float4 ld_cg(const float4 *p) { return __ldcg(p); }
 __device__ __forceinline__ double4_32a ld_cg(const double4_32a *p) {
     const double2 a = __ldcg(reinterpret_cast<const double2 *>(p));
@@ -319,29 +353,31 @@ __device__ __forceinline__ void store_quad(float4 *nodeQ, int pk, float sxx, flo
     nodeQ[2 * pk + 1] = make_float4(3.f * syz, 3.f * szz - tr, 0.f, 0.f);
 }
 
-__device__ __forceinline__ void store_cell(const Moments &m, int pk, Moments *mom, double4_32a *nodeA, float4 *) {
+__device__ __forceinline__ double4_32a store_cell(const Moments &m, int pk, Moments *mom, double4_32a *nodeA, float4 *) {
     mom[pk] = m;
-    nodeA[pk] = Prec<double>::make(m.cx, m.cy, m.cz, m.m);  // the f64 method is monopole only
+    return nodeA[pk] = Prec<double>::make(m.cx, m.cy, m.cz, m.m);  // the f64 method is monopole only
 }
 
-__device__ __forceinline__ void store_cell(const Moments &m, int pk, Rec32 *rec, float4 *nodeA, float4 *nodeQ) {
+__device__ __forceinline__ float4 store_cell(const Moments &m, int pk, Rec32 *rec, float4 *nodeA, float4 *nodeQ) {
     const float hx = float(m.cx), hy = float(m.cy), hz = float(m.cz), hm = float(m.m);
-    nodeA[pk] = make_float4(hx, hy, hz, hm);
+    const float4 a = make_float4(hx, hy, hz, hm);
+    nodeA[pk] = a;
     rec[pk].lo = make_float4(float(m.cx - hx), float(m.cy - hy), float(m.cz - hz), float(m.m - hm));
     rec[pk].s0 = make_float4(float(m.sxx), float(m.sxy), float(m.sxz), float(m.syy));
     rec[pk].s1 = make_float4(float(m.syz), float(m.szz), __int_as_float(int(m.count)), 0.f);
-    if (nodeQ)
-        store_quad(nodeQ, pk, float(m.sxx), float(m.sxy), float(m.sxz), float(m.syy), float(m.syz), float(m.szz));
+    store_quad(nodeQ, pk, float(m.sxx), float(m.sxy), float(m.sxz), float(m.syy), float(m.syz), float(m.szz));
+    return a;
 }
 
 // Leaves: a single body is its own cell data (no record: parents read nodeA; no
 // quadrupole: the walks read it for cells only); several (coincident, or closer
 // than the key resolution) get FP64 moments.
 template <class V4, class R>
-__device__ void leaf(int pk, int f, int e, const V4 *__restrict__ sbody, R *rec, V4 *nodeA, float4 *nodeQ) {
+__device__ __forceinline__ V4 leaf(int pk, int f, int e, const V4 *__restrict__ sbody, R *rec, V4 *nodeA, float4 *nodeQ) {
     if (e - f == 1) {
-        nodeA[pk] = sbody[f];
-        return;
+        const V4 p = sbody[f];
+        nodeA[pk] = p;
+        return p;
     }
     Moments m{};
     double sx = 0, sy = 0, sz = 0;
@@ -378,86 +414,62 @@ __device__ void leaf(int pk, int f, int e, const V4 *__restrict__ sbody, R *rec,
         m.syz += p.w * dy * dz;
         m.szz += p.w * dz * dz;
     }
-    store_cell(m, pk, rec, nodeA, nodeQ);
+    return store_cell(m, pk, rec, nodeA, nodeQ);
 }
 
-// Children of binary cell p: kid[8p .. 8p + nkid[p]) hold 2 x preorder index + 1 for
-// a single body (it has no record: its nodeA is its data). Filled in octree_links'
-// slot order, they are sorted back into preorder, the reference's child order, so
-// every sum runs in a fixed order; their loads are independent of each other.
-struct Kids {
-    int e[8];
-    int n;
+// One child of a cell, for the combination below.
+struct Child32 {
+    float4 a, lo, s0, s1;  // nodeA and Rec32
 };
+template <class T>
+using ChildOf = typename std::conditional<sizeof(T) == 4, Child32, Moments>::type;
 
-__device__ __forceinline__ void cswap(int &a, int &b) {
-    const int lo = min(a, b), hi = max(a, b);
-    a = lo, b = hi;
+// A single body, and a cell or several-body leaf from its record in global memory.
+__device__ __forceinline__ void child_single(float4 b, Child32 &c) {
+    c.a = b;
+    c.lo = c.s0 = make_float4(0.f, 0.f, 0.f, 0.f);
+    c.s1 = make_float4(0.f, 0.f, __int_as_float(1), 0.f);
 }
-
-__device__ __forceinline__ Kids load_kids(int p, const int *__restrict__ kid, const int *__restrict__ nkid) {
-    Kids K;
-    K.n = nkid[p];
-    const int4 a = reinterpret_cast<const int4 *>(kid)[2 * p];
-    const int4 b = reinterpret_cast<const int4 *>(kid)[2 * p + 1];
-    K.e[0] = a.x, K.e[1] = a.y, K.e[2] = a.z, K.e[3] = a.w, K.e[4] = b.x, K.e[5] = b.y, K.e[6] = b.z, K.e[7] = b.w;
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-        if (i >= K.n) K.e[i] = INT_MAX;
-    // Batcher's odd-even merge sort of 8 keys (19 compare-exchanges)
-    cswap(K.e[0], K.e[1]), cswap(K.e[2], K.e[3]), cswap(K.e[4], K.e[5]), cswap(K.e[6], K.e[7]);
-    cswap(K.e[0], K.e[2]), cswap(K.e[1], K.e[3]), cswap(K.e[4], K.e[6]), cswap(K.e[5], K.e[7]);
-    cswap(K.e[1], K.e[2]), cswap(K.e[5], K.e[6]);
-    cswap(K.e[0], K.e[4]), cswap(K.e[1], K.e[5]), cswap(K.e[2], K.e[6]), cswap(K.e[3], K.e[7]);
-    cswap(K.e[2], K.e[4]), cswap(K.e[3], K.e[5]);
-    cswap(K.e[1], K.e[2]), cswap(K.e[3], K.e[4]), cswap(K.e[5], K.e[6]);
-    return K;
+__device__ __forceinline__ void child_single(const double4_32a &b, Moments &c) {
+    c = Moments{};
+    c.cx = b.x, c.cy = b.y, c.cz = b.z, c.m = b.w, c.count = 1.0;
 }
+__device__ __forceinline__ void child_record(float4 a, const Rec32 *r, Child32 &c) {
+    c.a = a;
+    c.lo = ld_cg(&r->lo);
+    c.s0 = ld_cg(&r->s0);
+    c.s1 = ld_cg(&r->s1);
+}
+__device__ __forceinline__ void child_record(const double4_32a &, const Moments *r, Moments &c) { c = ld_cg(r); }
 
 // f32 trees: one pass over the children in FP32, sums about the cell's geometric
 // centre G, then moved to the centre of mass C by the parallel-axis rule
-// S_C = S_G - P P^T / M with P = sum m (c - G) = M (C - G).
-__device__ void cell(int pv, const Kids &K, const float4 *__restrict__ nodeG, Rec32 *rec, float4 *nodeA,
-                     float4 *nodeQ, int4 *nodeB) {
-    const float4 g = nodeG[pv];
+// S_C = S_G - P P^T / M with P = sum m (c - G) = M (C - G). *a gets nodeA.
+template <class Child>
+__device__ __forceinline__ Rec32 combine(float4 g, const Child &child, float4 *a) {
     float mh = 0.f, ml = 0.f, px = 0.f, py = 0.f, pz = 0.f;
     float sxx = 0.f, sxy = 0.f, sxz = 0.f, syy = 0.f, syz = 0.f, szz = 0.f;
     int count = 0;
-    // Straight-line over the 8 slots (no early exit): every slot's address is valid (an
-    // empty slot names the first child), so all the children's loads can be in flight at
-    // once; the sums still run slot by slot.
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const bool v = i < K.n;
-        const int ke = v ? K.e[i] : K.e[0];
-        const int c = ke >> 1;
-        const bool has_rec = v && !(ke & 1);
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 a = v ? ld_cg(nodeA + c) : zero;
-        float4 lo = zero, s0 = zero, s1 = zero;
-        int cn = 1;
-        if (has_rec) {
-            lo = ld_cg(&rec[c].lo);
-            s0 = ld_cg(&rec[c].s0);
-            s1 = ld_cg(&rec[c].s1);
-            cn = __float_as_int(s1.z);
-        }
-        if (!v) continue;
-        const float dx = __fsub_rn(a.x, g.x) + lo.x, dy = __fsub_rn(a.y, g.y) + lo.y, dz = __fsub_rn(a.z, g.z) + lo.z;
+        Child32 c;
+        if (!child(i, c)) continue;
+        const float dx = __fsub_rn(c.a.x, g.x) + c.lo.x, dy = __fsub_rn(c.a.y, g.y) + c.lo.y,
+                    dz = __fsub_rn(c.a.z, g.z) + c.lo.z;
         float e;
-        mh = two_sum(mh, a.w, e);
-        ml += e + lo.w;
-        const float mx = a.w * dx, my = a.w * dy, mz = a.w * dz;
+        mh = two_sum(mh, c.a.w, e);
+        ml += e + c.lo.w;
+        const float mx = c.a.w * dx, my = c.a.w * dy, mz = c.a.w * dz;
         px += mx;
         py += my;
         pz += mz;
-        sxx += s0.x + mx * dx;
-        sxy += s0.y + mx * dy;
-        sxz += s0.z + mx * dz;
-        syy += s0.w + my * dy;
-        syz += s1.x + my * dz;
-        szz += s1.y + mz * dz;
-        count += cn;
+        sxx += c.s0.x + mx * dx;
+        sxy += c.s0.y + mx * dy;
+        sxz += c.s0.z + mx * dz;
+        syy += c.s0.w + my * dy;
+        syz += c.s1.x + my * dz;
+        szz += c.s1.y + mz * dz;
+        count += __float_as_int(c.s1.z);
     }
     float e;
     const float M = two_sum(mh, ml, e);
@@ -474,66 +486,48 @@ __device__ void cell(int pv, const Kids &K, const float4 *__restrict__ nodeG, Re
         szz -= pz * oz;
     } else {  // massless: plain mean of the bodies (gravity/impls/mod.rs:127-129), a rare second pass
         float ux = 0.f, uy = 0.f, uz = 0.f;
-#pragma unroll
         for (int i = 0; i < 8; ++i) {
-            if (i >= K.n) break;
-            const int c = K.e[i] >> 1;
-            const float4 a = ld_cg(nodeA + c);
-            float4 lo = make_float4(0.f, 0.f, 0.f, 0.f);
-            float cn = 1.f;
-            if (!(K.e[i] & 1)) {
-                lo = ld_cg(&rec[c].lo);
-                cn = float(__float_as_int(ld_cg(&rec[c].s1).z));
-            }
-            ux += cn * (__fsub_rn(a.x, g.x) + lo.x);
-            uy += cn * (__fsub_rn(a.y, g.y) + lo.y);
-            uz += cn * (__fsub_rn(a.z, g.z) + lo.z);
+            Child32 c;
+            if (!child(i, c)) continue;
+            const float cn = float(__float_as_int(c.s1.z));
+            ux += cn * (__fsub_rn(c.a.x, g.x) + c.lo.x);
+            uy += cn * (__fsub_rn(c.a.y, g.y) + c.lo.y);
+            uz += cn * (__fsub_rn(c.a.z, g.z) + c.lo.z);
         }
         ox = ux / float(count), oy = uy / float(count), oz = uz / float(count);
     }
     float ex, ey, ez;
     const float hx = two_sum(g.x, ox, ex), hy = two_sum(g.y, oy, ey), hz = two_sum(g.z, oz, ez);
-    nodeA[pv] = make_float4(hx, hy, hz, M);
-    // a cell's nodeB.w (a leaf's body count) holds (M w^3)^(2/5): the error-bound
-    // opening radius^2 is this times (alpha |a|)^(-2/5) of the walking group
-    nodeB[pv].w = __float_as_int(M > 0.f ? __powf(M * g.w * g.w * g.w, 0.4f) : 0.f);
-    rec[pv].lo = make_float4(ex, ey, ez, Ml);
-    rec[pv].s0 = make_float4(sxx, sxy, sxz, syy);
-    rec[pv].s1 = make_float4(syz, szz, __int_as_float(count), 0.f);
-    if (nodeQ) store_quad(nodeQ, pv, sxx, sxy, sxz, syy, syz, szz);
+    *a = make_float4(hx, hy, hz, M);
+    Rec32 r;
+    r.lo = make_float4(ex, ey, ez, Ml);
+    r.s0 = make_float4(sxx, sxy, sxz, syy);
+    r.s1 = make_float4(syz, szz, __int_as_float(count), 0.f);
+    return r;
 }
 
 // f64 trees (DVec3 bodies): the same combination in FP64.
-__device__ void cell(int pv, const Kids &K, const double4_32a *__restrict__ nodeG, Moments *mom,
-                     double4_32a *nodeA, float4 *, int4 *) {
-    const double4_32a g = nodeG[pv];
+template <class Child>
+__device__ __forceinline__ Moments combine(double4_32a g, const Child &child, double4_32a *a) {
     const double gx = g.x, gy = g.y, gz = g.z;
     Moments m{};
     double px = 0, py = 0, pz = 0;
-    for (int i = 0; i < K.n; ++i) {
-        const int c = K.e[i] >> 1;
-        double cx, cy, cz, cmm, cn, sxx = 0, sxy = 0, sxz = 0, syy = 0, syz = 0, szz = 0;
-        if (K.e[i] & 1) {
-            const double4_32a a = ld_cg(nodeA + c);
-            cx = a.x, cy = a.y, cz = a.z, cmm = a.w, cn = 1.0;
-        } else {
-            const Moments cm = ld_cg(mom + c);
-            cx = cm.cx, cy = cm.cy, cz = cm.cz, cmm = cm.m, cn = cm.count;
-            sxx = cm.sxx, sxy = cm.sxy, sxz = cm.sxz, syy = cm.syy, syz = cm.syz, szz = cm.szz;
-        }
-        const double dx = cx - gx, dy = cy - gy, dz = cz - gz;
-        m.m += cmm;
-        m.count += cn;
-        const double mx = cmm * dx, my = cmm * dy, mz = cmm * dz;
+    for (int i = 0; i < 8; ++i) {
+        Moments c;
+        if (!child(i, c)) continue;
+        const double dx = c.cx - gx, dy = c.cy - gy, dz = c.cz - gz;
+        m.m += c.m;
+        m.count += c.count;
+        const double mx = c.m * dx, my = c.m * dy, mz = c.m * dz;
         px += mx;
         py += my;
         pz += mz;
-        m.sxx += sxx + mx * dx;
-        m.sxy += sxy + mx * dy;
-        m.sxz += sxz + mx * dz;
-        m.syy += syy + my * dy;
-        m.syz += syz + my * dz;
-        m.szz += szz + mz * dz;
+        m.sxx += c.sxx + mx * dx;
+        m.sxy += c.sxy + mx * dy;
+        m.sxz += c.sxz + mx * dz;
+        m.syy += c.syy + my * dy;
+        m.syz += c.syz + my * dz;
+        m.szz += c.szz + mz * dz;
     }
     if (m.m != 0.0) {
         const double inv = 1.0 / m.m;
@@ -549,140 +543,445 @@ __device__ void cell(int pv, const Kids &K, const double4_32a *__restrict__ node
         m.szz -= pz * oz;
     } else {  // massless: plain mean of the bodies (gravity/impls/mod.rs:127-129), a rare second pass
         double ux = 0, uy = 0, uz = 0;
-        for (int i = 0; i < K.n; ++i) {
-            const int c = K.e[i] >> 1;
-            double cx, cy, cz, cn;
-            if (K.e[i] & 1) {
-                const double4_32a a = ld_cg(nodeA + c);
-                cx = a.x, cy = a.y, cz = a.z, cn = 1.0;
-            } else {
-                const Moments cm = ld_cg(mom + c);
-                cx = cm.cx, cy = cm.cy, cz = cm.cz, cn = cm.count;
-            }
-            ux += cn * (cx - gx);
-            uy += cn * (cy - gy);
-            uz += cn * (cz - gz);
+        for (int i = 0; i < 8; ++i) {
+            Moments c;
+            if (!child(i, c)) continue;
+            ux += c.count * (c.cx - gx);
+            uy += c.count * (c.cy - gy);
+            uz += c.count * (c.cz - gz);
         }
         m.cx = gx + ux / m.count;
         m.cy = gy + uy / m.count;
         m.cz = gz + uz / m.count;
     }
-    store_cell(m, pv, mom, nodeA, nullptr);
+    *a = Prec<double>::make(m.cx, m.cy, m.cz, m.m);
+    return m;
+}
+
+// The same combinations by eight neighbouring lanes, one child to a lane (has: this lane has
+// one): the children's loads are all in flight and their sums form a tree, the same one
+// every time. All 32 lanes of the warp take part, each eight of them with a cell of its own;
+// every lane gets the result.
+__device__ __forceinline__ float sum8(float v) {
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ double sum8(double v) {
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ int sum8(int v) {
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__device__ __forceinline__ Rec32 combine8(float4 g, bool has, const Child32 &c, float4 *a) {
+    float dx = 0.f, dy = 0.f, dz = 0.f, m = 0.f, ml = 0.f;
+    int cn = 0;
+    if (has) {
+        dx = __fsub_rn(c.a.x, g.x) + c.lo.x;
+        dy = __fsub_rn(c.a.y, g.y) + c.lo.y;
+        dz = __fsub_rn(c.a.z, g.z) + c.lo.z;
+        m = c.a.w;
+        ml = c.lo.w;
+        cn = __float_as_int(c.s1.z);
+    }
+    const float mx = m * dx, my = m * dy, mz = m * dz;
+    const float px = sum8(mx), py = sum8(my), pz = sum8(mz);
+    float sxx = sum8((has ? c.s0.x : 0.f) + mx * dx), sxy = sum8((has ? c.s0.y : 0.f) + mx * dy),
+          sxz = sum8((has ? c.s0.z : 0.f) + mx * dz), syy = sum8((has ? c.s0.w : 0.f) + my * dy),
+          syz = sum8((has ? c.s1.x : 0.f) + my * dz), szz = sum8((has ? c.s1.y : 0.f) + mz * dz);
+    const int count = sum8(cn);
+    float mh = m, e;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        const float oh = __shfl_xor_sync(0xffffffffu, mh, o), ol = __shfl_xor_sync(0xffffffffu, ml, o);
+        mh = two_sum(mh, oh, e);
+        ml = (ml + ol) + e;
+    }
+    const float M = two_sum(mh, ml, e);
+    const float Ml = e;
+    float ux = 0.f, uy = 0.f, uz = 0.f;
+    if (__any_sync(0xffffffffu, M == 0.f)) {  // massless: plain mean of the bodies (gravity/impls/mod.rs:127-129)
+        ux = sum8(float(cn) * dx);
+        uy = sum8(float(cn) * dy);
+        uz = sum8(float(cn) * dz);
+    }
+    float ox, oy, oz;
+    if (M != 0.f) {
+        const float inv = 1.f / M;
+        ox = px * inv, oy = py * inv, oz = pz * inv;  // C - G
+        sxx -= px * ox;
+        sxy -= px * oy;
+        sxz -= px * oz;
+        syy -= py * oy;
+        syz -= py * oz;
+        szz -= pz * oz;
+    } else {
+        const float k = float(max(count, 1));
+        ox = ux / k, oy = uy / k, oz = uz / k;
+    }
+    float ex, ey, ez;
+    const float hx = two_sum(g.x, ox, ex), hy = two_sum(g.y, oy, ey), hz = two_sum(g.z, oz, ez);
+    *a = make_float4(hx, hy, hz, M);
+    Rec32 r;
+    r.lo = make_float4(ex, ey, ez, Ml);
+    r.s0 = make_float4(sxx, sxy, sxz, syy);
+    r.s1 = make_float4(syz, szz, __int_as_float(count), 0.f);
+    return r;
+}
+
+__device__ __forceinline__ Moments combine8(double4_32a g, bool has, const Moments &c, double4_32a *a) {
+    double dx = 0, dy = 0, dz = 0, m = 0, cn = 0;
+    if (has) dx = c.cx - g.x, dy = c.cy - g.y, dz = c.cz - g.z, m = c.m, cn = c.count;
+    const double mx = m * dx, my = m * dy, mz = m * dz;
+    Moments r{};
+    r.m = sum8(m);
+    r.count = sum8(cn);
+    const double px = sum8(mx), py = sum8(my), pz = sum8(mz);
+    r.sxx = sum8((has ? c.sxx : 0.0) + mx * dx), r.sxy = sum8((has ? c.sxy : 0.0) + mx * dy);
+    r.sxz = sum8((has ? c.sxz : 0.0) + mx * dz), r.syy = sum8((has ? c.syy : 0.0) + my * dy);
+    r.syz = sum8((has ? c.syz : 0.0) + my * dz), r.szz = sum8((has ? c.szz : 0.0) + mz * dz);
+    double ux = 0, uy = 0, uz = 0;
+    if (__any_sync(0xffffffffu, r.m == 0.0)) ux = sum8(cn * dx), uy = sum8(cn * dy), uz = sum8(cn * dz);
+    if (r.m != 0.0) {
+        const double inv = 1.0 / r.m;
+        const double ox = px * inv, oy = py * inv, oz = pz * inv;  // C - G
+        r.cx = g.x + ox;
+        r.cy = g.y + oy;
+        r.cz = g.z + oz;
+        r.sxx -= px * ox;
+        r.sxy -= px * oy;
+        r.sxz -= px * oz;
+        r.syy -= py * oy;
+        r.syz -= py * oz;
+        r.szz -= pz * oz;
+    } else {
+        const double k = fmax(r.count, 1.0);
+        r.cx = g.x + ux / k;
+        r.cy = g.y + uy / k;
+        r.cz = g.z + uz / k;
+    }
+    *a = Prec<double>::make(r.cx, r.cy, r.cz, r.m);
+    return r;
+}
+
+// A combined cell's node data (w its width). A cell's nodeB.w (a leaf's body count) holds
+// (M w^3)^(2/5): the error-bound opening radius^2 is this times (alpha |a|)^(-2/5) of the
+// walking group.
+__device__ __forceinline__ void put_cell(int pk, float w, float4 a, const Rec32 &r, float4 *nodeA, float4 *nodeQ,
+                                         int4 *nodeB) {
+    nodeA[pk] = a;
+    nodeB[pk].w = __float_as_int(a.w > 0.f ? __powf(a.w * w * w * w, 0.4f) : 0.f);
+    store_quad(nodeQ, pk, r.s0.x, r.s0.y, r.s0.z, r.s0.w, r.s1.x, r.s1.y);
+}
+__device__ __forceinline__ void put_cell(int pk, double, double4_32a a, const Moments &, double4_32a *nodeA, float4 *,
+                                         int4 *) {
+    nodeA[pk] = a;  // the f64 method is monopole only
 }
 
 template <class T>
 using Record = typename std::conditional<sizeof(T) == 4, Rec32, Moments>::type;
 
-// ---- 6. preorder layout (and the leaves' records) ---------------------------
+// Records of N cells in shared memory. Until a cell is combined its record holds its box
+// (centre, width).
+template <class T, int N>
+struct Records;
+template <int N>
+struct Records<float, N> {
+    float4 f[4][N];  // nodeA, lo, s0, s1
+    __device__ __forceinline__ void set_box(int l, float4 g) { f[0][l] = g; }
+    __device__ __forceinline__ float4 box(int l) const { return f[0][l]; }
+    __device__ __forceinline__ void set(int l, float4 a, const Rec32 &r) {
+        f[0][l] = a, f[1][l] = r.lo, f[2][l] = r.s0, f[3][l] = r.s1;
+    }
+    __device__ __forceinline__ void get(int l, Child32 &c) const {
+        c.a = f[0][l], c.lo = f[1][l], c.s0 = f[2][l], c.s1 = f[3][l];
+    }
+};
+template <int N>
+struct Records<double, N> {
+    double f[11][N];
+    __device__ __forceinline__ void set_box(int l, double4_32a g) {
+        f[0][l] = g.x, f[1][l] = g.y, f[2][l] = g.z, f[3][l] = g.w;
+    }
+    __device__ __forceinline__ double4_32a box(int l) const { return Prec<double>::make(f[0][l], f[1][l], f[2][l], f[3][l]); }
+    __device__ __forceinline__ void set(int l, double4_32a, const Moments &r) {
+        f[0][l] = r.m, f[1][l] = r.cx, f[2][l] = r.cy, f[3][l] = r.cz, f[4][l] = r.sxx, f[5][l] = r.sxy;
+        f[6][l] = r.sxz, f[7][l] = r.syy, f[8][l] = r.syz, f[9][l] = r.szz, f[10][l] = r.count;
+    }
+    __device__ __forceinline__ void get(int l, Moments &c) const {
+        c.m = f[0][l], c.cx = f[1][l], c.cy = f[2][l], c.cz = f[3][l], c.sxx = f[4][l], c.sxy = f[5][l];
+        c.sxz = f[6][l], c.syy = f[7][l], c.syz = f[8][l], c.szz = f[9][l], c.count = f[10][l];
+    }
+};
+
+// Cells bucketed by octree level in shared memory: count with add(), then every thread of the
+// block calls offsets(), then place().
+template <int N>
+struct LevelLists {
+    uint16_t list[N];
+    int cnt[LEVELS], start[LEVELS + 1];
+    __device__ __forceinline__ void clear() {
+        if (threadIdx.x < LEVELS) cnt[threadIdx.x] = 0;
+    }
+    __device__ __forceinline__ int add(int level) { return atomicAdd(&cnt[level], 1); }
+    __device__ __forceinline__ void offsets() {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int acc = 0;
+            for (int L = 0; L < LEVELS; ++L) {
+                start[L] = acc;
+                acc += cnt[L];
+            }
+            start[LEVELS] = acc;
+        }
+        __syncthreads();
+    }
+    __device__ __forceinline__ void place(int level, int rank, int l) { list[start[level] + rank] = uint16_t(l); }
+};
+
+// Child entries by octant digit, which is the children's preorder: a local cell, or a local
+// unit, of several bodies or one.
+constexpr unsigned KID_NONE = 0xffffu, KID_CELL = 0x8000u, KID_BUCKET = 0x4000u, KID_INDEX = 0x3fffu;
+static_assert(CHUNK <= int(KID_INDEX) && SPAN_CAP <= int(KID_INDEX), "local indices fit the child entries");
+
+template <class T>
+struct alignas(32) Chunk {
+    typename Prec<T>::V4 body[CHUNK];
+    Records<T, CHUNK> rec;
+    alignas(16) uint16_t kid[CHUNK][8];
+    int pre[CHUNK];      // the cells' preorder indices
+    LevelLists<CHUNK> lists;
+    uint8_t out[CHUNK];  // the cell's parent is of a later stage: its record goes to global memory
+};
+
+// A chunk cell's children.
+template <class T>
+struct ChunkKids {
+    const Chunk<T> &C;
+    int l;
+    const Record<T> *grec;  // several-body leaves have their record in global memory
+    const uint32_t *pscan, *starts;
+    int c0;
+    __device__ __forceinline__ bool operator()(int i, ChildOf<T> &c) const {
+        const unsigned e = C.kid[l][i];
+        if (e == KID_NONE) return false;
+        const int x = int(e & KID_INDEX), u = c0 + x;
+        if (e & KID_CELL) C.rec.get(x, c);
+        else if (e & KID_BUCKET) child_record(C.body[x], grec + (u + int(pscan[u]) + __popc(starts[u])), c);
+        else child_single(C.body[x], c);
+        return true;
+    }
+};
+
+// ---- 6. preorder layout, the leaves' records and the chunks' cells ------------
 // nodeB = {width bits, skip, first body (-1: internal cell), body count}.
 // counters[1] = T (cells + leaves), counters[2] = internal cells.
+// A block lays out the nodes of one chunk of CHUNK units (a binary node's index is one end of
+// its range, so a chunk's inner cells are among its own indices) and then combines the
+// chunk's inner cells level by level from shared memory. (As two passes over global memory, a
+// layout and a launch per level, they took 193 + 478 us of the launch list at N = 4M, 51 + 225
+// at N = 1M and 7 + 102 at N = 10000; layout and cells_span take 283 + 86, 84 + 58 and 22 +
+// 15.) A block waits on its own chain of loads, four blocks to an SM.
+constexpr int CHUNK_THREADS = 256;
+
 template <class T>
-__global__ void layout(int *counters, const int *__restrict__ bfirst,
-                       const int *__restrict__ blast, const int *__restrict__ bdelta,
-                       const uint8_t *__restrict__ top, const int *__restrict__ oparent,
-                       const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ pscan,
-                       const uint64_t *__restrict__ ukey, const uint32_t *__restrict__ ufirst,
-                       const T *__restrict__ box, int *__restrict__ pre, int4 *__restrict__ nodeB,
-                       typename Prec<T>::V4 *__restrict__ nodeG, int2 *__restrict__ nodeR,
-                       const int *__restrict__ loparent, const uint8_t *__restrict__ cslot,
-                       const uint8_t *__restrict__ lslot, int *__restrict__ kid, int *__restrict__ levels,
-                       int *__restrict__ by_level, const typename Prec<T>::V4 *__restrict__ sbody, Record<T> *rec,
-                       typename Prec<T>::V4 *nodeA, float4 *nodeQ) {
+__global__ void __launch_bounds__(CHUNK_THREADS)
+    layout(int *counters, const int *__restrict__ bfirst, const int *__restrict__ blast,
+           const int *__restrict__ bdelta, const uint8_t *__restrict__ top, const int *__restrict__ oparent,
+           const uint32_t *__restrict__ starts, const uint32_t *__restrict__ pscan, const uint64_t *__restrict__ ukey,
+           const uint32_t *__restrict__ ufirst, const T *__restrict__ box, int *__restrict__ pre, int4 *nodeB,
+           typename Prec<T>::V4 *__restrict__ nodeG, int2 *__restrict__ nodeR, const int *__restrict__ loparent,
+           int *__restrict__ kid, const typename Prec<T>::V4 *__restrict__ sbody, Record<T> *rec,
+           typename Prec<T>::V4 *nodeA, float4 *nodeQ) {
     using P = Prec<T>;
-    __shared__ int h[LEVELS], base[LEVELS];
-    if (threadIdx.x < LEVELS) h[threadIdx.x] = 0;
-    __syncthreads();
+    constexpr int PER = CHUNK / CHUNK_THREADS;
+    extern __shared__ __align__(32) unsigned char block_raw[];
+    Chunk<T> &C = *reinterpret_cast<Chunk<T> *>(block_raw);
     const int M = counters[0];
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    int lvl = -1, lrank = 0;  // this cell's octree level and rank among the block's
-    if (k == 0) {
+    const int c0 = blockIdx.x << CHUNK_SHIFT;
+    if (c0 >= M) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
         counters[1] = M + int(pscan[M]);
         counters[2] = int(pscan[M]);
     }
-    if (k < M - 1 && top[k]) {
-        const int b = bfirst[k];
-        int r = 0;
-        for (int p = oparent[k]; p >= 0 && bfirst[p] == b; p = oparent[p]) ++r;
-        const int pk = b + int(pscan[b]) + r;
-        pre[k] = pk;
-        const int after = blast[k] + 1;
-        const int skip = after + int(pscan[after]);
-        // Cell box at level L along the key's path: BoundingBox::width() of the
-        // reference cell (partition.rs:322-327) and its centre, replayed in the same
-        // f32 ops.
-        const int L = bdelta[k] / 3;
-        const uint64_t key = ukey[b];
-        T mn0 = box[0], mn1 = box[1], mn2 = box[2], mx0 = box[3], mx1 = box[4], mx2 = box[5];
-        for (int l = 0; l < L; ++l) {
-            const int o = 7 - int((key >> (3 * (LEVELS - 1 - l))) & 7u);
-            const T c0 = P::mul(P::add(mn0, mx0), T(0.5));
-            const T c1 = P::mul(P::add(mn1, mx1), T(0.5));
-            const T c2 = P::mul(P::add(mn2, mx2), T(0.5));
-            if (o & 1) mx0 = c0; else mn0 = c0;
-            if (o & 2) mx1 = c1; else mn1 = c1;
-            if (o & 4) mx2 = c2; else mn2 = c2;
+    C.lists.clear();
+    for (int i = threadIdx.x; i < CHUNK; i += CHUNK_THREADS)
+        reinterpret_cast<uint4 *>(C.kid)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    __syncthreads();
+    int lvl[PER], rank[PER];  // a chunk cell's octree level and rank among the chunk's of that level
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        const int lk = q * CHUNK_THREADS + threadIdx.x;
+        const int k = c0 + lk;
+        lvl[q] = -1;
+        const int cls = k < M - 1 ? top[k] : 0;
+        if (cls) {
+            const int b = bfirst[k], after = blast[k] + 1, op = oparent[k];
+            const int L = bdelta[k] / 3;
+            // the unit's shallower cells come first
+            const int pk = b + int(pscan[b]) + __popc(starts[b] & ((1u << L) - 1u));
+            const int skip = after + int(pscan[after]);
+            // Cell box at level L along the key's path: BoundingBox::width() of the
+            // reference cell (partition.rs:322-327) and its centre, replayed in the same
+            // f32 ops.
+            const uint64_t key = ukey[b];
+            T mn0 = box[0], mn1 = box[1], mn2 = box[2], mx0 = box[3], mx1 = box[4], mx2 = box[5];
+            for (int l = 0; l < L; ++l) {
+                const int o = 7 - digit_at(key, l);
+                const T x = P::mul(P::add(mn0, mx0), T(0.5));
+                const T y = P::mul(P::add(mn1, mx1), T(0.5));
+                const T z = P::mul(P::add(mn2, mx2), T(0.5));
+                if (o & 1) mx0 = x; else mn0 = x;
+                if (o & 2) mx1 = y; else mn1 = y;
+                if (o & 4) mx2 = z; else mn2 = z;
+            }
+            const T w = P::sub(mx0, mn0);
+            const auto g = P::make(T(0.5) * (mn0 + mx0), T(0.5) * (mn1 + mx1), T(0.5) * (mn2 + mx2), w);
+            // the f32 walk reads the width from nodeB.x; the f64 walk from nodeG.w
+            nodeB[pk] = make_int4(sizeof(T) == 4 ? __float_as_int(float(w)) : 0, skip, -1, 0);
+            nodeG[pk] = g;
+            nodeR[pk] = make_int2(int(ufirst[b]), int(ufirst[after]));
+            const bool out = op >= 0 && top[op] > cls;
+            const int digit = op >= 0 ? digit_at(key, bdelta[op] / 3) : 0;
+            if (out) kid[8 * size_t(op) + digit] = 2 * pk;
+            if (cls == 1) {
+                if (op >= 0 && !out) C.kid[op - c0][digit] = uint16_t(KID_CELL | unsigned(lk));
+                C.pre[lk] = pk;
+                C.out[lk] = out;
+                C.rec.set_box(lk, g);
+                lvl[q] = L;
+                rank[q] = C.lists.add(L);
+            } else {
+                pre[k] = pk;
+            }
         }
-        const T w = P::sub(mx0, mn0);
-        // the f32 walk reads the width from nodeB.x; the f64 walk from nodeG.w
-        nodeB[pk] = make_int4(sizeof(T) == 4 ? __float_as_int(float(w)) : 0, skip, -1, 0);
-        nodeG[pk] = P::make(T(0.5) * (mn0 + mx0), T(0.5) * (mn1 + mx1), T(0.5) * (mn2 + mx2), w);
-        nodeR[pk] = make_int2(int(ufirst[b]), int(ufirst[blast[k] + 1]));
-        // the cell's entry in its parent's child list
-        if (k != 0) kid[8 * oparent[k] + cslot[k]] = 2 * pk;
-        lvl = L;
-        lrank = atomicAdd(&h[L], 1);
+        if (k < M) {
+            const int pk = k + int(pscan[k]) + __popc(starts[k]);
+            const int f = int(ufirst[k]);
+            const int nb = int(ufirst[k + 1]) - f;
+            nodeB[pk] = make_int4(0, pk + 1, f, nb);
+            // (no nodeG / nodeR for leaves: the cell centre and body range are read for
+            // cells only, by the f64 walk's widths and the learned features and samples)
+            const int op = loparent[k];
+            C.body[lk] = leaf(pk, f, f + nb, sbody, rec, nodeA, nodeQ);  // the leaf's moment record
+            if (op >= 0) {
+                const int digit = digit_at(ukey[k], bdelta[op] / 3);
+                if (top[op] > 1) kid[8 * size_t(op) + digit] = 2 * pk + (nb == 1 ? 1 : 0);
+                else C.kid[op - c0][digit] = uint16_t((nb == 1 ? 0u : KID_BUCKET) | unsigned(lk));
+            }
+        }
     }
-    if (k < M) {
-        const int pk = k + int(pscan[k]) + int(cnt[k]);
-        const int f = int(ufirst[k]);
-        const int nb = int(ufirst[k + 1]) - f;
-        nodeB[pk] = make_int4(0, pk + 1, f, nb);
-        // (no nodeG / nodeR for leaves: the cell centre and body range are read for
-        // cells only, by the f64 walk's widths and the learned features and samples)
-        const int op = loparent[k];
-        if (op >= 0) kid[8 * op + lslot[k]] = 2 * pk + (nb == 1 ? 1 : 0);
-        leaf(pk, f, f + nb, sbody, rec, nodeA, nodeQ);  // the leaf's moment record
+    C.lists.offsets();
+#pragma unroll
+    for (int q = 0; q < PER; ++q)
+        if (lvl[q] >= 0) C.lists.place(lvl[q], rank[q], q * CHUNK_THREADS + threadIdx.x);
+    for (int L = LEVELS - 1; L >= 0; --L) {
+        const int s = C.lists.start[L], e = C.lists.start[L + 1];
+        if (s == e) continue;
+        __syncthreads();  // the list; the records of the levels below
+        for (int i = s + threadIdx.x; i < e; i += CHUNK_THREADS) {
+            const int l = C.lists.list[i], pk = C.pre[l];
+            const auto g = C.rec.box(l);
+            typename P::V4 a;
+            const Record<T> r = combine(g, ChunkKids<T>{C, l, rec, pscan, starts, c0}, &a);
+            put_cell(pk, g.w, a, r, nodeA, nodeQ, nodeB);
+            if (C.out[l]) rec[pk] = r;
+            C.rec.set(l, a, r);
+        }
     }
-    // cells bucketed by octree level (one range per level and block)
-    __syncthreads();
-    if (threadIdx.x < LEVELS && h[threadIdx.x])
-        base[threadIdx.x] = atomicAdd(&levels[2 * LEVELS + 2 + threadIdx.x], h[threadIdx.x]);
-    __syncthreads();
-    if (lvl >= 0) by_level[base[lvl] + lrank] = k;
 }
 
-// The cells of octree level L (levels below: done), one thread each.
+// The cells that span blocks of the stage before and lie in one of this stage's, a block of
+// threads for each such block. Children of the same stage are in shared memory, the others
+// have their records in global memory. (Climbing from child to parent through global memory
+// took 62 us at N = 10000 and 128 us at N = 4M, a cluster going level by level 177 us there:
+// a step up costs some five trips to L2 and two fences, 6 us. From shared memory, eight lanes
+// to a cell: 15 us at N = 10000, 29 + 35 + 22 us for the three stages at N = 4M.)
+constexpr int SPAN_THREADS = 512;
+
 template <class T>
-__global__ void __launch_bounds__(256)
-    cells_level(int L, const int *__restrict__ levels, const int *__restrict__ by_level,
-                const int *__restrict__ pre, const int *__restrict__ kid, const int *__restrict__ nkid,
-                const typename Prec<T>::V4 *__restrict__ nodeG, Record<T> *rec, typename Prec<T>::V4 *nodeA,
-                float4 *nodeQ, int4 *nodeB) {
-    const int begin = levels[LEVELS + 1 + L], end = begin + levels[L];
-    for (int i = begin + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x) {
-        const int k = by_level[i];
-        cell(pre[k], load_kids(k, kid, nkid), nodeG, rec, nodeA, nodeQ, nodeB);
+struct alignas(32) SpanBlock {
+    Records<T, SPAN_CAP> rec;
+    int kid[SPAN_CAP][8];  // 2 x preorder index + 1 for a single body, -1 none, -2 - x: local cell x
+    int pre[SPAN_CAP];     // preorder indices
+    LevelLists<SPAN_CAP> lists;
+    uint8_t out[SPAN_CAP]; // the cell's parent is of a later stage: its record goes to global memory
+};
+
+template <class T>
+__global__ void __launch_bounds__(SPAN_THREADS)
+    cells_span(int n, int stage, const int *__restrict__ nspan, const int *__restrict__ spans,
+               const int *__restrict__ bfirst, const int *__restrict__ bdelta, const uint8_t *__restrict__ top,
+               const uint64_t *__restrict__ ukey, const int *__restrict__ oparent, const int *__restrict__ pre,
+               const int *__restrict__ kid, const uint32_t *__restrict__ kmask, int *slot,
+               const typename Prec<T>::V4 *__restrict__ nodeG, Record<T> *rec, typename Prec<T>::V4 *nodeA,
+               float4 *nodeQ, int4 *nodeB) {
+    extern __shared__ __align__(32) unsigned char block_raw[];
+    SpanBlock<T> &C = *reinterpret_cast<SpanBlock<T> *>(block_raw);
+    const int blk = stage_first(n, stage) + blockIdx.x;
+    const int m = min(nspan[blk], SPAN_CAP);
+    if (m == 0) return;
+    constexpr int PER = (SPAN_CAP + SPAN_THREADS - 1) / SPAN_THREADS;
+    const int *cells = spans + size_t(blk) * SPAN_CAP;
+    C.lists.clear();
+    for (int x = threadIdx.x; x < 8 * m; x += SPAN_THREADS) {
+        const int i = x >> 3, d = x & 7, k = cells[i];
+        C.kid[i][d] = (kmask[k] >> d) & 1u ? kid[8 * size_t(k) + d] : -1;
+        if (d == 0) slot[k] = i;
     }
-}
-
-// Levels TOP_LEVELS - 1 .. 0 (at most 8^L cells each, 585 in all) in one block, a
-// barrier between levels: these levels hold few cells, and one launch each cost
-// ~17 us of latency at N = 4M. (Level 4 too, up to 4096 cells at several cells per
-// thread, made the block take 66 us.)
-constexpr int TOP_LEVELS = 4;
-
-template <class T>
-__global__ void __launch_bounds__(512)
-    cells_top(const int *__restrict__ levels, const int *__restrict__ by_level, const int *__restrict__ pre,
-              const int *__restrict__ kid, const int *__restrict__ nkid, const typename Prec<T>::V4 *__restrict__ nodeG,
-              Record<T> *rec, typename Prec<T>::V4 *nodeA, float4 *nodeQ, int4 *nodeB) {
-    for (int L = TOP_LEVELS - 1; L >= 0; --L) {
-        const int begin = levels[LEVELS + 1 + L], end = begin + levels[L];
-        for (int i = begin + threadIdx.x; i < end; i += blockDim.x) {
-            const int k = by_level[i];
-            cell(pre[k], load_kids(k, kid, nkid), nodeG, rec, nodeA, nodeQ, nodeB);
+    __syncthreads();
+    int lvl[PER], rank[PER];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        const int i = q * SPAN_THREADS + threadIdx.x;
+        if (i >= m) break;
+        const int k = cells[i], op = oparent[k], pk = pre[k];
+        const bool same = op >= 0 && top[op] == top[k];
+        C.pre[i] = pk;
+        C.out[i] = op >= 0 && !same;
+        C.rec.set_box(i, nodeG[pk]);
+        lvl[q] = bdelta[k] / 3;
+        rank[q] = C.lists.add(lvl[q]);
+        if (same) C.kid[slot[op]][digit_at(ukey[bfirst[k]], bdelta[op] / 3)] = -2 - i;
+    }
+    C.lists.offsets();
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        const int i = q * SPAN_THREADS + threadIdx.x;
+        if (i >= m) break;
+        C.lists.place(lvl[q], rank[q], i);
+    }
+    const int lane = threadIdx.x & 31, d = lane & 7;
+    for (int L = LEVELS - 1; L >= 0; --L) {
+        const int s = C.lists.start[L], e = C.lists.start[L + 1];
+        if (s == e) continue;
+        __syncthreads();  // the list; the records of the levels below
+        for (int i0 = s + (threadIdx.x >> 5) * 4; i0 < e; i0 += SPAN_THREADS / 8) {  // four cells to a warp
+            const bool valid = i0 + (lane >> 3) < e;
+            const int l = C.lists.list[valid ? i0 + (lane >> 3) : i0], x = C.kid[l][d];
+            const auto g = C.rec.box(l);
+            ChildOf<T> c;
+            if (x >= 0) {
+                const auto ca = ld_cg(nodeA + (x >> 1));
+                if (x & 1) child_single(ca, c);
+                else child_record(ca, rec + (x >> 1), c);
+            } else if (x < -1) {
+                C.rec.get(-2 - x, c);
+            }
+            typename Prec<T>::V4 a;
+            const Record<T> r = combine8(g, x != -1, c, &a);
+            if (valid && d == 0) {
+                const int pk = C.pre[l];
+                put_cell(pk, g.w, a, r, nodeA, nodeQ, nodeB);
+                if (C.out[l]) rec[pk] = r;
+                C.rec.set(l, a, r);
+            }
         }
-        __syncthreads();  // the level's records (global, read through L2) before its parents
     }
 }
 
@@ -701,8 +1000,6 @@ int build_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_src, int n) {
     PT_TRY(ensure_buf(ctx, S.keys, sizeof(uint64_t) * N));
     PT_TRY(ensure_buf(ctx, S.idx, sizeof(uint32_t) * N));
     PT_TRY(ensure_buf(ctx, sb, sizeof(V4) * N));
-    PT_TRY(ensure_buf(ctx, S.flags, sizeof(uint32_t) * N));
-    PT_TRY(ensure_buf(ctx, S.uscan, sizeof(uint32_t) * (N + 1)));
     PT_TRY(ensure_buf(ctx, S.ukey, sizeof(uint64_t) * N));
     PT_TRY(ensure_buf(ctx, S.ufirst, sizeof(uint32_t) * (N + 1)));
     PT_TRY(ensure_buf(ctx, S.bfirst, sizeof(int) * N));
@@ -713,15 +1010,12 @@ int build_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_src, int n) {
     PT_TRY(ensure_buf(ctx, S.top, N));
     PT_TRY(ensure_buf(ctx, S.oparent, sizeof(int) * N));
     PT_TRY(ensure_buf(ctx, S.loparent, sizeof(int) * N));
-    PT_TRY(ensure_buf(ctx, S.cnt, sizeof(uint32_t) * (N + 1)));
+    PT_TRY(ensure_buf(ctx, S.starts, sizeof(uint32_t) * (N + 1)));
     PT_TRY(ensure_buf(ctx, S.pscan, sizeof(uint32_t) * (N + 2)));
     PT_TRY(ensure_buf(ctx, S.pre, sizeof(int) * N));
-    PT_TRY(ensure_buf(ctx, S.nkid, sizeof(int) * N));
-    PT_TRY(ensure_buf(ctx, S.levels, sizeof(int) * (3 * LEVELS + 8)));
-    PT_TRY(ensure_buf(ctx, S.by_level, sizeof(int) * N));
+    PT_TRY(ensure_buf(ctx, S.kmask, sizeof(uint32_t) * N));
+    PT_TRY(ensure_buf(ctx, S.slot, sizeof(int) * N));
     PT_TRY(ensure_buf(ctx, S.kid, sizeof(int) * 8 * N));
-    PT_TRY(ensure_buf(ctx, S.cslot, N));
-    PT_TRY(ensure_buf(ctx, S.lslot, N));
     PT_TRY(ensure_buf(ctx, nA, sizeof(V4) * 2 * N));
     PT_TRY(ensure_buf(ctx, S.nodeB, sizeof(int4) * 2 * N));
     if (!F64) PT_TRY(ensure_buf(ctx, S.nodeQ, sizeof(float4) * 4 * N));
@@ -751,53 +1045,42 @@ int build_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_src, int n) {
     gather_bodies<V4><<<blocks(n), 256, 0, S.aux>>>(d_src, as<uint32_t>(S.idx), n, as<V4>(sb));
     PT_TRY(check_launch(ctx, "gather_bodies"));
     PT_CUDA(cudaEventRecord(S.join, S.aux));
-    unit_flags<<<blocks(n), 256, 0, st>>>(as<uint64_t>(S.keys), n, as<uint32_t>(S.flags));
-    PT_TRY(check_launch(ctx, "unit_flags"));
-    PT_TRY(scan_u32(ctx, S.prims, as<uint32_t>(S.flags), as<uint32_t>(S.uscan), n));
     int *counters = as<int>(S.counters);
-    unit_fill<<<blocks(n), 256, 0, st>>>(as<uint64_t>(S.keys), as<uint32_t>(S.flags), as<uint32_t>(S.uscan), n,
-                                        as<uint64_t>(S.ukey), as<uint32_t>(S.ufirst), counters);
-    PT_TRY(check_launch(ctx, "unit_fill"));
-    karras<<<blocks(n), 256, 0, st>>>(as<uint64_t>(S.ukey), counters, as<int>(S.bfirst), as<int>(S.blast),
-                                     as<int>(S.bdelta), as<int>(S.bparent), as<int>(S.lparent));
+    PT_TRY(scan_generated(ctx, S.prims, UnitHead{as<uint64_t>(S.keys)},
+                          UnitFill{as<uint64_t>(S.keys), n, as<uint64_t>(S.ukey), as<uint32_t>(S.ufirst), counters}, n));
+    const int nstages = stages(n), span_blocks = stage_first(n, nstages + 1);
+    PT_TRY(ensure_buf(ctx, S.nspan, sizeof(int) * size_t(std::max(1, span_blocks))));
+    PT_TRY(ensure_buf(ctx, S.spans, sizeof(int) * size_t(std::max(1, span_blocks)) * SPAN_CAP));
+    karras<<<blocks(n + 1), 256, 0, st>>>(as<uint64_t>(S.ukey), counters, n, as<int>(S.bfirst), as<int>(S.blast),
+                                          as<int>(S.bdelta), as<int>(S.bparent), as<int>(S.lparent),
+                                          as<uint8_t>(S.top), as<uint32_t>(S.starts), as<uint32_t>(S.kmask),
+                                          as<int>(S.nspan), span_blocks);
     PT_TRY(check_launch(ctx, "karras"));
-    octree_top<<<blocks(n), 256, 0, st>>>(counters, as<int>(S.bdelta), as<int>(S.bparent), as<uint8_t>(S.top));
-    PT_TRY(check_launch(ctx, "octree_top"));
-    PT_CUDA(cudaMemsetAsync(S.cnt.ptr, 0, sizeof(uint32_t) * (N + 1), st));
-    PT_CUDA(cudaMemsetAsync(S.nkid.ptr, 0, sizeof(int) * N, st));
-    PT_CUDA(cudaMemsetAsync(S.levels.ptr, 0, sizeof(int) * (3 * LEVELS + 8), st));
-    int *levels = as<int>(S.levels);
-    octree_links<<<blocks(n), 256, 0, st>>>(counters, as<int>(S.bfirst), as<int>(S.bparent), as<int>(S.lparent),
-                                           as<uint8_t>(S.top), as<int>(S.bdelta), as<int>(S.oparent),
-                                           as<int>(S.loparent), as<uint32_t>(S.cnt), as<int>(S.nkid),
-                                           as<uint8_t>(S.cslot), as<uint8_t>(S.lslot), levels);
+    octree_links<<<blocks(n), 256, 0, st>>>(counters, n, as<int>(S.bfirst), as<int>(S.bparent), as<int>(S.lparent),
+                                           as<uint8_t>(S.top), as<int>(S.bdelta), as<uint64_t>(S.ukey),
+                                           as<int>(S.oparent), as<int>(S.loparent), as<uint32_t>(S.starts),
+                                           as<uint32_t>(S.kmask), as<int>(S.nspan), as<int>(S.spans));
     PT_TRY(check_launch(ctx, "octree_links"));
-    level_offsets<<<1, 32, 0, st>>>(levels);
-    PT_TRY(check_launch(ctx, "level_offsets"));
-    PT_TRY(scan_u32(ctx, S.prims, as<uint32_t>(S.cnt), as<uint32_t>(S.pscan), n + 1));
+    PT_TRY(scan_generated(ctx, S.prims, CellStarts{as<uint32_t>(S.starts)},
+                          scan::WriteU32{as<uint32_t>(S.pscan), n + 1}, n + 1));
     PT_CUDA(cudaStreamWaitEvent(st, S.join, 0));  // the gathered bodies
-    layout<T><<<blocks(n), 256, 0, st>>>(counters, as<int>(S.bfirst), as<int>(S.blast), as<int>(S.bdelta),
-                                     as<uint8_t>(S.top), as<int>(S.oparent), as<uint32_t>(S.cnt),
-                                     as<uint32_t>(S.pscan), as<uint64_t>(S.ukey), as<uint32_t>(S.ufirst),
-                                     as<T>(S.box), as<int>(S.pre), as<int4>(S.nodeB), as<V4>(nG),
-                                     as<int2>(S.nodeR), as<int>(S.loparent), as<uint8_t>(S.cslot),
-                                     as<uint8_t>(S.lslot), as<int>(S.kid), levels, as<int>(S.by_level), as<V4>(sb),
-                                     as<Record<T>>(S.mom), as<V4>(nA), nodeQ);
+    PT_CUDA(cudaFuncSetAttribute(layout<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(Chunk<T>))));
+    layout<T><<<(n + CHUNK - 1) / CHUNK, CHUNK_THREADS, sizeof(Chunk<T>), st>>>(
+        counters, as<int>(S.bfirst), as<int>(S.blast), as<int>(S.bdelta), as<uint8_t>(S.top), as<int>(S.oparent),
+        as<uint32_t>(S.starts), as<uint32_t>(S.pscan), as<uint64_t>(S.ukey), as<uint32_t>(S.ufirst), as<T>(S.box),
+        as<int>(S.pre), as<int4>(S.nodeB), as<V4>(nG), as<int2>(S.nodeR), as<int>(S.loparent), as<int>(S.kid),
+        as<V4>(sb), as<Record<T>>(S.mom), as<V4>(nA), nodeQ);
     PT_TRY(check_launch(ctx, "layout"));
-
-    const int lvl_grid = std::max(1, std::min(blocks(n), 8 * ctx->sm_count));
-    for (int L = LEVELS - 1; L >= TOP_LEVELS; --L) {
-        // level L holds at most 8^L cells: shallow levels get a grid of their size
-        const long long cap = L < 10 ? (1ll << (3 * L)) : (long long)n;
-        const int grid = int(std::max(1ll, std::min<long long>(lvl_grid, (std::min<long long>(cap, n) + 255) / 256)));
-        cells_level<T><<<grid, 256, 0, st>>>(L, levels, as<int>(S.by_level), as<int>(S.pre), as<int>(S.kid),
-                                                as<int>(S.nkid), as<V4>(nG), as<Record<T>>(S.mom), as<V4>(nA),
-                                                nodeQ, as<int4>(S.nodeB));
-        PT_TRY(check_launch(ctx, "cells_level"));
+    if (nstages > 0)
+        PT_CUDA(cudaFuncSetAttribute(cells_span<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(sizeof(SpanBlock<T>))));
+    for (int stage = 1; stage <= nstages; ++stage) {
+        cells_span<T><<<stage_blocks(n, stage), SPAN_THREADS, sizeof(SpanBlock<T>), st>>>(
+            n, stage, as<int>(S.nspan), as<int>(S.spans), as<int>(S.bfirst), as<int>(S.bdelta), as<uint8_t>(S.top),
+            as<uint64_t>(S.ukey), as<int>(S.oparent), as<int>(S.pre), as<int>(S.kid), as<uint32_t>(S.kmask),
+            as<int>(S.slot), as<V4>(nG), as<Record<T>>(S.mom), as<V4>(nA), nodeQ, as<int4>(S.nodeB));
+        PT_TRY(check_launch(ctx, "cells_span"));
     }
-    cells_top<T><<<1, 512, 0, st>>>(levels, as<int>(S.by_level), as<int>(S.pre), as<int>(S.kid), as<int>(S.nkid),
-                                    as<V4>(nG), as<Record<T>>(S.mom), as<V4>(nA), nodeQ, as<int4>(S.nodeB));
-    PT_TRY(check_launch(ctx, "cells_top"));
     S.last_n_src = n;
     S.f64 = F64;
     S.user_tree = false;

@@ -1,7 +1,5 @@
-// Exclusive scan and stable LSD radix sort, written for the Barnes-Hut build.
+// Stable LSD radix sort, written for the Barnes-Hut build.
 //
-// scan_u32: blocks of SCAN_TILE items scan in shared memory and publish their
-// totals; the totals are scanned recursively and added back.
 // radix_sort_u64: 8-bit digits; per digit a histogram pass (per-tile counts), a row
 // scan (one block per digit value over the tiles) and a scatter pass. The scatter
 // ranks keys stably inside a tile (each warp its own run of keys, with warp
@@ -12,10 +10,6 @@
 namespace pt {
 namespace prims {
 
-constexpr int SCAN_THREADS = 512;
-constexpr int SCAN_ITEMS = 8;
-constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
-
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -24,54 +18,6 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
         if (lane >= o) v += t;
     }
     return v;
-}
-
-// Exclusive scan of one tile; writes out[i] and sums[blockIdx.x] = tile total.
-__global__ void __launch_bounds__(SCAN_THREADS)
-    scan_tiles(const uint32_t *__restrict__ in, uint32_t *__restrict__ out, int n, uint32_t *__restrict__ sums) {
-    __shared__ uint32_t tile[SCAN_TILE];
-    __shared__ uint32_t warp_tot[SCAN_THREADS / 32];
-    const size_t base = size_t(blockIdx.x) * SCAN_TILE;
-    for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS) {
-        const size_t i = base + k;
-        tile[k] = (i < size_t(n)) ? in[i] : 0u;
-    }
-    __syncthreads();
-    uint32_t local[SCAN_ITEMS];
-    uint32_t acc = 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-        local[k] = acc;
-        acc += tile[threadIdx.x * SCAN_ITEMS + k];
-    }
-    const uint32_t incl = warp_incl_scan(acc);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = (lane < SCAN_THREADS / 32) ? warp_tot[lane] : 0u;
-        const uint32_t wi = warp_incl_scan(w);
-        if (lane < SCAN_THREADS / 32) warp_tot[lane] = wi - w;
-        if (lane == SCAN_THREADS / 32 - 1) sums[blockIdx.x] = wi;
-    }
-    __syncthreads();
-    const uint32_t off = warp_tot[warp] + incl - acc;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) tile[threadIdx.x * SCAN_ITEMS + k] = off + local[k];
-    __syncthreads();
-    for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS) {
-        const size_t i = base + k;
-        if (i < size_t(n)) out[i] = tile[k];
-    }
-}
-
-__global__ void scan_add(uint32_t *__restrict__ out, int n, const uint32_t *__restrict__ offs) {
-    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < size_t(n)) out[i] += offs[i / SCAN_TILE];
-}
-
-__global__ void scan_total(uint32_t *__restrict__ out, int n, const uint32_t *__restrict__ sums) {
-    out[n] = sums[0];
 }
 
 // ---- radix sort ------------------------------------------------------------
@@ -216,49 +162,6 @@ __global__ void __launch_bounds__(RS_THREADS)
 }
 
 }  // namespace prims
-
-static int scan_rec(pt_ctx *ctx, uint32_t *tmp, size_t tmp_cap, const uint32_t *in, uint32_t *out, int n) {
-    using namespace prims;
-    cudaStream_t st = ctx->stream;
-    const int nb = (n + SCAN_TILE - 1) / SCAN_TILE;
-    if (size_t(2 * nb) > tmp_cap) return set_error(PT_ERR_INVALID, "scan scratch too small");
-    uint32_t *sums = tmp;
-    uint32_t *sums_scanned = tmp + nb;
-    scan_tiles<<<nb, SCAN_THREADS, 0, st>>>(in, out, n, sums);
-    PT_TRY(check_launch(ctx, "scan_tiles"));
-    if (nb == 1) {
-        scan_total<<<1, 1, 0, st>>>(out, n, sums);
-        return check_launch(ctx, "scan_total");
-    }
-    // sums_scanned gets nb + 1 entries: the scanned totals and the grand total.
-    PT_TRY(scan_rec(ctx, tmp + 2 * nb + 1, tmp_cap - (2 * nb + 1), sums, sums_scanned, nb));
-    scan_add<<<(n + 255) / 256, 256, 0, st>>>(out, n, sums_scanned);
-    PT_TRY(check_launch(ctx, "scan_add"));
-    scan_total<<<1, 1, 0, st>>>(out, n, sums_scanned + nb);
-    return check_launch(ctx, "scan_total");
-}
-
-static size_t scan_scratch_words(int n) {
-    size_t words = 0;
-    int m = n;
-    do {
-        const int nb = (m + prims::SCAN_TILE - 1) / prims::SCAN_TILE;
-        words += 2 * size_t(nb) + 1;
-        m = nb;
-        if (nb == 1) break;
-    } while (true);
-    return words + 16;
-}
-
-int scan_u32(pt_ctx *ctx, PrimScratch &s, const uint32_t *in, uint32_t *out, int n) {
-    if (n <= 0) {
-        PT_CUDA(cudaMemsetAsync(out, 0, sizeof(uint32_t), ctx->stream));
-        return PT_OK;
-    }
-    const size_t words = scan_scratch_words(n);
-    PT_TRY(ensure_buf(ctx, s.scan, words * sizeof(uint32_t)));
-    return scan_rec(ctx, static_cast<uint32_t *>(s.scan.ptr), words, in, out, n);
-}
 
 int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, int n, int bits) {
     using namespace prims;

@@ -1,0 +1,64 @@
+"""The tree build where its blocks end: chunks of 512 leaf units and blocks of 64 chunks
+(32768 units), full, one short and one over; massless and coincident bodies across them."""
+import numpy as np
+import pytest
+
+from particular_gb300 import AccelerationSoftened, cuda
+from test_bh_gpu import oracle_preorder
+
+pytestmark = pytest.mark.gpu
+
+
+def tree_of(res, b):
+    m = cuda.BarnesHut(0.5, res, AccelerationSoftened(0.01), quadrupole=True)
+    m.compute(b)
+    return m.export_tree()
+
+
+def clumpy(n, seed):
+    """Dense knots in a wide cloud: cells of many levels across every block boundary."""
+    r = np.random.RandomState(seed)
+    knot = r.uniform(-50, 50, (max(1, n // 700), 3))
+    x = knot[r.randint(0, len(knot), n)] + r.normal(size=(n, 3)) * 10.0 ** r.uniform(-3, 1, (n, 1))
+    return np.concatenate([x, r.uniform(0.5, 1.5, (n, 1))], 1).astype(np.float32)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 511, 512, 513, 1025, 32767, 32768, 32769, 70001])
+def test_tree_and_moments(res, oracle, n):
+    b = clumpy(n, n)
+    b[::7, 3] = 0.0  # massless bodies; below also whole massless cells
+    b[: n // 10, 3] = 0.0
+    g = tree_of(res, b)
+    order, e = oracle_preorder(oracle.Tree(b))
+    internal = e["internal"][order].astype(bool)
+    cells = g["links"][:, 2] < 0
+    assert np.array_equal(internal, cells)
+    skip = np.asarray(g["links"][:, 1], np.int64)
+    assert skip[0] == len(skip) and (skip > np.arange(len(skip))).all()
+    w_ref = (e["box"][order, 3] - e["box"][order, 0])[internal]
+    assert np.array_equal(g["width"][cells], w_ref.astype(np.float32))
+    assert np.array_equal(g["com_mass"][~cells], e["data"][order][~internal])
+    # mass and centre of mass of each cell's bodies (their plain mean where massless)
+    rng, bp = e["range"][order][internal], b[e["perm"]].astype(np.float64)
+    got, w = g["com_mass"][cells].astype(np.float64), g["width"][cells].astype(np.float64)
+    for k in np.unique(np.linspace(0, len(rng) - 1, 4000).astype(int)) if len(rng) else []:
+        x = bp[rng[k, 0]: rng[k, 0] + rng[k, 1]]
+        M = x[:, 3].sum()
+        com = (x[:, :3] * x[:, 3:]).sum(0) / M if M else x[:, :3].mean(0)
+        assert abs(got[k, 3] - M) <= 1e-6 * M
+        # f32 coordinates, and sums about the cell's centre
+        assert np.abs(got[k, :3] - com).max() <= 2.0 ** -23 * np.abs(com).max() + 1e-6 * w[k]
+
+
+@pytest.mark.parametrize("copies", [2, 600])
+def test_coincident_bodies_across_blocks(res, copies):
+    """Bodies that share a key make one leaf of several bodies, wherever its run lies."""
+    b = np.repeat(clumpy(40000 // copies, 5), copies, axis=0)
+    b[:, 3] = np.random.RandomState(6).uniform(0.5, 1.5, len(b))
+    g = tree_of(res, b)
+    cells = g["links"][:, 2] < 0
+    assert g["links"][~cells, 3].sum() == len(b) and (~cells).sum() == len(b) // copies
+    M = b[:, 3].astype(np.float64).sum()
+    com = (b[:, :3].astype(np.float64) * b[:, 3:]).sum(0) / M
+    assert abs(g["com_mass"][0, 3] - M) <= 1e-6 * M
+    assert np.abs(g["com_mass"][0, :3] - com).max() <= 1e-5
