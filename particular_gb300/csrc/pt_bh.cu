@@ -31,6 +31,11 @@ int validate(const char *fn, size_t n_aff, size_t n_src, uint32_t flags) {
     return PT_OK;
 }
 
+static int sort_error(const char *fn, int err) {
+    if (err & ERR_SORT_BARRIER) return set_error(PT_ERR_TIMEOUT, "%s: a grid barrier of the sort gave up", fn);
+    return PT_OK;
+}
+
 }  // namespace bh
 }  // namespace pt
 
@@ -173,6 +178,7 @@ int pt_bh_accel_f32(pt_ctx *ctx, const float *aff, size_t n_aff, const float *sr
     if (n_src) PT_CUDA(cudaMemcpyAsync(&err, static_cast<int *>(S->counters.ptr) + 3, sizeof(int),
                                        cudaMemcpyDeviceToHost, st));
     PT_CUDA(cudaStreamSynchronize(st));
+    PT_TRY(bh::sort_error("pt_bh_accel_f32", err));
     if (err & 2)
         return set_error(PT_ERR_CAPACITY, "pt_bh_accel_f32: learned-correction records overflowed");
     return PT_OK;
@@ -224,6 +230,7 @@ int pt_bh_accel_dvec3(pt_ctx *ctx, const double *aff, size_t n_aff, const double
     if (n_src) PT_CUDA(cudaMemcpyAsync(&err, static_cast<int *>(S->counters.ptr) + 3, sizeof(int),
                                        cudaMemcpyDeviceToHost, st));
     PT_CUDA(cudaStreamSynchronize(st));
+    PT_TRY(bh::sort_error("pt_bh_accel_dvec3", err));
     if (err & 1) return set_error(PT_ERR_CAPACITY, "pt_bh_accel_dvec3: a warp's stack ran out; its bodies are NaN");
     return PT_OK;
 }
@@ -244,6 +251,7 @@ int pt_bh_build_device(pt_ctx *ctx, const float *d_src, size_t n_src, uint64_t *
         ++S->generation;
     } else {
         mark(ctx, 0);
+        PT_TRY(bh::clear_errors(ctx, *S));
         PT_TRY(bh::build(ctx, *S, reinterpret_cast<const float4 *>(d_src), int(n_src)));
     }
     if (generation) *generation = S->generation;
@@ -272,6 +280,7 @@ int pt_bh_walk_device(pt_ctx *ctx, const float *d_aff, size_t n_aff, float theta
         return set_error(PT_ERR_INVALID,
                          "pt_bh_walk_device: a caller-built tree carries monopoles only (flags 0 or PT_BH_GROUP)");
     mark(ctx, 0);
+    PT_TRY(bh::clear_errors(ctx, *S));
     PT_TRY(bh::sort_targets(ctx, *S, reinterpret_cast<const float4 *>(d_aff), int(n_aff)));
     return bh::walk(ctx, *S, bh::as<float4>(S->tbody), bh::as<uint32_t>(S->tidx), int(n_aff), theta, softening,
                     flags, d_out);
@@ -434,6 +443,7 @@ int pt_bh_walk(pt_ctx *ctx, const float *aff, size_t n_aff, float theta, float s
     PT_CUDA(cudaMemcpyAsync(&err, static_cast<int *>(S->counters.ptr) + 3, sizeof(int), cudaMemcpyDeviceToHost,
                             st));
     PT_CUDA(cudaStreamSynchronize(st));
+    PT_TRY(bh::sort_error("pt_bh_walk", err));
     if (err & 2) return set_error(PT_ERR_CAPACITY, "pt_bh_walk: learned-correction records overflowed");
     return PT_OK;
 }

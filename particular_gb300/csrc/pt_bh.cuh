@@ -120,6 +120,7 @@ template <class T>
 int sort_targets_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_aff, int n);
 int sort_targets(pt_ctx *ctx, State &S, const float4 *d_aff, int n);
 // walks (pt_bh_walk.cu)
+int clear_errors(pt_ctx *ctx, State &S);
 int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n_aff, float theta,
          float softening, uint32_t flags, float *d_out);
 int run(pt_ctx *ctx, const float4 *d_aff, int n_aff, const float4 *d_src, int n_src, float theta, float softening,

@@ -128,17 +128,19 @@ __device__ __forceinline__ uint64_t key_of(T px, T py, T pz, const T *box) {
     return key;
 }
 
+// hist (small n): the counts of the sort's first digit by tile of RADIX_TILE keys.
 template <class T>
 __global__ void make_keys(const typename Prec<T>::V4 *__restrict__ bodies, int n, const T *__restrict__ box_g,
-                          uint64_t *__restrict__ keys, uint32_t *__restrict__ idx) {
+                          uint64_t *__restrict__ keys, uint32_t *__restrict__ hist, int shift) {
     __shared__ T box[6];
     if (threadIdx.x < 6) box[threadIdx.x] = box_g[threadIdx.x];
     __syncthreads();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const typename Prec<T>::V4 p = bodies[i];
-    keys[i] = key_of<T>(p.x, p.y, p.z, box);
-    idx[i] = uint32_t(i);
+    const uint64_t k = key_of<T>(p.x, p.y, p.z, box);
+    keys[i] = k;
+    if (hist) atomicAdd(&hist[(i / RADIX_TILE) * 256 + (int(k >> shift) & 255)], 1u);
 }
 
 template <class V4>
@@ -1030,9 +1032,13 @@ int build_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_src, int n) {
     PT_TRY(check_launch(ctx, "bbox_partial"));
     bbox_final<T><<<1, 256, 0, st>>>(as<T>(S.box_part), nb, as<T>(S.box));
     PT_TRY(check_launch(ctx, "bbox_final"));
-    make_keys<T><<<blocks(n), 256, 0, st>>>(d_src, n, as<T>(S.box), as<uint64_t>(S.keys), as<uint32_t>(S.idx));
+    RadixFirst rf{};
+    PT_TRY(radix_sort_prepare(ctx, S.prims, n, 3 * LEVELS, &rf));
+    make_keys<T><<<blocks(n), 256, 0, st>>>(d_src, n, as<T>(S.box), rf.keys ? rf.keys : as<uint64_t>(S.keys), rf.hist,
+                                            rf.shift);
     PT_TRY(check_launch(ctx, "make_keys"));
-    PT_TRY(radix_sort_u64(ctx, S.prims, as<uint64_t>(S.keys), as<uint32_t>(S.idx), n, 3 * LEVELS));
+    PT_TRY(radix_sort_u64(ctx, S.prims, as<uint64_t>(S.keys), as<uint32_t>(S.idx), n, 3 * LEVELS,
+                          as<int>(S.counters) + 3));
     // The bodies' gather into key order runs on a second stream beside the tree chain
     // (unit flags .. octree links) and joins before the layout, its first reader.
     if (!S.aux) {
@@ -1099,9 +1105,13 @@ int sort_targets_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_aff, int
     PT_TRY(ensure_buf(ctx, S.tkeys, sizeof(uint64_t) * size_t(n)));
     PT_TRY(ensure_buf(ctx, S.tidx, sizeof(uint32_t) * size_t(n)));
     PT_TRY(ensure_buf(ctx, tb, sizeof(V4) * size_t(n)));
-    make_keys<T><<<blocks(n), 256, 0, st>>>(d_aff, n, as<T>(S.box), as<uint64_t>(S.tkeys), as<uint32_t>(S.tidx));
+    RadixFirst rf{};
+    PT_TRY(radix_sort_prepare(ctx, S.prims, n, 3 * LEVELS, &rf));
+    make_keys<T><<<blocks(n), 256, 0, st>>>(d_aff, n, as<T>(S.box), rf.keys ? rf.keys : as<uint64_t>(S.tkeys), rf.hist,
+                                            rf.shift);
     PT_TRY(check_launch(ctx, "make_keys(targets)"));
-    PT_TRY(radix_sort_u64(ctx, S.prims, as<uint64_t>(S.tkeys), as<uint32_t>(S.tidx), n, 3 * LEVELS));
+    PT_TRY(radix_sort_u64(ctx, S.prims, as<uint64_t>(S.tkeys), as<uint32_t>(S.tidx), n, 3 * LEVELS,
+                          as<int>(S.counters) + 3));
     gather_bodies<V4><<<blocks(n), 256, 0, st>>>(d_aff, as<uint32_t>(S.tidx), n, as<V4>(tb));
     return check_launch(ctx, "gather_bodies(targets)");
 }

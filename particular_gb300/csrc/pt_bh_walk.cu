@@ -1772,6 +1772,14 @@ static GroupKernel group_kernel(bool quad, bool guard, bool learned, bool local,
 
 
 
+// Clears the error word (counters[3]) before a build or a walk of separate targets; within
+// a leapfrog sequence it collects every step's errors.
+int clear_errors(pt_ctx *ctx, State &S) {
+    PT_TRY(ensure_buf(ctx, S.counters, sizeof(unsigned long long) * 16));
+    if (!ctx->keep_errors) PT_CUDA(cudaMemsetAsync(as<int>(S.counters) + 3, 0, sizeof(int), ctx->stream));
+    return PT_OK;
+}
+
 int run(pt_ctx *ctx, const float4 *d_aff, int n_aff, const float4 *d_src, int n_src, float theta,
                float softening, uint32_t flags, float *d_out) {
     cudaStream_t st = ctx->stream;
@@ -1784,6 +1792,7 @@ int run(pt_ctx *ctx, const float4 *d_aff, int n_aff, const float4 *d_src, int n_
     if (!Sp) return set_error(PT_ERR_OOM, "Barnes-Hut state allocation failed");
     State &S = *Sp;
     mark(ctx, 0);
+    PT_TRY(clear_errors(ctx, S));
     PT_TRY(build(ctx, S, d_src, n_src));
     const bool same = (d_aff == d_src) && (n_aff == n_src);
     const float4 *tbody;
@@ -1822,6 +1831,7 @@ int run64(pt_ctx *ctx, const double4_32a *d_aff, int n_aff, const double4_32a *d
     if (!Sp) return set_error(PT_ERR_OOM, "Barnes-Hut state allocation failed");
     State &S = *Sp;
     mark(ctx, 0);
+    PT_TRY(clear_errors(ctx, S));
     PT_TRY(build_t<double>(ctx, S, d_src, n_src));
     const bool same = (d_aff == d_src) && (n_aff == n_src);
     if (!same) PT_TRY(sort_targets_t<double>(ctx, S, d_aff, n_aff));
@@ -1830,7 +1840,6 @@ int run64(pt_ctx *ctx, const double4_32a *d_aff, int n_aff, const double4_32a *d
     unsigned long long *stats = reinterpret_cast<unsigned long long *>(S.counters.ptr) + 2;
     int *err = as<int>(S.counters) + 3;
     PT_CUDA(cudaMemsetAsync(stats, 0, 9 * sizeof(unsigned long long), st));
-    PT_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
     mark(ctx, 1);
     const int lpb = lanes_per_body64(ctx, n_aff);
     auto kern = lpb == 4 ? bh_walk64<4> : lpb == 2 ? bh_walk64<2> : bh_walk64<1>;
@@ -1854,8 +1863,6 @@ int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n
     unsigned long long *stats = reinterpret_cast<unsigned long long *>(S.counters.ptr) + 2;
     int *err = as<int>(S.counters) + 3;
     PT_CUDA(cudaMemsetAsync(stats, 0, 9 * sizeof(unsigned long long), st));
-    // within a leapfrog sequence the error word collects every step's errors
-    if (!ctx->keep_errors) PT_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
     const float th2 = theta * theta;
     const float eps2 = softening * softening;
     const bool quad = flags & PT_BH_QUADRUPOLE;

@@ -1,11 +1,19 @@
-// Stable LSD radix sort, written for the Barnes-Hut build.
+// Stable radix sort of 63-bit keys and their bodies' indices, written for the Barnes-Hut build.
 //
-// radix_sort_u64: 8-bit digits; per digit a histogram pass (per-tile counts), a row
-// scan (one block per digit value over the tiles) and a scatter pass. The scatter
-// ranks keys stably inside a tile (each warp its own run of keys, with warp
-// match/popc), so equal digits keep their input order, stages the tile in shared
-// memory in digit order and writes every digit's run contiguously.
+// The upper HEAD_BITS bits are sorted by LSD passes of 8-bit digits; bodies that share them
+// are few and next to each other then, and rs_finish orders each such run by the whole key.
+// Where a run is longer than RUN_LIMIT (a cluster far smaller than 2^-13 of the box), it
+// raises a flag and rs_all, launched in any case, sorts everything by all eight digits.
+//
+// A pass ranks keys stably inside a tile (each warp its own run of keys, with warp
+// match/popc), so equal digits keep their input order, stages the tile in shared memory in
+// digit order and writes every digit's run contiguously. Up to DIRECT_TILES tiles a pass is
+// one launch: every block adds up the tiles' digit counts itself, and counts the digits of
+// the next pass as it writes. Above, a histogram pass (per-tile counts) and a row scan (one
+// block per digit value over the tiles) come before the scatter.
 #include "pt_prims.cuh"
+
+#include <algorithm>
 
 namespace pt {
 namespace prims {
@@ -27,7 +35,11 @@ constexpr int RS_THREADS = 256;
 #endif
 constexpr int RS_ROUNDS = PT_RS_ROUNDS;  // keys per thread of a tile
 constexpr int RS_TILE = RS_THREADS * RS_ROUNDS;
+static_assert(RS_TILE == RADIX_TILE, "the producer of the keys counts their first digits by tile");
 constexpr int RS_WARPS = RS_THREADS / 32;
+
+// Tiles up to which a pass is one launch.
+constexpr int DIRECT_TILES = 64;
 
 // Exclusive scan of one value per thread over the 256 threads of a block; wsum holds
 // RS_WARPS + 1 words. Every thread of the block must call it.
@@ -49,68 +61,77 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *wsum, 
     return r;
 }
 
+__device__ __forceinline__ uint32_t digit_of(uint64_t key, int shift) { return uint32_t(key >> shift) & 255u; }
+
 // hist[d * nblocks + b] = count of digit d in tile b.
-__global__ void __launch_bounds__(RS_THREADS)
-    rs_hist(const uint64_t *__restrict__ keys, int n, int shift, uint32_t *__restrict__ hist, int nblocks) {
-    __shared__ uint32_t cnt[256];
+__device__ __forceinline__ void hist_tile(const uint64_t *__restrict__ keys, int n, int shift,
+                                          uint32_t *__restrict__ hist, int nblocks, int b, uint32_t *cnt) {
     cnt[threadIdx.x] = 0;
     __syncthreads();
-    const size_t base = size_t(blockIdx.x) * RS_TILE;
+    const size_t base = size_t(b) * RS_TILE;
 #pragma unroll 4
     for (int r = 0; r < RS_ROUNDS; ++r) {
         const size_t i = base + size_t(r) * RS_THREADS + threadIdx.x;
-        if (i < size_t(n)) atomicAdd(&cnt[(keys[i] >> shift) & 255u], 1u);
+        if (i < size_t(n)) atomicAdd(&cnt[digit_of(__ldcg(keys + i), shift)], 1u);
     }
     __syncthreads();
-    hist[size_t(threadIdx.x) * nblocks + blockIdx.x] = cnt[threadIdx.x];
+    hist[size_t(threadIdx.x) * nblocks + b] = cnt[threadIdx.x];
 }
 
-// One block per digit d: offs[d * nblocks + b] = count of digit d in tiles before b,
-// rowsum[d] = count of digit d.
 __global__ void __launch_bounds__(RS_THREADS)
-    rs_rowscan(const uint32_t *__restrict__ hist, uint32_t *__restrict__ offs, uint32_t *__restrict__ rowsum,
-               int nblocks) {
-    __shared__ uint32_t wsum[RS_WARPS + 1];
-    const int d = blockIdx.x;
+    rs_hist(const uint64_t *__restrict__ keys, int n, int shift, uint32_t *__restrict__ hist, int nblocks) {
+    __shared__ uint32_t cnt[256];
+    hist_tile(keys, n, shift, hist, nblocks, blockIdx.x, cnt);
+}
+
+// Digit d: offs[d * nblocks + b] = count of digit d in tiles before b, rowsum[d] = count of
+// digit d.
+__device__ __forceinline__ void scan_row(const uint32_t *__restrict__ hist, uint32_t *__restrict__ offs,
+                                         uint32_t *__restrict__ rowsum, int nblocks, int d, uint32_t *wsum) {
     const uint32_t *row = hist + size_t(d) * nblocks;
     uint32_t *orow = offs + size_t(d) * nblocks;
     const int q = (nblocks + RS_THREADS - 1) / RS_THREADS;
     const int b0 = min(nblocks, int(threadIdx.x) * q), b1 = min(nblocks, b0 + q);
     uint32_t s = 0;
-    for (int b = b0; b < b1; ++b) s += row[b];
+    for (int b = b0; b < b1; ++b) s += __ldcg(row + b);
     uint32_t total;
     uint32_t acc = block_excl_scan(s, wsum, &total);
     for (int b = b0; b < b1; ++b) {
-        const uint32_t h = row[b];
+        const uint32_t h = __ldcg(row + b);
         orow[b] = acc;
         acc += h;
     }
     if (threadIdx.x == 0) rowsum[d] = total;
 }
 
-// Ranks the tile's keys stably by digit, stages them in shared memory in digit order,
-// then writes each digit's run to its global range (consecutive threads write
-// consecutive addresses). Warp w owns the tile's w-th run of 32 * RS_ROUNDS keys and
-// ranks them round by round with warp match/popc against its own digit counters (no
-// block barrier between rounds); one scan over the warps per digit then orders the
-// warps, so equal digits keep their input order.
 __global__ void __launch_bounds__(RS_THREADS)
-    rs_scatter(const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin, uint64_t *__restrict__ kout,
-               uint32_t *__restrict__ vout, int n, int shift, const uint32_t *__restrict__ offs,
-               const uint32_t *__restrict__ rowsum, int nblocks) {
-    __shared__ uint64_t skeys[RS_TILE];
-    __shared__ uint32_t svals[RS_TILE];
-    __shared__ uint32_t wcnt[RS_WARPS][256];
-    __shared__ uint32_t tstart[256], gbase[256];
+    rs_rowscan(const uint32_t *__restrict__ hist, uint32_t *__restrict__ offs, uint32_t *__restrict__ rowsum,
+               int nblocks) {
     __shared__ uint32_t wsum[RS_WARPS + 1];
+    scan_row(hist, offs, rowsum, nblocks, blockIdx.x, wsum);
+}
+
+struct ScatterShared {
+    uint64_t skeys[RS_TILE];
+    uint32_t svals[RS_TILE];
+    uint32_t wcnt[RS_WARPS][256];
+    uint32_t tstart[256], gbase[256];
+    uint32_t wsum[RS_WARPS + 1];
+};
+
+// Tile b's part of a pass: ranks its keys stably by digit, stages them in shared memory in
+// digit order, then writes each digit's run to its global range (consecutive threads write
+// consecutive addresses). Warp w owns the tile's w-th run of 32 * RS_ROUNDS keys and ranks
+// them round by round with warp match/popc against its own digit counters (no block barrier
+// between rounds); one scan over the warps per digit then orders the warps, so equal digits
+// keep their input order. gstart(t): where digit t's keys of this tile go. vin null: a key's
+// value is its index. next: null, or the digit counts by tile of the pass at next_shift. (All
+// reads go to L2: within rs_all other blocks have written what an earlier pass read.)
+template <class Start>
+__device__ __forceinline__ void scatter_tile(ScatterShared &S, const uint64_t *kin, const uint32_t *vin,
+                                             uint64_t *kout, uint32_t *vout, int n, int shift, int b,
+                                             const Start &gstart, uint32_t *next, int next_shift) {
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    const int b = blockIdx.x;
-    // digit t's global start for this tile: all smaller digits, then earlier tiles
-    gbase[t] = block_excl_scan(rowsum[t], wsum, nullptr) + offs[size_t(t) * nblocks + b];
-#pragma unroll
-    for (int w = 0; w < RS_WARPS; ++w) wcnt[w][t] = 0;
-    __syncthreads();
-    const uint32_t lt = (1u << lane) - 1u;
     const size_t wbase = size_t(b) * RS_TILE + size_t(warp) * (32 * RS_ROUNDS);
     uint64_t key[RS_ROUNDS];
     uint32_t val[RS_ROUNDS], rank[RS_ROUNDS];
@@ -118,14 +139,23 @@ __global__ void __launch_bounds__(RS_THREADS)
     for (int r = 0; r < RS_ROUNDS; ++r) {
         const size_t i = wbase + size_t(r) * 32 + lane;
         const bool valid = i < size_t(n);
-        key[r] = valid ? kin[i] : 0ull;
-        val[r] = valid ? vin[i] : 0u;
-        const uint32_t d = valid ? uint32_t((key[r] >> shift) & 255u) : 256u;
+        key[r] = valid ? __ldcg(kin + i) : 0ull;
+        val[r] = valid ? (vin ? __ldcg(vin + i) : uint32_t(i)) : 0u;
+    }
+    S.gbase[t] = gstart(t);
+#pragma unroll
+    for (int w = 0; w < RS_WARPS; ++w) S.wcnt[w][t] = 0;
+    __syncthreads();
+    const uint32_t lt = (1u << lane) - 1u;
+#pragma unroll
+    for (int r = 0; r < RS_ROUNDS; ++r) {
+        const bool valid = wbase + size_t(r) * 32 + lane < size_t(n);
+        const uint32_t d = valid ? digit_of(key[r], shift) : 256u;
         const uint32_t peers = __match_any_sync(0xffffffffu, d);
         // keys of digit d in this warp's earlier rounds, then the lanes below
-        const uint32_t before = valid ? wcnt[warp][d] : 0u;
+        const uint32_t before = valid ? S.wcnt[warp][d] : 0u;
         __syncwarp();
-        if (valid && (peers & lt) == 0u) wcnt[warp][d] = before + __popc(peers);
+        if (valid && (peers & lt) == 0u) S.wcnt[warp][d] = before + __popc(peers);
         __syncwarp();
         rank[r] = before + __popc(peers & lt);
     }
@@ -134,66 +164,241 @@ __global__ void __launch_bounds__(RS_THREADS)
     uint32_t tot = 0;
 #pragma unroll
     for (int w = 0; w < RS_WARPS; ++w) {
-        const uint32_t c = wcnt[w][t];
-        wcnt[w][t] = tot;
+        const uint32_t c = S.wcnt[w][t];
+        S.wcnt[w][t] = tot;
         tot += c;
     }
-    tstart[t] = block_excl_scan(tot, wsum, nullptr);
+    S.tstart[t] = block_excl_scan(tot, S.wsum, nullptr);
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < RS_ROUNDS; ++r) {
-        const size_t i = wbase + size_t(r) * 32 + lane;
-        if (i < size_t(n)) {
-            const uint32_t d = uint32_t((key[r] >> shift) & 255u);
-            const uint32_t pos = tstart[d] + wcnt[warp][d] + rank[r];
-            skeys[pos] = key[r];
-            svals[pos] = val[r];
+        if (wbase + size_t(r) * 32 + lane < size_t(n)) {
+            const uint32_t d = digit_of(key[r], shift);
+            const uint32_t pos = S.tstart[d] + S.wcnt[warp][d] + rank[r];
+            S.skeys[pos] = key[r];
+            S.svals[pos] = val[r];
         }
     }
     __syncthreads();
     const int cnt = int(min(size_t(RS_TILE), size_t(n) - size_t(b) * RS_TILE));
     for (int i = t; i < cnt; i += RS_THREADS) {
-        const uint64_t k = skeys[i];
-        const uint32_t d = uint32_t(k >> shift) & 255u;
-        const uint32_t pos = gbase[d] + (uint32_t(i) - tstart[d]);
+        const uint64_t k = S.skeys[i];
+        const uint32_t d = digit_of(k, shift);
+        const uint32_t pos = S.gbase[d] + (uint32_t(i) - S.tstart[d]);
         kout[pos] = k;
-        vout[pos] = svals[i];
+        vout[pos] = S.svals[i];
+        if (next) atomicAdd(&next[(pos / RS_TILE) * 256 + digit_of(k, next_shift)], 1u);
     }
+}
+
+__global__ void __launch_bounds__(RS_THREADS)
+    rs_scatter(const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin, uint64_t *__restrict__ kout,
+               uint32_t *__restrict__ vout, int n, int shift, const uint32_t *__restrict__ offs,
+               const uint32_t *__restrict__ rowsum, int nblocks) {
+    __shared__ ScatterShared S;
+    const int b = blockIdx.x;
+    // all smaller digits, then earlier tiles
+    scatter_tile(S, kin, vin, kout, vout, n, shift, b,
+                 [&](int t) { return block_excl_scan(rowsum[t], S.wsum, nullptr) + offs[size_t(t) * nblocks + b]; },
+                 nullptr, 0);
+}
+
+// One pass in one launch: hist[b * 256 + d] holds the tiles' digit counts.
+__global__ void __launch_bounds__(RS_THREADS)
+    rs_pass(const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin, uint64_t *__restrict__ kout,
+            uint32_t *__restrict__ vout, int n, int shift, const uint32_t *__restrict__ hist, int nblocks,
+            uint32_t *__restrict__ next, int next_shift) {
+    __shared__ ScatterShared S;
+    const int b = blockIdx.x;
+    scatter_tile(S, kin, vin, kout, vout, n, shift, b,
+                 [&](int t) {
+                     uint32_t before = 0, total = 0;
+#pragma unroll 8
+                     for (int j = 0; j < nblocks; ++j) {
+                         const uint32_t h = hist[j * 256 + t];
+                         if (j < b) before += h;
+                         total += h;
+                     }
+                     return block_excl_scan(total, S.wsum, nullptr) + before;
+                 },
+                 next, next_shift);
+}
+
+// Orders every run of keys with the same upper bits (key >> shift) by the whole key, stably:
+// each key counts those of its run that come before it. Raises *redo (and leaves the output
+// to rs_all) where a run reaches further than RUN_LIMIT keys to one side.
+constexpr int RUN_LIMIT = 48;
+
+__global__ void __launch_bounds__(256)
+    rs_finish(const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin, int n, int shift,
+              uint64_t *__restrict__ kout, uint32_t *__restrict__ vout, int *__restrict__ redo) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const uint64_t k = kin[i], h = k >> shift;
+    int lo = i, hi = i, before = 0;
+    while (lo > 0 && i - lo < RUN_LIMIT) {
+        const uint64_t x = kin[lo - 1];
+        if ((x >> shift) != h) break;
+        --lo;
+        before += x <= k;
+    }
+    while (hi + 1 < n && hi - i < RUN_LIMIT) {
+        const uint64_t x = kin[hi + 1];
+        if ((x >> shift) != h) break;
+        ++hi;
+        before += x < k;
+    }
+    if (i - lo >= RUN_LIMIT || hi - i >= RUN_LIMIT) *redo = 1;
+    const int pos = lo + before;  // in [lo, hi]
+    kout[pos] = k;
+    vout[pos] = vin[i];
+}
+
+// A barrier over the grid of a cooperative launch: ctrl[0] arrivals, ctrl[1] generation. It
+// gives up after SPIN_LIMIT waits (all blocks then leave): returns false.
+constexpr int SPIN_LIMIT = 1 << 24;
+__device__ bool grid_barrier(unsigned *ctrl, volatile unsigned *failed) {
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        volatile unsigned *gen = ctrl + 1;
+        const unsigned g = *gen;
+        __threadfence();
+        if (atomicAdd(ctrl, 1u) == gridDim.x - 1) {
+            atomicExch(ctrl, 0u);
+            __threadfence();
+            atomicAdd(ctrl + 1, 1u);
+        } else {
+            int it = 0;
+            while (*gen == g) {
+                if (++it > SPIN_LIMIT || *failed) {
+                    *failed = 1u;
+                    break;
+                }
+                __nanosleep(64);
+            }
+        }
+        __threadfence();
+        ok = *failed == 0u;
+    }
+    __syncthreads();
+    return ok;
+}
+
+// When *redo is set: sorts (kb, vb) by all eight digits into (ka, va), one cooperative launch.
+// ctrl: arrivals, generation, failed; a barrier that gave up is told in *err. When *redo is
+// not set every block leaves at once.
+__global__ void __launch_bounds__(RS_THREADS)
+    rs_all(uint64_t *ka, uint32_t *va, uint64_t *kb, uint32_t *vb, int n, int passes, uint32_t *hist, uint32_t *offs,
+           uint32_t *rowsum, int nblocks, const int *redo, unsigned *ctrl, int *err) {
+    if (*redo == 0) return;
+    auto barrier = [&]() {
+        const bool ok = grid_barrier(ctrl, ctrl + 2);
+        if (!ok && threadIdx.x == 0) atomicOr(err, ERR_SORT_BARRIER);
+        return ok;
+    };
+    __shared__ ScatterShared S;
+    uint64_t *kin = kb, *kout = ka;
+    uint32_t *vin = vb, *vout = va;
+    for (int p = 0; p < passes; ++p) {
+        for (int b = blockIdx.x; b < nblocks; b += gridDim.x) {
+            hist_tile(kin, n, 8 * p, hist, nblocks, b, S.tstart);
+            __syncthreads();
+        }
+        if (!barrier()) return;
+        for (int d = blockIdx.x; d < 256; d += gridDim.x) scan_row(hist, offs, rowsum, nblocks, d, S.wsum);
+        if (!barrier()) return;
+        for (int b = blockIdx.x; b < nblocks; b += gridDim.x) {
+            scatter_tile(S, kin, vin, kout, vout, n, 8 * p, b,
+                         [&](int t) {
+                             return block_excl_scan(__ldcg(rowsum + t), S.wsum, nullptr) +
+                                    __ldcg(offs + size_t(t) * nblocks + b);
+                         },
+                         nullptr, 0);
+            __syncthreads();
+        }
+        if (!barrier()) return;
+        uint64_t *tk = kin;
+        kin = kout;
+        kout = tk;
+        uint32_t *tv = vin;
+        vin = vout;
+        vout = tv;
+    }
+    if (kin == kb)  // the last pass wrote the other pair
+        for (int i = blockIdx.x * RS_THREADS + threadIdx.x; i < n; i += gridDim.x * RS_THREADS) {
+            ka[i] = __ldcg(kb + i);
+            va[i] = __ldcg(vb + i);
+        }
 }
 
 }  // namespace prims
 
-int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, int n, int bits) {
+// The first sorted bit of n keys: five digits from the top (13 octree levels and a bit) leave
+// runs of a few bodies at 4M bulge+disk; a sixth from 8M on.
+static int head_shift(int n, int bits) { return std::max(0, bits - 8 * (n >= (1 << 23) ? 6 : 5)); }
+
+int radix_sort_prepare(pt_ctx *ctx, PrimScratch &s, int n, int bits, RadixFirst *first) {
     using namespace prims;
-    if (n <= 1) return PT_OK;
     const int nblocks = (n + RS_TILE - 1) / RS_TILE;
+    const int shift = head_shift(n, bits), passes = (bits - shift + 7) / 8;
     const size_t nhist = 256 * size_t(nblocks);
+    // histograms: per pass of the direct passes, or counts + offsets + row sums
+    const size_t words = std::max(size_t(passes) * nhist, 2 * nhist + 256) + 64;
     PT_TRY(ensure_buf(ctx, s.keys2, sizeof(uint64_t) * size_t(n)));
     PT_TRY(ensure_buf(ctx, s.vals2, sizeof(uint32_t) * size_t(n)));
-    PT_TRY(ensure_buf(ctx, s.hist, sizeof(uint32_t) * (2 * nhist + 256)));
+    PT_TRY(ensure_buf(ctx, s.hist, sizeof(uint32_t) * words));
+    // the last 64 words: the redo flag and the barrier of rs_all
+    const bool direct = nblocks <= DIRECT_TILES;
     uint32_t *hist = static_cast<uint32_t *>(s.hist.ptr);
-    uint32_t *offs = hist + nhist;
-    uint32_t *rowsum = offs + nhist;
-    uint64_t *ka = keys, *kb = static_cast<uint64_t *>(s.keys2.ptr);
-    uint32_t *va = vals, *vb = static_cast<uint32_t *>(s.vals2.ptr);
-    const int passes = (bits + 7) / 8;
+    uint32_t *tail = hist + (words - 64);
+    if (direct) PT_CUDA(cudaMemsetAsync(hist, 0, sizeof(uint32_t) * words, ctx->stream));
+    else PT_CUDA(cudaMemsetAsync(tail, 0, sizeof(uint32_t) * 64, ctx->stream));
+    // an odd number of passes ends in the pair that the finishing pass reads
+    first->keys = (passes & 1) ? nullptr : static_cast<uint64_t *>(s.keys2.ptr);
+    first->hist = direct ? hist : nullptr;
+    first->shift = shift;
+    return PT_OK;
+}
+
+int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, int n, int bits, int *err) {
+    using namespace prims;
+    const int nblocks = (n + RS_TILE - 1) / RS_TILE;
+    const int shift0 = head_shift(n, bits), passes = (bits - shift0 + 7) / 8;
+    const size_t nhist = 256 * size_t(nblocks);
+    const size_t words = std::max(size_t(passes) * nhist, 2 * nhist + 256) + 64;
+    uint32_t *hist = static_cast<uint32_t *>(s.hist.ptr);
+    int *redo = reinterpret_cast<int *>(hist + (words - 64));
+    unsigned *ctrl = reinterpret_cast<unsigned *>(redo + 16);
+    uint32_t *offs = hist + nhist, *rowsum = offs + nhist;
+    uint64_t *kb = static_cast<uint64_t *>(s.keys2.ptr), *k[2] = {keys, kb};
+    uint32_t *vb = static_cast<uint32_t *>(s.vals2.ptr), *v[2] = {vals, vb};
     cudaStream_t st = ctx->stream;
-    for (int p = 0; p < passes; ++p) {
-        const int shift = 8 * p;
-        rs_hist<<<nblocks, RS_THREADS, 0, st>>>(ka, n, shift, hist, nblocks);
+    int in = (passes & 1) ? 0 : 1;  // the passes end in (kb, vb)
+    for (int p = 0; p < passes; ++p, in ^= 1) {
+        const int shift = shift0 + 8 * p;
+        const uint32_t *vin = p == 0 ? nullptr : v[in];
+        if (nblocks <= DIRECT_TILES) {
+            uint32_t *next = p + 1 < passes ? hist + (p + 1) * nhist : nullptr;
+            rs_pass<<<nblocks, RS_THREADS, 0, st>>>(k[in], vin, k[in ^ 1], v[in ^ 1], n, shift, hist + p * nhist,
+                                                    nblocks, next, shift + 8);
+            PT_TRY(check_launch(ctx, "rs_pass"));
+            continue;
+        }
+        rs_hist<<<nblocks, RS_THREADS, 0, st>>>(k[in], n, shift, hist, nblocks);
         PT_TRY(check_launch(ctx, "rs_hist"));
         rs_rowscan<<<256, RS_THREADS, 0, st>>>(hist, offs, rowsum, nblocks);
         PT_TRY(check_launch(ctx, "rs_rowscan"));
-        rs_scatter<<<nblocks, RS_THREADS, 0, st>>>(ka, va, kb, vb, n, shift, offs, rowsum, nblocks);
+        rs_scatter<<<nblocks, RS_THREADS, 0, st>>>(k[in], vin, k[in ^ 1], v[in ^ 1], n, shift, offs, rowsum, nblocks);
         PT_TRY(check_launch(ctx, "rs_scatter"));
-        std::swap(ka, kb);
-        std::swap(va, vb);
     }
-    if (ka != keys) {
-        PT_CUDA(cudaMemcpyAsync(keys, ka, sizeof(uint64_t) * size_t(n), cudaMemcpyDeviceToDevice, st));
-        PT_CUDA(cudaMemcpyAsync(vals, va, sizeof(uint32_t) * size_t(n), cudaMemcpyDeviceToDevice, st));
-    }
-    return PT_OK;
+    rs_finish<<<(n + 255) / 256, 256, 0, st>>>(kb, vb, n, shift0, keys, vals, redo);
+    PT_TRY(check_launch(ctx, "rs_finish"));
+    int all = (bits + 7) / 8, nb = nblocks;
+    void *args[] = {&keys, &vals, &kb, &vb, &n, &all, &hist, &offs, &rowsum, &nb, &redo, &ctrl, &err};
+    const int grid = std::min(nblocks, 2 * std::max(1, ctx->sm_count));  // 2 of 36 KB fit every SM
+    PT_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(rs_all), dim3(grid), dim3(RS_THREADS), args, 0, st));
+    return check_launch(ctx, "rs_all");
 }
 
 void prim_free(pt_ctx *ctx, PrimScratch &s) {

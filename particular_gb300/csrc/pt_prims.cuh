@@ -1,5 +1,5 @@
 // Device-wide primitives used by the Barnes-Hut build: scratch for the scans of pt_scan.cuh
-// and a stable LSD radix sort of (u64 key, u32 value) pairs.
+// and a stable radix sort of u64 keys and their indices.
 #pragma once
 
 #include "pt_common.cuh"
@@ -9,14 +9,26 @@ namespace pt {
 // Scratch for the primitives; grow-only, owned by a subsystem.
 struct PrimScratch {
     DevBuf scan;   // tile totals of a scan
-    DevBuf hist;   // radix histograms / offsets
+    DevBuf hist;   // radix histograms / offsets, the flags of a sort
     DevBuf keys2;  // ping-pong keys
     DevBuf vals2;  // ping-pong values
 };
 
-// Sorts keys (and their values) ascending by the low `bits` bits, stably. The
-// result ends in keys/vals.
-int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, int n, int bits);
+// Sorting n keys takes two calls: radix_sort_prepare before the keys are produced tells the
+// producer where to put them (first->keys, or the caller's own array where that is null) and,
+// for small n, to count their first digits: hist[(i / RADIX_TILE) * 256 + (key >> shift &
+// 255)] for key i where hist is not null. radix_sort_u64 then leaves the keys ascending by
+// their low `bits` bits in keys, equal ones in the order of their index, and their indices in
+// vals. *err (device) gets ERR_SORT_BARRIER where a grid barrier of the general path gave up.
+constexpr int ERR_SORT_BARRIER = 4;
+constexpr int RADIX_TILE = 2048;
+struct RadixFirst {
+    uint64_t *keys;
+    uint32_t *hist;
+    int shift;
+};
+int radix_sort_prepare(pt_ctx *ctx, PrimScratch &s, int n, int bits, RadixFirst *first);
+int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, int n, int bits, int *err);
 
 void prim_free(pt_ctx *ctx, PrimScratch &s);
 

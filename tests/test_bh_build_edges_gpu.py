@@ -62,3 +62,43 @@ def test_coincident_bodies_across_blocks(res, copies):
     com = (b[:, :3].astype(np.float64) * b[:, 3:]).sum(0) / M
     assert abs(g["com_mass"][0, 3] - M) <= 1e-6 * M
     assert np.abs(g["com_mass"][0, :3] - com).max() <= 1e-5
+
+
+def reference_order(b):
+    """Bodies in ascending key order: the root box and 21 subdivisions in the build's f32 ops."""
+    x = b[:, :3]
+    mn, mx = x.min(0), x.max(0)
+    c = (mn + mx) * np.float32(0.5)
+    half = np.float32((mx - mn).max()) * np.float32(0.5)
+    lo, hi = np.tile(c - half, (len(b), 1)), np.tile(c + half, (len(b), 1))
+    key = np.zeros(len(b), np.uint64)
+    for _ in range(21):
+        c = (lo + hi) * np.float32(0.5)
+        left = x < c
+        hi, lo = np.where(left, c, hi), np.where(left, lo, c)
+        o = left[:, 0] + 2 * left[:, 1].astype(int) + 4 * left[:, 2].astype(int)
+        key = (key << np.uint64(3)) | (7 - o).astype(np.uint64)
+    return np.argsort(key, kind="stable"), key
+
+
+# tiles of 2048 keys, one launch a pass up to 64 of them; and clusters so much smaller than
+# the box that their keys share the upper bits the passes sort, in runs short and long
+@pytest.mark.parametrize("n", [2047, 2048, 2049, 131072, 131073])
+@pytest.mark.parametrize("kind", ["cube", "runs", "core"])
+def test_bodies_are_in_key_order(res, n, kind):
+    r = np.random.RandomState(n)
+    x = r.uniform(-1, 1, (n, 3))
+    if kind == "runs":  # knots of 1 to 30 bodies, 1e-5 of the box wide
+        x = np.repeat(x, r.randint(1, 31, n), axis=0)[:n] + r.uniform(-1e-5, 1e-5, (n, 3))
+        x = x[r.permutation(n)]
+    elif kind == "core":  # all but a few within 1e-5 of the box
+        x[20:] *= 1e-5
+    b = np.concatenate([x, np.ones((n, 1))], 1).astype(np.float32)
+    order, key = reference_order(b)
+    g = tree_of(res, b)
+    leaves = g["links"][:, 2] < 0
+    first, count = g["links"][~leaves, 2], g["links"][~leaves, 3]
+    assert count.sum() == n and np.array_equal(first, np.cumsum(count) - count)
+    assert np.array_equal(count, np.unique(key, return_counts=True)[1])
+    single = count == 1
+    assert np.array_equal(g["com_mass"][~leaves][single], b[order[first[single]]])
