@@ -166,6 +166,20 @@ struct RegSums {
         for (int i = 0; i < TPL; ++i) csum_zero(c[i]);
     }
     __device__ __forceinline__ void fold(int i, f2 tx, f2 ty, f2 tz) { csum_fold(c[i], tx, ty, tz); }
+    // adds up the sums of the LPB lanes that share body i; each of them gets the result
+    template <int LPB>
+    __device__ __forceinline__ void gather(int i) {
+        float *s[3] = {&c[i].sx, &c[i].sy, &c[i].sz}, *e[3] = {&c[i].cx, &c[i].cy, &c[i].cz};
+#pragma unroll
+        for (int o = 1; o < LPB; o <<= 1)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float os = __shfl_xor_sync(0xffffffffu, *s[a], o), oe = __shfl_xor_sync(0xffffffffu, *e[a], o);
+                float r = *e[a] + oe;
+                two_sum_acc(*s[a], r, os);
+                *e[a] = r;
+            }
+    }
     __device__ __forceinline__ void total(int i, float &x, float &y, float &z) const {
         x = c[i].sx + c[i].cx;
         y = c[i].sy + c[i].cy;
@@ -1086,21 +1100,17 @@ __global__ void __launch_bounds__(128)
 }
 
 // ---- masked group walk: the reference's rule, per body, with shared traversal ----
-// The default method (no PT_BH_GROUP). One warp walks for MW_TPL x 32 key-adjacent
-// bodies (MW_TPL per lane) like bh_walk_group, but every stack range carries the
+// The default method (no PT_BH_GROUP). One warp walks for 64 key-adjacent
+// bodies (two per lane; fewer in small calls) like bh_walk_group, but every stack range carries the
 // masks of the bodies that still descend into it, and every list entry the masks of
 // the bodies that accept it: each body's accepted set is exactly the reference's
 // (sequential.rs:470-505: skip a node at d^2 == 0, open a cell when theta^2 d^2 <
 // w^2, else accept). A list entry is evaluated for every body and weighted by the
 // body's mask bit. Sums run in list order instead of the reference's visit order
 // (rounding-level differences).
-// Warps (groups) per CTA of the masked walk: one, so that a finished group's slot is
-// refilled at once (walk at N = 4M, 4 / 2 / 1 warps per CTA: theta 0.5 14.57 / 14.46 /
-// 14.26 ms, with quadrupoles 22.79 / 22.60 / 22.64, theta 0.3 40.06 / 40.36 / 39.87).
-#ifndef PT_MW_WARPS
-#define PT_MW_WARPS 1
-#endif
-constexpr int MW_WARPS = PT_MW_WARPS;
+// One warp (group) per CTA, so that a finished group's slot is refilled at once (walk at N =
+// 4M, 4 / 2 / 1 warps per CTA: theta 0.5 14.57 / 14.46 / 14.26 ms, with quadrupoles 22.79 /
+// 22.60 / 22.64, theta 0.3 40.06 / 40.36 / 39.87).
 // Stack ranges per warp of the masked walk: 320 fit 20 one-warp CTAs per SM in shared
 // memory (384: 18). Walk at N = 4M, 384 -> 320: theta 0.5 13.96 -> 13.81 ms, with
 // quadrupoles 22.51 -> 22.38, theta 0.3 39.40 -> 39.03 (12 of 65536 warps then run out
@@ -1117,17 +1127,18 @@ constexpr int MW_STACK = PT_MW_STACK;
 #ifndef PT_MW_BODIES
 #define PT_MW_BODIES 128
 #endif
-constexpr int MW_TPL = 2;  // bodies per lane; mask word i covers bodies g0 + 32 i + lane
+// A warp walks for 32 TPL / LPB bodies: TPL bodies to a lane, mask word i covering bodies g0 +
+// 32 i + lane, or, in small calls, one body to LPB lanes, which carry the same mask bits,
+// vote alike and split the list entries among them.
 
 // Entry pair (packed lo/hi) for one body, weighted by the body's bits of the two
 // entries' masks (qm = the pair's mask words for this body's word).
-template <int NF, bool GUARD>
+template <int NF>
 __device__ __forceinline__ void eval_pair_masked(const f2 *q, f2 qm, f2 px, f2 py, f2 pz, f2 e2, f2 &ax, f2 &ay,
                                                  f2 &az) {
-    const int lane = threadIdx.x & 31;
+    const unsigned mine = 1u << (threadIdx.x & 31);
     float m0, m1;
     upk2(qm, m0, m1);
-    const f2 bit = pk2(float((__float_as_uint(m0) >> lane) & 1u), float((__float_as_uint(m1) >> lane) & 1u));
     const f2 dx = sub2(q[0], px);
     const f2 dy = sub2(q[1], py);
     const f2 dz = sub2(q[2], pz);
@@ -1135,11 +1146,11 @@ __device__ __forceinline__ void eval_pair_masked(const f2 *q, f2 qm, f2 px, f2 p
     float r0, r1;
     upk2(r2, r0, r1);
     float i0 = rsqrt_ftz(r0), i1 = rsqrt_ftz(r1);
-    if (GUARD) {
-        i0 = (r0 > 0.0f) ? i0 : 0.0f;
-        i1 = (r1 > 0.0f) ? i1 : 0.0f;
-    }
-    const f2 inv = mul2(pk2(i0, i1), bit);  // a body outside the entry's mask adds exactly 0
+    // a body outside the entry's mask adds exactly 0 (a body at r = 0 is never in it); a select
+    // on the mask word, where a factor made of the bit took a conversion on the MUFU pipe
+    i0 = (__float_as_uint(m0) & mine) ? i0 : 0.0f;
+    i1 = (__float_as_uint(m1) & mine) ? i1 : 0.0f;
+    const f2 inv = pk2(i0, i1);
     const f2 inv2 = mul2(inv, inv);
     const f2 sc = mul2(mul2(q[3], inv), inv2);
     if constexpr (NF == 10) {
@@ -1160,70 +1171,69 @@ __device__ __forceinline__ void eval_pair_masked(const f2 *q, f2 qm, f2 px, f2 p
     }
 }
 
-// Lists hold NF fields then MW_TPL mask words per entry.
-template <int NF, int CAP, bool GUARD>
-__device__ __forceinline__ void eval_list_masked(IList<NF + MW_TPL, CAP> &Lst, int cnt, const f2 (&px)[MW_TPL],
-                                                 const f2 (&py)[MW_TPL], const f2 (&pz)[MW_TPL], f2 e2,
-                                                 RegSums<MW_TPL> &acc) {
+// Lists hold NF fields then TPL mask words per entry.
+template <int NF, int TPL, int LPB, int CAP>
+__device__ __forceinline__ void eval_list_masked(IList<NF + TPL, CAP> &Lst, int cnt, const f2 (&px)[TPL],
+                                                 const f2 (&py)[TPL], const f2 (&pz)[TPL], f2 e2,
+                                                 RegSums<TPL> &acc) {
     const int lane = threadIdx.x & 31;
-    f2 ax[MW_TPL], ay[MW_TPL], az[MW_TPL];
+    f2 ax[TPL], ay[TPL], az[TPL];
 #pragma unroll
-    for (int i = 0; i < MW_TPL; ++i) ax[i] = ay[i] = az[i] = pk2(0.f, 0.f);
+    for (int i = 0; i < TPL; ++i) ax[i] = ay[i] = az[i] = pk2(0.f, 0.f);
     __syncwarp();
-    if (cnt & 1) {  // pad: far away, massless, empty masks
-        if (lane < NF + MW_TPL) Lst.f[lane][cnt] = (lane < 3) ? 1e30f : 0.0f;
+    const int end = (cnt + 2 * LPB - 1) / (2 * LPB) * (2 * LPB);
+    if (end != cnt) {  // pad: far away, massless, empty masks
+        for (int x = lane; x < (NF + TPL) * (end - cnt); x += 32)
+            Lst.f[x % (NF + TPL)][cnt + x / (NF + TPL)] = (x % (NF + TPL) < 3) ? 1e30f : 0.0f;
         __syncwarp();
-        ++cnt;
     }
 #pragma unroll 2
-    for (int e = 0; e < cnt; e += 2) {
-        f2 q[NF + MW_TPL];
+    for (int e = 2 * (lane % LPB); e < end; e += 2 * LPB) {
+        f2 q[NF + TPL];
 #pragma unroll
-        for (int k = 0; k < NF + MW_TPL; ++k) q[k] = *reinterpret_cast<const f2 *>(&Lst.f[k][e]);
+        for (int k = 0; k < NF + TPL; ++k) q[k] = *reinterpret_cast<const f2 *>(&Lst.f[k][e]);
 #pragma unroll
-        for (int i = 0; i < MW_TPL; ++i)
-            eval_pair_masked<NF, GUARD>(q, q[NF + i], px[i], py[i], pz[i], e2, ax[i], ay[i], az[i]);
+        for (int i = 0; i < TPL; ++i)
+            eval_pair_masked<NF>(q, q[NF + i], px[i], py[i], pz[i], e2, ax[i], ay[i], az[i]);
     }
 #pragma unroll
-    for (int i = 0; i < MW_TPL; ++i) acc.fold(i, ax[i], ay[i], az[i]);
+    for (int i = 0; i < TPL; ++i) acc.fold(i, ax[i], ay[i], az[i]);
     __syncwarp();
 }
 
-template <bool QUAD, bool GUARD>
-__global__ void __launch_bounds__(32 * MW_WARPS)
+template <bool QUAD, int TPL, int LPB>
+__global__ void __launch_bounds__(32)
     bh_walk_masked(const float4 *__restrict__ tbody, const uint32_t *__restrict__ tidx, int n_aff,
                    const float4 *__restrict__ nodeA, const int4 *__restrict__ nodeB,
                    const float4 *__restrict__ nodeQ, const float4 *__restrict__ sbody,
                    const int *__restrict__ counters, float th2, float eps2, float *__restrict__ out,
                    unsigned long long *__restrict__ stats) {
     constexpr int NFC = QUAD ? 10 : 4;
-    constexpr int TPL = MW_TPL;
-    static_assert(TPL == 2, "stack entries hold two mask words");
-    using CellList = IList<NFC + TPL, PT_MW_CELLS>;  // + the masks of the accepting bodies
-    using BodyList = IList<4 + TPL, PT_MW_BODIES>;
-    __shared__ int4 s_stack[MW_WARPS][MW_STACK];  // (first, end, mask word 0, mask word 1)
-    __shared__ __align__(16) CellList s_cells[MW_WARPS];
-    __shared__ __align__(16) BodyList s_bodies[MW_WARPS];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g0 = (blockIdx.x * MW_WARPS + warp) * 32 * TPL;
+    static_assert((TPL == 2 && LPB == 1) || (TPL == 1 && LPB <= 4), "two mask words, lists padded by 2 LPB - 1");
+    using CellList = IList<NFC + TPL, PT_MW_CELLS + (LPB > 1 ? 2 * LPB - 2 : 0)>;  // + the masks of the accepting bodies
+    using BodyList = IList<4 + TPL, PT_MW_BODIES + (LPB > 1 ? 2 * LPB - 2 : 0)>;
+    constexpr int CELLS = PT_MW_CELLS, BODIES = PT_MW_BODIES;  // the rest is padding
+    __shared__ int4 stack[MW_STACK];  // (first, end, mask word 0, mask word 1)
+    __shared__ __align__(16) CellList Lc;
+    __shared__ __align__(16) BodyList Lb;
+    const int lane = threadIdx.x;
+    const int g0 = blockIdx.x * (32 * TPL / LPB);
     if (g0 >= n_aff) return;
     float4 p[TPL];
     bool valid[TPL];
     unsigned vmask[TPL];
 #pragma unroll
     for (int i = 0; i < TPL; ++i) {
-        const int t = g0 + 32 * i + lane;
+        const int t = g0 + 32 * i + lane / LPB;
         valid[i] = t < n_aff;
         p[i] = tbody[valid[i] ? t : g0];
         vmask[i] = __ballot_sync(0xffffffffu, valid[i]);
     }
     const unsigned lt = (1u << lane) - 1u;
-    int4 *stack = s_stack[warp];
     const int T = counters[1];
-    CellList &Lc = s_cells[warp];
-    BodyList &Lb = s_bodies[warp];
-    float mn0 = fminf(p[0].x, p[1].x), mn1 = fminf(p[0].y, p[1].y), mn2 = fminf(p[0].z, p[1].z);
-    float mx0 = fmaxf(p[0].x, p[1].x), mx1 = fmaxf(p[0].y, p[1].y), mx2 = fmaxf(p[0].z, p[1].z);
+    const float4 pl = p[TPL - 1];
+    float mn0 = fminf(p[0].x, pl.x), mn1 = fminf(p[0].y, pl.y), mn2 = fminf(p[0].z, pl.z);
+    float mx0 = fmaxf(p[0].x, pl.x), mx1 = fmaxf(p[0].y, pl.y), mx2 = fmaxf(p[0].z, pl.z);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         mn0 = fminf(mn0, __shfl_xor_sync(0xffffffffu, mn0, o));
@@ -1243,7 +1253,7 @@ __global__ void __launch_bounds__(32 * MW_WARPS)
         py[i] = pk2(p[i].y, p[i].y);
         pz[i] = pk2(p[i].z, p[i].z);
     }
-    if (lane == 0) stack[0] = make_int4(0, T, int(vmask[0]), int(vmask[1]));
+    if (lane == 0) stack[0] = make_int4(0, T, int(vmask[0]), TPL == 2 ? int(vmask[TPL - 1]) : 0);
     __syncwarp();
     int S = 1, Nc = 0, Nb = 0;
     unsigned long long acc_pairs = 0, cell_pairs = 0, visit_pairs = 0;
@@ -1316,27 +1326,33 @@ __global__ void __launch_bounds__(32 * MW_WARPS)
                 }
             }
         }
+        // The voted nodes are read back from the stack's free slots (the popped ranges' and
+        // the room k left above them: at least 3 k, for 2 k nodes at most). A leaf's width is
+        // 0: no body opens it.
         unsigned vm = __ballot_sync(0xffffffffu, need);
-        while (vm) {
+        if (need) stack[S + __popc(vm & lt)] = make_int4(__float_as_int(A.x), __float_as_int(A.y), __float_as_int(A.z),
+                                                         __float_as_int(w * w));
+        __syncwarp();
+        for (int v = S; vm; ++v) {
             const int j = __ffs(vm) - 1;
             vm &= vm - 1;
-            const float cx = __shfl_sync(0xffffffffu, A.x, j);
-            const float cy = __shfl_sync(0xffffffffu, A.y, j);
-            const float cz = __shfl_sync(0xffffffffu, A.z, j);
-            const float cw = __shfl_sync(0xffffffffu, w, j);
-            const unsigned mj0 = __shfl_sync(0xffffffffu, mk0, j), mj1 = __shfl_sync(0xffffffffu, mk1, j);
-            const bool cj = __shfl_sync(0xffffffffu, cell, j);
-            const f2 dx = sub2(pk2(cx, cx), pk2(p[0].x, p[1].x));
-            const f2 dy = sub2(pk2(cy, cy), pk2(p[0].y, p[1].y));
-            const f2 dz = sub2(pk2(cz, cz), pk2(p[0].z, p[1].z));
+            const int4 c = stack[v];
+            const float cx = __int_as_float(c.x), cy = __int_as_float(c.y), cz = __int_as_float(c.z),
+                        cw2 = __int_as_float(c.w);
+            const unsigned mj0 = __shfl_sync(0xffffffffu, mk0, j);
+            const f2 dx = sub2(pk2(cx, cx), pk2(p[0].x, pl.x));
+            const f2 dy = sub2(pk2(cy, cy), pk2(p[0].y, pl.y));
+            const f2 dz = sub2(pk2(cz, cz), pk2(p[0].z, pl.z));
             float d0, d1;
             upk2(fma2(dx, dx, fma2(dy, dy, mul2(dz, dz))), d0, d1);
-            const bool in0 = (mj0 >> lane) & 1u, in1 = (mj1 >> lane) & 1u;
-            const bool o0 = in0 && cj && d0 > 0.0f && th2 * d0 < cw * cw;
-            const bool o1 = in1 && cj && d1 > 0.0f && th2 * d1 < cw * cw;
-            const unsigned om0 = __ballot_sync(0xffffffffu, o0), om1 = __ballot_sync(0xffffffffu, o1);
-            const unsigned am0 = __ballot_sync(0xffffffffu, in0 && !o0 && d0 > 0.0f);
-            const unsigned am1 = __ballot_sync(0xffffffffu, in1 && !o1 && d1 > 0.0f);
+            const unsigned om0 = mj0 & __ballot_sync(0xffffffffu, d0 > 0.0f && th2 * d0 < cw2);
+            const unsigned am0 = mj0 & ~om0 & __ballot_sync(0xffffffffu, d0 > 0.0f);
+            unsigned om1 = 0u, am1 = 0u;
+            if (TPL == 2) {
+                const unsigned mj1 = __shfl_sync(0xffffffffu, mk1, j);
+                om1 = mj1 & __ballot_sync(0xffffffffu, d1 > 0.0f && th2 * d1 < cw2);
+                am1 = mj1 & ~om1 & __ballot_sync(0xffffffffu, d1 > 0.0f);
+            }
             if (lane == j) {
                 op0 = om0;
                 op1 = om1;
@@ -1344,6 +1360,7 @@ __global__ void __launch_bounds__(32 * MW_WARPS)
                 ac1 = am1;
             }
         }
+        __syncwarp();
         // push: later siblings share the parent's masks; children get the opening bodies
         const bool rest = have && !handed && (mk0 | mk1) && B.y < r.y;
         const bool opn = (op0 | op1) != 0u;
@@ -1370,8 +1387,8 @@ __global__ void __launch_bounds__(32 * MW_WARPS)
         if (cellacc) cell_pairs += na;
         const unsigned mc = __ballot_sync(0xffffffffu, cellacc);
         const int nc1 = __popc(mc);
-        if (Nc + nc1 > CellList::CAP) {
-            eval_list_masked<NFC, CellList::CAP, GUARD>(Lc, Nc, px, py, pz, e2, bsum);
+        if (Nc + nc1 > CELLS) {
+            eval_list_masked<NFC, TPL, LPB>(Lc, Nc, px, py, pz, e2, bsum);
             Nc = 0;
         }
         if (cellacc) {
@@ -1391,13 +1408,13 @@ __global__ void __launch_bounds__(32 * MW_WARPS)
                 Lc.f[9][e] = -q1.y;
             }
             Lc.f[NFC][e] = __uint_as_float(ac0);
-            Lc.f[NFC + 1][e] = __uint_as_float(ac1);
+            if (TPL == 2) Lc.f[NFC + TPL - 1][e] = __uint_as_float(ac1);
         }
         Nc += nc1;
         const unsigned mb1 = __ballot_sync(0xffffffffu, bodyacc);
         const int nb1 = __popc(mb1);
-        if (Nb + nb1 > BodyList::CAP) {
-            eval_list_masked<4, BodyList::CAP, GUARD>(Lb, Nb, px, py, pz, e2, bsum);
+        if (Nb + nb1 > BODIES) {
+            eval_list_masked<4, TPL, LPB>(Lb, Nb, px, py, pz, e2, bsum);
             Nb = 0;
         }
         if (bodyacc) {
@@ -1407,7 +1424,7 @@ __global__ void __launch_bounds__(32 * MW_WARPS)
             Lb.f[2][e] = A.z;
             Lb.f[3][e] = A.w;
             Lb.f[4][e] = __uint_as_float(ac0);
-            Lb.f[5][e] = __uint_as_float(ac1);
+            if (TPL == 2) Lb.f[3 + TPL][e] = __uint_as_float(ac1);
         }
         Nb += nb1;
         unsigned mbk = __ballot_sync(0xffffffffu, bucket);
@@ -1419,29 +1436,43 @@ __global__ void __launch_bounds__(32 * MW_WARPS)
             const unsigned b0 = __shfl_sync(0xffffffffu, ac0, src), b1 = __shfl_sync(0xffffffffu, ac1, src);
             for (int base = 0; base < c; base += 32) {
                 const int n = min(32, c - base);
-                if (Nb + n > BodyList::CAP) {
-                    eval_list_masked<4, BodyList::CAP, GUARD>(Lb, Nb, px, py, pz, e2, bsum);
+                if (Nb + n > BODIES) {
+                    eval_list_masked<4, TPL, LPB>(Lb, Nb, px, py, pz, e2, bsum);
                     Nb = 0;
                 }
+                float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (lane < n) q = __ldg(sbody + f + base + lane);
+                unsigned q0 = 0u, q1 = 0u;
+                for (int j = 0; j < n; ++j) {  // a body does not meet itself in the leaf
+                    const float cx = __shfl_sync(0xffffffffu, q.x, j), cy = __shfl_sync(0xffffffffu, q.y, j),
+                                cz = __shfl_sync(0xffffffffu, q.z, j);
+                    const float x0 = cx - p[0].x, y0 = cy - p[0].y, z0 = cz - p[0].z;
+                    const float x1 = cx - pl.x, y1 = cy - pl.y, z1 = cz - pl.z;
+                    const unsigned m0 = __ballot_sync(0xffffffffu, fmaf(x0, x0, fmaf(y0, y0, z0 * z0)) > 0.f);
+                    const unsigned m1 = __ballot_sync(0xffffffffu, fmaf(x1, x1, fmaf(y1, y1, z1 * z1)) > 0.f);
+                    if (lane == j) q0 = b0 & m0, q1 = b1 & m1;
+                }
                 if (lane < n) {
-                    const float4 q = __ldg(sbody + f + base + lane);
                     Lb.f[0][Nb + lane] = q.x;
                     Lb.f[1][Nb + lane] = q.y;
                     Lb.f[2][Nb + lane] = q.z;
                     Lb.f[3][Nb + lane] = q.w;
-                    Lb.f[4][Nb + lane] = __uint_as_float(b0);
-                    Lb.f[5][Nb + lane] = __uint_as_float(b1);
+                    Lb.f[4][Nb + lane] = __uint_as_float(q0);
+                    if (TPL == 2) Lb.f[3 + TPL][Nb + lane] = __uint_as_float(q1);
                 }
                 Nb += n;
             }
         }
         __syncwarp();
     }
-    eval_list_masked<NFC, CellList::CAP, GUARD>(Lc, Nc, px, py, pz, e2, bsum);
-    eval_list_masked<4, BodyList::CAP, GUARD>(Lb, Nb, px, py, pz, e2, bsum);
+    eval_list_masked<NFC, TPL, LPB>(Lc, Nc, px, py, pz, e2, bsum);
+    eval_list_masked<4, TPL, LPB>(Lb, Nb, px, py, pz, e2, bsum);
     float rx[TPL], ry[TPL], rz[TPL];
 #pragma unroll
-    for (int i = 0; i < TPL; ++i) bsum.total(i, rx[i], ry[i], rz[i]);
+    for (int i = 0; i < TPL; ++i) {
+        if (LPB > 1) bsum.template gather<LPB>(i);
+        bsum.total(i, rx[i], ry[i], rz[i]);
+    }
     if (failed) {  // the stack ran out: the per-body cursor walk instead (warp-uniform)
         unsigned na = 0, nv = 0, nc = 0;
 #pragma unroll
@@ -1463,16 +1494,17 @@ __global__ void __launch_bounds__(32 * MW_WARPS)
 #pragma unroll
     for (int i = 0; i < TPL; ++i)
         if (valid[i]) {
-            const uint32_t o = tidx[g0 + 32 * i + lane];
+            if (LPB > 1 && lane % LPB != 0) continue;
+            const uint32_t o = tidx[g0 + 32 * i + lane / LPB];
             out[3 * size_t(o) + 0] = rx[i];
             out[3 * size_t(o) + 1] = ry[i];
             out[3 * size_t(o) + 2] = rz[i];
         }
     if (stats && lane == 0) {
-        atomicAdd(stats + 0, acc_pairs);
-        atomicAdd(stats + 1, visit_pairs);
+        atomicAdd(stats + 0, acc_pairs / LPB);
+        atomicAdd(stats + 1, visit_pairs / LPB);
         atomicAdd(stats + 2, 1ull);
-        atomicAdd(stats + 5, cell_pairs);
+        atomicAdd(stats + 5, cell_pairs / LPB);
         if (failed) atomicAdd(stats + 6, 1ull);
     }
 }
@@ -1752,9 +1784,16 @@ using GroupKernel = void (*)(const float4 *, const uint32_t *, int, const float4
                              const float4 *, const float4 *, const int *, float, float, LearnedRecords, float,
                              float *, unsigned long long *, int *, int, float, const float *, float);
 
-static WalkKernel masked_kernel(bool quad, bool guard) {
-    if (quad) return guard ? bh_walk_masked<true, true> : bh_walk_masked<true, false>;
-    return guard ? bh_walk_masked<false, true> : bh_walk_masked<false, false>;
+// bodies: per warp, 64, 32, 16 or 8
+template <bool QUAD>
+static WalkKernel masked_kernel_q(int bodies) {
+    return bodies == 64   ? bh_walk_masked<QUAD, 2, 1>
+           : bodies == 32 ? bh_walk_masked<QUAD, 1, 1>
+           : bodies == 16 ? bh_walk_masked<QUAD, 1, 2>
+                          : bh_walk_masked<QUAD, 1, 4>;
+}
+static WalkKernel masked_kernel(bool quad, int bodies) {
+    return quad ? masked_kernel_q<true>(bodies) : masked_kernel_q<false>(bodies);
 }
 
 template <bool LEARNED, bool LOCAL, bool REL>
@@ -1771,6 +1810,20 @@ static GroupKernel group_kernel(bool quad, bool guard, bool learned, bool local,
 }
 
 
+
+// Bodies per warp of the masked walk. A warp alone waits on its own loads and votes, so small
+// calls want many warps with little to evaluate in each: 8 or 16 bodies, 4 or 2 lanes to a
+// body, while these warps are all resident at once (20 per SM). 32 bodies, one to a lane,
+// meet fewer nodes than 64 (which share a traversal over more bodies) and end sooner; from
+// some 110 warps per SM on the traversals saved count for more. Whole call at 64 / 32 / 16 /
+// 8 bodies, us: N = 3000 theta 0.7 271 / 232 / 213 / 200; N = 30000 theta 0.5 552 / 436 / 391
+// / 392; N = 65536 theta 0.7 422 / 372 / 379 / 424; N = 262144 theta 0.5 1208 / 1163 / 1389 /
+// 1829; N = 524288 theta 0.8 1034 / 1027 / 1229 / 1653; N = 1M theta 0.5 3686 / 3759 / 4796 /
+// 6834.
+static int masked_bodies(const pt_ctx *ctx, int n_aff) {
+    const long long sms = std::max(1, ctx->sm_count);
+    return n_aff <= 8 * 20 * sms ? 8 : n_aff <= 16 * 20 * sms ? 16 : n_aff <= 32 * 110 * sms ? 32 : 64;
+}
 
 // Clears the error word (counters[3]) before a build or a walk of separate targets; within
 // a leapfrog sequence it collects every step's errors.
@@ -1928,8 +1981,8 @@ int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n
         mark(ctx, 2);
         return PT_OK;
     }
-    masked_kernel(quad, eps2 == 0.0f)<<<(n_aff + 32 * MW_TPL * MW_WARPS - 1) / (32 * MW_TPL * MW_WARPS),
-                                        32 * MW_WARPS, 0, st>>>(
+    const int bodies = masked_bodies(ctx, n_aff);
+    masked_kernel(quad, bodies)<<<(n_aff + bodies - 1) / bodies, 32, 0, st>>>(
         tbody, tidx, n_aff, as<float4>(S.nodeA), as<int4>(S.nodeB), as<float4>(S.nodeQ), as<float4>(S.sbody),
         as<int>(S.counters), th2, eps2, d_out, stats);
     PT_TRY(check_launch(ctx, "bh_walk_masked"));
