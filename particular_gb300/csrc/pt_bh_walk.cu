@@ -124,12 +124,40 @@ __device__ __forceinline__ void lane_walk(float4 p, bool valid, int T, const flo
 constexpr int GW_WARPS = PT_GW_WARPS;
 
 
-// Interaction lists in structure-of-arrays form. Cells carry their quadrupole
-// when QUAD; single bodies never need one.
+// Interaction lists. Cells carry their quadrupole when QUAD; single bodies never need one.
+// pair(): two entries' fields, packed.
 template <int NF, int CAP_>
-struct IList {
-    static constexpr int CAP = CAP_;
+struct IList {  // an array per field
+    static constexpr int FIELDS = NF, CAP = CAP_;
     float f[NF][CAP + 2];
+    __device__ __forceinline__ void put(int k, int e, float x) { f[k][e] = x; }
+    __device__ __forceinline__ void pair(int e, f2 (&q)[NF]) const {
+#pragma unroll
+        for (int k = 0; k < NF; ++k) q[k] = *reinterpret_cast<const f2 *>(&f[k][e]);
+    }
+};
+
+// The same with a field's two values of a pair of entries side by side, so that one 16-byte
+// read gives two fields. In the walks with local expansions this is the faster of the two (N
+// = 4M error bound: walk 5205 -> 5000 us), in the others its wider registers spill or it is 1-3 %
+// slower.
+template <int NF, int CAP_>
+struct PList {
+    static_assert(NF % 2 == 0, "two fields to a 16-byte read");
+    static constexpr int FIELDS = NF, CAP = CAP_;
+    float4 v[(CAP + 2) / 2 * (NF / 2)];
+    __device__ __forceinline__ void put(int k, int e, float x) {
+        reinterpret_cast<float *>(v)[(e >> 1) * (2 * NF) + 2 * k + (e & 1)] = x;
+    }
+    __device__ __forceinline__ void pair(int e, f2 (&q)[NF]) const {
+        const float4 *p = v + (e >> 1) * (NF / 2);
+#pragma unroll
+        for (int k = 0; k < NF / 2; ++k) {
+            const float4 t = p[k];
+            q[2 * k] = pk2(t.x, t.y);
+            q[2 * k + 1] = pk2(t.z, t.w);
+        }
+    }
 };
 
 // A body's acceleration as a compensated FP32 sum (running sum s, rounding errors c).
@@ -251,24 +279,24 @@ __device__ __forceinline__ void eval_pair(const f2 (&q)[NF], f2 px, f2 py, f2 pz
 // Evaluates entries [0, cnt) of a list for this lane's TPL targets, two entries per
 // packed instruction; each pair of entries is read from shared memory once for all
 // of the lane's targets.
-template <int NF, int CAP, bool GUARD, int TPL, class Sums>
-__device__ __forceinline__ void eval_list(IList<NF, CAP> &Lst, int cnt, const f2 (&px)[TPL], const f2 (&py)[TPL],
+template <bool GUARD, int TPL, class List, class Sums>
+__device__ __forceinline__ void eval_list(List &Lst, int cnt, const f2 (&px)[TPL], const f2 (&py)[TPL],
                                           const f2 (&pz)[TPL], f2 e2, Sums &acc) {
+    constexpr int NF = List::FIELDS;
     const int lane = threadIdx.x & 31;
     f2 ax[TPL], ay[TPL], az[TPL];
 #pragma unroll
     for (int i = 0; i < TPL; ++i) ax[i] = ay[i] = az[i] = pk2(0.f, 0.f);
     __syncwarp();
     if (cnt & 1) {  // pad with a massless entry far away: contributes exactly 0
-        if (lane < NF) Lst.f[lane][cnt] = (lane < 3) ? 1e30f : 0.0f;
+        if (lane < NF) Lst.put(lane, cnt, (lane < 3) ? 1e30f : 0.0f);
         __syncwarp();
         ++cnt;
     }
 #pragma unroll 2
     for (int e = 0; e < cnt; e += 2) {
         f2 q[NF];
-#pragma unroll
-        for (int k = 0; k < NF; ++k) q[k] = *reinterpret_cast<const f2 *>(&Lst.f[k][e]);
+        Lst.pair(e, q);
 #pragma unroll
         for (int i = 0; i < TPL; ++i) eval_pair<NF, GUARD>(q, px[i], py[i], pz[i], e2, ax[i], ay[i], az[i]);
     }
@@ -542,8 +570,8 @@ __global__ void __launch_bounds__(32 * GW_WARPS, (LOCAL ? PT_GW_LMINB : PT_GW_MI
     static_assert(!(LEARNED && REL), "PT_BH_LEARNED and PT_BH_RELATIVE are exclusive");
     constexpr int NFC = QUAD ? 10 : 4;
     constexpr int TPL = GW_TPL;
-    using CellList = IList<NFC, LOCAL ? PT_GW_LCELLS : 96>;
-    using BodyList = IList<4, LOCAL ? PT_GW_LBODIES : 128>;
+    using CellList = typename std::conditional<LOCAL, PList<NFC, PT_GW_LCELLS>, IList<NFC, 96>>::type;
+    using BodyList = typename std::conditional<LOCAL, PList<4, PT_GW_LBODIES>, IList<4, 128>>::type;
     // PT_BH_LOCAL keeps its 19 expansion coefficients per lane in shared memory
     // ([coefficient][lane]: no bank conflicts) and queues far nodes (up to 63) so that
     // they are expanded 32 at a time, one per lane, instead of by the few lanes that
@@ -839,26 +867,26 @@ __global__ void __launch_bounds__(32 * GW_WARPS, (LOCAL ? PT_GW_LMINB : PT_GW_MI
         const unsigned mc = __ballot_sync(0xffffffffu, cellacc);
         const int nc1 = __popc(mc);
         if (Nc + nc1 > CellList::CAP) {
-            eval_list<NFC, CellList::CAP, GUARD, TPL>(Lc, Nc, px, py, pz, e2, bsum);
+            eval_list<GUARD, TPL>(Lc, Nc, px, py, pz, e2, bsum);
             entries += Nc;
             centries += Nc;
             Nc = 0;
         }
         if (cellacc) {
             const int e = Nc + __popc(mc & lt);
-            Lc.f[0][e] = A.x;
-            Lc.f[1][e] = A.y;
-            Lc.f[2][e] = A.z;
-            Lc.f[3][e] = A.w;
+            Lc.put(0, e, A.x);
+            Lc.put(1, e, A.y);
+            Lc.put(2, e, A.z);
+            Lc.put(3, e, A.w);
             if constexpr (QUAD) {  // negated: the list evaluation's form
                 const float4 q0 = __ldg(nodeQ + 2 * node);
                 const float4 q1 = __ldg(nodeQ + 2 * node + 1);
-                Lc.f[4][e] = -q0.x;
-                Lc.f[5][e] = -q0.y;
-                Lc.f[6][e] = -q0.z;
-                Lc.f[7][e] = -q0.w;
-                Lc.f[8][e] = -q1.x;
-                Lc.f[9][e] = -q1.y;
+                Lc.put(4, e, -q0.x);
+                Lc.put(5, e, -q0.y);
+                Lc.put(6, e, -q0.z);
+                Lc.put(7, e, -q0.w);
+                Lc.put(8, e, -q1.x);
+                Lc.put(9, e, -q1.y);
             }
         }
         Nc += nc1;
@@ -866,16 +894,16 @@ __global__ void __launch_bounds__(32 * GW_WARPS, (LOCAL ? PT_GW_LMINB : PT_GW_MI
         const unsigned mb1 = __ballot_sync(0xffffffffu, bodyacc);
         const int nb1 = __popc(mb1);
         if (Nb + nb1 > BodyList::CAP) {
-            eval_list<4, BodyList::CAP, GUARD, TPL>(Lb, Nb, px, py, pz, e2, bsum);
+            eval_list<GUARD, TPL>(Lb, Nb, px, py, pz, e2, bsum);
             entries += Nb;
             Nb = 0;
         }
         if (bodyacc) {
             const int e = Nb + __popc(mb1 & lt);
-            Lb.f[0][e] = A.x;
-            Lb.f[1][e] = A.y;
-            Lb.f[2][e] = A.z;
-            Lb.f[3][e] = A.w;
+            Lb.put(0, e, A.x);
+            Lb.put(1, e, A.y);
+            Lb.put(2, e, A.z);
+            Lb.put(3, e, A.w);
         }
         Nb += nb1;
         // bodies [f, f + c) of the key-ordered array -> the body list (warp-uniform f, c)
@@ -883,16 +911,16 @@ __global__ void __launch_bounds__(32 * GW_WARPS, (LOCAL ? PT_GW_LMINB : PT_GW_MI
             for (int base = 0; base < c; base += 32) {
                 const int n = min(32, c - base);
                 if (Nb + n > BodyList::CAP) {
-                    eval_list<4, BodyList::CAP, GUARD, TPL>(Lb, Nb, px, py, pz, e2, bsum);
+                    eval_list<GUARD, TPL>(Lb, Nb, px, py, pz, e2, bsum);
                     entries += Nb;
                     Nb = 0;
                 }
                 if (lane < n) {
                     const float4 q = __ldg(sbody + f + base + lane);
-                    Lb.f[0][Nb + lane] = q.x;
-                    Lb.f[1][Nb + lane] = q.y;
-                    Lb.f[2][Nb + lane] = q.z;
-                    Lb.f[3][Nb + lane] = q.w;
+                    Lb.put(0, Nb + lane, q.x);
+                    Lb.put(1, Nb + lane, q.y);
+                    Lb.put(2, Nb + lane, q.z);
+                    Lb.put(3, Nb + lane, q.w);
                 }
                 Nb += n;
             }
@@ -937,16 +965,16 @@ __global__ void __launch_bounds__(32 * GW_WARPS, (LOCAL ? PT_GW_LMINB : PT_GW_MI
                 const unsigned m1 = __ballot_sync(0xffffffffu, one);
                 const int n1 = __popc(m1);
                 if (Nb + n1 > BodyList::CAP) {
-                    eval_list<4, BodyList::CAP, GUARD, TPL>(Lb, Nb, px, py, pz, e2, bsum);
+                    eval_list<GUARD, TPL>(Lb, Nb, px, py, pz, e2, bsum);
                     entries += Nb;
                     Nb = 0;
                 }
                 if (one) {
                     const int e = Nb + __popc(m1 & lt);
-                    Lb.f[0][e] = la.x;
-                    Lb.f[1][e] = la.y;
-                    Lb.f[2][e] = la.z;
-                    Lb.f[3][e] = la.w;
+                    Lb.put(0, e, la.x);
+                    Lb.put(1, e, la.y);
+                    Lb.put(2, e, la.z);
+                    Lb.put(3, e, la.w);
                 }
                 Nb += n1;
                 unsigned mm = __ballot_sync(0xffffffffu, lb.z >= 0 && lb.w > 1);
@@ -959,8 +987,8 @@ __global__ void __launch_bounds__(32 * GW_WARPS, (LOCAL ? PT_GW_LMINB : PT_GW_MI
         }
         __syncwarp();
     }
-    eval_list<NFC, CellList::CAP, GUARD, TPL>(Lc, Nc, px, py, pz, e2, bsum);
-    eval_list<4, BodyList::CAP, GUARD, TPL>(Lb, Nb, px, py, pz, e2, bsum);
+    eval_list<GUARD, TPL>(Lc, Nc, px, py, pz, e2, bsum);
+    eval_list<GUARD, TPL>(Lb, Nb, px, py, pz, e2, bsum);
     entries += Nc + Nb;
     centries += Nc;
     float rx[TPL], ry[TPL], rz[TPL];
@@ -1171,7 +1199,7 @@ __device__ __forceinline__ void eval_pair_masked(const f2 *q, f2 qm, f2 px, f2 p
     }
 }
 
-// Lists hold NF fields then TPL mask words per entry.
+// Lists hold NF fields, then TPL mask words per entry.
 template <int NF, int TPL, int LPB, int CAP>
 __device__ __forceinline__ void eval_list_masked(IList<NF + TPL, CAP> &Lst, int cnt, const f2 (&px)[TPL],
                                                  const f2 (&py)[TPL], const f2 (&pz)[TPL], f2 e2,
@@ -1184,14 +1212,13 @@ __device__ __forceinline__ void eval_list_masked(IList<NF + TPL, CAP> &Lst, int 
     const int end = (cnt + 2 * LPB - 1) / (2 * LPB) * (2 * LPB);
     if (end != cnt) {  // pad: far away, massless, empty masks
         for (int x = lane; x < (NF + TPL) * (end - cnt); x += 32)
-            Lst.f[x % (NF + TPL)][cnt + x / (NF + TPL)] = (x % (NF + TPL) < 3) ? 1e30f : 0.0f;
+            Lst.put(x % (NF + TPL), cnt + x / (NF + TPL), (x % (NF + TPL) < 3) ? 1e30f : 0.0f);
         __syncwarp();
     }
 #pragma unroll 2
     for (int e = 2 * (lane % LPB); e < end; e += 2 * LPB) {
         f2 q[NF + TPL];
-#pragma unroll
-        for (int k = 0; k < NF + TPL; ++k) q[k] = *reinterpret_cast<const f2 *>(&Lst.f[k][e]);
+        Lst.pair(e, q);
 #pragma unroll
         for (int i = 0; i < TPL; ++i)
             eval_pair_masked<NF>(q, q[NF + i], px[i], py[i], pz[i], e2, ax[i], ay[i], az[i]);
@@ -1393,22 +1420,22 @@ __global__ void __launch_bounds__(32)
         }
         if (cellacc) {
             const int e = Nc + __popc(mc & lt);
-            Lc.f[0][e] = A.x;
-            Lc.f[1][e] = A.y;
-            Lc.f[2][e] = A.z;
-            Lc.f[3][e] = A.w;
+            Lc.put(0, e, A.x);
+            Lc.put(1, e, A.y);
+            Lc.put(2, e, A.z);
+            Lc.put(3, e, A.w);
             if constexpr (QUAD) {  // negated: the list evaluation's form
                 const float4 q0 = __ldg(nodeQ + 2 * node);
                 const float4 q1 = __ldg(nodeQ + 2 * node + 1);
-                Lc.f[4][e] = -q0.x;
-                Lc.f[5][e] = -q0.y;
-                Lc.f[6][e] = -q0.z;
-                Lc.f[7][e] = -q0.w;
-                Lc.f[8][e] = -q1.x;
-                Lc.f[9][e] = -q1.y;
+                Lc.put(4, e, -q0.x);
+                Lc.put(5, e, -q0.y);
+                Lc.put(6, e, -q0.z);
+                Lc.put(7, e, -q0.w);
+                Lc.put(8, e, -q1.x);
+                Lc.put(9, e, -q1.y);
             }
-            Lc.f[NFC][e] = __uint_as_float(ac0);
-            if (TPL == 2) Lc.f[NFC + TPL - 1][e] = __uint_as_float(ac1);
+            Lc.put(NFC, e, __uint_as_float(ac0));
+            if (TPL == 2) Lc.put(NFC + 1, e, __uint_as_float(ac1));
         }
         Nc += nc1;
         const unsigned mb1 = __ballot_sync(0xffffffffu, bodyacc);
@@ -1419,12 +1446,12 @@ __global__ void __launch_bounds__(32)
         }
         if (bodyacc) {
             const int e = Nb + __popc(mb1 & lt);
-            Lb.f[0][e] = A.x;
-            Lb.f[1][e] = A.y;
-            Lb.f[2][e] = A.z;
-            Lb.f[3][e] = A.w;
-            Lb.f[4][e] = __uint_as_float(ac0);
-            if (TPL == 2) Lb.f[3 + TPL][e] = __uint_as_float(ac1);
+            Lb.put(0, e, A.x);
+            Lb.put(1, e, A.y);
+            Lb.put(2, e, A.z);
+            Lb.put(3, e, A.w);
+            Lb.put(4, e, __uint_as_float(ac0));
+            if (TPL == 2) Lb.put(5, e, __uint_as_float(ac1));
         }
         Nb += nb1;
         unsigned mbk = __ballot_sync(0xffffffffu, bucket);
@@ -1453,12 +1480,12 @@ __global__ void __launch_bounds__(32)
                     if (lane == j) q0 = b0 & m0, q1 = b1 & m1;
                 }
                 if (lane < n) {
-                    Lb.f[0][Nb + lane] = q.x;
-                    Lb.f[1][Nb + lane] = q.y;
-                    Lb.f[2][Nb + lane] = q.z;
-                    Lb.f[3][Nb + lane] = q.w;
-                    Lb.f[4][Nb + lane] = __uint_as_float(q0);
-                    if (TPL == 2) Lb.f[3 + TPL][Nb + lane] = __uint_as_float(q1);
+                    Lb.put(0, Nb + lane, q.x);
+                    Lb.put(1, Nb + lane, q.y);
+                    Lb.put(2, Nb + lane, q.z);
+                    Lb.put(3, Nb + lane, q.w);
+                    Lb.put(4, Nb + lane, __uint_as_float(q0));
+                    if (TPL == 2) Lb.put(5, Nb + lane, __uint_as_float(q1));
                 }
                 Nb += n;
             }
