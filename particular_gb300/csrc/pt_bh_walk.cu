@@ -538,7 +538,7 @@ static_assert(GW_GROUP == (1 << GW_SHIFT), "targets per lane: 1, 2 or 4");
 #define PT_GW_LCELLS 64
 #endif
 #ifndef PT_GW_LBODIES
-#define PT_GW_LBODIES 88
+#define PT_GW_LBODIES 80
 #endif
 // Stack ranges per warp of the PT_BH_LOCAL walk. (21 warps per SM, with lists of 56
 // cells / 80 bodies and 272 ranges, measured the same as 20: 5.21 against 5.20 ms.)
@@ -577,8 +577,11 @@ __global__ void __launch_bounds__(32 * GW_WARPS, (LOCAL ? PT_GW_LMINB : PT_GW_MI
     // they are expanded 32 at a time, one per lane, instead of by the few lanes that
     // popped them; the stack is trimmed to 288 ranges so that 20 warps stay resident per SM.
     constexpr int STK = LOCAL ? PT_GW_LSTACK : GW_STACK;
+    // A pop of k <= (cap - S) / 2 ranges leaves 3 k slots free below the cap and may vote on
+    // min(32, 2 k) cells of two slots, from an even slot on: 17 slots past the cap at most.
+    constexpr int VOTE_SLACK = 18;
     stack_cap = min(stack_cap, STK);
-    __shared__ int2 s_stack[GW_WARPS][STK];
+    __shared__ __align__(16) int2 s_stack[GW_WARPS][STK + VOTE_SLACK];
     __shared__ __align__(16) CellList s_cells[GW_WARPS];
     __shared__ __align__(16) BodyList s_bodies[GW_WARPS];
     __shared__ float s_lx[GW_WARPS][LOCAL ? 19 : 1][32];
@@ -749,17 +752,18 @@ __global__ void __launch_bounds__(32 * GW_WARPS, (LOCAL ? PT_GW_LMINB : PT_GW_MI
         }
         open = sure;
         bool marginal = false;
+        // the cells to vote on are read back from the stack's free slots, two each
         unsigned amb = __ballot_sync(0xffffffffu, maybe && !sure);
-        while (amb) {
+        float4 *voted = reinterpret_cast<float4 *>(stack + ((S + 1) & ~1));
+        if (maybe && !sure) voted[__popc(amb & lt)] = make_float4(A.x, A.y, A.z, w * w);
+        __syncwarp();
+        for (int v = 0; amb; ++v) {
             const int j = __ffs(amb) - 1;
             amb &= amb - 1;
-            const float cx = __shfl_sync(0xffffffffu, A.x, j);
-            const float cy = __shfl_sync(0xffffffffu, A.y, j);
-            const float cz = __shfl_sync(0xffffffffu, A.z, j);
-            const float cw = __shfl_sync(0xffffffffu, w, j);
+            const float4 cell = voted[v];
+            const float cx = cell.x, cy = cell.y, cz = cell.z, cw2 = cell.w;
             const float crr = REL ? __shfl_sync(0xffffffffu, rr2, j) : 0.f;
             bool o1 = false, i1 = false;
-            const float cw2 = cw * cw;
             if constexpr (TPL == 2) {  // both targets in one packed pass (same IEEE ops)
                 const f2 dx = sub2(pk2(cx, cx), vx01), dy = sub2(pk2(cy, cy), vy01), dz = sub2(pk2(cz, cz), vz01);
                 float d0, d1;
@@ -784,6 +788,7 @@ __global__ void __launch_bounds__(32 * GW_WARPS, (LOCAL ? PT_GW_LMINB : PT_GW_MI
                 if (lane == j) marginal = vo == 0u && vi != 0u && A.w > 0.0f;
             }
         }
+        __syncwarp();
         if (LEARNED) {
             const unsigned mm = __ballot_sync(0xffffffffu, marginal);
             const int nm = __popc(mm);
@@ -818,21 +823,16 @@ __global__ void __launch_bounds__(32 * GW_WARPS, (LOCAL ? PT_GW_LMINB : PT_GW_MI
         // of the tree's last levels.
         const bool flat = GW_FLAT > 0 && open && B.y - node - 1 <= GW_FLAT;
         const bool kids = open && !flat;
-        const int np = int(rest) + int(kids);
         // each lane's pushes follow those of the lanes below it
         const unsigned mrest = __ballot_sync(0xffffffffu, rest), mopen = __ballot_sync(0xffffffffu, kids);
         const int total = __popc(mrest) + __popc(mopen);
-        int slot = S + __popc(mrest & lt) + __popc(mopen & lt);
-        if (slot + np > stack_cap) {
+        if (S + total > stack_cap) {
             failed = true;  // never written out of bounds
-        } else {
-            if (rest) stack[slot++] = make_int2(B.y, range.y);
-            if (kids) stack[slot++] = make_int2(node + 1, B.y);  // children on top: popped first
-        }
-        if (__any_sync(0xffffffffu, failed)) {
-            failed = true;
             break;
         }
+        int slot = S + __popc(mrest & lt) + __popc(mopen & lt);
+        if (rest) stack[slot++] = make_int2(B.y, range.y);
+        if (kids) stack[slot++] = make_int2(node + 1, B.y);  // children on top: popped first
         S += total;
         maxS = max(maxS, S);
         const bool acc = have && !open;
@@ -934,7 +934,7 @@ __global__ void __launch_bounds__(32 * GW_WARPS, (LOCAL ? PT_GW_LMINB : PT_GW_MI
         // Small opened subtrees, all of this pop's at once: their nodes are numbered
         // across the warp (a prefix sum of the subtrees' sizes) and loaded 32 at a
         // time, one per lane; the leaves' bodies go to the body list.
-        if constexpr (GW_FLAT > 0) {
+        if (GW_FLAT > 0 && __any_sync(0xffffffffu, flat)) {
             const int fcnt = flat ? B.y - node - 1 : 0;
             int fincl = fcnt;
 #pragma unroll
@@ -1240,7 +1240,8 @@ __global__ void __launch_bounds__(32)
     using CellList = IList<NFC + TPL, PT_MW_CELLS + (LPB > 1 ? 2 * LPB - 2 : 0)>;  // + the masks of the accepting bodies
     using BodyList = IList<4 + TPL, PT_MW_BODIES + (LPB > 1 ? 2 * LPB - 2 : 0)>;
     constexpr int CELLS = PT_MW_CELLS, BODIES = PT_MW_BODIES;  // the rest is padding
-    __shared__ int4 stack[MW_STACK];  // (first, end, mask word 0, mask word 1)
+    // (first, end, mask word 0, mask word 1); one more: a pop from a full stack votes on two nodes
+    __shared__ int4 stack[MW_STACK + 1];
     __shared__ __align__(16) CellList Lc;
     __shared__ __align__(16) BodyList Lb;
     const int lane = threadIdx.x;
@@ -1354,7 +1355,7 @@ __global__ void __launch_bounds__(32)
             }
         }
         // The voted nodes are read back from the stack's free slots (the popped ranges' and
-        // the room k left above them: at least 3 k, for 2 k nodes at most). A leaf's width is
+        // the room k left above them, for 2 k nodes at most). A leaf's width is
         // 0: no body opens it.
         unsigned vm = __ballot_sync(0xffffffffu, need);
         if (need) stack[S + __popc(vm & lt)] = make_int4(__float_as_int(A.x), __float_as_int(A.y), __float_as_int(A.z),
@@ -1393,17 +1394,13 @@ __global__ void __launch_bounds__(32)
         const bool opn = (op0 | op1) != 0u;
         const unsigned mrest = __ballot_sync(0xffffffffu, rest), mopen = __ballot_sync(0xffffffffu, opn);
         const int total = __popc(mrest) + __popc(mopen);
-        int slot = S + __popc(mrest & lt) + __popc(mopen & lt);
-        if (slot + int(rest) + int(opn) > MW_STACK) {
-            failed = true;
-        } else {
-            if (rest) stack[slot++] = make_int4(B.y, r.y, int(mk0), int(mk1));
-            if (opn) stack[slot++] = make_int4(node + 1, B.y, int(op0), int(op1));
-        }
-        if (__any_sync(0xffffffffu, failed)) {
+        if (S + total > MW_STACK) {
             failed = true;
             break;
         }
+        int slot = S + __popc(mrest & lt) + __popc(mopen & lt);
+        if (rest) stack[slot++] = make_int4(B.y, r.y, int(mk0), int(mk1));
+        if (opn) stack[slot++] = make_int4(node + 1, B.y, int(op0), int(op1));
         S += total;
         const int na = __popc(ac0) + __popc(ac1);
         acc_pairs += na;
