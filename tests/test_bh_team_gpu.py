@@ -1,0 +1,43 @@
+"""The group walk with 8, 4 or 1 warps per group, which the number of groups decides: the
+same groups are walked among few, some and many others and keep their accelerations."""
+import numpy as np
+import pytest
+
+from particular_gb300 import Acceleration, AccelerationSoftened, Between, cuda
+
+pytestmark = pytest.mark.gpu
+
+
+def scattered(r, n, lo, hi, mass):
+    return np.concatenate([r.uniform(lo, hi, (n, 3)), np.full((n, 1), mass)], 1).astype(np.float32)
+
+
+@pytest.mark.parametrize("soft", [0.0, 0.01])
+@pytest.mark.parametrize("kw", [{}, {"quadrupole": True}, {"quadrupole": True, "local": True},
+                                {"relative": 2.5e-3}, {"quadrupole": True, "local": True, "relative": 2.5e-3}])
+def test_team_sizes_agree(res, kw, soft):
+    r = np.random.RandomState(4)
+    src = scattered(r, 30000, -1, 1, 1 / 30000)
+    src[0, :3], src[1, :3] = -1, 1  # a root box about the origin
+    # 50 full groups of targets in the half x < 0, sources among them; the others' keys are
+    # the highest (x, y, z >= 0), so they fill groups of their own
+    tgt = src[src[:, 0] < -0.05][:3200]
+    assert len(tgt) == 3200
+    it = AccelerationSoftened(soft) if soft else Acceleration.checked()
+    m = cuda.BarnesHut(0.7, res, it, group=True, **kw)
+    tree = m.build(src)
+    sms = res.sm_count
+    got = {}
+    for groups in (50, 5 * sms // 2 + 1, 11 * sms + 1):  # 8, 4 and 1 warps per group
+        more = scattered(r, 64 * (groups - 50), 0.1, 1, 0)
+        out = m.compute(Between(np.concatenate([tgt, more]), tree))
+        assert np.isfinite(out).all()
+        st = m.stats()
+        assert st["overflow"] == 0 and st["warps"] == groups
+        got[groups] = out[:3200]
+    want = got[11 * sms + 1].astype(np.float64)
+    # the same nodes, added in another order: compensated sums, local expansions to a few
+    # roundings of their 19 coefficients
+    scale = np.linalg.norm(want, axis=1) + np.median(np.linalg.norm(want, axis=1))
+    for out in got.values():
+        assert (np.linalg.norm(out - want, axis=1) <= 2e-6 * scale).all()
