@@ -258,27 +258,37 @@ __device__ __forceinline__ void eval_list_masked(IList<NF + TPL, CAP> &Lst, int 
     __syncwarp();
 }
 
-template <bool QUAD, int TPL, int LPB>
-__global__ void __launch_bounds__(32)
-    bh_walk_masked(const float4 *__restrict__ tbody, const uint32_t *__restrict__ tidx, int n_aff,
-                   const float4 *__restrict__ nodeA, const int4 *__restrict__ nodeB,
-                   const float4 *__restrict__ nodeQ, const float4 *__restrict__ sbody,
-                   const int *__restrict__ counters, float th2, float eps2, float *__restrict__ out,
-                   unsigned long long *__restrict__ stats) {
-    constexpr int NFC = QUAD ? 10 : 4;
-    static_assert((TPL == 2 && LPB == 1) || (TPL == 1 && LPB <= 4), "two mask words, lists padded by 2 LPB - 1");
+// Shared memory of a warp that walks for `BODIES` bodies (64, 32, 16 or 8).
+template <bool QUAD, int BODIES>
+struct Masked {
+    static constexpr int TPL = BODIES == 64 ? 2 : 1, LPB = BODIES >= 32 ? 1 : 32 / BODIES;
+    static_assert(32 * TPL / LPB == BODIES && LPB <= 4, "64, 32, 16 or 8 bodies");
+    static constexpr int NFC = QUAD ? 10 : 4;
     // (smaller lists with one body per lane, whose fewer registers leave room for more warps)
-    constexpr int CELLS = TPL == 1 ? 64 : PT_MW_CELLS, BODIES = TPL == 1 ? 96 : PT_MW_BODIES;
-    constexpr int PAD = LPB > 1 ? 2 * LPB - 2 : 0;
+    static constexpr int CELLS = TPL == 1 ? 64 : PT_MW_CELLS, LEAVES = TPL == 1 ? 96 : PT_MW_BODIES;
+    static constexpr int PAD = LPB > 1 ? 2 * LPB - 2 : 0;
     using CellList = IList<NFC + TPL, CELLS + PAD>;  // + the masks of the accepting bodies
-    using BodyList = IList<4 + TPL, BODIES + PAD>;
+    using BodyList = IList<4 + TPL, LEAVES + PAD>;
     // (first, end, mask word 0, mask word 1); one more: a pop from a full stack votes on two nodes
-    __shared__ int4 stack[MW_STACK + 1];
-    __shared__ __align__(16) CellList Lc;
-    __shared__ __align__(16) BodyList Lb;
+    int4 stack[MW_STACK + 1];
+    alignas(16) CellList cells;
+    alignas(16) BodyList leaves;
+};
+
+// The walk for the bodies from g0 on.
+template <bool QUAD, int NB>
+__device__ __forceinline__ void
+    walk_masked(Masked<QUAD, NB> &Sh, int g0, const float4 *__restrict__ tbody, const uint32_t *__restrict__ tidx,
+                int n_aff, const float4 *__restrict__ nodeA, const int4 *__restrict__ nodeB,
+                const float4 *__restrict__ nodeQ, const float4 *__restrict__ sbody,
+                const int *__restrict__ counters, float th2, float eps2, float *__restrict__ out,
+                unsigned long long *__restrict__ stats) {
+    using M = Masked<QUAD, NB>;
+    constexpr int NFC = M::NFC, TPL = M::TPL, LPB = M::LPB, CELLS = M::CELLS, BODIES = M::LEAVES;
+    int4 *stack = Sh.stack;
+    auto &Lc = Sh.cells;
+    auto &Lb = Sh.leaves;
     const int lane = threadIdx.x;
-    const int g0 = blockIdx.x * (32 * TPL / LPB);
-    if (g0 >= n_aff) return;
     float4 p[TPL];
     bool valid[TPL];
     unsigned vmask[TPL];
@@ -565,6 +575,34 @@ __global__ void __launch_bounds__(32)
     }
 }
 
+// BIG bodies a warp for the first big_groups blocks, SMALL for the rest: the last warps to
+// start are short, so that the chip does not idle for the length of a whole warp's walk at
+// the end.
+template <bool QUAD, int BIG, int SMALL>
+__global__ void __launch_bounds__(32)
+    bh_walk_masked(int big_groups, const float4 *__restrict__ tbody, const uint32_t *__restrict__ tidx, int n_aff,
+                   const float4 *__restrict__ nodeA, const int4 *__restrict__ nodeB,
+                   const float4 *__restrict__ nodeQ, const float4 *__restrict__ sbody,
+                   const int *__restrict__ counters, float th2, float eps2, float *__restrict__ out,
+                   unsigned long long *__restrict__ stats) {
+    __shared__ union {
+        __align__(16) unsigned char raw[1];
+        Masked<QUAD, BIG> big;
+        Masked<QUAD, SMALL> small;
+    } Sh;
+    const int b = blockIdx.x;
+    if (BIG == SMALL || b < big_groups) {
+        if (b * BIG < n_aff)
+            walk_masked<QUAD, BIG>(Sh.big, b * BIG, tbody, tidx, n_aff, nodeA, nodeB, nodeQ, sbody, counters, th2, eps2,
+                                   out, stats);
+    } else {
+        const int g0 = big_groups * BIG + (b - big_groups) * SMALL;
+        if (g0 < n_aff)
+            walk_masked<QUAD, SMALL>(Sh.small, g0, tbody, tidx, n_aff, nodeA, nodeB, nodeQ, sbody, counters, th2, eps2,
+                                     out, stats);
+    }
+}
+
 // ---- the reference rule over DVec3 bodies (f64 method) -------------------------
 // As bh_walk_masked with one body per lane, in double: node data, widths and the
 // per-pair kernel (impl_acceleration_cpu_scalar!(DVec3, f64): d * (m / (n_s sqrt n_s)))
@@ -834,18 +872,14 @@ __global__ void __launch_bounds__(32)
 }
 
 
-using WalkKernel = void (*)(const float4 *, const uint32_t *, int, const float4 *, const int4 *, const float4 *,
+using WalkKernel = void (*)(int, const float4 *, const uint32_t *, int, const float4 *, const int4 *, const float4 *,
                             const float4 *, const int *, float, float, float *, unsigned long long *);
-// bodies: per warp, 64, 32, 16 or 8
 template <bool QUAD>
-static WalkKernel masked_kernel_q(int bodies) {
-    return bodies == 64   ? bh_walk_masked<QUAD, 2, 1>
-           : bodies == 32 ? bh_walk_masked<QUAD, 1, 1>
-           : bodies == 16 ? bh_walk_masked<QUAD, 1, 2>
-                          : bh_walk_masked<QUAD, 1, 4>;
-}
-static WalkKernel masked_kernel(bool quad, int bodies) {
-    return quad ? masked_kernel_q<true>(bodies) : masked_kernel_q<false>(bodies);
+static WalkKernel masked_kernel_q(int big) {
+    return big == 64   ? bh_walk_masked<QUAD, 64, 32>
+           : big == 32 ? bh_walk_masked<QUAD, 32, 16>
+           : big == 16 ? bh_walk_masked<QUAD, 16, 16>
+                       : bh_walk_masked<QUAD, 8, 8>;
 }
 
 static GroupKernel group_kernel(bool quad, bool guard, bool learned, bool local, bool rel, int team) {
@@ -867,16 +901,30 @@ static int team_of(const pt_ctx *ctx, int groups) {
 
 // Bodies per warp of the masked walk. A warp alone waits on its own loads and votes, so small
 // calls want many warps with little to evaluate in each: 8 or 16 bodies, 4 or 2 lanes to a
-// body, while these warps are all resident at once (20 per SM). 32 bodies, one to a lane,
+// body, while these warps are (nearly) all resident at once, 20 per SM. 32 bodies, one to a lane,
 // meet fewer nodes than 64 (which share a traversal over more bodies) and end sooner; from
 // some 110 warps per SM on the traversals saved count for more. Whole call at 64 / 32 / 16 /
 // 8 bodies, us: N = 3000 theta 0.7 271 / 232 / 213 / 200; N = 30000 theta 0.5 552 / 436 / 391
 // / 392; N = 65536 theta 0.7 422 / 372 / 379 / 424; N = 262144 theta 0.5 1208 / 1163 / 1389 /
 // 1829; N = 524288 theta 0.8 1034 / 1027 / 1229 / 1653; N = 1M theta 0.5 3686 / 3759 / 4796 /
 // 6834.
-static int masked_bodies(const pt_ctx *ctx, int n_aff) {
+// The last groups, half a wave of 64 bodies or a quarter of one of 32, are walked in halves,
+// so that the warps that end last are short (whole / halves: N = 262144 theta 0.5 1091 / 1064
+// us; N = 800000 theta 0.6 1929 / 1883; N = 1M theta 0.5 3409 / 3292).
+struct MaskedPlan {
+    int big, big_groups, small_groups;  // bodies per warp of the first groups (then half of it from 32 on)
+};
+
+static MaskedPlan masked_plan(const pt_ctx *ctx, int n_aff) {
     const long long sms = std::max(1, ctx->sm_count);
-    return n_aff <= 8 * 20 * sms ? 8 : n_aff <= 16 * 20 * sms ? 16 : n_aff <= 32 * 110 * sms ? 32 : 64;
+    MaskedPlan p{};
+    p.big = n_aff <= 8 * 20 * sms ? 8 : n_aff <= 16 * 27 * sms ? 16 : n_aff <= 32 * 110 * sms ? 32 : 64;
+    const int all = (n_aff + p.big - 1) / p.big;
+    const int halved = p.big == 64 ? int(10 * sms) : p.big == 32 ? int(5 * sms) : 0;
+    p.big_groups = std::max(0, all - halved);
+    p.small_groups = (std::max(0, n_aff - p.big_groups * p.big) + p.big / 2 - 1) / (p.big / 2);
+    if (!halved) p.small_groups = 0;
+    return p;
 }
 
 // Clears the error word (counters[3]) before a build or a walk of separate targets; within
@@ -1036,9 +1084,10 @@ int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n
         mark(ctx, 2);
         return PT_OK;
     }
-    const int bodies = masked_bodies(ctx, n_aff);
-    masked_kernel(quad, bodies)<<<(n_aff + bodies - 1) / bodies, 32, 0, st>>>(
-        tbody, tidx, n_aff, as<float4>(S.nodeA), as<int4>(S.nodeB), as<float4>(S.nodeQ), as<float4>(S.sbody),
+    const MaskedPlan p = masked_plan(ctx, n_aff);
+    auto kern = quad ? masked_kernel_q<true>(p.big) : masked_kernel_q<false>(p.big);
+    kern<<<p.big_groups + p.small_groups, 32, 0, st>>>(
+        p.big_groups, tbody, tidx, n_aff, as<float4>(S.nodeA), as<int4>(S.nodeB), as<float4>(S.nodeQ), as<float4>(S.sbody),
         as<int>(S.counters), th2, eps2, d_out, stats);
     PT_TRY(check_launch(ctx, "bh_walk_masked"));
     mark(ctx, 2);
