@@ -246,10 +246,14 @@ __device__ __forceinline__ void each_pair(const SoaTile &T, int cnt, const f2 (&
 // Sources are read as rows and transposed on their way into shared memory, one tile ahead:
 // the next tile's rows are in registers while this tile is evaluated.
 // part (when non-null): [gridDim.y][2][n_aff] float4 = per-slice (sum, compensation).
-template <int K, bool GUARD>
+// NEXT: launched by launch_next (small calls: the wait at the start costs the compiled inner
+// loop some registers' worth of order, 127 -> 140 us at N = 16384, but a short call 2-3 us
+// less, 12.3 -> 9.4 at N = 1024).
+template <int K, bool GUARD, bool NEXT>
 __global__ void __launch_bounds__(THREADS, K == 1 ? 8 : 1)
     bf_fast(const float4 *__restrict__ aff, int n_aff, const float4 *__restrict__ src, int n_src, float eps2,
             int slice_len, float4 *__restrict__ part, float *__restrict__ out) {
+    if (NEXT) wait_previous();
     __shared__ __align__(16) SoaTile tiles[2];
     const int i0 = blockIdx.x * (THREADS * K);
     const int j0 = blockIdx.y * slice_len;
@@ -444,6 +448,7 @@ __global__ void __launch_bounds__(THREADS)
 // Sources (x, y, z, mu) rows -> four padded arrays (tail zero-filled, never read
 // as sources because every loop is bounded by n_src).
 __global__ void bf_to_soa(const float4 *__restrict__ src, int n, int n_pad, float *__restrict__ soa) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_pad) return;
     const float4 p = (i < n) ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -455,6 +460,7 @@ __global__ void bf_to_soa(const float4 *__restrict__ src, int n, int n_pad, floa
 
 // Combines the slices' (sum, compensation) pairs in slice order, in double.
 __global__ void bf_fixup(const float4 *__restrict__ part, int n_aff, int slices, float *__restrict__ out) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_aff) return;
     double x = 0.0, y = 0.0, z = 0.0;
@@ -693,16 +699,16 @@ __global__ void __launch_bounds__(ORD_THREADS)
 
 using FastKernel = void (*)(const float4 *, int, const float4 *, int, float, int, float4 *, float *);
 
-template <int K>
+template <int K, bool NEXT>
 FastKernel pick(bool guard) {
-    return guard ? bf_fast<K, true> : bf_fast<K, false>;
+    return guard ? bf_fast<K, true, NEXT> : bf_fast<K, false, NEXT>;
 }
 
 FastKernel fast_kernel(int K, bool guard) {
     switch (K) {
-        case 1: return pick<1>(guard);
-        case 2: return pick<2>(guard);
-        default: return pick<4>(guard);
+        case 1: return pick<1, false>(guard);
+        case 2: return pick<2, false>(guard);
+        default: return pick<4, false>(guard);
     }
 }
 
@@ -718,9 +724,10 @@ RingKernel ring_kernel(int K) {
 
 // Unguarded sums over this many sources and more take bf_fast_ring: it needs a launch to
 // lay the sources out, and its inner loop holds 9 blocks per SM where bf_fast's holds 8
-// (K = 1; N = 24001: 254 us against 263, N = 65000: 1593 against 1668, N = 131072: 6273
-// against 6510; at N = 16384 the launch costs more than the loop gains, 137 against 129).
-constexpr int RING_MIN_SRC = 20480;
+// (ring / bf_fast at K = 1: N = 131072 6275 / 6650 us, 65000 1585 / 1668, 22000 209 / 223,
+// 19000 172 / 174, 17000 138 / 143; at N = 16384 the launch costs more than the loop gains,
+// 137 / 127).
+constexpr int RING_MIN_SRC = 16640;
 
 static bool use_ring(bool guard, int n_src) { return !guard && n_src >= RING_MIN_SRC; }
 
@@ -780,6 +787,18 @@ static Plan plan(const pt_ctx *ctx, int n_aff, int n_src, bool guard, int force_
     p.slice_len = len_tiles * TILE;
     p.slices = (n_src + p.slice_len - 1) / p.slice_len;
     return p;
+}
+
+// Pairs up to which a call is short enough for its launches to show.
+constexpr double NEXT_MAX_PAIRS = 4096.0 * 4096.0;
+
+static void launch_fast(const Plan &p, bool guard, cudaStream_t st, const float4 *aff, int n_aff, const float4 *src,
+                        int n_src, float eps2, int slice_len, float4 *part, float *out) {
+    const dim3 grid(p.n_ib, p.slices);
+    if (p.K == 1 && double(n_aff) * n_src <= NEXT_MAX_PAIRS)
+        launch_next(pick<1, true>(guard), grid, THREADS, 0, st, aff, n_aff, src, n_src, eps2, slice_len, part, out);
+    else
+        fast_kernel(p.K, guard)<<<grid, THREADS, 0, st>>>(aff, n_aff, src, n_src, eps2, slice_len, part, out);
 }
 
 // Below this many targets the terms and the sum run in different warps (bf_ordered); from
@@ -843,17 +862,17 @@ int bf_launch_f32(pt_ctx *ctx, const float4 *aff, int n_aff, const float4 *src, 
         const int n_pad = (n_src + TILE - 1) / TILE * TILE;
         PT_TRY(ensure(ctx, BUF_SOA, sizeof(float) * 4 * size_t(n_pad)));
         float *soa = static_cast<float *>(ctx->bufs[BUF_SOA].ptr);
-        bf_to_soa<<<(n_pad + 255) / 256, 256, 0, st>>>(src, n_src, n_pad, soa);
+        launch_next(bf_to_soa, (n_pad + 255) / 256, 256, 0, st, src, n_src, n_pad, soa);
         PT_TRY(check_launch(ctx, "bf_to_soa"));
         mark(ctx, 1);
         ring_kernel(p.K)<<<grid, THREADS, 0, st>>>(aff, n_aff, soa, n_src, n_pad, soft2, p.slice_len, part, out);
     } else {
         mark(ctx, 1);
-        fast_kernel(p.K, guard)<<<grid, THREADS, 0, st>>>(aff, n_aff, src, n_src, soft2, p.slice_len, part, out);
+        launch_fast(p, guard, st, aff, n_aff, src, n_src, soft2, p.slice_len, part, out);
     }
     PT_TRY(check_launch(ctx, "bf_fast"));
     if (part) {
-        bf_fixup<<<(n_aff + 255) / 256, 256, 0, st>>>(part, n_aff, p.slices, out);
+        launch_next(bf_fixup, (n_aff + 255) / 256, 256, 0, st, part, n_aff, p.slices, out);
         PT_TRY(check_launch(ctx, "bf_fixup"));
     }
     mark(ctx, 2);
@@ -1125,15 +1144,15 @@ extern "C" int pt_bf_accel_f32_noalloc(const float *d_aff, size_t n_aff, const f
     if (use_ring(guard, ns)) {
         const int n_pad = (ns + TILE - 1) / TILE * TILE;
         float *soa = reinterpret_cast<float *>(scratch);
-        bf_to_soa<<<(n_pad + 255) / 256, 256, 0, st>>>(src, ns, n_pad, soa);
+        launch_next(bf_to_soa, (n_pad + 255) / 256, 256, 0, st, src, ns, n_pad, soa);
         PT_CUDA(cudaGetLastError());
         ring_kernel(p.K)<<<grid, THREADS, 0, st>>>(aff, na, soa, ns, n_pad, soft2, p.slice_len, part, d_out);
     } else {
-        fast_kernel(p.K, guard)<<<grid, THREADS, 0, st>>>(aff, na, src, ns, soft2, p.slice_len, part, d_out);
+        launch_fast(p, guard, st, aff, na, src, ns, soft2, p.slice_len, part, d_out);
     }
     PT_CUDA(cudaGetLastError());
     if (part) {
-        bf_fixup<<<(na + 255) / 256, 256, 0, st>>>(part, na, p.slices, d_out);
+        launch_next(bf_fixup, (na + 255) / 256, 256, 0, st, part, na, p.slices, d_out);
         PT_CUDA(cudaGetLastError());
     }
     return PT_OK;

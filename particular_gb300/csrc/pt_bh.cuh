@@ -17,6 +17,7 @@ namespace pt {
 namespace bh {
 
 constexpr int LEVELS = 21;   // 63-bit keys
+constexpr int WALK_STATS = 9;  // the walk's u64 counters behind counters[0..3]
 
 struct Moments {  // FP64 cell data used while combining children (DVec3 trees, bucket leaves)
     double m, cx, cy, cz;
@@ -84,10 +85,6 @@ struct State {
     float theta_inner = 0.5f;
     int cap_n = 0;
     int last_n_src = 0;
-    // a second stream for build work that does not depend on the tree chain (the
-    // sorted bodies' gather), joined back before the layout
-    cudaStream_t aux = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
 };
 
 inline State *state(pt_ctx *ctx) {

@@ -32,9 +32,13 @@ namespace pt {
 namespace bh {
 
 // ---- 1. root box -----------------------------------------------------------
+// Also clears the sort's words.
 template <class T>
-__global__ void bbox_partial(const typename Prec<T>::V4 *__restrict__ src, int n, T *__restrict__ part) {
+__global__ void bbox_partial(const typename Prec<T>::V4 *__restrict__ src, int n, T *__restrict__ part,
+                             uint32_t *__restrict__ zero, int zero_words) {
     using P = Prec<T>;
+    after_previous();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < zero_words; i += gridDim.x * blockDim.x) zero[i] = 0u;
     T mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const typename P::V4 p = src[i];
@@ -68,6 +72,7 @@ __global__ void bbox_partial(const typename Prec<T>::V4 *__restrict__ src, int n
 // order), then thread 0 forms the reference's square root box.
 template <class T>
 __global__ void bbox_final(const T *__restrict__ part, int nb, T *__restrict__ box) {
+    after_previous();
     using P = Prec<T>;
     T mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (int b = threadIdx.x; b < nb; b += blockDim.x)
@@ -132,6 +137,7 @@ __device__ __forceinline__ uint64_t key_of(T px, T py, T pz, const T *box) {
 template <class T>
 __global__ void make_keys(const typename Prec<T>::V4 *__restrict__ bodies, int n, const T *__restrict__ box_g,
                           uint64_t *__restrict__ keys, uint32_t *__restrict__ hist, int shift) {
+    after_previous();
     __shared__ T box[6];
     if (threadIdx.x < 6) box[threadIdx.x] = box_g[threadIdx.x];
     __syncthreads();
@@ -143,10 +149,17 @@ __global__ void make_keys(const typename Prec<T>::V4 *__restrict__ bodies, int n
     if (hist) atomicAdd(&hist[(i / RADIX_TILE) * 256 + (int(k >> shift) & 255)], 1u);
 }
 
+// The walk's counters (counters + 4 ints) start from zero.
+__device__ __forceinline__ void clear_stats(int *counters, int i) {
+    if (i < WALK_STATS) (reinterpret_cast<unsigned long long *>(counters) + 2)[i] = 0ull;
+}
+
 template <class V4>
 __global__ void gather_bodies(const V4 *__restrict__ src, const uint32_t *__restrict__ idx, int n,
-                              V4 *__restrict__ out) {
+                              V4 *__restrict__ out, int *__restrict__ counters) {
+    after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    clear_stats(counters, k);
     if (k < n) out[k] = src[idx[k]];
 }
 
@@ -214,14 +227,19 @@ __device__ __forceinline__ int stage_of(int first, int last) {
 // cell: the root, or a node whose common-prefix level (delta / 3) exceeds its parent's. The
 // parent's prefix is the longer of those that the range shares with its neighbours, so no
 // second pass over the parents is needed. top[i] = 1 + stage for a cell, else 0. Thread i
-// also clears what the next pass counts.
-__global__ void karras(const uint64_t *__restrict__ ukey, const int *__restrict__ counters, int n,
+// also clears what the next pass counts, and moves body i of the key order to its place: a
+// random read beside the search's chain of dependent ones.
+template <class V4>
+__global__ void karras(const V4 *__restrict__ src, const uint32_t *__restrict__ idx, V4 *__restrict__ sbody,
+                       const uint64_t *__restrict__ ukey, const int *__restrict__ counters, int n,
                        int *__restrict__ bfirst, int *__restrict__ blast, int *__restrict__ bdelta,
                        int *__restrict__ bparent, int *__restrict__ lparent, uint8_t *__restrict__ top,
                        uint32_t *__restrict__ starts, uint32_t *__restrict__ kmask, int *__restrict__ nspan,
                        int span_blocks) {
+    after_previous();
     const int M = counters[0];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) sbody[i] = src[idx[i]];
     if (i <= n) starts[i] = 0u;
     if (i < span_blocks) nspan[i] = 0;
     if (i >= M - 1) return;
@@ -277,6 +295,7 @@ __global__ void octree_links(const int *__restrict__ counters, int n, const int 
                              const uint64_t *__restrict__ ukey, int *__restrict__ oparent, int *__restrict__ loparent,
                              uint32_t *__restrict__ starts, uint32_t *__restrict__ kmask, int *__restrict__ nspan,
                              int *__restrict__ spans) {
+    after_previous();
     const int M = counters[0];
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < M - 1 && top[k]) {
@@ -800,6 +819,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS)
            typename Prec<T>::V4 *__restrict__ nodeG, int2 *__restrict__ nodeR, const int *__restrict__ loparent,
            int *__restrict__ kid, const typename Prec<T>::V4 *__restrict__ sbody, Record<T> *rec,
            typename Prec<T>::V4 *nodeA, float4 *nodeQ) {
+    after_previous();
     using P = Prec<T>;
     constexpr int PER = CHUNK / CHUNK_THREADS;
     extern __shared__ __align__(32) unsigned char block_raw[];
@@ -807,6 +827,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS)
     const int M = counters[0];
     const int c0 = blockIdx.x << CHUNK_SHIFT;
     if (c0 >= M) return;
+    if (blockIdx.x == 0) clear_stats(counters, threadIdx.x);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         counters[1] = M + int(pscan[M]);
         counters[2] = int(pscan[M]);
@@ -923,6 +944,7 @@ __global__ void __launch_bounds__(SPAN_THREADS)
                const int *__restrict__ kid, const uint32_t *__restrict__ kmask, int *slot,
                const typename Prec<T>::V4 *__restrict__ nodeG, Record<T> *rec, typename Prec<T>::V4 *nodeA,
                float4 *nodeQ, int4 *nodeB) {
+    after_previous();
     extern __shared__ __align__(32) unsigned char block_raw[];
     SpanBlock<T> &C = *reinterpret_cast<SpanBlock<T> *>(block_raw);
     const int blk = stage_first(n, stage) + blockIdx.x;
@@ -1027,52 +1049,39 @@ int build_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_src, int n) {
     PT_TRY(ensure_buf(ctx, S.mom, sizeof(Moments) * 2 * N));
     PT_TRY(ensure_buf(ctx, S.counters, sizeof(unsigned long long) * 16));
 
-    const int nb = std::min(1024, blocks(n));
-    bbox_partial<T><<<nb, 256, 0, st>>>(d_src, n, as<T>(S.box_part));
-    PT_TRY(check_launch(ctx, "bbox_partial"));
-    bbox_final<T><<<1, 256, 0, st>>>(as<T>(S.box_part), nb, as<T>(S.box));
-    PT_TRY(check_launch(ctx, "bbox_final"));
     RadixFirst rf{};
     PT_TRY(radix_sort_prepare(ctx, S.prims, n, 3 * LEVELS, &rf));
-    make_keys<T><<<blocks(n), 256, 0, st>>>(d_src, n, as<T>(S.box), rf.keys ? rf.keys : as<uint64_t>(S.keys), rf.hist,
-                                            rf.shift);
+    const int nb = std::min(1024, blocks(n));
+    launch_next(bbox_partial<T>, nb, 256, 0, st, d_src, n, as<T>(S.box_part), rf.zero, rf.zero_words);
+    PT_TRY(check_launch(ctx, "bbox_partial"));
+    launch_next(bbox_final<T>, 1, 256, 0, st, as<T>(S.box_part), nb, as<T>(S.box));
+    PT_TRY(check_launch(ctx, "bbox_final"));
+    launch_next(make_keys<T>, blocks(n), 256, 0, st, d_src, n, as<T>(S.box),
+                rf.keys ? rf.keys : as<uint64_t>(S.keys), rf.hist, rf.shift);
     PT_TRY(check_launch(ctx, "make_keys"));
     PT_TRY(radix_sort_u64(ctx, S.prims, as<uint64_t>(S.keys), as<uint32_t>(S.idx), n, 3 * LEVELS,
                           as<int>(S.counters) + 3));
-    // The bodies' gather into key order runs on a second stream beside the tree chain
-    // (unit flags .. octree links) and joins before the layout, its first reader.
-    if (!S.aux) {
-        PT_CUDA(cudaStreamCreateWithFlags(&S.aux, cudaStreamNonBlocking));
-        PT_CUDA(cudaEventCreateWithFlags(&S.fork, cudaEventDisableTiming));
-        PT_CUDA(cudaEventCreateWithFlags(&S.join, cudaEventDisableTiming));
-    }
-    PT_CUDA(cudaEventRecord(S.fork, st));
-    PT_CUDA(cudaStreamWaitEvent(S.aux, S.fork, 0));
-    gather_bodies<V4><<<blocks(n), 256, 0, S.aux>>>(d_src, as<uint32_t>(S.idx), n, as<V4>(sb));
-    PT_TRY(check_launch(ctx, "gather_bodies"));
-    PT_CUDA(cudaEventRecord(S.join, S.aux));
     int *counters = as<int>(S.counters);
     PT_TRY(scan_generated(ctx, S.prims, UnitHead{as<uint64_t>(S.keys)},
                           UnitFill{as<uint64_t>(S.keys), n, as<uint64_t>(S.ukey), as<uint32_t>(S.ufirst), counters}, n));
     const int nstages = stages(n), span_blocks = stage_first(n, nstages + 1);
     PT_TRY(ensure_buf(ctx, S.nspan, sizeof(int) * size_t(std::max(1, span_blocks))));
     PT_TRY(ensure_buf(ctx, S.spans, sizeof(int) * size_t(std::max(1, span_blocks)) * SPAN_CAP));
-    karras<<<blocks(n + 1), 256, 0, st>>>(as<uint64_t>(S.ukey), counters, n, as<int>(S.bfirst), as<int>(S.blast),
-                                          as<int>(S.bdelta), as<int>(S.bparent), as<int>(S.lparent),
-                                          as<uint8_t>(S.top), as<uint32_t>(S.starts), as<uint32_t>(S.kmask),
-                                          as<int>(S.nspan), span_blocks);
+    launch_next(karras<V4>, blocks(n + 1), 256, 0, st, d_src, as<uint32_t>(S.idx), as<V4>(sb), as<uint64_t>(S.ukey),
+                counters, n, as<int>(S.bfirst), as<int>(S.blast), as<int>(S.bdelta), as<int>(S.bparent),
+                as<int>(S.lparent), as<uint8_t>(S.top), as<uint32_t>(S.starts), as<uint32_t>(S.kmask),
+                as<int>(S.nspan), span_blocks);
     PT_TRY(check_launch(ctx, "karras"));
-    octree_links<<<blocks(n), 256, 0, st>>>(counters, n, as<int>(S.bfirst), as<int>(S.bparent), as<int>(S.lparent),
+    launch_next(octree_links, blocks(n), 256, 0, st, counters, n, as<int>(S.bfirst), as<int>(S.bparent), as<int>(S.lparent),
                                            as<uint8_t>(S.top), as<int>(S.bdelta), as<uint64_t>(S.ukey),
                                            as<int>(S.oparent), as<int>(S.loparent), as<uint32_t>(S.starts),
                                            as<uint32_t>(S.kmask), as<int>(S.nspan), as<int>(S.spans));
     PT_TRY(check_launch(ctx, "octree_links"));
     PT_TRY(scan_generated(ctx, S.prims, CellStarts{as<uint32_t>(S.starts)},
                           scan::WriteU32{as<uint32_t>(S.pscan), n + 1}, n + 1));
-    PT_CUDA(cudaStreamWaitEvent(st, S.join, 0));  // the gathered bodies
     PT_CUDA(cudaFuncSetAttribute(layout<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(Chunk<T>))));
-    layout<T><<<(n + CHUNK - 1) / CHUNK, CHUNK_THREADS, sizeof(Chunk<T>), st>>>(
-        counters, as<int>(S.bfirst), as<int>(S.blast), as<int>(S.bdelta), as<uint8_t>(S.top), as<int>(S.oparent),
+    launch_next(
+        layout<T>, (n + CHUNK - 1) / CHUNK, CHUNK_THREADS, sizeof(Chunk<T>), st, counters, as<int>(S.bfirst), as<int>(S.blast), as<int>(S.bdelta), as<uint8_t>(S.top), as<int>(S.oparent),
         as<uint32_t>(S.starts), as<uint32_t>(S.pscan), as<uint64_t>(S.ukey), as<uint32_t>(S.ufirst), as<T>(S.box),
         as<int>(S.pre), as<int4>(S.nodeB), as<V4>(nG), as<int2>(S.nodeR), as<int>(S.loparent), as<int>(S.kid),
         as<V4>(sb), as<Record<T>>(S.mom), as<V4>(nA), nodeQ);
@@ -1081,8 +1090,8 @@ int build_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_src, int n) {
         PT_CUDA(cudaFuncSetAttribute(cells_span<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      int(sizeof(SpanBlock<T>))));
     for (int stage = 1; stage <= nstages; ++stage) {
-        cells_span<T><<<stage_blocks(n, stage), SPAN_THREADS, sizeof(SpanBlock<T>), st>>>(
-            n, stage, as<int>(S.nspan), as<int>(S.spans), as<int>(S.bfirst), as<int>(S.bdelta), as<uint8_t>(S.top),
+        launch_next(
+            cells_span<T>, stage_blocks(n, stage), SPAN_THREADS, sizeof(SpanBlock<T>), st, n, stage, as<int>(S.nspan), as<int>(S.spans), as<int>(S.bfirst), as<int>(S.bdelta), as<uint8_t>(S.top),
             as<uint64_t>(S.ukey), as<int>(S.oparent), as<int>(S.pre), as<int>(S.kid), as<uint32_t>(S.kmask),
             as<int>(S.slot), as<V4>(nG), as<Record<T>>(S.mom), as<V4>(nA), nodeQ, as<int4>(S.nodeB));
         PT_TRY(check_launch(ctx, "cells_span"));
@@ -1107,12 +1116,13 @@ int sort_targets_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_aff, int
     PT_TRY(ensure_buf(ctx, tb, sizeof(V4) * size_t(n)));
     RadixFirst rf{};
     PT_TRY(radix_sort_prepare(ctx, S.prims, n, 3 * LEVELS, &rf));
-    make_keys<T><<<blocks(n), 256, 0, st>>>(d_aff, n, as<T>(S.box), rf.keys ? rf.keys : as<uint64_t>(S.tkeys), rf.hist,
-                                            rf.shift);
+    PT_CUDA(cudaMemsetAsync(rf.zero, 0, sizeof(uint32_t) * size_t(rf.zero_words), st));
+    launch_next(make_keys<T>, blocks(n), 256, 0, st, d_aff, n, as<T>(S.box),
+                rf.keys ? rf.keys : as<uint64_t>(S.tkeys), rf.hist, rf.shift);
     PT_TRY(check_launch(ctx, "make_keys(targets)"));
     PT_TRY(radix_sort_u64(ctx, S.prims, as<uint64_t>(S.tkeys), as<uint32_t>(S.tidx), n, 3 * LEVELS,
                           as<int>(S.counters) + 3));
-    gather_bodies<V4><<<blocks(n), 256, 0, st>>>(d_aff, as<uint32_t>(S.tidx), n, as<V4>(tb));
+    launch_next(gather_bodies<V4>, blocks(n), 256, 0, st, d_aff, as<uint32_t>(S.tidx), n, as<V4>(tb), as<int>(S.counters));
     return check_launch(ctx, "gather_bodies(targets)");
 }
 

@@ -493,6 +493,7 @@ __global__ void __launch_bounds__(32 * W, (LOCAL ? PT_GW_LMINB : PT_GW_MINB) * 4
                   float th2, float th_in2, LearnedRecords LR, float eps2, float *__restrict__ out,
                   unsigned long long *__restrict__ stats, int *__restrict__ err, int stack_cap,
                   float local_ratio, const float *__restrict__ gscale, float mono_beta) {
+    after_previous();
     static_assert(!(LEARNED && LOCAL), "PT_BH_LEARNED and PT_BH_LOCAL are exclusive");
     static_assert(!(LEARNED && REL), "PT_BH_LEARNED and PT_BH_RELATIVE are exclusive");
     static_assert(!(LEARNED && W > 1), "one warp chains a group's records");

@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(128)
     bh_group_scale(const float4 *__restrict__ tbody, int n_aff, const float4 *__restrict__ nodeA,
                    const int4 *__restrict__ nodeB, const int *__restrict__ counters, float eps2, float alpha,
                    float *__restrict__ gscale) {
+    after_previous();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int g0 = g * GW_GROUP;
     if (g0 >= n_aff) return;
@@ -585,6 +586,7 @@ __global__ void __launch_bounds__(32)
                    const float4 *__restrict__ nodeQ, const float4 *__restrict__ sbody,
                    const int *__restrict__ counters, float th2, float eps2, float *__restrict__ out,
                    unsigned long long *__restrict__ stats) {
+    after_previous();
     __shared__ union {
         __align__(16) unsigned char raw[1];
         Masked<QUAD, BIG> big;
@@ -696,6 +698,7 @@ __global__ void __launch_bounds__(32)
               const double4_32a *__restrict__ nodeG, const double4_32a *__restrict__ sbody,
               const int *__restrict__ counters, double th2, double eps2, double *__restrict__ out,
               unsigned long long *__restrict__ stats, int *__restrict__ err) {
+    after_previous();
     __shared__ int4 stack[W64_STACK];
     __shared__ List64 Lst;
     const int lane = threadIdx.x;
@@ -994,12 +997,11 @@ int run64(pt_ctx *ctx, const double4_32a *d_aff, int n_aff, const double4_32a *d
     const uint32_t *tidx = same ? as<uint32_t>(S.idx) : as<uint32_t>(S.tidx);
     unsigned long long *stats = reinterpret_cast<unsigned long long *>(S.counters.ptr) + 2;
     int *err = as<int>(S.counters) + 3;
-    PT_CUDA(cudaMemsetAsync(stats, 0, 9 * sizeof(unsigned long long), st));
     mark(ctx, 1);
     const int lpb = lanes_per_body64(ctx, n_aff);
     auto kern = lpb == 4 ? bh_walk64<4> : lpb == 2 ? bh_walk64<2> : bh_walk64<1>;
-    kern<<<(n_aff + 32 / lpb - 1) / (32 / lpb), 32, 0, st>>>(
-        tbody, tidx, n_aff, as<double4_32a>(S.nodeA64), as<int4>(S.nodeB), as<double4_32a>(S.nodeG64),
+    launch_next(
+        kern, (n_aff + 32 / lpb - 1) / (32 / lpb), 32, 0, st, tbody, tidx, n_aff, as<double4_32a>(S.nodeA64), as<int4>(S.nodeB), as<double4_32a>(S.nodeG64),
         as<double4_32a>(S.sbody64), as<int>(S.counters), theta * theta, softening * softening, d_out, stats, err);
     PT_TRY(check_launch(ctx, "bh_walk64"));
     mark(ctx, 2);
@@ -1014,10 +1016,10 @@ int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n
     if (S.f64) return set_error(PT_ERR_INVALID, "the context's tree holds DVec3 bodies: walk it with the f64 method");
     // counters: int[4] = {leaves, nodes, cells, error} then u64[8] = {interactions,
     // visits, warps, max group stack, learned records, cell interactions, warps that
-    // fell back to the per-body walk, far nodes taken by the local expansion}
+    // fell back to the per-body walk, far nodes taken by the local expansion}, cleared by the
+    // layout or the targets' gather before
     unsigned long long *stats = reinterpret_cast<unsigned long long *>(S.counters.ptr) + 2;
     int *err = as<int>(S.counters) + 3;
-    PT_CUDA(cudaMemsetAsync(stats, 0, 9 * sizeof(unsigned long long), st));
     const float th2 = theta * theta;
     const float eps2 = softening * softening;
     const bool quad = flags & PT_BH_QUADRUPOLE;
@@ -1037,7 +1039,7 @@ int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n
         const float *gscale = nullptr;
         if (flags & PT_BH_RELATIVE) {
             PT_TRY(ensure_buf(ctx, S.gscale, sizeof(float) * size_t(groups)));
-            bh_group_scale<<<blocks(groups, 128), 128, 0, st>>>(tbody, n_aff, as<float4>(S.nodeA), as<int4>(S.nodeB),
+            launch_next(bh_group_scale, blocks(groups, 128), 128, 0, st, tbody, n_aff, as<float4>(S.nodeA), as<int4>(S.nodeB),
                                                                 as<int>(S.counters), eps2, S.rel_alpha,
                                                                 as<float>(S.gscale));
             PT_TRY(check_launch(ctx, "bh_group_scale"));
@@ -1054,9 +1056,9 @@ int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n
                 PT_CUDA(cudaMemsetAsync(LR.used, 0, sizeof(int), st));
             }
             const int team = learned ? 1 : team_of(ctx, groups);
-            group_kernel(quad, eps2 == 0.0f, learned, flags & PT_BH_LOCAL, gscale != nullptr, team)<<<groups, 32 * team,
-                                                                                                      0, st>>>(
-                tbody, tidx, n_aff, as<float4>(S.nodeA), as<int4>(S.nodeB), as<float4>(S.nodeQ), as<float4>(S.nodeG),
+            launch_next(
+                group_kernel(quad, eps2 == 0.0f, learned, flags & PT_BH_LOCAL, gscale != nullptr, team), groups,
+                32 * team, 0, st, tbody, tidx, n_aff, as<float4>(S.nodeA), as<int4>(S.nodeB), as<float4>(S.nodeQ), as<float4>(S.nodeG),
                 as<float4>(S.sbody), as<int>(S.counters), th2, S.theta_inner * S.theta_inner, LR, eps2, d_out, stats,
                 err, S.stack_cap > 0 ? S.stack_cap : INT_MAX, S.local_ratio, gscale, S.rel_mono);
             PT_TRY(check_launch(ctx, "bh_walk_group"));
@@ -1070,7 +1072,7 @@ int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n
             if (used <= S.lcap) break;
             S.lcap = used + used / 4;
             PT_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
-            PT_CUDA(cudaMemsetAsync(stats, 0, 9 * sizeof(unsigned long long), st));
+            PT_CUDA(cudaMemsetAsync(stats, 0, WALK_STATS * sizeof(unsigned long long), st));
         }
         if (learned) {
             bh_learned_eval<<<ctx->sm_count * 4, 128, 0, st>>>(LR, as<float4>(S.nodeA), as<float4>(S.nodeQ),
@@ -1086,8 +1088,8 @@ int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n
     }
     const MaskedPlan p = masked_plan(ctx, n_aff);
     auto kern = quad ? masked_kernel_q<true>(p.big) : masked_kernel_q<false>(p.big);
-    kern<<<p.big_groups + p.small_groups, 32, 0, st>>>(
-        p.big_groups, tbody, tidx, n_aff, as<float4>(S.nodeA), as<int4>(S.nodeB), as<float4>(S.nodeQ), as<float4>(S.sbody),
+    launch_next(
+        kern, p.big_groups + p.small_groups, 32, 0, st, p.big_groups, tbody, tidx, n_aff, as<float4>(S.nodeA), as<int4>(S.nodeB), as<float4>(S.nodeQ), as<float4>(S.sbody),
         as<int>(S.counters), th2, eps2, d_out, stats);
     PT_TRY(check_launch(ctx, "bh_walk_masked"));
     mark(ctx, 2);

@@ -82,6 +82,35 @@ inline void mark(pt_ctx *ctx, int k) {
     if (ctx->timing) cudaEventRecord(ctx->ev[k], ctx->stream);
 }
 
+// Launches a kernel that may start while the one before it on the stream is ending (programmatic
+// stream serialization): its first statement is after_previous(), which waits until that one
+// has ended and its writes are visible. A chain of short kernels loses some 2 us less between
+// each two.
+template <class... P, class... A>
+inline void launch_next(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);  // check_launch() reads the error
+}
+
+#ifdef __CUDACC__
+// Waits for the kernel before this one on the stream (see launch_next); after_previous() then
+// lets the one after it be scheduled once every block of this one has come here.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void after_previous() {
+    wait_previous();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Barnes-Hut settings held by the context that its launches take as parameters

@@ -24,6 +24,7 @@ namespace lf {
 // v += a * kick; x += v * dt   (kick = dt/2 for the first step, dt afterwards)
 __global__ void kick_drift(float4 *__restrict__ body, float4 *__restrict__ vel, const float *__restrict__ acc,
                            int n, float kick, float dt) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float4 v = vel[i];
@@ -39,6 +40,7 @@ __global__ void kick_drift(float4 *__restrict__ body, float4 *__restrict__ vel, 
 }
 
 __global__ void kick(float4 *__restrict__ vel, const float *__restrict__ acc, int n, float k) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float4 v = vel[i];
@@ -106,11 +108,11 @@ static int enqueue_steps(pt_ctx *ctx, float4 *body, float4 *vel, float *acc, siz
                          int method, float theta, float softening, uint32_t flags) {
     const int blocks = int((n + 255) / 256);
     for (int s = 0; s < steps; ++s) {
-        kick_drift<<<blocks, 256, 0, ctx->stream>>>(body, vel, acc, int(n), s == 0 ? 0.5f * dt : dt, dt);
+        launch_next(kick_drift, blocks, 256, 0, ctx->stream, body, vel, acc, int(n), s == 0 ? 0.5f * dt : dt, dt);
         PT_TRY(check_launch(ctx, "kick_drift"));
         PT_TRY(accel(ctx, reinterpret_cast<float *>(body), acc, n, method, theta, softening, flags));
     }
-    kick<<<blocks, 256, 0, ctx->stream>>>(vel, acc, int(n), 0.5f * dt);
+    launch_next(kick, blocks, 256, 0, ctx->stream, vel, acc, int(n), 0.5f * dt);
     return check_launch(ctx, "kick");
 }
 

@@ -80,6 +80,7 @@ __device__ __forceinline__ void hist_tile(const uint64_t *__restrict__ keys, int
 
 __global__ void __launch_bounds__(RS_THREADS)
     rs_hist(const uint64_t *__restrict__ keys, int n, int shift, uint32_t *__restrict__ hist, int nblocks) {
+    after_previous();
     __shared__ uint32_t cnt[256];
     hist_tile(keys, n, shift, hist, nblocks, blockIdx.x, cnt);
 }
@@ -107,6 +108,7 @@ __device__ __forceinline__ void scan_row(const uint32_t *__restrict__ hist, uint
 __global__ void __launch_bounds__(RS_THREADS)
     rs_rowscan(const uint32_t *__restrict__ hist, uint32_t *__restrict__ offs, uint32_t *__restrict__ rowsum,
                int nblocks) {
+    after_previous();
     __shared__ uint32_t wsum[RS_WARPS + 1];
     scan_row(hist, offs, rowsum, nblocks, blockIdx.x, wsum);
 }
@@ -195,6 +197,7 @@ __global__ void __launch_bounds__(RS_THREADS)
     rs_scatter(const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin, uint64_t *__restrict__ kout,
                uint32_t *__restrict__ vout, int n, int shift, const uint32_t *__restrict__ offs,
                const uint32_t *__restrict__ rowsum, int nblocks) {
+    after_previous();
     __shared__ ScatterShared S;
     const int b = blockIdx.x;
     // all smaller digits, then earlier tiles
@@ -208,6 +211,7 @@ __global__ void __launch_bounds__(RS_THREADS)
     rs_pass(const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin, uint64_t *__restrict__ kout,
             uint32_t *__restrict__ vout, int n, int shift, const uint32_t *__restrict__ hist, int nblocks,
             uint32_t *__restrict__ next, int next_shift) {
+    after_previous();
     __shared__ ScatterShared S;
     const int b = blockIdx.x;
     scatter_tile(S, kin, vin, kout, vout, n, shift, b,
@@ -232,6 +236,7 @@ constexpr int RUN_LIMIT = 48;
 __global__ void __launch_bounds__(256)
     rs_finish(const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin, int n, int shift,
               uint64_t *__restrict__ kout, uint32_t *__restrict__ vout, int *__restrict__ redo) {
+    after_previous();
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= n) return;
     const uint64_t k = kin[i], h = k >> shift;
@@ -352,8 +357,8 @@ int radix_sort_prepare(pt_ctx *ctx, PrimScratch &s, int n, int bits, RadixFirst 
     const bool direct = nblocks <= DIRECT_TILES;
     uint32_t *hist = static_cast<uint32_t *>(s.hist.ptr);
     uint32_t *tail = hist + (words - 64);
-    if (direct) PT_CUDA(cudaMemsetAsync(hist, 0, sizeof(uint32_t) * words, ctx->stream));
-    else PT_CUDA(cudaMemsetAsync(tail, 0, sizeof(uint32_t) * 64, ctx->stream));
+    first->zero = direct ? hist : tail;
+    first->zero_words = direct ? int(words) : 64;
     // an odd number of passes ends in the pair that the finishing pass reads
     first->keys = (passes & 1) ? nullptr : static_cast<uint64_t *>(s.keys2.ptr);
     first->hist = direct ? hist : nullptr;
@@ -380,19 +385,19 @@ int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, 
         const uint32_t *vin = p == 0 ? nullptr : v[in];
         if (nblocks <= DIRECT_TILES) {
             uint32_t *next = p + 1 < passes ? hist + (p + 1) * nhist : nullptr;
-            rs_pass<<<nblocks, RS_THREADS, 0, st>>>(k[in], vin, k[in ^ 1], v[in ^ 1], n, shift, hist + p * nhist,
+            launch_next(rs_pass, nblocks, RS_THREADS, 0, st, k[in], vin, k[in ^ 1], v[in ^ 1], n, shift, hist + p * nhist,
                                                     nblocks, next, shift + 8);
             PT_TRY(check_launch(ctx, "rs_pass"));
             continue;
         }
-        rs_hist<<<nblocks, RS_THREADS, 0, st>>>(k[in], n, shift, hist, nblocks);
+        launch_next(rs_hist, nblocks, RS_THREADS, 0, st, k[in], n, shift, hist, nblocks);
         PT_TRY(check_launch(ctx, "rs_hist"));
-        rs_rowscan<<<256, RS_THREADS, 0, st>>>(hist, offs, rowsum, nblocks);
+        launch_next(rs_rowscan, 256, RS_THREADS, 0, st, hist, offs, rowsum, nblocks);
         PT_TRY(check_launch(ctx, "rs_rowscan"));
-        rs_scatter<<<nblocks, RS_THREADS, 0, st>>>(k[in], vin, k[in ^ 1], v[in ^ 1], n, shift, offs, rowsum, nblocks);
+        launch_next(rs_scatter, nblocks, RS_THREADS, 0, st, k[in], vin, k[in ^ 1], v[in ^ 1], n, shift, offs, rowsum, nblocks);
         PT_TRY(check_launch(ctx, "rs_scatter"));
     }
-    rs_finish<<<(n + 255) / 256, 256, 0, st>>>(kb, vb, n, shift0, keys, vals, redo);
+    launch_next(rs_finish, (n + 255) / 256, 256, 0, st, kb, vb, n, shift0, keys, vals, redo);
     PT_TRY(check_launch(ctx, "rs_finish"));
     int all = (bits + 7) / 8, nb = nblocks;
     void *args[] = {&keys, &vals, &kb, &vb, &n, &all, &hist, &offs, &rowsum, &nb, &redo, &ctrl, &err};

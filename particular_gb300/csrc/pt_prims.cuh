@@ -26,6 +26,8 @@ struct RadixFirst {
     uint64_t *keys;
     uint32_t *hist;
     int shift;
+    uint32_t *zero;  // words that have to be zero before the keys are produced
+    int zero_words;
 };
 int radix_sort_prepare(pt_ctx *ctx, PrimScratch &s, int n, int bits, RadixFirst *first);
 int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, int n, int bits, int *err);

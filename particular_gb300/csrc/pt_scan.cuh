@@ -55,6 +55,7 @@ __device__ __forceinline__ int first_item(int tile) {
 
 template <class In>
 __global__ void __launch_bounds__(THREADS) tile_sums(In in, int n, uint32_t *__restrict__ sums) {
+    after_previous();
     const int i0 = first_item(blockIdx.x);
     uint32_t s = 0;
 #pragma unroll
@@ -68,6 +69,7 @@ __global__ void __launch_bounds__(THREADS) tile_sums(In in, int n, uint32_t *__r
 template <class In, class Out>
 __global__ void __launch_bounds__(THREADS)
     scan_apply(In in, Out out, int n, const uint32_t *__restrict__ sums, int scanned) {
+    after_previous();
     uint32_t before = 0;
     if (scanned) {
         before = sums[blockIdx.x];
@@ -122,7 +124,7 @@ template <class In, class Out>
 int run(pt_ctx *ctx, const In &in, const Out &out, int n, uint32_t *tmp) {
     const int tiles = (n + TILE - 1) / TILE;
     uint32_t *sums = tmp;
-    tile_sums<<<tiles, THREADS, 0, ctx->stream>>>(in, n, sums);
+    launch_next(tile_sums<In>, tiles, THREADS, 0, ctx->stream, in, n, sums);
     PT_TRY(check_launch(ctx, "tile_sums"));
     const uint32_t *pre = sums;
     if (tiles > SCAN_DIRECT) {
@@ -130,7 +132,7 @@ int run(pt_ctx *ctx, const In &in, const Out &out, int n, uint32_t *tmp) {
         PT_TRY(run(ctx, ReadU32{sums}, WriteU32{scanned, tiles}, tiles, tmp + 2 * size_t(tiles) + 2));
         pre = scanned;
     }
-    scan_apply<<<tiles, THREADS, 0, ctx->stream>>>(in, out, n, pre, tiles > SCAN_DIRECT);
+    launch_next(scan_apply<In, Out>, tiles, THREADS, 0, ctx->stream, in, out, n, pre, int(tiles > SCAN_DIRECT));
     return check_launch(ctx, "scan_apply");
 }
 
