@@ -42,7 +42,7 @@ inline int size_class(uint32_t n) {
 }
 
 struct Tile {
-    float c[4][TILE + 2];
+    float c[4][TILE + 4];
 };
 
 // Accelerations of targets [s0+t0, s0+t0+cnt) from every body of the system [s0, s0+n),
@@ -75,20 +75,26 @@ __device__ void accel_item(const float4 *__restrict__ body, float *__restrict__ 
             T.c[2][e] = q.z;
             T.c[3][e] = q.w;
         }
-        if ((cj & 1) && tid == 0) {  // massless pad far away: contributes exactly 0
-            T.c[0][cj] = T.c[1][cj] = T.c[2][cj] = 1e30f;
-            T.c[3][cj] = 0.f;
+        if (tid < (-cj & 3)) {  // massless pad far away: contributes exactly 0
+            T.c[0][cj + tid] = T.c[1][cj + tid] = T.c[2][cj + tid] = 1e30f;
+            T.c[3][cj + tid] = 0.f;
         }
         __syncthreads();
-        const int c2 = (cj + 1) & ~1;
-#pragma unroll 4
-        for (int e = 0; e < c2; e += 2) {
-            const f2 xj = *reinterpret_cast<const f2 *>(&T.c[0][e]);
-            const f2 yj = *reinterpret_cast<const f2 *>(&T.c[1][e]);
-            const f2 zj = *reinterpret_cast<const f2 *>(&T.c[2][e]);
-            const f2 mj = *reinterpret_cast<const f2 *>(&T.c[3][e]);
+        const float4 *X = reinterpret_cast<const float4 *>(T.c[0]), *Y = reinterpret_cast<const float4 *>(T.c[1]);
+        const float4 *Z = reinterpret_cast<const float4 *>(T.c[2]), *M = reinterpret_cast<const float4 *>(T.c[3]);
+        const int quads = (cj + 3) >> 2;
+        // bound by the FMA pipe; four sources a step, one 16-byte read per component (by two, 8
+        // bytes each, 1024 systems of 64-8192 bodies took 31.6 ms for 10 steps, now 29.9)
+#pragma unroll 2
+        for (int q = 0; q < quads; ++q) {
+            const float4 x = X[q], y = Y[q], z = Z[q], m = M[q];
 #pragma unroll
-            for (int k = 0; k < K; ++k) interact2<GUARD>(xj, yj, zj, mj, xi[k], yi[k], zi[k], ax[k], ay[k], az[k], e2);
+            for (int k = 0; k < K; ++k) {
+                interact2<GUARD>(pk2(x.x, x.y), pk2(y.x, y.y), pk2(z.x, z.y), pk2(m.x, m.y), xi[k], yi[k], zi[k],
+                                 ax[k], ay[k], az[k], e2);
+                interact2<GUARD>(pk2(x.z, x.w), pk2(y.z, y.w), pk2(z.z, z.w), pk2(m.z, m.w), xi[k], yi[k], zi[k],
+                                 ax[k], ay[k], az[k], e2);
+            }
         }
 #pragma unroll
         for (int k = 0; k < K; ++k) {
@@ -132,7 +138,15 @@ __device__ __forceinline__ void run_item(const int4 w, const float4 *__restrict_
     else run_item_k<1, GUARD>(jc, w, cnt, body, acc, eps2, T);
 }
 
-// ctrl: [0] barrier arrivals, [1] barrier generation, [2 + p] queue of phase p.
+// ctrl: [0] barrier arrivals, [1] barrier generation, [PLACE ..] the blocks' places, then
+// [QUEUE + p] queue of phase p.
+// Places: blocks are ordered by how many others came to their SM before them, so that the
+// items that the first blocks take, the largest, are spread over the SMs however the launch
+// filled these (it fills an SM before the next: in block order the largest systems' items
+// shared a few SMs; 40 systems of 64-8192 bodies, 10 steps, 4.07 -> 2.85 ms).
+constexpr int RANKS = 32, PLACE_SMS = 512, PLACE = 2, QUEUE = PLACE + RANKS + PLACE_SMS;
+constexpr size_t ctrl_words(int steps) { return size_t(QUEUE) + size_t(steps) + 1; }
+
 // Returns false (in every thread) once any block has recorded an error.
 __device__ bool grid_sync(unsigned *ctrl, int *err, long long spin_limit, unsigned expected) {
     __shared__ int s_ok;
@@ -169,9 +183,23 @@ __global__ void __launch_bounds__(THREADS)
     __shared__ __align__(16) Tile T;
     __shared__ int s_item;
     const unsigned expected = gridDim.x + (stall ? 1u : 0u);  // stall: a barrier nothing completes
+    unsigned *place = ctrl + PLACE;
+    unsigned rank = 0, nth = 0;
+    if (threadIdx.x == 0) {
+        unsigned sm;
+        asm("mov.u32 %0, %smid;" : "=r"(sm));
+        rank = min(atomicAdd(place + RANKS + sm % PLACE_SMS, 1u), unsigned(RANKS - 1));
+        nth = atomicAdd(place + rank, 1u);
+    }
+    if (!grid_sync(ctrl, err, spin_limit, expected)) return;
+    int first = 0;
+    if (threadIdx.x == 0) {
+        first = int(nth);
+        for (unsigned r = 0; r < rank; ++r) first += int(*reinterpret_cast<volatile unsigned *>(place + r));
+    }
     for (int phase = 0; phase <= steps; ++phase) {
-        for (;;) {
-            if (threadIdx.x == 0) s_item = int(atomicAdd(ctrl + 2 + phase, 1u));
+        for (bool begin = true;; begin = false) {
+            if (threadIdx.x == 0) s_item = begin ? first : int(gridDim.x + atomicAdd(ctrl + QUEUE + phase, 1u));
             __syncthreads();
             const int it = s_item;
             __syncthreads();
@@ -230,7 +258,11 @@ static State *state(pt_ctx *ctx) {
     return static_cast<State *>(ctx->ens);
 }
 
-static int default_k(int cls) { return cls >= 5 ? 2 : 1; }  // >= 2048 bodies: 2 targets per thread
+// One target per thread for every size: with the blocks spread over the SMs the shorter items
+// balance better than two targets' fewer shared-memory reads gain (10 steps, ms, one / two
+// from 2048 bodies on: 1024 systems of 64-8192 29.9 / 30.5; 130 systems 4.6 / 5.1; 40 systems
+// 2.0 / 2.8; 100 systems of 64-3000 0.90 / 1.17).
+static int default_k(int) { return 1; }
 
 // Items sorted by cost (targets x sources), largest first.
 static void build_items(const uint32_t *offsets, uint32_t n_sys, const int *table, const int *tiles,
@@ -296,11 +328,11 @@ static int launch(pt_ctx *ctx, State &S, float4 *body, float4 *vel, int n_bodies
     PT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, THREADS, 0));
     if (occ < 1) return set_error(PT_ERR_CUDA, "ensemble kernel does not fit on an SM");
     int grid = std::max(1, std::min(occ * ctx->sm_count, std::max(S.n_items, 1)));
-    PT_CUDA(cudaMemsetAsync(S.ctrl.ptr, 0, sizeof(unsigned) * size_t(steps + 3) + 16, ctx->stream));
+    PT_CUDA(cudaMemsetAsync(S.ctrl.ptr, 0, sizeof(unsigned) * ens::ctrl_words(steps) + 16, ctx->stream));
     const int4 *items = static_cast<const int4 *>(S.items.ptr);
     float *acc = static_cast<float *>(S.acc.ptr);
     unsigned *ctrl = static_cast<unsigned *>(S.ctrl.ptr);
-    int *err = reinterpret_cast<int *>(static_cast<char *>(S.ctrl.ptr) + sizeof(unsigned) * size_t(steps + 3));
+    int *err = reinterpret_cast<int *>(static_cast<char *>(S.ctrl.ptr) + sizeof(unsigned) * ens::ctrl_words(steps));
     int n_items = S.n_items;
     long long spin = S.spin_limit;
     int stall = S.stall;
@@ -342,11 +374,11 @@ extern "C" int pt_ensemble_run(pt_ctx *ctx, const uint32_t *offsets, uint32_t n_
     if (n == 0) return PT_OK;
     PT_TRY(ens::upload_items(ctx, *S, offsets, n_sys));
     PT_TRY(ensure_buf(ctx, S->acc, 12 * size_t(n)));
-    PT_TRY(ensure_buf(ctx, S->ctrl, sizeof(unsigned) * size_t(steps + 3) + 16));
+    PT_TRY(ensure_buf(ctx, S->ctrl, sizeof(unsigned) * ens::ctrl_words(steps) + 16));
     float4 *body = reinterpret_cast<float4 *>(d_bodies);
     float4 *vel = reinterpret_cast<float4 *>(d_vel);
     const float eps2 = softening * softening;
-    int *err = reinterpret_cast<int *>(static_cast<char *>(S->ctrl.ptr) + sizeof(unsigned) * size_t(steps + 3));
+    int *err = reinterpret_cast<int *>(static_cast<char *>(S->ctrl.ptr) + sizeof(unsigned) * ens::ctrl_words(steps));
     if (!use_graph) {
         PT_TRY(ens::launch(ctx, *S, body, vel, n, steps, dt, eps2));
     } else {
