@@ -165,16 +165,15 @@ int pt_bh_accel_f32(pt_ctx *ctx, const float *aff, size_t n_aff, const float *sr
     float *d_aff = static_cast<float *>(S->aff_h.ptr);
     float *d_src = same ? d_aff : static_cast<float *>(S->src_h.ptr);
     float *d_out = static_cast<float *>(S->out.ptr);
-    cudaStream_t st = ctx->stream;
-    PT_CUDA(cudaMemcpyAsync(d_aff, aff, 16 * n_aff, cudaMemcpyHostToDevice, st));
-    if (!same && n_src) PT_CUDA(cudaMemcpyAsync(d_src, src, 16 * n_src, cudaMemcpyHostToDevice, st));
+    Staging copies(ctx, 16 * n_aff + (same ? 0 : 16 * n_src) + 12 * n_aff + sizeof(int));
+    PT_TRY(copies.to_device(d_aff, aff, 16 * n_aff));
+    if (!same && n_src) PT_TRY(copies.to_device(d_src, src, 16 * n_src));
     PT_TRY(bh::run(ctx, reinterpret_cast<const float4 *>(d_aff), int(n_aff), reinterpret_cast<const float4 *>(d_src),
                    int(n_src), theta, softening, flags, d_out));
-    PT_CUDA(cudaMemcpyAsync(out, d_out, 12 * n_aff, cudaMemcpyDeviceToHost, st));
+    PT_TRY(copies.to_host(out, d_out, 12 * n_aff));
     int err = 0;
-    if (n_src) PT_CUDA(cudaMemcpyAsync(&err, static_cast<int *>(S->counters.ptr) + 3, sizeof(int),
-                                       cudaMemcpyDeviceToHost, st));
-    PT_CUDA(cudaStreamSynchronize(st));
+    if (n_src) PT_TRY(copies.to_host(&err, static_cast<int *>(S->counters.ptr) + 3, sizeof(int)));
+    PT_TRY(copies.finish());
     PT_TRY(bh::sort_error("pt_bh_accel_f32", err));
     if (err & 2)
         return set_error(PT_ERR_CAPACITY, "pt_bh_accel_f32: learned-correction records overflowed");
@@ -217,16 +216,15 @@ int pt_bh_accel_dvec3(pt_ctx *ctx, const double *aff, size_t n_aff, const double
     double *d_aff = static_cast<double *>(S->aff_h.ptr);
     double *d_src = same ? d_aff : static_cast<double *>(S->src_h.ptr);
     double *d_out = static_cast<double *>(S->out.ptr);
-    cudaStream_t st = ctx->stream;
-    PT_CUDA(cudaMemcpyAsync(d_aff, aff, 32 * n_aff, cudaMemcpyHostToDevice, st));
-    if (!same && n_src) PT_CUDA(cudaMemcpyAsync(d_src, src, 32 * n_src, cudaMemcpyHostToDevice, st));
+    Staging copies(ctx, 32 * n_aff + (same ? 0 : 32 * n_src) + 24 * n_aff + sizeof(int));
+    PT_TRY(copies.to_device(d_aff, aff, 32 * n_aff));
+    if (!same && n_src) PT_TRY(copies.to_device(d_src, src, 32 * n_src));
     PT_TRY(bh::run64(ctx, reinterpret_cast<const double4_32a *>(d_aff), int(n_aff),
                      reinterpret_cast<const double4_32a *>(d_src), int(n_src), theta, softening, d_out));
-    PT_CUDA(cudaMemcpyAsync(out, d_out, 24 * n_aff, cudaMemcpyDeviceToHost, st));
+    PT_TRY(copies.to_host(out, d_out, 24 * n_aff));
     int err = 0;
-    if (n_src) PT_CUDA(cudaMemcpyAsync(&err, static_cast<int *>(S->counters.ptr) + 3, sizeof(int),
-                                       cudaMemcpyDeviceToHost, st));
-    PT_CUDA(cudaStreamSynchronize(st));
+    if (n_src) PT_TRY(copies.to_host(&err, static_cast<int *>(S->counters.ptr) + 3, sizeof(int)));
+    PT_TRY(copies.finish());
     PT_TRY(bh::sort_error("pt_bh_accel_dvec3", err));
     if (err & 1) return set_error(PT_ERR_CAPACITY, "pt_bh_accel_dvec3: a warp's stack ran out; its bodies are NaN");
     return PT_OK;
@@ -432,14 +430,13 @@ int pt_bh_walk(pt_ctx *ctx, const float *aff, size_t n_aff, float theta, float s
     PT_TRY(ensure_buf(ctx, S->out, 12 * n_aff));
     float *d_aff = static_cast<float *>(S->aff_h.ptr);
     float *d_out = static_cast<float *>(S->out.ptr);
-    cudaStream_t st = ctx->stream;
-    PT_CUDA(cudaMemcpyAsync(d_aff, aff, 16 * n_aff, cudaMemcpyHostToDevice, st));
+    Staging copies(ctx, 16 * n_aff + 12 * n_aff + sizeof(int));
+    PT_TRY(copies.to_device(d_aff, aff, 16 * n_aff));
     PT_TRY(pt_bh_walk_device(ctx, d_aff, n_aff, theta, softening, flags, d_out));
-    PT_CUDA(cudaMemcpyAsync(out, d_out, 12 * n_aff, cudaMemcpyDeviceToHost, st));
+    PT_TRY(copies.to_host(out, d_out, 12 * n_aff));
     int err = 0;
-    PT_CUDA(cudaMemcpyAsync(&err, static_cast<int *>(S->counters.ptr) + 3, sizeof(int), cudaMemcpyDeviceToHost,
-                            st));
-    PT_CUDA(cudaStreamSynchronize(st));
+    PT_TRY(copies.to_host(&err, static_cast<int *>(S->counters.ptr) + 3, sizeof(int)));
+    PT_TRY(copies.finish());
     PT_TRY(bh::sort_error("pt_bh_walk", err));
     if (err & 2) return set_error(PT_ERR_CAPACITY, "pt_bh_walk: learned-correction records overflowed");
     return PT_OK;

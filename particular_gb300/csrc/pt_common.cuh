@@ -50,6 +50,10 @@ struct pt_ctx {
     // that captured buffer addresses are captured again when it has moved.
     unsigned long long buf_epoch = 0;
     pt::DevBuf bufs[pt::BUF_COUNT];
+    // Small brute-force calls: slices ended per block of targets (DONE_COUNTERS, zero between calls).
+    unsigned *slices_done = nullptr;
+    // Page-locked host memory (Staging) and its device address.
+    void *pinned = nullptr, *pinned_dev = nullptr;
     // Extra subsystems hang off the context lazily.
     void *bh = nullptr;
     void *lf = nullptr;
@@ -72,6 +76,34 @@ int ensure(pt_ctx *ctx, int slot, size_t bytes);
 // Generic grow-only buffer (for subsystems that keep their own DevBufs).
 int ensure_buf(pt_ctx *ctx, DevBuf &b, size_t bytes);
 void free_buf(pt_ctx *ctx, DevBuf &b);
+constexpr int DONE_COUNTERS = 2048;
+// The copies of one host call of `bytes` in all (each rounded up to 16): through the context's
+// page-locked memory while they fit in it, so that none of them waits for the driver's own
+// staging, else straight from and to the caller's memory. finish() waits for the stream.
+// Brute force with and without, us: 20.5/26.8 at N = 64, 27.4/34.2 at 1024, 45/49 at 4000,
+// 113/115 at 12000, but 505/478 at 32000: hence the limit.
+constexpr size_t PINNED_BYTES = size_t(384) << 10;
+struct Staging {
+    Staging(pt_ctx *c, size_t bytes);
+    int to_device(void *dev, const void *host, size_t n);
+    int to_host(void *host, const void *dev, size_t n);
+    // Where a kernel may itself write n bytes for host: page-locked memory, or dev with a copy
+    // that the caller asks for by to_host. nullptr where it has to be the latter.
+    void *kernel_output(void *host, size_t n);
+    int finish();
+
+   private:
+    char *take(size_t n);
+    pt_ctx *ctx;
+    size_t used = 0;
+    bool pinned;
+    int n_out = 0;
+    struct {
+        void *host;
+        const char *from;
+        size_t n;
+    } outs[2];
+};
 
 // Checks the launch just made; counts it.
 int check_launch(pt_ctx *ctx, const char *what);

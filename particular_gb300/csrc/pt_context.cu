@@ -82,6 +82,60 @@ void free_buf(pt_ctx *ctx, DevBuf &b) {
     b.cap = 0;
 }
 
+Staging::Staging(pt_ctx *c, size_t bytes) : ctx(c), pinned(bytes + 64 <= PINNED_BYTES) {
+    if (!pinned || ctx->pinned) return;
+    void *h = nullptr, *d = nullptr;
+    cudaError_t e = cudaHostAlloc(&h, PINNED_BYTES, cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&d, h, 0);
+    if (e != cudaSuccess) {  // the call does without
+        cudaGetLastError();
+        if (h) cudaFreeHost(h);
+        pinned = false;
+        return;
+    }
+    ctx->pinned = h;
+    ctx->pinned_dev = d;
+}
+
+char *Staging::take(size_t n) {
+    char *h = static_cast<char *>(ctx->pinned) + used;
+    used += (n + 15) / 16 * 16;
+    return h;
+}
+
+int Staging::to_device(void *dev, const void *host, size_t n) {
+    if (pinned) {
+        char *h = take(n);
+        std::memcpy(h, host, n);
+        host = h;
+    }
+    PT_CUDA(cudaMemcpyAsync(dev, host, n, cudaMemcpyHostToDevice, ctx->stream));
+    return PT_OK;
+}
+
+int Staging::to_host(void *host, const void *dev, size_t n) {
+    char *h = static_cast<char *>(host);
+    if (pinned) {
+        h = take(n);
+        outs[n_out++] = {host, h, n};
+    }
+    PT_CUDA(cudaMemcpyAsync(h, dev, n, cudaMemcpyDeviceToHost, ctx->stream));
+    return PT_OK;
+}
+
+void *Staging::kernel_output(void *host, size_t n) {
+    if (!pinned) return nullptr;
+    const char *h = take(n);
+    outs[n_out++] = {host, h, n};
+    return static_cast<char *>(ctx->pinned_dev) + (h - static_cast<char *>(ctx->pinned));
+}
+
+int Staging::finish() {
+    PT_CUDA(cudaStreamSynchronize(ctx->stream));
+    for (int i = 0; i < n_out; ++i) std::memcpy(outs[i].host, outs[i].from, outs[i].n);
+    return PT_OK;
+}
+
 int ensure(pt_ctx *ctx, int slot, size_t bytes) { return ensure_buf(ctx, ctx->bufs[slot], bytes); }
 
 }  // namespace pt
@@ -118,6 +172,16 @@ int pt_ctx_create(pt_ctx **out, int device) {
         return pt::check_cuda(e, "pt_ctx_create");
     }
     c->stream = c->own_stream;
+    // Without the counters small calls add their slices in a kernel of their own.
+    void *done = nullptr;
+    if (cudaMalloc(&done, sizeof(unsigned) * pt::DONE_COUNTERS) != cudaSuccess ||
+        cudaMemsetAsync(done, 0, sizeof(unsigned) * pt::DONE_COUNTERS, c->own_stream) != cudaSuccess ||
+        cudaStreamSynchronize(c->own_stream) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(done);
+        done = nullptr;
+    }
+    c->slices_done = static_cast<unsigned *>(done);
     *out = c;
     return PT_OK;
 }
@@ -131,6 +195,8 @@ void pt_ctx_destroy(pt_ctx *ctx) {
     pt_bh_state_free(ctx);
     pt_mlp_state_free(ctx);
     for (auto &b : ctx->bufs) pt::free_buf(ctx, b);
+    if (ctx->pinned) cudaFreeHost(ctx->pinned);
+    cudaFree(ctx->slices_done);
     for (auto &e : ctx->ev)
         if (e) cudaEventDestroy(e);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);

@@ -59,3 +59,23 @@ def test_fast_sums_at_tile_edges(res, oracle, n_src, soft):
     scale = (src[None, :, 3] * np.sqrt(r2) / np.where(r2 > 0, r2 + eps * eps, 1.0) ** 1.5).sum(1)
     assert np.isfinite(got).all()
     assert (np.abs(got - want).max(1) <= 1e-5 * scale + 1e-30).all()
+
+
+# Slices added by the last block of a small call or by a kernel of its own (up to 4096 x 4096
+# pairs and beyond), host calls through page-locked memory or without (14043 bodies and beyond):
+# the same sums in the same order, also when a call follows one of another shape.
+@pytest.mark.parametrize("n", [1, 127, 129, 257, 1024, 4096, 4097, 14042, 14044])
+def test_small_calls_add_their_slices_in_the_same_order(res, native_lib, n):
+    import torch
+    from particular_gb300 import _native as N
+
+    b = bodies(n, n)
+    d = torch.from_numpy(b).cuda()
+    own = torch.empty((n, 3), device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    N.check(native_lib.pt_bf_accel_f32_noalloc(d.data_ptr(), n, d.data_ptr(), n, 0.01, 1, own.data_ptr(), stream))
+    want = own.cpu().numpy()
+    method = cuda.BruteForce(res, AccelerationSoftened(0.01))
+    for m in (n, 300, n, n):
+        got = method.compute(b[:m])
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
