@@ -246,7 +246,6 @@ int pt_bh_build_device(pt_ctx *ctx, const float *d_src, size_t n_src, uint64_t *
         ++S->generation;
     } else {
         mark(ctx, 0);
-        PT_TRY(bh::clear_errors(ctx, *S));
         PT_TRY(bh::build(ctx, *S, reinterpret_cast<const float4 *>(d_src), int(n_src)));
     }
     if (generation) *generation = S->generation;

@@ -18,6 +18,7 @@ namespace bh {
 
 constexpr int LEVELS = 21;   // 63-bit keys
 constexpr int WALK_STATS = 9;  // the walk's u64 counters behind counters[0..3]
+constexpr int ROOT_BOX_DONE = 30;  // root_box's word of counters
 
 struct Moments {  // FP64 cell data used while combining children (DVec3 trees, bucket leaves)
     double m, cx, cy, cz;
@@ -117,6 +118,7 @@ template <class T>
 int sort_targets_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_aff, int n);
 int sort_targets(pt_ctx *ctx, State &S, const float4 *d_aff, int n);
 // walks (pt_bh_walk.cu)
+int ensure_counters(pt_ctx *ctx, State &S);
 int clear_errors(pt_ctx *ctx, State &S);
 int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n_aff, float theta,
          float softening, uint32_t flags, float *d_out);

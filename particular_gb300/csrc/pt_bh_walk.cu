@@ -930,10 +930,17 @@ static MaskedPlan masked_plan(const pt_ctx *ctx, int n_aff) {
     return p;
 }
 
-// Clears the error word (counters[3]) before a build or a walk of separate targets; within
-// a leapfrog sequence it collects every step's errors.
-int clear_errors(pt_ctx *ctx, State &S) {
+int ensure_counters(pt_ctx *ctx, State &S) {
+    if (S.counters.ptr) return PT_OK;
     PT_TRY(ensure_buf(ctx, S.counters, sizeof(unsigned long long) * 16));
+    PT_CUDA(cudaMemsetAsync(S.counters.ptr, 0, sizeof(unsigned long long) * 16, ctx->stream));
+    return PT_OK;
+}
+
+// Clears the error word (counters[3]) before a walk of separate targets, as a build does by
+// itself; within a leapfrog sequence it collects every step's errors.
+int clear_errors(pt_ctx *ctx, State &S) {
+    PT_TRY(ensure_counters(ctx, S));
     if (!ctx->keep_errors) PT_CUDA(cudaMemsetAsync(as<int>(S.counters) + 3, 0, sizeof(int), ctx->stream));
     return PT_OK;
 }
@@ -950,7 +957,6 @@ int run(pt_ctx *ctx, const float4 *d_aff, int n_aff, const float4 *d_src, int n_
     if (!Sp) return set_error(PT_ERR_OOM, "Barnes-Hut state allocation failed");
     State &S = *Sp;
     mark(ctx, 0);
-    PT_TRY(clear_errors(ctx, S));
     PT_TRY(build(ctx, S, d_src, n_src));
     const bool same = (d_aff == d_src) && (n_aff == n_src);
     const float4 *tbody;
@@ -989,7 +995,6 @@ int run64(pt_ctx *ctx, const double4_32a *d_aff, int n_aff, const double4_32a *d
     if (!Sp) return set_error(PT_ERR_OOM, "Barnes-Hut state allocation failed");
     State &S = *Sp;
     mark(ctx, 0);
-    PT_TRY(clear_errors(ctx, S));
     PT_TRY(build_t<double>(ctx, S, d_src, n_src));
     const bool same = (d_aff == d_src) && (n_aff == n_src);
     if (!same) PT_TRY(sort_targets_t<double>(ctx, S, d_aff, n_aff));

@@ -7,7 +7,7 @@
 //
 // A pass ranks keys stably inside a tile (each warp its own run of keys, with warp
 // match/popc), so equal digits keep their input order, stages the tile in shared memory in
-// digit order and writes every digit's run contiguously. Up to DIRECT_TILES tiles a pass is
+// digit order and writes every digit's run contiguously. Up to 262144 keys a pass is
 // one launch: every block adds up the tiles' digit counts itself, and counts the digits of
 // the next pass as it writes. Above, a histogram pass (per-tile counts) and a row scan (one
 // block per digit value over the tiles) come before the scatter.
@@ -30,16 +30,16 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
 
 // ---- radix sort ------------------------------------------------------------
 constexpr int RS_THREADS = 256;
-#ifndef PT_RS_ROUNDS
-#define PT_RS_ROUNDS 8
-#endif
-constexpr int RS_ROUNDS = PT_RS_ROUNDS;  // keys per thread of a tile
+constexpr int RS_ROUNDS = 8;  // keys per thread of a tile
 constexpr int RS_TILE = RS_THREADS * RS_ROUNDS;
-static_assert(RS_TILE == RADIX_TILE, "the producer of the keys counts their first digits by tile");
 constexpr int RS_WARPS = RS_THREADS / 32;
 
-// Tiles up to which a pass is one launch.
-constexpr int DIRECT_TILES = 64;
+// Keys per thread of a tile of the direct passes, or 0 from where a pass takes three launches.
+// Few tiles keep the sum over them short, many keep the chip busy. A whole call at 10000 bodies
+// takes 179 us with tiles of 256 keys and 187 with 2048, at 65536 274 with 1024 and 280 with
+// 2048 (318 with 256), at 131072 350 with 2048 and 355 with 1024; at 262144 534 against 541
+// with three launches a pass.
+static int direct_rounds(int n) { return n <= 64 * 256 ? 1 : n <= 64 * 1024 ? 4 : n <= 128 * 2048 ? 8 : 0; }
 
 // Exclusive scan of one value per thread over the 256 threads of a block; wsum holds
 // RS_WARPS + 1 words. Every thread of the block must call it.
@@ -113,10 +113,11 @@ __global__ void __launch_bounds__(RS_THREADS)
     scan_row(hist, offs, rowsum, nblocks, blockIdx.x, wsum);
 }
 
+template <int ROUNDS>
 struct ScatterShared {
-    uint64_t skeys[RS_TILE];
-    uint32_t svals[RS_TILE];
-    uint32_t wcnt[RS_WARPS][256];
+    uint64_t skeys[RS_THREADS * ROUNDS];
+    uint32_t svals[RS_THREADS * ROUNDS];
+    alignas(16) uint32_t wcnt[RS_WARPS][256];
     uint32_t tstart[256], gbase[256];
     uint32_t wsum[RS_WARPS + 1];
 };
@@ -129,16 +130,17 @@ struct ScatterShared {
 // keep their input order. gstart(t): where digit t's keys of this tile go. vin null: a key's
 // value is its index. next: null, or the digit counts by tile of the pass at next_shift. (All
 // reads go to L2: within rs_all other blocks have written what an earlier pass read.)
-template <class Start>
-__device__ __forceinline__ void scatter_tile(ScatterShared &S, const uint64_t *kin, const uint32_t *vin,
+template <int ROUNDS, class Start>
+__device__ __forceinline__ void scatter_tile(ScatterShared<ROUNDS> &S, const uint64_t *kin, const uint32_t *vin,
                                              uint64_t *kout, uint32_t *vout, int n, int shift, int b,
                                              const Start &gstart, uint32_t *next, int next_shift) {
+    constexpr int TILE = RS_THREADS * ROUNDS;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    const size_t wbase = size_t(b) * RS_TILE + size_t(warp) * (32 * RS_ROUNDS);
-    uint64_t key[RS_ROUNDS];
-    uint32_t val[RS_ROUNDS], rank[RS_ROUNDS];
+    const size_t wbase = size_t(b) * TILE + size_t(warp) * (32 * ROUNDS);
+    uint64_t key[ROUNDS];
+    uint32_t val[ROUNDS], rank[ROUNDS];
 #pragma unroll
-    for (int r = 0; r < RS_ROUNDS; ++r) {
+    for (int r = 0; r < ROUNDS; ++r) {
         const size_t i = wbase + size_t(r) * 32 + lane;
         const bool valid = i < size_t(n);
         key[r] = valid ? __ldcg(kin + i) : 0ull;
@@ -150,7 +152,7 @@ __device__ __forceinline__ void scatter_tile(ScatterShared &S, const uint64_t *k
     __syncthreads();
     const uint32_t lt = (1u << lane) - 1u;
 #pragma unroll
-    for (int r = 0; r < RS_ROUNDS; ++r) {
+    for (int r = 0; r < ROUNDS; ++r) {
         const bool valid = wbase + size_t(r) * 32 + lane < size_t(n);
         const uint32_t d = valid ? digit_of(key[r], shift) : 256u;
         const uint32_t peers = __match_any_sync(0xffffffffu, d);
@@ -173,7 +175,7 @@ __device__ __forceinline__ void scatter_tile(ScatterShared &S, const uint64_t *k
     S.tstart[t] = block_excl_scan(tot, S.wsum, nullptr);
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < RS_ROUNDS; ++r) {
+    for (int r = 0; r < ROUNDS; ++r) {
         if (wbase + size_t(r) * 32 + lane < size_t(n)) {
             const uint32_t d = digit_of(key[r], shift);
             const uint32_t pos = S.tstart[d] + S.wcnt[warp][d] + rank[r];
@@ -182,14 +184,14 @@ __device__ __forceinline__ void scatter_tile(ScatterShared &S, const uint64_t *k
         }
     }
     __syncthreads();
-    const int cnt = int(min(size_t(RS_TILE), size_t(n) - size_t(b) * RS_TILE));
+    const int cnt = int(min(size_t(TILE), size_t(n) - size_t(b) * TILE));
     for (int i = t; i < cnt; i += RS_THREADS) {
         const uint64_t k = S.skeys[i];
         const uint32_t d = digit_of(k, shift);
         const uint32_t pos = S.gbase[d] + (uint32_t(i) - S.tstart[d]);
         kout[pos] = k;
         vout[pos] = S.svals[i];
-        if (next) atomicAdd(&next[(pos / RS_TILE) * 256 + digit_of(k, next_shift)], 1u);
+        if (next) atomicAdd(&next[(pos / TILE) * 256 + digit_of(k, next_shift)], 1u);
     }
 }
 
@@ -198,7 +200,7 @@ __global__ void __launch_bounds__(RS_THREADS)
                uint32_t *__restrict__ vout, int n, int shift, const uint32_t *__restrict__ offs,
                const uint32_t *__restrict__ rowsum, int nblocks) {
     after_previous();
-    __shared__ ScatterShared S;
+    __shared__ ScatterShared<RS_ROUNDS> S;
     const int b = blockIdx.x;
     // all smaller digits, then earlier tiles
     scatter_tile(S, kin, vin, kout, vout, n, shift, b,
@@ -207,23 +209,39 @@ __global__ void __launch_bounds__(RS_THREADS)
 }
 
 // One pass in one launch: hist[b * 256 + d] holds the tiles' digit counts.
+template <int ROUNDS>
 __global__ void __launch_bounds__(RS_THREADS)
     rs_pass(const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin, uint64_t *__restrict__ kout,
             uint32_t *__restrict__ vout, int n, int shift, const uint32_t *__restrict__ hist, int nblocks,
             uint32_t *__restrict__ next, int next_shift) {
     after_previous();
-    __shared__ ScatterShared S;
+    __shared__ ScatterShared<ROUNDS> S;
     const int b = blockIdx.x;
     scatter_tile(S, kin, vin, kout, vout, n, shift, b,
                  [&](int t) {
-                     uint32_t before = 0, total = 0;
+                     // four digits a load, every fourth tile
+                     const int g = t >> 6, q = t & 63;
+                     uint4 before = make_uint4(0, 0, 0, 0), total = before;
 #pragma unroll 8
-                     for (int j = 0; j < nblocks; ++j) {
-                         const uint32_t h = hist[j * 256 + t];
-                         if (j < b) before += h;
-                         total += h;
+                     for (int j = g; j < nblocks; j += 4) {
+                         const uint4 h = reinterpret_cast<const uint4 *>(hist)[j * 64 + q];
+                         if (j < b) {
+                             before.x += h.x;
+                             before.y += h.y;
+                             before.z += h.z;
+                             before.w += h.w;
+                         }
+                         total.x += h.x;
+                         total.y += h.y;
+                         total.z += h.z;
+                         total.w += h.w;
                      }
-                     return block_excl_scan(total, S.wsum, nullptr) + before;
+                     reinterpret_cast<uint4 *>(S.wcnt[g])[q] = before;
+                     reinterpret_cast<uint4 *>(S.wcnt[4 + g])[q] = total;
+                     __syncthreads();
+                     const uint32_t sum = S.wcnt[4][t] + S.wcnt[5][t] + S.wcnt[6][t] + S.wcnt[7][t];
+                     const uint32_t mine = S.wcnt[0][t] + S.wcnt[1][t] + S.wcnt[2][t] + S.wcnt[3][t];
+                     return block_excl_scan(sum, S.wsum, nullptr) + mine;
                  },
                  next, next_shift);
 }
@@ -302,7 +320,7 @@ __global__ void __launch_bounds__(RS_THREADS)
         if (!ok && threadIdx.x == 0) atomicOr(err, ERR_SORT_BARRIER);
         return ok;
     };
-    __shared__ ScatterShared S;
+    __shared__ ScatterShared<RS_ROUNDS> S;
     uint64_t *kin = kb, *kout = ka;
     uint32_t *vin = vb, *vout = va;
     for (int p = 0; p < passes; ++p) {
@@ -343,39 +361,52 @@ __global__ void __launch_bounds__(RS_THREADS)
 // runs of a few bodies at 4M bulge+disk; a sixth from 8M on.
 static int head_shift(int n, int bits) { return std::max(0, bits - 8 * (n >= (1 << 23) ? 6 : 5)); }
 
+namespace prims {
+// How a sort of n keys is laid out: tiles of the direct passes (rounds = 0: three launches a
+// pass) and words of histograms.
+struct SortPlan {
+    int shift, passes, rounds, tile, tiles, blocks;
+    size_t nhist, words;
+    SortPlan(int n, int bits)
+        : shift(head_shift(n, bits)),
+          passes((bits - shift + 7) / 8),
+          rounds(direct_rounds(n)),
+          tile(RS_THREADS * (rounds ? rounds : RS_ROUNDS)),
+          tiles((n + tile - 1) / tile),
+          blocks((n + RS_TILE - 1) / RS_TILE),
+          nhist(256 * size_t(blocks)) {
+        // counts per pass of the direct passes; counts, offsets and row sums; then the redo
+        // flag and the barrier of rs_all
+        words = std::max(rounds ? size_t(passes) * 256 * tiles : 0, 2 * nhist + 256) + 64;
+    }
+};
+}  // namespace prims
+
 int radix_sort_prepare(pt_ctx *ctx, PrimScratch &s, int n, int bits, RadixFirst *first) {
     using namespace prims;
-    const int nblocks = (n + RS_TILE - 1) / RS_TILE;
-    const int shift = head_shift(n, bits), passes = (bits - shift + 7) / 8;
-    const size_t nhist = 256 * size_t(nblocks);
-    // histograms: per pass of the direct passes, or counts + offsets + row sums
-    const size_t words = std::max(size_t(passes) * nhist, 2 * nhist + 256) + 64;
+    const SortPlan p(n, bits);
     PT_TRY(ensure_buf(ctx, s.keys2, sizeof(uint64_t) * size_t(n)));
     PT_TRY(ensure_buf(ctx, s.vals2, sizeof(uint32_t) * size_t(n)));
-    PT_TRY(ensure_buf(ctx, s.hist, sizeof(uint32_t) * words));
-    // the last 64 words: the redo flag and the barrier of rs_all
-    const bool direct = nblocks <= DIRECT_TILES;
+    PT_TRY(ensure_buf(ctx, s.hist, sizeof(uint32_t) * p.words));
     uint32_t *hist = static_cast<uint32_t *>(s.hist.ptr);
-    uint32_t *tail = hist + (words - 64);
-    first->zero = direct ? hist : tail;
-    first->zero_words = direct ? int(words) : 64;
+    first->zero = p.rounds ? hist : hist + (p.words - 64);
+    first->zero_words = p.rounds ? int(p.words) : 64;
     // an odd number of passes ends in the pair that the finishing pass reads
-    first->keys = (passes & 1) ? nullptr : static_cast<uint64_t *>(s.keys2.ptr);
-    first->hist = direct ? hist : nullptr;
-    first->shift = shift;
+    first->keys = (p.passes & 1) ? nullptr : static_cast<uint64_t *>(s.keys2.ptr);
+    first->hist = p.rounds ? hist : nullptr;
+    first->shift = p.shift;
+    first->tile = p.tile;
     return PT_OK;
 }
 
 int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, int n, int bits, int *err) {
     using namespace prims;
-    const int nblocks = (n + RS_TILE - 1) / RS_TILE;
-    const int shift0 = head_shift(n, bits), passes = (bits - shift0 + 7) / 8;
-    const size_t nhist = 256 * size_t(nblocks);
-    const size_t words = std::max(size_t(passes) * nhist, 2 * nhist + 256) + 64;
+    const SortPlan sp(n, bits);
+    const int nblocks = sp.blocks, shift0 = sp.shift, passes = sp.passes;
     uint32_t *hist = static_cast<uint32_t *>(s.hist.ptr);
-    int *redo = reinterpret_cast<int *>(hist + (words - 64));
+    int *redo = reinterpret_cast<int *>(hist + (sp.words - 64));
     unsigned *ctrl = reinterpret_cast<unsigned *>(redo + 16);
-    uint32_t *offs = hist + nhist, *rowsum = offs + nhist;
+    uint32_t *offs = hist + sp.nhist, *rowsum = offs + sp.nhist;
     uint64_t *kb = static_cast<uint64_t *>(s.keys2.ptr), *k[2] = {keys, kb};
     uint32_t *vb = static_cast<uint32_t *>(s.vals2.ptr), *v[2] = {vals, vb};
     cudaStream_t st = ctx->stream;
@@ -383,10 +414,14 @@ int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, 
     for (int p = 0; p < passes; ++p, in ^= 1) {
         const int shift = shift0 + 8 * p;
         const uint32_t *vin = p == 0 ? nullptr : v[in];
-        if (nblocks <= DIRECT_TILES) {
-            uint32_t *next = p + 1 < passes ? hist + (p + 1) * nhist : nullptr;
-            launch_next(rs_pass, nblocks, RS_THREADS, 0, st, k[in], vin, k[in ^ 1], v[in ^ 1], n, shift, hist + p * nhist,
-                                                    nblocks, next, shift + 8);
+        if (sp.rounds) {
+            const size_t direct = 256 * size_t(sp.tiles);
+            uint32_t *next = p + 1 < passes ? hist + (p + 1) * direct : nullptr;
+            launch_next(sp.rounds == 1   ? rs_pass<1>
+                        : sp.rounds == 4 ? rs_pass<4>
+                                         : rs_pass<8>,
+                        sp.tiles, RS_THREADS, 0, st, k[in], vin, k[in ^ 1], v[in ^ 1], n, shift, hist + p * direct,
+                        sp.tiles, next, shift + 8);
             PT_TRY(check_launch(ctx, "rs_pass"));
             continue;
         }
@@ -394,7 +429,8 @@ int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, 
         PT_TRY(check_launch(ctx, "rs_hist"));
         launch_next(rs_rowscan, 256, RS_THREADS, 0, st, hist, offs, rowsum, nblocks);
         PT_TRY(check_launch(ctx, "rs_rowscan"));
-        launch_next(rs_scatter, nblocks, RS_THREADS, 0, st, k[in], vin, k[in ^ 1], v[in ^ 1], n, shift, offs, rowsum, nblocks);
+        launch_next(rs_scatter, nblocks, RS_THREADS, 0, st, k[in], vin, k[in ^ 1], v[in ^ 1], n, shift, offs, rowsum,
+                    nblocks);
         PT_TRY(check_launch(ctx, "rs_scatter"));
     }
     launch_next(rs_finish, (n + 255) / 256, 256, 0, st, kb, vb, n, shift0, keys, vals, redo);

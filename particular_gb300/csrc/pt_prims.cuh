@@ -16,16 +16,15 @@ struct PrimScratch {
 
 // Sorting n keys takes two calls: radix_sort_prepare before the keys are produced tells the
 // producer where to put them (first->keys, or the caller's own array where that is null) and,
-// for small n, to count their first digits: hist[(i / RADIX_TILE) * 256 + (key >> shift &
-// 255)] for key i where hist is not null. radix_sort_u64 then leaves the keys ascending by
+// for small n, to count their first digits: hist[(i / tile) * 256 + (key >> shift & 255)]
+// for key i where hist is not null. radix_sort_u64 then leaves the keys ascending by
 // their low `bits` bits in keys, equal ones in the order of their index, and their indices in
 // vals. *err (device) gets ERR_SORT_BARRIER where a grid barrier of the general path gave up.
 constexpr int ERR_SORT_BARRIER = 4;
-constexpr int RADIX_TILE = 2048;
 struct RadixFirst {
     uint64_t *keys;
     uint32_t *hist;
-    int shift;
+    int shift, tile;
     uint32_t *zero;  // words that have to be zero before the keys are produced
     int zero_words;
 };

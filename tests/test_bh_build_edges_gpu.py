@@ -81,9 +81,11 @@ def reference_order(b):
     return np.argsort(key, kind="stable"), key
 
 
-# tiles of 2048 keys, one launch a pass up to 64 of them; and clusters so much smaller than
-# the box that their keys share the upper bits the passes sort, in runs short and long
-@pytest.mark.parametrize("n", [2047, 2048, 2049, 131072, 131073])
+# tiles of 256 keys, from 16385 on of 1024, from 65537 on of 2048, three launches a pass from
+# 262145 on; and clusters so much smaller than the box that their keys share the upper bits
+# the passes sort, in runs short and long
+@pytest.mark.parametrize("n", [1, 255, 257, 2047, 2048, 2049, 16384, 16385, 65536, 65537, 131072, 131073, 262144,
+                               262145])
 @pytest.mark.parametrize("kind", ["cube", "runs", "core"])
 def test_bodies_are_in_key_order(res, n, kind):
     r = np.random.RandomState(n)
