@@ -123,7 +123,7 @@ void pt_bh_state_free(pt_ctx *ctx) {
                      &S->nodeA,  &S->nodeB,  &S->nodeQ,  &S->nodeG, &S->nodeR, &S->mom,     &S->tkeys,  &S->tidx,
                      &S->tbody,    &S->counters, &S->out,  &S->aff_h,  &S->src_h, &S->lrec, &S->lgroup,
                      &S->lnext,    &S->lpart,  &S->lhead, &S->lcentre, &S->lused, &S->sbody64, &S->nodeA64,
-                     &S->nodeG64,  &S->tbody64, &S->gscale};
+                     &S->nodeG64,  &S->tbody64, &S->gscale,  &S->gorder};
     for (DevBuf *b : all) free_buf(ctx, *b);
     delete S;
     ctx->bh = nullptr;
@@ -372,7 +372,7 @@ int pt_bh_load_tree(pt_ctx *ctx, const int32_t *orthant, const float *bbox, cons
         PT_TRY(ensure_buf(ctx, S->nodeQ, 32 * T));
         PT_TRY(ensure_buf(ctx, S->sbody, 16 * std::max<size_t>(L, 1)));
     }
-    PT_TRY(ensure_buf(ctx, S->counters, sizeof(unsigned long long) * 16));
+    PT_TRY(ensure_buf(ctx, S->counters, bh::COUNTER_BYTES));
     PT_TRY(ensure_buf(ctx, S->box, sizeof(float) * 8));
     cudaStream_t st = ctx->stream;
     const int counts[4] = {int(L), int(T), cells, 0};
@@ -382,7 +382,7 @@ int pt_bh_load_tree(pt_ctx *ctx, const int32_t *orthant, const float *bbox, cons
         PT_CUDA(cudaMemsetAsync(S->nodeQ.ptr, 0, 32 * T, st));
         if (L) PT_CUDA(cudaMemcpyAsync(S->sbody.ptr, leaves.data(), 16 * L, cudaMemcpyHostToDevice, st));
     }
-    PT_CUDA(cudaMemsetAsync(S->counters.ptr, 0, sizeof(unsigned long long) * 16, st));
+    PT_CUDA(cudaMemsetAsync(S->counters.ptr, 0, bh::COUNTER_BYTES, st));
     PT_CUDA(cudaMemcpyAsync(S->counters.ptr, counts, sizeof(counts), cudaMemcpyHostToDevice, st));
     PT_CUDA(cudaMemcpyAsync(S->box.ptr, box, sizeof(box), cudaMemcpyHostToDevice, st));
     PT_CUDA(cudaStreamSynchronize(st));  // the host arrays are freed on return

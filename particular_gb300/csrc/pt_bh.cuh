@@ -19,6 +19,9 @@ namespace bh {
 constexpr int LEVELS = 21;   // 63-bit keys
 constexpr int WALK_STATS = 9;  // the walk's u64 counters behind counters[0..3]
 constexpr int ROOT_BOX_DONE = 30;  // root_box's word of counters
+// Group walk in order of work: the counts and cursors of its buckets, behind counters[0..31].
+constexpr int ORDER_BUCKETS = 128, ORDER_WORDS = 2 * ORDER_BUCKETS;
+constexpr size_t COUNTER_BYTES = sizeof(int) * (32 + ORDER_WORDS);
 
 struct Moments {  // FP64 cell data used while combining children (DVec3 trees, bucket leaves)
     double m, cx, cy, cz;
@@ -71,7 +74,7 @@ struct State {
     DevBuf out;
     DevBuf aff_h, src_h;  // staging for the host-pointer entry point
     DevBuf lrec, lgroup, lnext, lpart, lhead, lcentre, lused;  // learned-correction records
-    DevBuf gscale;                    // PT_BH_RELATIVE: 1 / (alpha |a|) per group
+    DevBuf gscale, gorder;            // PT_BH_RELATIVE: 1 / (alpha |a|) per group, groups by it
     int lcap = 0;                     // record chunks allocated
     int lcap_fixed = 0;               // > 0: record chunks fixed by pt_bh_set_learned_capacity
     int stack_cap = 0;                // group-walk stack ranges per warp in use (0 = all)

@@ -492,7 +492,8 @@ __global__ void __launch_bounds__(32 * W, (LOCAL ? PT_GW_LMINB : PT_GW_MINB) * 4
                   const float4 *__restrict__ nodeG, const float4 *__restrict__ sbody, const int *__restrict__ counters,
                   float th2, float th_in2, LearnedRecords LR, float eps2, float *__restrict__ out,
                   unsigned long long *__restrict__ stats, int *__restrict__ err, int stack_cap,
-                  float local_ratio, const float *__restrict__ gscale, float mono_beta) {
+                  float local_ratio, const float *__restrict__ gscale, float mono_beta,
+                  const int *__restrict__ gorder) {
     after_previous();
     static_assert(!(LEARNED && LOCAL), "PT_BH_LEARNED and PT_BH_LOCAL are exclusive");
     static_assert(!(LEARNED && REL), "PT_BH_LEARNED and PT_BH_RELATIVE are exclusive");
@@ -523,7 +524,7 @@ __global__ void __launch_bounds__(32 * W, (LOCAL ? PT_GW_LMINB : PT_GW_MINB) * 4
     __shared__ __align__(16) Shared s_warp[W];
     __shared__ int s_push[W];
     const int warp = W > 1 ? threadIdx.x >> 5 : 0, lane = threadIdx.x & 31;
-    const int group = blockIdx.x;
+    const int group = REL && gorder ? gorder[blockIdx.x] : blockIdx.x;
     const int g0 = group * GW_GROUP;
     if (g0 >= n_aff) return;
     Shared &my = s_warp[warp];
@@ -1049,7 +1050,7 @@ __global__ void __launch_bounds__(32 * W, (LOCAL ? PT_GW_LMINB : PT_GW_MINB) * 4
 
 using GroupKernel = void (*)(const float4 *, const uint32_t *, int, const float4 *, const int4 *, const float4 *,
                              const float4 *, const float4 *, const int *, float, float, LearnedRecords, float,
-                             float *, unsigned long long *, int *, int, float, const float *, float);
+                             float *, unsigned long long *, int *, int, float, const float *, float, const int *);
 
 template <bool LEARNED, bool LOCAL, bool REL, int W>
 inline GroupKernel group_kernel_q(bool quad, bool guard) {

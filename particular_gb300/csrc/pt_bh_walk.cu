@@ -126,6 +126,12 @@ __device__ __forceinline__ void scale_cursor_walk(float cx, float cy, float cz, 
     }
 }
 
+// Two octaves of the scale (positive, or infinite) to a bucket, the largest first.
+static_assert(ORDER_BUCKETS == 128, "a float's sign and upper exponent bits");
+__device__ __forceinline__ int order_bucket(float scale) {
+    return ORDER_BUCKETS - 1 - ((__float_as_int(scale) & 0x7fffffff) >> 24);
+}
+
 // One thread per group: the group's box, then the cursor walk from its centre. (One
 // warp per group walking with a range stack, one node per lane and pop, was slower at
 // N = 4M: the walk phase, which includes this kernel, went from 5.68 to 5.85 ms. Its
@@ -135,13 +141,15 @@ __device__ __forceinline__ void scale_cursor_walk(float cx, float cy, float cz, 
 // own octant holds most of the visits. Four lanes per group popping up to four ranges
 // of a shared-memory stack per step took 0.18 ms: a walk from one point keeps few
 // ranges open, so the steps stayed nearly as many and each cost more.)
+// buckets: null, or counts the groups by order_bucket.
 __global__ void __launch_bounds__(128)
     bh_group_scale(const float4 *__restrict__ tbody, int n_aff, const float4 *__restrict__ nodeA,
                    const int4 *__restrict__ nodeB, const int *__restrict__ counters, float eps2, float alpha,
-                   float *__restrict__ gscale) {
+                   float *__restrict__ gscale, unsigned *__restrict__ buckets) {
     after_previous();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int g0 = g * GW_GROUP;
+    const unsigned active = __ballot_sync(0xffffffffu, g0 < n_aff);
     if (g0 >= n_aff) return;
     const int g1 = min(n_aff, g0 + GW_GROUP);
     float4 p = tbody[g0];
@@ -155,7 +163,51 @@ __global__ void __launch_bounds__(128)
     scale_cursor_walk(0.5f * (mn0 + mx0), 0.5f * (mn1 + mx1), 0.5f * (mn2 + mx2), nodeA, nodeB, counters[1], eps2,
                       ax, ay, az);
     const float a = sqrtf(fmaf(ax, ax, fmaf(ay, ay, az * az)));
-    gscale[g] = 1.f / (alpha * fmaxf(a, 1e-30f));
+    const float s = 1.f / (alpha * fmaxf(a, 1e-30f));
+    gscale[g] = s;
+    if (!buckets) return;
+    __syncwarp(active);
+    const int b = order_bucket(s);
+    const unsigned peers = __match_any_sync(active, b);
+    if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(buckets + b, __popc(peers));
+}
+
+// The groups by descending scale, for the walk to take them in: a group whose error bound is
+// small next to its forces opens the most cells (rank correlation with its walk 0.75), and one
+// that starts last holds up the call. Within a bucket they stay about in key order, so that
+// neighbours still share what they read. Whole call in key order and so ordered, us: N = 262144
+// KA / KB, 524288 KC / KD, 1048576 KE / KF, 4194304 KG / KH. While all groups start at once there is nothing to order.
+__global__ void __launch_bounds__(256)
+    bh_group_order(const float *__restrict__ gscale, int groups, unsigned *__restrict__ buckets,
+                   int *__restrict__ gorder) {
+    after_previous();
+    __shared__ unsigned first[ORDER_BUCKETS], wsum[4];
+    const int t = threadIdx.x, lane = t & 31, i = blockIdx.x * blockDim.x + t;
+    unsigned c = 0, incl = 0;
+    if (t < ORDER_BUCKETS) {
+        c = incl = buckets[t];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31) wsum[t >> 5] = incl;
+    }
+    __syncthreads();
+    if (t < ORDER_BUCKETS) {
+        for (int w = 0; w < t >> 5; ++w) incl += wsum[w];
+        first[t] = incl - c;
+    }
+    __syncthreads();
+    const unsigned active = __ballot_sync(0xffffffffu, i < groups);
+    if (i >= groups) return;
+    const int b = order_bucket(gscale[i]);
+    const unsigned peers = __match_any_sync(active, b);
+    const int leader = __ffs(peers) - 1;
+    unsigned at = 0;
+    if (lane == leader) at = atomicAdd(buckets + ORDER_BUCKETS + b, __popc(peers));
+    at = __shfl_sync(peers, at, leader);
+    gorder[first[b] + at + __popc(peers & ((1u << lane) - 1u))] = i;
 }
 
 // ---- masked group walk: the reference's rule, per body, with shared traversal ----
@@ -932,8 +984,8 @@ static MaskedPlan masked_plan(const pt_ctx *ctx, int n_aff) {
 
 int ensure_counters(pt_ctx *ctx, State &S) {
     if (S.counters.ptr) return PT_OK;
-    PT_TRY(ensure_buf(ctx, S.counters, sizeof(unsigned long long) * 16));
-    PT_CUDA(cudaMemsetAsync(S.counters.ptr, 0, sizeof(unsigned long long) * 16, ctx->stream));
+    PT_TRY(ensure_buf(ctx, S.counters, COUNTER_BYTES));
+    PT_CUDA(cudaMemsetAsync(S.counters.ptr, 0, COUNTER_BYTES, ctx->stream));
     return PT_OK;
 }
 
@@ -1042,13 +1094,24 @@ int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n
             else if (S.lcap == 0) S.lcap = std::max(1024, 2 * groups);
         }
         const float *gscale = nullptr;
+        const int *gorder = nullptr;
         if (flags & PT_BH_RELATIVE) {
             PT_TRY(ensure_buf(ctx, S.gscale, sizeof(float) * size_t(groups)));
+            unsigned *buckets = nullptr;
+            if (groups > 20 * std::max(1, ctx->sm_count)) {  // more than start at once
+                PT_TRY(ensure_buf(ctx, S.gorder, sizeof(int) * size_t(groups)));
+                buckets = reinterpret_cast<unsigned *>(as<int>(S.counters) + 32);
+            }
             launch_next(bh_group_scale, blocks(groups, 128), 128, 0, st, tbody, n_aff, as<float4>(S.nodeA), as<int4>(S.nodeB),
                                                                 as<int>(S.counters), eps2, S.rel_alpha,
-                                                                as<float>(S.gscale));
+                                                                as<float>(S.gscale), buckets);
             PT_TRY(check_launch(ctx, "bh_group_scale"));
             gscale = as<float>(S.gscale);
+            if (buckets) {
+                launch_next(bh_group_order, blocks(groups), 256, 0, st, gscale, groups, buckets, as<int>(S.gorder));
+                PT_TRY(check_launch(ctx, "bh_group_order"));
+                gorder = as<int>(S.gorder);
+            }
         }
         for (int attempt = 0;; ++attempt) {
             if (learned) {
@@ -1065,7 +1128,7 @@ int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n
                 group_kernel(quad, eps2 == 0.0f, learned, flags & PT_BH_LOCAL, gscale != nullptr, team), groups,
                 32 * team, 0, st, tbody, tidx, n_aff, as<float4>(S.nodeA), as<int4>(S.nodeB), as<float4>(S.nodeQ), as<float4>(S.nodeG),
                 as<float4>(S.sbody), as<int>(S.counters), th2, S.theta_inner * S.theta_inner, LR, eps2, d_out, stats,
-                err, S.stack_cap > 0 ? S.stack_cap : INT_MAX, S.local_ratio, gscale, S.rel_mono);
+                err, S.stack_cap > 0 ? S.stack_cap : INT_MAX, S.local_ratio, gscale, S.rel_mono, gorder);
             PT_TRY(check_launch(ctx, "bh_walk_group"));
             // Outside stream capture (and with the automatic capacity) the record count
             // is checked and the walk rerun with room for all records; otherwise an
