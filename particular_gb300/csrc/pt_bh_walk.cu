@@ -176,7 +176,8 @@ __global__ void __launch_bounds__(128)
 // small next to its forces opens the most cells (rank correlation with its walk 0.75), and one
 // that starts last holds up the call. Within a bucket they stay about in key order, so that
 // neighbours still share what they read. Whole call in key order and so ordered, us: N = 262144
-// KA / KB, 524288 KC / KD, 1048576 KE / KF, 4194304 KG / KH. While all groups start at once there is nothing to order.
+// 974 / 872, 524288 1513 / 1209, 1048576 1824 / 1825, 2097152 3880 / 3290, 4194304 6008 / 6020.
+// While all groups start at once there is nothing to order.
 __global__ void __launch_bounds__(256)
     bh_group_order(const float *__restrict__ gscale, int groups, unsigned *__restrict__ buckets,
                    int *__restrict__ gorder) {

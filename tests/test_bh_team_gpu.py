@@ -41,3 +41,25 @@ def test_team_sizes_agree(res, kw, soft):
     scale = np.linalg.norm(want, axis=1) + np.median(np.linalg.norm(want, axis=1))
     for out in got.values():
         assert (np.linalg.norm(out - want, axis=1) <= 2e-6 * scale).all()
+
+
+@pytest.mark.parametrize("kw", [{}, {"quadrupole": True}, {"quadrupole": True, "local": True}])
+def test_order_of_the_groups_does_not_show(res, kw):
+    """From 20 groups per SM on the error-bound walk takes them by their scale; every group
+    keeps its accelerations, to the bit, and none is left out."""
+    r = np.random.RandomState(5)
+    src = scattered(r, 30000, -1, 1, 1 / 30000)
+    src[0, :3], src[1, :3] = -1, 1
+    tgt = src[src[:, 0] < -0.05][:3200]
+    m = cuda.BarnesHut(0.7, res, AccelerationSoftened(0.01), group=True, relative=2.5e-3, **kw)
+    tree = m.build(src)
+    sms = res.sm_count
+    want = None
+    for groups, last in ((20 * sms, 64), (20 * sms + 1, 64), (20 * sms + 257, 1)):
+        more = scattered(r, 64 * (groups - 51) + last, 0.1, 1, 0)
+        more[::3, :3] *= 1000.0 / more[::3, :3].max()  # far outside the box: scales of many octaves
+        out = m.compute(Between(np.concatenate([tgt, more]), tree))
+        assert m.stats()["warps"] == groups
+        assert np.isfinite(out).all() and (out != 0).any(1).all()
+        want = out[:3200] if want is None else want
+        assert np.array_equal(out[:3200].view(np.uint32), want.view(np.uint32))
