@@ -123,6 +123,7 @@ int sort_targets(pt_ctx *ctx, State &S, const float4 *d_aff, int n);
 // walks (pt_bh_walk.cu)
 int ensure_counters(pt_ctx *ctx, State &S);
 int clear_errors(pt_ctx *ctx, State &S);
+inline unsigned *order_buckets(State &S) { return static_cast<unsigned *>(S.counters.ptr) + 32; }
 int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n_aff, float theta,
          float softening, uint32_t flags, float *d_out);
 int run(pt_ctx *ctx, const float4 *d_aff, int n_aff, const float4 *d_src, int n_src, float theta, float softening,

@@ -524,9 +524,9 @@ __global__ void __launch_bounds__(32 * W, (LOCAL ? PT_GW_LMINB : PT_GW_MINB) * 4
     __shared__ __align__(16) Shared s_warp[W];
     __shared__ int s_push[W];
     const int warp = W > 1 ? threadIdx.x >> 5 : 0, lane = threadIdx.x & 31;
-    const int group = REL && gorder ? gorder[blockIdx.x] : blockIdx.x;
+    const int group = gorder ? gorder[blockIdx.x] : blockIdx.x;
     const int g0 = group * GW_GROUP;
-    if (g0 >= n_aff) return;
+    if (unsigned(g0) >= unsigned(n_aff)) return;
     Shared &my = s_warp[warp];
     // this lane's targets: g0 + lane, g0 + 32 + lane, ...
     float4 p[TPL];

@@ -172,10 +172,11 @@ __global__ void __launch_bounds__(128)
     if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(buckets + b, __popc(peers));
 }
 
-// The groups by descending scale, for the walk to take them in: a group whose error bound is
-// small next to its forces opens the most cells (rank correlation with its walk 0.75), and one
-// that starts last holds up the call. Within a bucket they stay about in key order, so that
-// neighbours still share what they read. Whole call in key order and so ordered, us: N = 262144
+// The groups by descending key, for the walk to take them in: one that opens many cells and
+// starts last holds up the call. In the error-bound walk the key is the group's scale: one whose
+// error bound is small next to its forces opens the most (rank correlation with its walk 0.75).
+// Within a bucket they stay about in tree order, so that neighbours still share what they read.
+// Whole error-bound call in tree order and so ordered, us: N = 262144
 // 974 / 872, 524288 1513 / 1209, 1048576 1824 / 1825, 2097152 3880 / 3290, 4194304 6008 / 6020.
 // While all groups start at once there is nothing to order.
 __global__ void __launch_bounds__(256)
@@ -208,7 +209,61 @@ __global__ void __launch_bounds__(256)
     unsigned at = 0;
     if (lane == leader) at = atomicAdd(buckets + ORDER_BUCKETS + b, __popc(peers));
     at = __shfl_sync(peers, at, leader);
-    gorder[first[b] + at + __popc(peers & ((1u << lane) - 1u))] = i;
+    const unsigned pos = first[b] + at + __popc(peers & ((1u << lane) - 1u));
+    if (pos < unsigned(groups)) gorder[pos] = i;  // (always: the buckets are cleared before they count)
+}
+
+// The key of the walks by opening angle: a group's squared width over its squared distance from
+// the root's centre of mass, the angle under which the mass sees it (rank correlation with the
+// walk 0.57 to 0.68; of the longest 5 % of the walks, 74 to 90 % are in the first fifth). Whole
+// call in tree order and so ordered, us: masked N = 131072 theta 0.8 347 / 334, N = 262144 theta
+// 0.5 1018 / 964, N = 1M 3226 / 3170; group walk N = 262144 theta 0.6 725 / 699, N = 524288 with
+// local expansions 1435 / 1319, N = 1M 3000 / 2930. (The error-bound walk by this key: N = 1M
+// 1825 -> 1739, 4M 6015 -> 6127.)
+__global__ void __launch_bounds__(256)
+    bh_group_width(const float4 *__restrict__ tbody, int n_aff, int groups, int size,
+                   const float4 *__restrict__ nodeA, float *__restrict__ ratio, unsigned *__restrict__ buckets) {
+    after_previous();
+    __shared__ unsigned cnt[ORDER_BUCKETS];
+    for (int i = threadIdx.x; i < ORDER_BUCKETS; i += blockDim.x) cnt[i] = 0;
+    __syncthreads();
+    const int lanes = min(32, size);  // a power of two
+    const float4 root = nodeA[0];
+    const int step = gridDim.x * blockDim.x / lanes;
+    const int l = threadIdx.x % lanes;
+    const int rounds = (groups + step - 1) / step;
+    int g = (blockIdx.x * blockDim.x + threadIdx.x) / lanes;
+    for (int r = 0; r < rounds; ++r, g += step) {  // as many for every thread: the shuffles need the warp
+        float mn0 = INFINITY, mn1 = INFINITY, mn2 = INFINITY, mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY;
+        if (g < groups)
+            for (int t = g * size + l; t < min(n_aff, (g + 1) * size); t += lanes) {
+                const float4 p = tbody[t];
+                mn0 = fminf(mn0, p.x), mn1 = fminf(mn1, p.y), mn2 = fminf(mn2, p.z);
+                mx0 = fmaxf(mx0, p.x), mx1 = fmaxf(mx1, p.y), mx2 = fmaxf(mx2, p.z);
+            }
+        for (int o = lanes / 2; o > 0; o >>= 1) {
+            mn0 = fminf(mn0, __shfl_xor_sync(0xffffffffu, mn0, o));
+            mn1 = fminf(mn1, __shfl_xor_sync(0xffffffffu, mn1, o));
+            mn2 = fminf(mn2, __shfl_xor_sync(0xffffffffu, mn2, o));
+            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
+            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
+            mx2 = fmaxf(mx2, __shfl_xor_sync(0xffffffffu, mx2, o));
+        }
+        if (l == 0 && g < groups) {
+            const float w0 = mx0 - mn0, w1 = mx1 - mn1, w2 = mx2 - mn2;
+            const float d0 = 0.5f * (mn0 + mx0) - root.x, d1 = 0.5f * (mn1 + mx1) - root.y,
+                        d2 = 0.5f * (mn2 + mx2) - root.z;
+            const float s = fmaf(w0, w0, fmaf(w1, w1, w2 * w2)) / fmaf(d0, d0, fmaf(d1, d1, d2 * d2));
+            // two buckets an octave from 2^-20 to 2^12, as order_bucket takes two octaves
+            const float q = fminf(fmaxf(s, 9.5367431640625e-7f), 4096.f);
+            const float key = __int_as_float(((__float_as_int(q) - 0x35800000) >> 22) << 24);
+            ratio[g] = key;
+            atomicAdd(&cnt[order_bucket(key)], 1u);
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < ORDER_BUCKETS; i += blockDim.x)
+        if (cnt[i]) atomicAdd(buckets + i, cnt[i]);
 }
 
 // ---- masked group walk: the reference's rule, per body, with shared traversal ----
@@ -634,7 +689,7 @@ __device__ __forceinline__ void
 // the end.
 template <bool QUAD, int BIG, int SMALL>
 __global__ void __launch_bounds__(32)
-    bh_walk_masked(int big_groups, const float4 *__restrict__ tbody, const uint32_t *__restrict__ tidx, int n_aff,
+    bh_walk_masked(int big_groups, const int *__restrict__ order, const float4 *__restrict__ tbody, const uint32_t *__restrict__ tidx, int n_aff,
                    const float4 *__restrict__ nodeA, const int4 *__restrict__ nodeB,
                    const float4 *__restrict__ nodeQ, const float4 *__restrict__ sbody,
                    const int *__restrict__ counters, float th2, float eps2, float *__restrict__ out,
@@ -647,12 +702,14 @@ __global__ void __launch_bounds__(32)
     } Sh;
     const int b = blockIdx.x;
     if (BIG == SMALL || b < big_groups) {
-        if (b * BIG < n_aff)
-            walk_masked<QUAD, BIG>(Sh.big, b * BIG, tbody, tidx, n_aff, nodeA, nodeB, nodeQ, sbody, counters, th2, eps2,
+        const int g0 = (order ? order[b] : b) * BIG;
+        if (unsigned(g0) < unsigned(n_aff))
+            walk_masked<QUAD, BIG>(Sh.big, g0, tbody, tidx, n_aff, nodeA, nodeB, nodeQ, sbody, counters, th2, eps2,
                                    out, stats);
     } else {
-        const int g0 = big_groups * BIG + (b - big_groups) * SMALL;
-        if (g0 < n_aff)
+        const int half = b - big_groups, whole = big_groups + (half >> 1);
+        const int g0 = (order ? order[whole] : whole) * BIG + (half & 1) * SMALL;
+        if (unsigned(g0) < unsigned(n_aff))
             walk_masked<QUAD, SMALL>(Sh.small, g0, tbody, tidx, n_aff, nodeA, nodeB, nodeQ, sbody, counters, th2, eps2,
                                      out, stats);
     }
@@ -928,7 +985,7 @@ __global__ void __launch_bounds__(32)
 }
 
 
-using WalkKernel = void (*)(int, const float4 *, const uint32_t *, int, const float4 *, const int4 *, const float4 *,
+using WalkKernel = void (*)(int, const int *, const float4 *, const uint32_t *, int, const float4 *, const int4 *, const float4 *,
                             const float4 *, const int *, float, float, float *, unsigned long long *);
 template <bool QUAD>
 static WalkKernel masked_kernel_q(int big) {
@@ -964,9 +1021,9 @@ static int team_of(const pt_ctx *ctx, int groups) {
 // / 392; N = 65536 theta 0.7 422 / 372 / 379 / 424; N = 262144 theta 0.5 1208 / 1163 / 1389 /
 // 1829; N = 524288 theta 0.8 1034 / 1027 / 1229 / 1653; N = 1M theta 0.5 3686 / 3759 / 4796 /
 // 6834.
-// The last groups, half a wave of 64 bodies or a quarter of one of 32, are walked in halves,
-// so that the warps that end last are short (whole / halves: N = 262144 theta 0.5 1091 / 1064
-// us; N = 800000 theta 0.6 1929 / 1883; N = 1M theta 0.5 3409 / 3292).
+// The last five groups per SM are walked in halves, so that the warps that end last are short
+// (whole call without, 5 and 10 per SM, us: N = 131072 theta 0.8 339 / 333 / 347; N = 262144
+// theta 0.5 970 / 963 / 979; N = 1M theta 0.5 3192 / 3170 / 3182).
 struct MaskedPlan {
     int big, big_groups, small_groups;  // bodies per warp of the first groups (then half of it from 32 on)
 };
@@ -976,10 +1033,9 @@ static MaskedPlan masked_plan(const pt_ctx *ctx, int n_aff) {
     MaskedPlan p{};
     p.big = n_aff <= 8 * 20 * sms ? 8 : n_aff <= 16 * 27 * sms ? 16 : n_aff <= 32 * 110 * sms ? 32 : 64;
     const int all = (n_aff + p.big - 1) / p.big;
-    const int halved = p.big == 64 ? int(10 * sms) : p.big == 32 ? int(5 * sms) : 0;
+    const int halved = p.big >= 32 ? int(5 * sms) : 0;
     p.big_groups = std::max(0, all - halved);
-    p.small_groups = (std::max(0, n_aff - p.big_groups * p.big) + p.big / 2 - 1) / (p.big / 2);
-    if (!halved) p.small_groups = 0;
+    p.small_groups = halved ? 2 * (all - p.big_groups) : 0;
     return p;
 }
 
@@ -996,6 +1052,29 @@ int clear_errors(pt_ctx *ctx, State &S) {
     PT_TRY(ensure_counters(ctx, S));
     if (!ctx->keep_errors) PT_CUDA(cudaMemsetAsync(as<int>(S.counters) + 3, 0, sizeof(int), ctx->stream));
     return PT_OK;
+}
+
+// The order of the groups whose keys are in S.gscale and counted in the buckets.
+static int place_groups(pt_ctx *ctx, State &S, int groups, const int **order) {
+    PT_TRY(ensure_buf(ctx, S.gorder, sizeof(int) * size_t(groups)));
+    launch_next(bh_group_order, blocks(groups), 256, 0, ctx->stream, as<float>(S.gscale), groups, order_buckets(S),
+                as<int>(S.gorder));
+    *order = as<int>(S.gorder);
+    return check_launch(ctx, "bh_group_order");
+}
+
+// The order of groups of `size` bodies by width over distance, or null while all start at once:
+// from 24 a SM on (20 or 24 are resident; N = 50000, 3125 groups of 16, took 237 us without and
+// 240 with it, N = 65536, 4096 groups, 266 and 265).
+static int order_groups(pt_ctx *ctx, State &S, const float4 *tbody, int n_aff, int size, const int **order) {
+    const int sms = std::max(1, ctx->sm_count), groups = (n_aff + size - 1) / size;
+    *order = nullptr;
+    if (groups <= 24 * sms) return PT_OK;
+    PT_TRY(ensure_buf(ctx, S.gscale, sizeof(float) * size_t(groups)));
+    launch_next(bh_group_width, std::min(2 * sms, blocks(groups * std::min(32, size))), 256, 0, ctx->stream, tbody,
+                n_aff, groups, size, as<float4>(S.nodeA), as<float>(S.gscale), order_buckets(S));
+    PT_TRY(check_launch(ctx, "bh_group_width"));
+    return place_groups(ctx, S, groups, order);
 }
 
 int run(pt_ctx *ctx, const float4 *d_aff, int n_aff, const float4 *d_src, int n_src, float theta,
@@ -1098,21 +1177,15 @@ int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n
         const int *gorder = nullptr;
         if (flags & PT_BH_RELATIVE) {
             PT_TRY(ensure_buf(ctx, S.gscale, sizeof(float) * size_t(groups)));
-            unsigned *buckets = nullptr;
-            if (groups > 20 * std::max(1, ctx->sm_count)) {  // more than start at once
-                PT_TRY(ensure_buf(ctx, S.gorder, sizeof(int) * size_t(groups)));
-                buckets = reinterpret_cast<unsigned *>(as<int>(S.counters) + 32);
-            }
-            launch_next(bh_group_scale, blocks(groups, 128), 128, 0, st, tbody, n_aff, as<float4>(S.nodeA), as<int4>(S.nodeB),
-                                                                as<int>(S.counters), eps2, S.rel_alpha,
-                                                                as<float>(S.gscale), buckets);
+            const bool ordered = groups > 20 * std::max(1, ctx->sm_count);  // more than start at once
+            launch_next(bh_group_scale, blocks(groups, 128), 128, 0, st, tbody, n_aff, as<float4>(S.nodeA),
+                        as<int4>(S.nodeB), as<int>(S.counters), eps2, S.rel_alpha, as<float>(S.gscale),
+                        ordered ? order_buckets(S) : nullptr);
             PT_TRY(check_launch(ctx, "bh_group_scale"));
             gscale = as<float>(S.gscale);
-            if (buckets) {
-                launch_next(bh_group_order, blocks(groups), 256, 0, st, gscale, groups, buckets, as<int>(S.gorder));
-                PT_TRY(check_launch(ctx, "bh_group_order"));
-                gorder = as<int>(S.gorder);
-            }
+            if (ordered) PT_TRY(place_groups(ctx, S, groups, &gorder));
+        } else {
+            PT_TRY(order_groups(ctx, S, tbody, n_aff, GW_GROUP, &gorder));
         }
         for (int attempt = 0;; ++attempt) {
             if (learned) {
@@ -1157,8 +1230,10 @@ int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n
     }
     const MaskedPlan p = masked_plan(ctx, n_aff);
     auto kern = quad ? masked_kernel_q<true>(p.big) : masked_kernel_q<false>(p.big);
+    const int *order = nullptr;
+    PT_TRY(order_groups(ctx, S, tbody, n_aff, p.big, &order));
     launch_next(
-        kern, p.big_groups + p.small_groups, 32, 0, st, p.big_groups, tbody, tidx, n_aff, as<float4>(S.nodeA), as<int4>(S.nodeB), as<float4>(S.nodeQ), as<float4>(S.sbody),
+        kern, p.big_groups + p.small_groups, 32, 0, st, p.big_groups, order, tbody, tidx, n_aff, as<float4>(S.nodeA), as<int4>(S.nodeB), as<float4>(S.nodeQ), as<float4>(S.sbody),
         as<int>(S.counters), th2, eps2, d_out, stats);
     PT_TRY(check_launch(ctx, "bh_walk_masked"));
     mark(ctx, 2);

@@ -43,23 +43,48 @@ def test_team_sizes_agree(res, kw, soft):
         assert (np.linalg.norm(out - want, axis=1) <= 2e-6 * scale).all()
 
 
-@pytest.mark.parametrize("kw", [{}, {"quadrupole": True}, {"quadrupole": True, "local": True}])
+@pytest.mark.parametrize("kw", [{"relative": 2.5e-3}, {"quadrupole": True, "relative": 2.5e-3},
+                                {"quadrupole": True, "local": True, "relative": 2.5e-3}, {},
+                                {"quadrupole": True, "local": True}])
 def test_order_of_the_groups_does_not_show(res, kw):
-    """From 20 groups per SM on the error-bound walk takes them by their scale; every group
-    keeps its accelerations, to the bit, and none is left out."""
+    """From 20 groups per SM on (24 without an error bound) the walk takes them by how much each
+    is likely to open; every group keeps its accelerations, to the bit, and none is left out."""
     r = np.random.RandomState(5)
     src = scattered(r, 30000, -1, 1, 1 / 30000)
     src[0, :3], src[1, :3] = -1, 1
     tgt = src[src[:, 0] < -0.05][:3200]
-    m = cuda.BarnesHut(0.7, res, AccelerationSoftened(0.01), group=True, relative=2.5e-3, **kw)
+    m = cuda.BarnesHut(0.7, res, AccelerationSoftened(0.01), group=True, **kw)
     tree = m.build(src)
-    sms = res.sm_count
+    turn = (20 if "relative" in kw else 24) * res.sm_count
     want = None
-    for groups, last in ((20 * sms, 64), (20 * sms + 1, 64), (20 * sms + 257, 1)):
+    for groups, last in ((turn, 64), (turn + 1, 64), (turn + 257, 1)):
         more = scattered(r, 64 * (groups - 51) + last, 0.1, 1, 0)
-        more[::3, :3] *= 1000.0 / more[::3, :3].max()  # far outside the box: scales of many octaves
+        more[::3, :3] *= 1000.0 / more[::3, :3].max()  # far outside the box: keys of many octaves
         out = m.compute(Between(np.concatenate([tgt, more]), tree))
         assert m.stats()["warps"] == groups
         assert np.isfinite(out).all() and (out != 0).any(1).all()
         want = out[:3200] if want is None else want
         assert np.array_equal(out[:3200].view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("quadrupole", [False, True])
+def test_order_of_the_masked_walk_does_not_show(res, quadrupole):
+    """The same for the reference's rule: 16 bodies a warp in tree order and by width, 32 and 64
+    by width with the last ones in halves."""
+    r = np.random.RandomState(6)
+    src = scattered(r, 30000, -1, 1, 1 / 30000)
+    src[0, :3], src[1, :3] = -1, 1
+    tgt = src[src[:, 0] < -0.05][:3200]
+    m = cuda.BarnesHut(0.7, res, AccelerationSoftened(0.01), quadrupole=quadrupole)
+    tree = m.build(src)
+    want = None
+    for n in (24 * 16 * res.sm_count, 24 * 16 * res.sm_count + 1, 24 * 32 * res.sm_count + 31,
+              110 * 32 * res.sm_count + 1):
+        more = scattered(r, n - 3200, 0.1, 1, 0)
+        more[::3, :3] *= 1000.0 / more[::3, :3].max()
+        out = m.compute(Between(np.concatenate([tgt, more]), tree))
+        assert np.isfinite(out).all() and (out != 0).any(1).all()
+        got, want = out[:3200].astype(np.float64), out[:3200].astype(np.float64) if want is None else want
+        # the same nodes, added in another order: compensated sums
+        scale = np.linalg.norm(want, axis=1) + np.median(np.linalg.norm(want, axis=1))
+        assert (np.linalg.norm(got - want, axis=1) <= 2e-6 * scale).all()
