@@ -811,6 +811,7 @@ __global__ void __launch_bounds__(32)
     after_previous();
     __shared__ int4 stack[W64_STACK];
     __shared__ List64 Lst;
+    __shared__ float4 vote[64];
     const int lane = threadIdx.x;
     const int group = blockIdx.x;
     constexpr int BODIES = 32 / LPB;
@@ -831,6 +832,14 @@ __global__ void __launch_bounds__(32)
         mx1 = fmax(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
         mx2 = fmax(mx2, __shfl_xor_sync(0xffffffffu, mx2, o));
     }
+    // for the votes: this lane's body and the farthest one about the box's centre, in FP32
+    const double g0 = 0.5 * (mn0 + mx0), g1 = 0.5 * (mn1 + mx1), g2 = 0.5 * (mn2 + mx2);
+    const float px = float(p.x - g0), py = float(p.y - g1), pz = float(p.z - g2);
+    float rg2 = fmaf(px, px, fmaf(py, py, pz * pz));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) rg2 = fmaxf(rg2, __shfl_xor_sync(0xffffffffu, rg2, o));
+    const float th2f = float(th2);
+    const bool th2_ok = th2 == 0.0 || th2f > 1e-30f;
     double ax = 0.0, ay = 0.0, az = 0.0;
     if (lane == 0) stack[0] = make_int4(0, T, int(valid_mask), 0);
     __syncwarp();
@@ -876,9 +885,40 @@ __global__ void __launch_bounds__(32)
             }
         }
         unsigned vm = __ballot_sync(0xffffffffu, need);
+        // Each node that the box left open is put to the bodies in FP32 first. With c and b the
+        // node and a body about the box's centre, rounded to 24 bits each, |c - b|^2 is off by
+        // less than 2^-20 (|c|^2 + |b|^2), its product with theta^2 by 2^-22 of the same more
+        // and w^2 by 2^-22 of itself (and by 1e-37 where they are denormal). Within twice that
+        // of the decision (or of zero distance, or where a product could overflow) all bodies
+        // decide in FP64, so that the accepted sets stay the reference's. A vote in FP64 keeps
+        // that pipe, two lane-operations a cycle, for a quarter of what a pair does: whole host
+        // call at N = 50021, theta 0.5, 6.15 -> 5.23 ms, 10000 at 0.6 1.20 -> 0.93.
+        if (need) {
+            const float cx = float(A.x - g0), cy = float(A.y - g1), cz = float(A.z - g2), wf = float(w);
+            const float c2 = fmaf(cx, cx, fmaf(cy, cy, cz * cz)) + rg2, lim = wf * wf;
+            const bool ok = th2_ok && c2 < 1e37f && lim < 1e37f;
+            vote[2 * lane] = make_float4(cx, cy, cz, cell ? lim : -1.f);
+            vote[2 * lane + 1] = make_float4(ok ? fmaf(c2, 0x1p-19f, 1e-36f) : INFINITY,
+                                             fmaf(fmaf(th2f, c2, lim), 0x1p-19f, fmaf(th2f, 1e-36f, 1e-36f)),
+                                             __uint_as_float(mask), 0.f);
+        }
+        __syncwarp();
         while (vm) {
             const int j = __ffs(vm) - 1;
             vm &= vm - 1;
+            const float4 v0 = vote[2 * j], v1 = vote[2 * j + 1];
+            const float fx = v0.x - px, fy = v0.y - py, fz = v0.z - pz;
+            const float f2 = fmaf(fx, fx, fmaf(fy, fy, fz * fz)), side = fmaf(th2f, f2, -v0.w);
+            const bool in = (__float_as_uint(v1.z) >> lane) & 1u;
+            const bool leaf = v0.w < 0.f;
+            if (__all_sync(0xffffffffu, !in || (f2 > v1.x && (leaf || fabsf(side) > v1.y)))) {
+                const unsigned om = __ballot_sync(0xffffffffu, in && !leaf && side < 0.f);
+                if (lane == j) {
+                    open_m = om;
+                    acc_m = mask & ~om;
+                }
+                continue;
+            }
             const double cx = __shfl_sync(0xffffffffu, A.x, j), cy = __shfl_sync(0xffffffffu, A.y, j);
             const double cz = __shfl_sync(0xffffffffu, A.z, j), cw = __shfl_sync(0xffffffffu, w, j);
             const unsigned mj = __shfl_sync(0xffffffffu, mask, j);
