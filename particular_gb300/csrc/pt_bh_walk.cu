@@ -832,12 +832,17 @@ __global__ void __launch_bounds__(32)
         mx1 = fmax(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
         mx2 = fmax(mx2, __shfl_xor_sync(0xffffffffu, mx2, o));
     }
-    // for the votes: this lane's body and the farthest one about the box's centre, in FP32
+    // for the decisions: this lane's body and the box's half widths about its centre, in FP32
     const double g0 = 0.5 * (mn0 + mx0), g1 = 0.5 * (mn1 + mx1), g2 = 0.5 * (mn2 + mx2);
     const float px = float(p.x - g0), py = float(p.y - g1), pz = float(p.z - g2);
-    float rg2 = fmaf(px, px, fmaf(py, py, pz * pz));
+    float h0 = fabsf(px), h1 = fabsf(py), h2 = fabsf(pz);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) rg2 = fmaxf(rg2, __shfl_xor_sync(0xffffffffu, rg2, o));
+    for (int o = 16; o > 0; o >>= 1) {
+        h0 = fmaxf(h0, __shfl_xor_sync(0xffffffffu, h0, o));
+        h1 = fmaxf(h1, __shfl_xor_sync(0xffffffffu, h1, o));
+        h2 = fmaxf(h2, __shfl_xor_sync(0xffffffffu, h2, o));
+    }
+    const float rg2 = fmaf(h0, h0, fmaf(h1, h1, h2 * h2));
     const float th2f = float(th2);
     const bool th2_ok = th2 == 0.0 || th2f > 1e-30f;
     double ax = 0.0, ay = 0.0, az = 0.0;
@@ -867,41 +872,41 @@ __global__ void __launch_bounds__(32)
         const bool cell = B.z < 0;
         unsigned open_m = 0, acc_m = 0;
         bool need = false;
+        // The box, then each node that it leaves open the bodies, decide in FP32. With c and b
+        // the node and a body (or a point of the box) about the box's centre, rounded to 24 bits
+        // each, |c - b|^2 is off by less than 2^-20 (|c|^2 + |b|^2), its product with theta^2 by
+        // 2^-22 of the same more and w^2 by 2^-22 of itself (and by 1e-37 where they are
+        // denormal). Within twice that of the decision (or of zero distance, or where a product
+        // could overflow) the bodies decide in FP64, so that the accepted sets stay the
+        // reference's. A vote in FP64 keeps that pipe, two lane-operations a cycle, for a
+        // quarter of what a pair does: whole host call at N = 50021, theta 0.5, 6.15 -> 5.23 ms,
+        // 10000 at 0.6 1.20 -> 0.93; the box in FP32 too: 4.86 and 0.79.
         if (have && mask) {
-            const double e0 = fmax(fmax(mn0 - A.x, A.x - mx0), 0.0);
-            const double e1 = fmax(fmax(mn1 - A.y, A.y - mx1), 0.0);
-            const double e2b = fmax(fmax(mn2 - A.z, A.z - mx2), 0.0);
-            const double db2 = __dadd_rn(__dadd_rn(__dmul_rn(e0, e0), __dmul_rn(e1, e1)), __dmul_rn(e2b, e2b));
-            if (!(db2 > 0.0)) {
-                need = true;
-            } else if (!cell || !(__dmul_rn(th2, db2) < __dmul_rn(w, w))) {
-                acc_m = mask;
-            } else {
-                const double f0 = fmax(A.x - mn0, mx0 - A.x), f1 = fmax(A.y - mn1, mx1 - A.y);
-                const double f2b = fmax(A.z - mn2, mx2 - A.z);
-                const double dm2 = __dadd_rn(__dadd_rn(__dmul_rn(f0, f0), __dmul_rn(f1, f1)), __dmul_rn(f2b, f2b));
-                if (__dmul_rn(th2, dm2) < __dmul_rn(w, w)) open_m = mask;
-                else need = true;
-            }
-        }
-        unsigned vm = __ballot_sync(0xffffffffu, need);
-        // Each node that the box left open is put to the bodies in FP32 first. With c and b the
-        // node and a body about the box's centre, rounded to 24 bits each, |c - b|^2 is off by
-        // less than 2^-20 (|c|^2 + |b|^2), its product with theta^2 by 2^-22 of the same more
-        // and w^2 by 2^-22 of itself (and by 1e-37 where they are denormal). Within twice that
-        // of the decision (or of zero distance, or where a product could overflow) all bodies
-        // decide in FP64, so that the accepted sets stay the reference's. A vote in FP64 keeps
-        // that pipe, two lane-operations a cycle, for a quarter of what a pair does: whole host
-        // call at N = 50021, theta 0.5, 6.15 -> 5.23 ms, 10000 at 0.6 1.20 -> 0.93.
-        if (need) {
             const float cx = float(A.x - g0), cy = float(A.y - g1), cz = float(A.z - g2), wf = float(w);
             const float c2 = fmaf(cx, cx, fmaf(cy, cy, cz * cz)) + rg2, lim = wf * wf;
             const bool ok = th2_ok && c2 < 1e37f && lim < 1e37f;
-            vote[2 * lane] = make_float4(cx, cy, cz, cell ? lim : -1.f);
-            vote[2 * lane + 1] = make_float4(ok ? fmaf(c2, 0x1p-19f, 1e-36f) : INFINITY,
-                                             fmaf(fmaf(th2f, c2, lim), 0x1p-19f, fmaf(th2f, 1e-36f, 1e-36f)),
-                                             __uint_as_float(mask), 0.f);
+            const float zero = ok ? fmaf(c2, 0x1p-19f, 1e-36f) : INFINITY;
+            const float line = fmaf(fmaf(th2f, c2, lim), 0x1p-19f, fmaf(th2f, 1e-36f, 1e-36f));
+            const float x0 = fabsf(cx), x1 = fabsf(cy), x2 = fabsf(cz);
+            const float n0 = fmaxf(x0 - h0, 0.f), n1 = fmaxf(x1 - h1, 0.f), n2 = fmaxf(x2 - h2, 0.f);
+            const float near2 = fmaf(n0, n0, fmaf(n1, n1, n2 * n2));
+            const float far2 = fmaf(x0 + h0, x0 + h0, fmaf(x1 + h1, x1 + h1, (x2 + h2) * (x2 + h2)));
+            need = true;
+            if (near2 > zero) {
+                if (!cell || fmaf(th2f, near2, -lim) > line) {
+                    acc_m = mask;
+                    need = false;
+                } else if (fmaf(th2f, far2, -lim) < -line) {
+                    open_m = mask;
+                    need = false;
+                }
+            }
+            if (need) {
+                vote[2 * lane] = make_float4(cx, cy, cz, cell ? lim : -1.f);
+                vote[2 * lane + 1] = make_float4(zero, line, __uint_as_float(mask), 0.f);
+            }
         }
+        unsigned vm = __ballot_sync(0xffffffffu, need);
         __syncwarp();
         while (vm) {
             const int j = __ffs(vm) - 1;
