@@ -626,7 +626,7 @@ __device__ __forceinline__ void exact_term(Row64 p, double xi, double yi, double
                                            double &ax, double &ay, double &az) {
     const double dx = __dsub_rn(p.x, xi), dy = __dsub_rn(p.y, yi), dz = __dsub_rn(p.z, zi);
     const double n = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-    if (checked && n == 0.0) {
+    if (checked && __double_as_longlong(n) == 0) {  // n is not -0; no compare on the FP64 pipe
         ax = dx;
         ay = dy;
         az = dz;
@@ -650,7 +650,7 @@ __device__ __forceinline__ double ord_add(double a, double b) { return __dadd_rn
 // Targets per block, warps that form terms (one more adds them up), sources per round.
 // Swept over 4-32 targets, 4-16 warps and 32-128 sources: these are fastest or within 3 %
 // at N = 4999, 10007 and 32768 (f32: 80 / 239 / 2210 us; 32 targets: 189 / 389 / 2641) and
-// at N = 1000 and 6007 (f64: 95 / 2404 us; 32 targets: 315 / 3692).
+// at N = 1000 and 6007 (f64: 95 / 2404 us then; 32 targets: 315 / 3692).
 constexpr int ORD_TG = 8;
 constexpr int ORD_WARPS = 8;
 constexpr int ORD_J = 64;
@@ -665,8 +665,8 @@ static_assert(32 % ORD_TG == 0 && 3 * ORD_TG <= 32, "one warp adds the terms");
 // A thread per target that does both waits on its own divide and square root for every
 // source (10 % of the issue slots at N = 10007, 13 % of the FP64 pipe at N = 6007): f32
 // N = 1024 / 10007 / 32768 took 119 / 1126 / 3882 us and take 14 / 239 / 2210; f64 N =
-// 1000 / 6007 took 1247 / 7485 and take 95 / 2404, where the FP64 pipe is the bound (about
-// 40 of its lane-operations a pair).
+// 1000 / 6007 took 1247 / 7485 and take 88 / 2230, where the FP64 pipe is the bound (some 35
+// of its lane-operations a pair; with the test for zero on it too 95 / 2301).
 template <class T, bool VEC3A>
 __global__ void __launch_bounds__(ORD_THREADS)
     bf_ordered(const T *__restrict__ aff, int n_aff, const T *__restrict__ src, int n_src, T soft2, int checked,

@@ -727,10 +727,17 @@ constexpr int W64_STACK = 384;
 // y^3 (1 + 3/2 e + 15/8 e^2). y has 24 bits, so y^2 is exact; |e| < 7e-7, so the series'
 // remainder is below 2^-60. The rounding errors left are those of the four operations that
 // the square root, product, divide form has too: against 80-bit values over 2e6 random pairs
-// 0.734 units of 2^-53 rms, where sqrt and divide give 0.735.
+// 0.734 units of 2^-53 rms, where sqrt and divide give 0.735. Conversions and compares run on
+// the integer pipe, by the bits: on the FP64 pipe they were 5 of a pair's 22 operations (whole
+// host call at N = 50021, theta 0.5, 4.86 -> 3.91 ms, 10000 at 0.6 0.79 -> 0.71).
 __device__ __forceinline__ double inv_cube64(double ns, double m) {
-    if (!(ns > 1e-36 && ns < 1e36)) return __ddiv_rn(m, __dmul_rn(ns, __dsqrt_rn(ns)));  // outside FP32's range
-    const double y = double(rsqrt_ftz(float(ns)));
+    const unsigned hi = __double2hiint(ns), lo = __double2loint(ns);
+    // 2^-119 <= ns < 2^119 by its exponent; outside FP32's range:
+    if (hi - ((1023u - 119u) << 20) >= (238u << 20)) return __ddiv_rn(m, __dmul_rn(ns, __dsqrt_rn(ns)));
+    // ns to FP32 (a half rounded up) and y back by their bits: the exponents differ by 896
+    const float nf = __uint_as_float(__funnelshift_l(lo, hi, 3) - (896u << 23) + ((lo >> 28) & 1u));
+    const unsigned yb = __float_as_uint(rsqrt_ftz(nf));
+    const double y = __hiloint2double((yb >> 3) + (896u << 20), yb << 29);
     const double y2 = y * y;
     const double e = fma(-ns, y2, 1.0);
     const double my3 = m * (y2 * y);
@@ -741,7 +748,7 @@ __device__ __forceinline__ void pair64(double px, double py, double pz, double c
                                        double eps2, double &ax, double &ay, double &az) {
     const double dx = cx - px, dy = cy - py, dz = cz - pz;
     const double n = fma(dx, dx, fma(dy, dy, dz * dz));
-    if (n == 0.0) return;  // checked: d itself, which is zero
+    if (__double_as_longlong(n) == 0) return;  // checked: d itself, which is zero (n is not -0)
     const double s = inv_cube64(n + eps2, m);
     ax = fma(dx, s, ax);
     ay = fma(dy, s, ay);
@@ -768,7 +775,7 @@ __device__ __forceinline__ unsigned transpose32(unsigned x) {
 }
 
 // Each lane evaluates its own body's accepted entries of the list, in list order. The pair
-// costs some 40 lane-operations of an FP64 pipe that does two a cycle, so a lane whose body
+// costs 17 lane-operations of an FP64 pipe that does two a cycle, so a lane whose body
 // does not accept an entry goes on to its own next entry instead of waiting for the lanes
 // whose bodies do: the list takes as many rounds as the body with the most accepted entries
 // has, not as many as it holds. (Entry by entry with the mask's lanes on, N = 50021 at theta
