@@ -786,7 +786,7 @@ __device__ __forceinline__ void eval_list64(const List64 &Lst, int cnt, double p
                                             double &ax, double &ay, double &az) {
     const int lane = threadIdx.x & 31;
     constexpr int WORDS = List64::CAP / 32;
-    constexpr unsigned share = LPB == 1 ? 0xffffffffu : LPB == 2 ? 0x55555555u : 0x11111111u;
+    constexpr unsigned share = 0xffffffffu / ((1u << LPB) - 1u);  // every LPB-th bit
     __syncwarp();
     unsigned w[WORDS];  // bit e of word k: this lane's body accepts entry 32 k + e
 #pragma unroll
@@ -1156,14 +1156,17 @@ int run(pt_ctx *ctx, const float4 *d_aff, int n_aff, const float4 *d_src, int n_
     return walk(ctx, S, tbody, tidx, n_aff, theta, softening, flags, d_out);
 }
 
-// Lanes that share a body in bh_walk64: as many as keep every warp resident at once (20 per
-// SM by registers). One warp of a small call is bound by its own FP64 latency, so more
-// warps, each with fewer list entries per lane, win until the chip is full (N = 5000 at
-// theta 0.6, host API, 1 / 2 / 4 lanes: 1995 / 1438 / 1207 us; N = 20000 2836 / 2327 / 2298);
-// beyond that they only repeat the traversal (N = 50021 at theta 0.9: 2458 / 2641 / 2934).
+// Lanes that share a body in bh_walk64. A warp of a small call is bound by its own FP64 latency,
+// so as many lanes, up to 16, as keep every warp resident at once (20 per SM by registers); once
+// the chip is full more lanes repeat the traversal but end more evenly. Whole host call, us, at
+// 1 / 2 / 4 / 8 / 16 lanes: N = 2000 theta 0.6 - / - / 445 / 373 / 329, 5000 1206 / 787 / 589 /
+// 500 / 462, 10000 1462 / 895 / 712 / 651 / 693, 20000 1806 / 1258 / 1101 / 1132 / 1204; N = 50021
+// theta 0.5 3918 / 3413 / 3370, theta 0.9 1423 / 1395 / 1416; N = 100000 theta 0.5 7258 / 6923 /
+// 6845, theta 0.9 2491 / 2407 / 2490; N = 300000 theta 0.7 10970 / 10961 / 11416; N = 1M theta
+// 0.9 22528 / 23063.
 static int lanes_per_body64(const pt_ctx *ctx, int n_aff) {
-    const long long slots = 20ll * std::max(1, ctx->sm_count) * 32;
-    return 4ll * n_aff <= slots ? 4 : 2ll * n_aff <= slots ? 2 : 1;
+    const long long slots = 20ll * std::max(1, ctx->sm_count) * 32, n = n_aff;
+    return 16 * n <= slots ? 16 : 8 * n <= slots ? 8 : 8 * n <= 5 * slots ? 4 : n <= 4 * slots ? 2 : 1;
 }
 
 // The f64 method: build over DVec3 bodies, walk with the reference rule in double.
@@ -1188,7 +1191,11 @@ int run64(pt_ctx *ctx, const double4_32a *d_aff, int n_aff, const double4_32a *d
     int *err = as<int>(S.counters) + 3;
     mark(ctx, 1);
     const int lpb = lanes_per_body64(ctx, n_aff);
-    auto kern = lpb == 4 ? bh_walk64<4> : lpb == 2 ? bh_walk64<2> : bh_walk64<1>;
+    auto kern = lpb == 16 ? bh_walk64<16>
+                : lpb == 8  ? bh_walk64<8>
+                : lpb == 4  ? bh_walk64<4>
+                : lpb == 2  ? bh_walk64<2>
+                            : bh_walk64<1>;
     launch_next(
         kern, (n_aff + 32 / lpb - 1) / (32 / lpb), 32, 0, st, tbody, tidx, n_aff, as<double4_32a>(S.nodeA64), as<int4>(S.nodeB), as<double4_32a>(S.nodeG64),
         as<double4_32a>(S.sbody64), as<int>(S.counters), theta * theta, softening * softening, d_out, stats, err);

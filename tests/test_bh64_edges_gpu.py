@@ -1,4 +1,4 @@
-"""The f64 Barnes-Hut walk where the number of lanes per body changes (4, 2, 1 by the number of
+"""The f64 Barnes-Hut walk where the number of lanes per body changes (16 to 1 by the number of
 targets), in a last warp that is not full, and with softened distances outside FP32's range."""
 import numpy as np
 import pytest
@@ -27,6 +27,22 @@ def test_walk_matches_reference(res, oracle, n_aff, scale):
     # terms cancel lose digits in both, so against the typical acceleration
     mag = np.linalg.norm(want, axis=1)
     assert (np.linalg.norm(got - want, axis=1) <= 1e-13 * np.maximum(mag, np.median(mag))).all()
+
+
+# 16, 8, 4, 2 and 1 lanes per body: the same accepted sets on either side of each turn
+@pytest.mark.parametrize("lanes", [16, 8, 4, 2])
+def test_lanes_per_body_agree(res, oracle, lanes):
+    slots = 20 * 32 * res.sm_count
+    turn = {16: slots // 16, 8: slots // 8, 4: 5 * slots // 8, 2: 4 * slots}[lanes]
+    src = cloud(300, 6)
+    aff = cloud(turn + 1, 7)
+    m = cuda.BarnesHut(0.7, res, AccelerationSoftened(0.0), dvec3=True)
+    want, acc = oracle.bh_dvec3(aff, src, 0.7, 0.0, True, accepted=True)
+    for n in (turn, turn + 1):
+        got = m.compute(Between(aff[:n], src))
+        assert m.stats()["interactions"] == int(acc[:n].sum())
+        mag = np.linalg.norm(want[:n], axis=1)
+        assert (np.linalg.norm(got - want[:n], axis=1) <= 1e-13 * np.maximum(mag, np.median(mag))).all()
 
 
 def accepted_pairs(g, b, theta):
