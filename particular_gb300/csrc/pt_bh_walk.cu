@@ -367,11 +367,11 @@ __device__ __forceinline__ void eval_list_masked(IList<NF + TPL, CAP> &Lst, int 
     __syncwarp();
 }
 
-// Shared memory of a warp that walks for `BODIES` bodies (64, 32, 16 or 8).
+// Shared memory of a warp that walks for `BODIES` bodies (64 to 2).
 template <bool QUAD, int BODIES>
 struct Masked {
     static constexpr int TPL = BODIES == 64 ? 2 : 1, LPB = BODIES >= 32 ? 1 : 32 / BODIES;
-    static_assert(32 * TPL / LPB == BODIES && LPB <= 4, "64, 32, 16 or 8 bodies");
+    static_assert(32 * TPL / LPB == BODIES && LPB <= 16, "64 to 2 bodies");
     static constexpr int NFC = QUAD ? 10 : 4;
     // (smaller lists with one body per lane, whose fewer registers leave room for more warps)
     static constexpr int CELLS = TPL == 1 ? 64 : PT_MW_CELLS, LEAVES = TPL == 1 ? 96 : PT_MW_BODIES;
@@ -1044,7 +1044,9 @@ static WalkKernel masked_kernel_q(int big) {
     return big == 64   ? bh_walk_masked<QUAD, 64, 32>
            : big == 32 ? bh_walk_masked<QUAD, 32, 16>
            : big == 16 ? bh_walk_masked<QUAD, 16, 16>
-                       : bh_walk_masked<QUAD, 8, 8>;
+           : big == 8  ? bh_walk_masked<QUAD, 8, 8>
+           : big == 4  ? bh_walk_masked<QUAD, 4, 4>
+                       : bh_walk_masked<QUAD, 2, 2>;
 }
 
 static GroupKernel group_kernel(bool quad, bool guard, bool learned, bool local, bool rel, int team) {
@@ -1065,8 +1067,10 @@ static int team_of(const pt_ctx *ctx, int groups) {
 }
 
 // Bodies per warp of the masked walk. A warp alone waits on its own loads and votes, so small
-// calls want many warps with little to evaluate in each: 8 or 16 bodies, 4 or 2 lanes to a
-// body, while these warps are (nearly) all resident at once, 20 per SM. 32 bodies, one to a lane,
+// calls want many warps with little to evaluate in each: 2 to 16 bodies, 16 to 2 lanes to a
+// body, while these warps are (nearly) all resident at once, 20 per SM (host call at 8 / 4 / 2
+// bodies, theta 0.7, us: N = 500 104.5 / 100.9 / 100.6; 3000 143 / 139 / 130; 10000 177 / 169 /
+// 183; 20000 205 / 220 / 243). 32 bodies, one to a lane,
 // meet fewer nodes than 64 (which share a traversal over more bodies) and end sooner; from
 // some 110 warps per SM on the traversals saved count for more. Whole call at 64 / 32 / 16 /
 // 8 bodies, us: N = 3000 theta 0.7 271 / 232 / 213 / 200; N = 30000 theta 0.5 552 / 436 / 391
@@ -1083,7 +1087,7 @@ struct MaskedPlan {
 static MaskedPlan masked_plan(const pt_ctx *ctx, int n_aff) {
     const long long sms = std::max(1, ctx->sm_count);
     MaskedPlan p{};
-    p.big = n_aff <= 8 * 20 * sms ? 8 : n_aff <= 16 * 27 * sms ? 16 : n_aff <= 32 * 110 * sms ? 32 : 64;
+    p.big = n_aff <= 2 * 20 * sms ? 2 : n_aff <= 4 * 20 * sms ? 4 : n_aff <= 8 * 20 * sms ? 8 : n_aff <= 16 * 27 * sms ? 16 : n_aff <= 32 * 110 * sms ? 32 : 64;
     const int all = (n_aff + p.big - 1) / p.big;
     const int halved = p.big >= 32 ? int(5 * sms) : 0;
     p.big_groups = std::max(0, all - halved);

@@ -1,5 +1,5 @@
-"""The reference-rule walk where the bodies per warp change with the number of targets (8, 16,
-32, 64, the last groups of the larger two in halves), in last warps that are not full."""
+"""The reference-rule walk where the bodies per warp change with the number of targets (2 to
+64, the last groups of the larger two in halves), in last warps that are not full."""
 import numpy as np
 import pytest
 
@@ -16,7 +16,7 @@ def test_sizes_agree_with_the_oracle(res, oracle, quad):
     m = cuda.BarnesHut(0.8, res, Acceleration.checked(), quadrupole=quad)
     tree = m.build(src)
     sms = res.sm_count
-    sizes = [1, 9, 160 * sms, 160 * sms + 1, 432 * sms + 17, 3520 * sms, 3520 * sms + 33]
+    sizes = [1, 3, 9, 40 * sms, 40 * sms + 1, 80 * sms, 80 * sms + 1, 160 * sms, 160 * sms + 1, 432 * sms + 17, 3520 * sms, 3520 * sms + 33]
     probe = np.concatenate([src[:200], np.concatenate([r.normal(size=(56, 3)), np.zeros((56, 1))], 1)]).astype(np.float32)
     want = cuda.BarnesHut(0.8, res, Acceleration.checked(), quadrupole=quad).compute(Between(probe, src))
     tree = m.build(src)
