@@ -617,8 +617,17 @@ __device__ __forceinline__ void
                 }
                 float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (lane < n) q = __ldg(sbody + f + base + lane);
-                unsigned q0 = 0u, q1 = 0u;
-                for (int j = 0; j < n; ++j) {  // a body does not meet itself in the leaf
+                unsigned q0 = b0, q1 = b1;
+                // A body does not meet itself in the leaf: only one in the group's box can be at
+                // a body of the group. (Voting on every leaf body: 1M bodies, all but 20 within
+                // 1e-5 of the box, 14.5 ms a walk, and 8.9 like this.)
+                const float e0 = fmaxf(fmaxf(mn0 - q.x, q.x - mx0), 0.0f);
+                const float e1 = fmaxf(fmaxf(mn1 - q.y, q.y - mx1), 0.0f);
+                const float e2b = fmaxf(fmaxf(mn2 - q.z, q.z - mx2), 0.0f);
+                unsigned vote = __ballot_sync(0xffffffffu, lane < n && !(fmaf(e0, e0, fmaf(e1, e1, e2b * e2b)) > 0.0f));
+                while (vote) {
+                    const int j = __ffs(vote) - 1;
+                    vote &= vote - 1;
                     const float cx = __shfl_sync(0xffffffffu, q.x, j), cy = __shfl_sync(0xffffffffu, q.y, j),
                                 cz = __shfl_sync(0xffffffffu, q.z, j);
                     const float x0 = cx - p[0].x, y0 = cy - p[0].y, z0 = cz - p[0].z;

@@ -323,17 +323,31 @@ __global__ void __launch_bounds__(RS_THREADS)
     __shared__ ScatterShared<RS_ROUNDS> S;
     uint64_t *kin = kb, *kout = ka;
     uint32_t *vin = vb, *vout = va;
+    const bool few = nblocks <= 64;  // the blocks add up the tiles' counts themselves: few blocks
+                                     // would each scan many rows
     for (int p = 0; p < passes; ++p) {
         for (int b = blockIdx.x; b < nblocks; b += gridDim.x) {
             hist_tile(kin, n, 8 * p, hist, nblocks, b, S.tstart);
             __syncthreads();
         }
         if (!barrier()) return;
-        for (int d = blockIdx.x; d < 256; d += gridDim.x) scan_row(hist, offs, rowsum, nblocks, d, S.wsum);
-        if (!barrier()) return;
+        if (!few) {
+            for (int d = blockIdx.x; d < 256; d += gridDim.x) scan_row(hist, offs, rowsum, nblocks, d, S.wsum);
+            if (!barrier()) return;
+        }
         for (int b = blockIdx.x; b < nblocks; b += gridDim.x) {
             scatter_tile(S, kin, vin, kout, vout, n, 8 * p, b,
                          [&](int t) {
+                             if (few) {
+                                 uint32_t before = 0, total = 0;
+#pragma unroll 8
+                                 for (int j = 0; j < nblocks; ++j) {
+                                     const uint32_t h = __ldcg(hist + t * nblocks + j);
+                                     if (j < b) before += h;
+                                     total += h;
+                                 }
+                                 return block_excl_scan(total, S.wsum, nullptr) + before;
+                             }
                              return block_excl_scan(__ldcg(rowsum + t), S.wsum, nullptr) +
                                     __ldcg(offs + size_t(t) * nblocks + b);
                          },
@@ -437,7 +451,11 @@ int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, 
     PT_TRY(check_launch(ctx, "rs_finish"));
     int all = (bits + 7) / 8, nb = nblocks;
     void *args[] = {&keys, &vals, &kb, &vb, &n, &all, &hist, &offs, &rowsum, &nb, &redo, &ctrl, &err};
-    const int grid = std::min(nblocks, 2 * std::max(1, ctx->sm_count));  // 2 of 36 KB fit every SM
+    static const int per_sm = [] {  // blocks that are resident together
+        int b = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rs_all, RS_THREADS, 0) == cudaSuccess ? std::max(1, b) : 1;
+    }();
+    const int grid = std::min(nblocks, per_sm * std::max(1, ctx->sm_count));
     PT_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(rs_all), dim3(grid), dim3(RS_THREADS), args, 0, st));
     return check_launch(ctx, "rs_all");
 }
