@@ -1047,7 +1047,7 @@ int build_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_src, int n) {
     PT_TRY(ensure_buf(ctx, nG, sizeof(V4) * 2 * N));
     float4 *nodeQ = F64 ? nullptr : as<float4>(S.nodeQ);
     PT_TRY(ensure_buf(ctx, S.nodeR, sizeof(int2) * 2 * N));
-    PT_TRY(ensure_buf(ctx, S.mom, sizeof(Moments) * 2 * N));
+    PT_TRY(ensure_buf(ctx, S.mom, sizeof(Record<T>) * 2 * N));
     PT_TRY(ensure_counters(ctx, S));
 
     RadixFirst rf{};
