@@ -392,7 +392,7 @@ int pt_mlp_predict_tc(pt_ctx *ctx, const float *features, int n, float *out);
 /* Phase timing of the last pt_bf_* / pt_bh_* call, from CUDA events recorded on
  * the context's stream when enabled: for Barnes-Hut, build = tree construction
  * and moments, walk = the traversal kernel; for the brute force, build = source
- * layout conversion, walk = the pair kernel(s). */
+ * layout conversion (0 where the pair kernel reads the rows), walk = the pair kernel(s). */
 typedef struct pt_timing {
     float build_ms;
     float walk_ms;

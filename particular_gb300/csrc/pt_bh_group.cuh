@@ -106,9 +106,9 @@ __device__ __forceinline__ void lane_walk(float4 p, bool valid, int T, const flo
 // its targets against all entries, two entries per packed f32x2 instruction.
 // Warps (groups) per CTA of the group walk. A CTA's slot is held until its slowest
 // warp ends, so with one warp per CTA no warp slot idles behind a neighbouring group's
-// longer walk; the local-expansion lists are sized (64 cells, 88 bodies) so that 20
+// longer walk; the local-expansion lists are sized (64 cells, 80 bodies) so that 20
 // one-warp CTAs fit an SM's shared memory. Measured at N = 4M (walk ms): headline
-// configuration 5.40 with 2 warps per CTA (72 / 96 entries) -> 5.25 with 1 (64 / 88);
+// configuration 5.40 with 2 warps per CTA (72 / 96 entries) -> 5.25 with 1 (then 64 / 88);
 // quadrupole + group + local at theta 0.52 12.19 -> 11.74; quadrupole + group at theta
 // 0.52 16.30 -> 15.19 (4 warps per CTA: 5.47, 12.43, 16.40). Persistent warps taking
 // groups from a counter instead spilled (96 -> 116 bytes) and were slower (5.85 ms).
