@@ -810,6 +810,7 @@ struct ChunkKids {
 // at N = 1M and 7 + 102 at N = 10000; layout and cells_span take 283 + 86, 84 + 58 and 22 +
 // 15.) A block waits on its own chain of loads, four blocks to an SM.
 constexpr int CHUNK_THREADS = 256;
+constexpr int SPREAD = 8;
 
 template <class T>
 __global__ void __launch_bounds__(CHUNK_THREADS)
@@ -826,7 +827,10 @@ __global__ void __launch_bounds__(CHUNK_THREADS)
     extern __shared__ __align__(32) unsigned char block_raw[];
     Chunk<T> &C = *reinterpret_cast<Chunk<T> *>(block_raw);
     const int M = counters[0];
-    const int c0 = blockIdx.x << CHUNK_SHIFT;
+    // Neighbouring chunks go to blocks SPREAD apart: where bodies share keys only the first few
+    // chunks hold units, and the first blocks start on the same SMs (1M bodies within 1e-5 of the
+    // box: build 2.13 ms in block order, 0.91 so).
+    const int c0 = int(blockIdx.x % SPREAD * (gridDim.x / SPREAD) + blockIdx.x / SPREAD) << CHUNK_SHIFT;
     if (c0 >= M) return;
     if (blockIdx.x == 0) clear_stats(counters, threadIdx.x);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1079,9 +1083,10 @@ int build_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_src, int n) {
     PT_TRY(check_launch(ctx, "octree_links"));
     PT_TRY(scan_generated(ctx, S.prims, CellStarts{as<uint32_t>(S.starts)},
                           scan::WriteU32{as<uint32_t>(S.pscan), n + 1}, n + 1));
+    const int chunks = ((n + CHUNK - 1) / CHUNK + SPREAD - 1) / SPREAD * SPREAD;
     PT_CUDA(cudaFuncSetAttribute(layout<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(Chunk<T>))));
     launch_next(
-        layout<T>, (n + CHUNK - 1) / CHUNK, CHUNK_THREADS, sizeof(Chunk<T>), st, counters, as<int>(S.bfirst), as<int>(S.blast), as<int>(S.bdelta), as<uint8_t>(S.top), as<int>(S.oparent),
+        layout<T>, chunks, CHUNK_THREADS, sizeof(Chunk<T>), st, counters, as<int>(S.bfirst), as<int>(S.blast), as<int>(S.bdelta), as<uint8_t>(S.top), as<int>(S.oparent),
         as<uint32_t>(S.starts), as<uint32_t>(S.pscan), as<uint64_t>(S.ukey), as<uint32_t>(S.ufirst), as<T>(S.box),
         as<int>(S.pre), as<int4>(S.nodeB), as<V4>(nG), as<int2>(S.nodeR), as<int>(S.loparent), as<int>(S.kid),
         as<V4>(sb), as<Record<T>>(S.mom), as<V4>(nA), nodeQ);
