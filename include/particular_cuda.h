@@ -315,8 +315,8 @@ int pt_leapfrog(pt_ctx *ctx, float *bodies, float *vel, size_t n, float dt, int 
  * holding the accelerations of the current positions, updated to the final ones).
  * use_graph != 0 captures the whole `steps`-step sequence into a CUDA graph on first
  * use for this (pointers, n, steps, method, dt, theta, softening, flags, stream and,
- * for Barnes-Hut, the context's local ratio, error-bound factor, stack limit and
- * learned model; any reallocation of a context buffer in between) and replays it
+ * for Barnes-Hut, the context's local ratio, error-bound and monopole factors, stack
+ * limit and learned model; any reallocation of a context buffer in between) and replays it
  * afterwards; that first call also recomputes `acc` from the positions
  * before capturing, so every buffer is sized outside the capture.
  * With PT_BH_LEARNED the call synchronises at the end and fails with PT_ERR_CAPACITY

@@ -42,14 +42,15 @@ static int sort_error(const char *fn, int err) {
 namespace pt {
 
 // The Barnes-Hut settings that captured launches carry as parameters (local ratio,
-// error-bound factor, learned inner angle, stack cap, model weights): a CUDA graph
-// captured under other values has to be captured again.
+// error-bound and monopole factors, learned inner angle, stack cap, model weights): a CUDA
+// graph captured under other values has to be captured again.
 BhTuning bh_tuning(pt_ctx *ctx) {
     BhTuning t{};
     const auto *S = static_cast<const bh::State *>(ctx->bh);
     if (S) {
         t.local_ratio = S->local_ratio;
         t.rel_alpha = S->rel_alpha;
+        t.rel_mono = S->rel_mono;
         t.theta_inner = S->theta_inner;
         t.stack_cap = S->stack_cap;
         t.learned_cap = S->lcap_fixed;

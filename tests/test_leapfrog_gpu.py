@@ -139,6 +139,38 @@ def test_graph_recaptured_when_settings_change(res):
     assert np.array_equal(outs[0][1], outs[1][1])
 
 
+@pytest.mark.parametrize("setter,values,restore", [("pt_bh_set_relative_monopole", (0.0, 1.0), 0.1),
+                                                   ("pt_bh_set_stack_limit", (0, 8), 0)])
+def test_graph_recaptured_when_one_setting_changes(res, setter, values, restore):
+    """Each setting by itself: the monopole factor and the stack limit are launch
+    parameters too."""
+    import torch
+    d = ics.plummer(20000, seed=57)
+    L = N.lib()
+    fl = N.PT_BH_QUADRUPOLE | N.PT_BH_GROUP | N.PT_BH_RELATIVE
+    outs = []
+    try:
+        for use_graph in (0, 1):
+            b = torch.from_numpy(d["bodies"]).cuda()
+            v = torch.zeros((20000, 4), device="cuda")
+            v[:, :3] = torch.from_numpy(d["vel"]).cuda()
+            a = torch.zeros((20000, 3), device="cuda")
+            torch.cuda.synchronize()
+            for value in values:
+                N.check(getattr(L, setter)(res.handle, value))
+                N.check(L.pt_bh_accel_f32_device(res.handle, b.data_ptr(), 20000, b.data_ptr(), 20000,
+                                                 1.0, 0.01, fl, a.data_ptr()))
+                for _ in range(2):
+                    N.check(L.pt_leapfrog_device(res.handle, b.data_ptr(), v.data_ptr(), a.data_ptr(), 20000,
+                                                 1e-3, 3, N.PT_METHOD_BARNES_HUT, 1.0, 0.01, fl, use_graph))
+            res.synchronize()
+            outs.append((b.cpu().numpy(), v.cpu().numpy()))
+    finally:
+        N.check(getattr(L, setter)(res.handle, restore))
+    assert np.array_equal(outs[0][0], outs[1][0])
+    assert np.array_equal(outs[0][1], outs[1][1])
+
+
 def test_graph_recaptured_when_buffers_grow():
     """A captured leapfrog holds the addresses of the context's grow-only buffers. A
     bigger Barnes-Hut call on the same context between two replays reallocates them
