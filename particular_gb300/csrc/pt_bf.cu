@@ -78,11 +78,6 @@ __device__ __forceinline__ void for_each_tile(float4 (*tiles)[TILE], const float
     cp_async_wait<0>();
 }
 
-// A slice's last, shorter tile is added in plain FP32 runs of TAIL_RUN sources (padded to
-// whole runs). Where it is the slice's only tile every source is compensated: there is no
-// whole tile whose rounding would hide that of the runs.
-constexpr int TAIL_RUN = 8;
-
 // A tile of sources in structure-of-arrays form, so that one LDS.128 yields two packed
 // source pairs.
 struct SoaTile {
@@ -117,8 +112,8 @@ __device__ __forceinline__ void stage_tile(SoaTile &T, const float4 (&pre)[TILE 
 // N = 65536, the rest lost to operand reads and the two-sum folds). What else a call paid
 // for, and no longer does: the launch that laid the sources out, the coincidence test's
 // selects on every pair, and a scalar loop over the sources of a last, shorter tile
-// (1000003 targets x 3001 sources: unsoftened 1424 -> 1109 us, softened 1251 -> 1114; N =
-// 4999 45 -> 39 us).
+// (1000003 targets x 3001 sources: unsoftened 1424 -> 1203 us, softened 1251 -> 1196; N =
+// 4999 45 -> 38 us).
 
 // Four sources against a thread's K targets, in packed lo/hi partials.
 template <int K, bool GUARD>
@@ -143,15 +138,14 @@ __device__ __forceinline__ void tile_quad(const SoaTile &T, int q, const f2 (&xi
                    e2, ax, ay, az);
 }
 
-// Adds a run's partials (quads [q0, q1) of the tile) to the targets' compensated sums and
-// zeroes them.
-// GUARD (checked, eps == 0): runs are evaluated without the test for coincidence, which
-// costs two selects per pair. A coincident pair then always makes the run's sum NaN
-// (0 times an infinite s, or 0 times NaN), so only a run whose sum is not finite is done
-// again with the test, by the threads that met it: one run per target that is its own
+// Adds a whole tile's partials to the targets' compensated sums and zeroes them.
+// GUARD (checked, eps == 0): tiles are evaluated without the test for coincidence, which
+// costs two selects per pair. A coincident pair then always makes the tile's sum NaN
+// (0 times an infinite s, or 0 times NaN), so only a tile whose sum is not finite is done
+// again with the test, by the threads that met it: one tile per target that is its own
 // source. A sum that is not finite for another reason comes out the same again.
 template <int K, bool GUARD>
-__device__ __forceinline__ void fold_run(const SoaTile &T, int q0, int q1, const f2 (&xi)[K], const f2 (&yi)[K],
+__device__ __forceinline__ void fold_tile(const SoaTile &T, const f2 (&xi)[K], const f2 (&yi)[K],
                                          const f2 (&zi)[K], f2 e2, f2 (&ax)[K], f2 (&ay)[K], f2 (&az)[K],
                                          float (&sx)[K], float (&sy)[K], float (&sz)[K], float (&cx)[K],
                                          float (&cy)[K], float (&cz)[K]) {
@@ -175,7 +169,7 @@ __device__ __forceinline__ void fold_run(const SoaTile &T, int q0, int q1, const
 #pragma unroll
             for (int k = 0; k < K; ++k) ax[k] = ay[k] = az[k] = zero2;
 #pragma unroll 1
-            for (int q = q0; q < q1; ++q) tile_quad<K, true>(T, q, xi, yi, zi, e2, ax, ay, az);
+            for (int q = 0; q < TILE / 4; ++q) tile_quad<K, true>(T, q, xi, yi, zi, e2, ax, ay, az);
 #pragma unroll
             for (int k = 0; k < K; ++k) {
                 float l, h;
@@ -205,27 +199,38 @@ __device__ __forceinline__ void two_sum_acc2(f2 &s, f2 &c, f2 t) {
     s = sn;
 }
 
-// The first cnt sources of a tile, each added with its rounding error kept: pairs of them
-// in packed sums, whose halves then enter the targets' sums.
+// The cnt sources of a slice's last, shorter tile, each added with its rounding error kept: in
+// packed sums, one half of which goes on from the targets' sums. Four sources a step, for a
+// short call waits on the steps' latency (5003 targets x 317 sources 7.2 us, two a step 7.7).
+// In plain runs of eight, only the runs' errors kept, 1000003 x 3001 took 1107 us where it
+// takes 1203, but the rms error was up to 0.9 % higher at 257 to 511 sources.
 template <int K, bool GUARD>
-__device__ __forceinline__ void each_pair(const SoaTile &T, int cnt, const f2 (&xi)[K], const f2 (&yi)[K],
-                                          const f2 (&zi)[K], f2 e2, float (&sx)[K], float (&sy)[K], float (&sz)[K],
-                                          float (&cx)[K], float (&cy)[K], float (&cz)[K]) {
+__device__ __forceinline__ void each_source(const SoaTile &T, int cnt, const f2 (&xi)[K], const f2 (&yi)[K],
+                                            const f2 (&zi)[K], f2 e2, float (&sx)[K], float (&sy)[K], float (&sz)[K],
+                                            float (&cx)[K], float (&cy)[K], float (&cz)[K]) {
     const f2 zero2 = pk2(0.f, 0.f);
     f2 s[K][3], c[K][3];
 #pragma unroll
-    for (int k = 0; k < K; ++k) s[k][0] = s[k][1] = s[k][2] = c[k][0] = c[k][1] = c[k][2] = zero2;
+    for (int k = 0; k < K; ++k) {
+        s[k][0] = pk2(sx[k], 0.f), s[k][1] = pk2(sy[k], 0.f), s[k][2] = pk2(sz[k], 0.f);
+        c[k][0] = pk2(cx[k], 0.f), c[k][1] = pk2(cy[k], 0.f), c[k][2] = pk2(cz[k], 0.f);
+    }
 #pragma unroll 1
-    for (int e = 0; e < cnt; e += 2) {
-        const f2 x = *reinterpret_cast<const f2 *>(&T.c[0][e]), y = *reinterpret_cast<const f2 *>(&T.c[1][e]);
-        const f2 z = *reinterpret_cast<const f2 *>(&T.c[2][e]), m = *reinterpret_cast<const f2 *>(&T.c[3][e]);
+    for (int e = 0; e < cnt; e += 4) {
+        const float4 x = *reinterpret_cast<const float4 *>(&T.c[0][e]), y = *reinterpret_cast<const float4 *>(&T.c[1][e]);
+        const float4 z = *reinterpret_cast<const float4 *>(&T.c[2][e]), m = *reinterpret_cast<const float4 *>(&T.c[3][e]);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            f2 ax = zero2, ay = zero2, az = zero2;
-            interact2<GUARD>(x, y, z, m, xi[k], yi[k], zi[k], ax, ay, az, e2);
-            two_sum_acc2(s[k][0], c[k][0], ax);
-            two_sum_acc2(s[k][1], c[k][1], ay);
-            two_sum_acc2(s[k][2], c[k][2], az);
+            f2 a[3] = {zero2, zero2, zero2}, b[3] = {zero2, zero2, zero2};
+            interact2<GUARD>(pk2(x.x, x.y), pk2(y.x, y.y), pk2(z.x, z.y), pk2(m.x, m.y), xi[k], yi[k], zi[k], a[0],
+                             a[1], a[2], e2);
+            interact2<GUARD>(pk2(x.z, x.w), pk2(y.z, y.w), pk2(z.z, z.w), pk2(m.z, m.w), xi[k], yi[k], zi[k], b[0],
+                             b[1], b[2], e2);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                two_sum_acc2(s[k][i], c[k][i], a[i]);
+                two_sum_acc2(s[k][i], c[k][i], b[i]);
+            }
         }
     }
 #pragma unroll
@@ -233,12 +238,11 @@ __device__ __forceinline__ void each_pair(const SoaTile &T, int cnt, const f2 (&
         float *sum[3] = {&sx[k], &sy[k], &sz[k]}, *err[3] = {&cx[k], &cy[k], &cz[k]};
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            float l, h, cl, ch;
-            upk2(s[k][a], l, h);
-            upk2(c[k][a], cl, ch);
-            two_sum_acc(*sum[a], *err[a], l);
+            float h, ch;
+            upk2(s[k][a], *sum[a], h);
+            upk2(c[k][a], *err[a], ch);
             two_sum_acc(*sum[a], *err[a], h);
-            *err[a] += cl + ch;
+            *err[a] += ch;
         }
     }
 }
@@ -311,24 +315,14 @@ __global__ void __launch_bounds__(THREADS, K == 1 ? 8 : 1)
         const float4 *M = reinterpret_cast<const float4 *>(T.c[3]);
 #pragma unroll 2
         for (int q = 0; q < TILE / 4; ++q) quad<K, false>(X[q], Y[q], Z[q], M[q], xi2, yi2, zi2, e2, ax, ay, az);
-        fold_run<K, GUARD>(T, 0, TILE / 4, xi2, yi2, zi2, e2, ax, ay, az, sx, sy, sz, cx, cy, cz);
+        fold_tile<K, GUARD>(T, xi2, yi2, zi2, e2, ax, ay, az, sx, sy, sz, cx, cy, cz);
     }
     if (whole < ntiles) {  // the last, shorter tile
         SoaTile &T = tiles[whole & 1];
         stage_tile<THREADS>(T, pre);
         __syncthreads();
         const int cnt = j_end - (j0 + whole * TILE);
-        if (whole == 0) {
-            each_pair<K, GUARD>(T, cnt, xi2, yi2, zi2, e2, sx, sy, sz, cx, cy, cz);
-        } else {
-#pragma unroll 1
-            for (int q = 0; 4 * q < cnt; q += TAIL_RUN / 4) {
-#pragma unroll
-                for (int r = 0; r < TAIL_RUN / 4; ++r)
-                    tile_quad<K, false>(T, q + r, xi2, yi2, zi2, e2, ax, ay, az);
-                fold_run<K, GUARD>(T, q, q + TAIL_RUN / 4, xi2, yi2, zi2, e2, ax, ay, az, sx, sy, sz, cx, cy, cz);
-            }
-        }
+        each_source<K, GUARD>(T, cnt, xi2, yi2, zi2, e2, sx, sy, sz, cx, cy, cz);
     }
 
 #pragma unroll

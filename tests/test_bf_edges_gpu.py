@@ -79,3 +79,29 @@ def test_small_calls_add_their_slices_in_the_same_order(res, native_lib, n):
     for m in (n, 300, n, n):
         got = method.compute(b[:m])
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+# The sources of a last, shorter tile behind whole ones: each one's rounding error is kept. Two
+# that cancel with a small one between them, in every place of the tile.
+@pytest.mark.parametrize("targets_per_thread", [1, 2, 4])
+@pytest.mark.parametrize("soft", [0.0, 0.05])
+@pytest.mark.parametrize("tail", [3, 16, 21, 255])
+def test_each_source_of_a_short_tile_is_compensated(res, native_lib, targets_per_thread, soft, tail):
+    from particular_gb300 import _native as N
+
+    src = bodies(256 + tail, 3)
+    src[:, 3] = 0.0
+    big, small = 256 + np.array([0, tail - 1]), 256 + tail // 2
+    src[big] = [[1, 0, 0, 1e6], [-1, 0, 0, 1e6]]
+    src[small] = [1, 0, 0, 1e-2]
+    aff = bodies(300, 4)
+    aff[::7, :3] = 0.0
+    it = AccelerationSoftened(soft) if soft else Acceleration.checked()
+    try:
+        N.check(native_lib.pt_bf_set_plan(res.handle, targets_per_thread, 1))
+        got = cuda.BruteForce(res, it).compute(Between(aff, src))[::7]
+    finally:
+        N.check(native_lib.pt_bf_set_plan(res.handle, 0, 0))
+    want = 1e-2 / (1.0 + float(np.float32(soft)) ** 2) ** 1.5
+    # the two cancel exactly; the small one's three rsqrt factors (2^-22 each) remain
+    assert (np.abs(got[:, 0] - want) <= 2e-6 * want).all() and (got[:, 1:] == 0).all()
