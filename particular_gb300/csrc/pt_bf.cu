@@ -84,15 +84,15 @@ struct SoaTile {
     float c[4][TILE];
 };
 
-// This thread's sources of tile t of [j0, j_end), past the end massless ones far away: they
-// add exactly 0 (r^2 overflows, 1 / r is 0).
+// This thread's sources of tile t of [j0, j_end), past the end zeros (each_source leaves them
+// out).
 template <int TH>
 __device__ __forceinline__ void fetch_tile(float4 (&pre)[TILE / TH], const float4 *__restrict__ src, int j0, int j_end,
                                            int t) {
 #pragma unroll
     for (int c = 0; c < TILE / TH; ++c) {
         const int j = j0 + t * TILE + c * TH + threadIdx.x;
-        pre[c] = j < j_end ? __ldg(src + j) : make_float4(1e30f, 1e30f, 1e30f, 0.f);
+        pre[c] = j < j_end ? __ldg(src + j) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
 
@@ -223,9 +223,9 @@ __device__ __forceinline__ void each_source(const SoaTile &T, int cnt, const f2 
         for (int k = 0; k < K; ++k) {
             f2 a[3] = {zero2, zero2, zero2}, b[3] = {zero2, zero2, zero2};
             interact2<GUARD>(pk2(x.x, x.y), pk2(y.x, y.y), pk2(z.x, z.y), pk2(m.x, m.y), xi[k], yi[k], zi[k], a[0],
-                             a[1], a[2], e2);
+                             a[1], a[2], e2, true, e + 1 < cnt);
             interact2<GUARD>(pk2(x.z, x.w), pk2(y.z, y.w), pk2(z.z, z.w), pk2(m.z, m.w), xi[k], yi[k], zi[k], b[0],
-                             b[1], b[2], e2);
+                             b[1], b[2], e2, e + 2 < cnt, e + 3 < cnt);
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
                 two_sum_acc2(s[k][i], c[k][i], a[i]);

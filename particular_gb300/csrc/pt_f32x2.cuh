@@ -56,10 +56,11 @@ __device__ __forceinline__ void two_sum_acc(float &s, float &c, float t) {
 // Two pairs (one target; sources in the lo and hi lanes) of the per-pair kernel
 // a = d * mu / n_s^1.5 with n_s = |d|^2 + eps^2 (particular/src/gravity/impls/mod.rs:
 // 156-165): 12 FMA-pipe lane-ops as 6 f32x2 instructions + 2 MUFU. GUARD zeroes
-// the contribution of n_s == 0 (checked with eps == 0: the body itself).
+// the contribution of n_s == 0 (checked with eps == 0: the body itself). lo, hi: there is a
+// source in that lane; else a massless one with finite coordinates adds exactly 0.
 template <bool GUARD>
 __device__ __forceinline__ void interact2(f2 xj, f2 yj, f2 zj, f2 mj, f2 xi, f2 yi, f2 zi, f2 &ax, f2 &ay,
-                                          f2 &az, f2 e2) {
+                                          f2 &az, f2 e2, bool lo = true, bool hi = true) {
     const f2 dx = sub2(xj, xi);
     const f2 dy = sub2(yj, yi);
     const f2 dz = sub2(zj, zi);
@@ -71,6 +72,8 @@ __device__ __forceinline__ void interact2(f2 xj, f2 yj, f2 zj, f2 mj, f2 xi, f2 
         i0 = (r0 > 0.0f) ? i0 : 0.0f;
         i1 = (r1 > 0.0f) ? i1 : 0.0f;
     }
+    i0 = lo ? i0 : 0.0f;
+    i1 = hi ? i1 : 0.0f;
     const f2 inv = pk2(i0, i1);
     const f2 s = mul2(mul2(mj, inv), mul2(inv, inv));
     ax = fma2(dx, s, ax);

@@ -105,3 +105,24 @@ def test_each_source_of_a_short_tile_is_compensated(res, native_lib, targets_per
     want = 1e-2 / (1.0 + float(np.float32(soft)) ** 2) ** 1.5
     # the two cancel exactly; the small one's three rsqrt factors (2^-22 each) remain
     assert (np.abs(got[:, 0] - want) <= 2e-6 * want).all() and (got[:, 1:] == 0).all()
+
+
+# The places of a short tile behind its last source hold no source: a target anywhere, at the
+# origin and far outside the others too, meets the sources alone (unchecked and unsoftened, where a
+# pair at one place would be NaN).
+@pytest.mark.parametrize("n_src", [1, 2, 3, 255, 257, 300, 1022])
+@pytest.mark.parametrize("at", [0.0, 1e30, -1e30, 3.4e38])
+def test_no_source_behind_the_last_one(res, oracle, n_src, at):
+    src = bodies(n_src, n_src)
+    aff = bodies(40, 8)
+    aff[::3, :3] = at
+    got = cuda.BruteForce(res, Acceleration.unchecked()).compute(Between(aff, src))
+    want = oracle.bf_f64(aff, src, 0.0, False)
+    assert np.isfinite(got).all()
+    if at:  # r^2 overflows in f32: exactly 0
+        assert (got[::3] == 0).all()
+    rest = np.ones(len(aff), bool)
+    rest[::3] = at == 0
+    scale = np.linalg.norm(want[rest], axis=1)
+    # one sum of at most 256 terms' rounding, rsqrt factors of 2^-22
+    assert (np.linalg.norm(got[rest] - want[rest], axis=1) <= 1e-4 * scale + 1e-5 * n_src).all()
