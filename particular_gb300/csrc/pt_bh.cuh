@@ -19,9 +19,7 @@ namespace bh {
 constexpr int LEVELS = 21;   // 63-bit keys
 constexpr int WALK_STATS = 9;  // the walk's u64 counters behind counters[0..3]
 constexpr int ROOT_BOX_DONE = 30;  // root_box's word of counters
-// Group walk in order of work: the counts and cursors of its buckets, behind counters[0..31].
-constexpr int ORDER_BUCKETS = 128, ORDER_WORDS = 2 * ORDER_BUCKETS;
-constexpr size_t COUNTER_BYTES = sizeof(int) * (32 + ORDER_WORDS);
+constexpr size_t COUNTER_BYTES = sizeof(int) * 32;
 
 struct Moments {  // FP64 cell data used while combining children (DVec3 trees, bucket leaves)
     double m, cx, cy, cz;
@@ -74,7 +72,7 @@ struct State {
     DevBuf out;
     DevBuf aff_h, src_h;  // staging for the host-pointer entry point
     DevBuf lrec, lgroup, lnext, lpart, lhead, lcentre, lused;  // learned-correction records
-    DevBuf gscale, gorder;            // PT_BH_RELATIVE: 1 / (alpha |a|) per group, groups by it
+    DevBuf gscale, gorder;            // key per group (PT_BH_RELATIVE: 1 / (alpha |a|)), groups by it
     int lcap = 0;                     // record chunks allocated
     int lcap_fixed = 0;               // > 0: record chunks fixed by pt_bh_set_learned_capacity
     int stack_cap = 0;                // group-walk stack ranges per warp in use (0 = all)
@@ -123,7 +121,6 @@ int sort_targets(pt_ctx *ctx, State &S, const float4 *d_aff, int n);
 // walks (pt_bh_walk.cu)
 int ensure_counters(pt_ctx *ctx, State &S);
 int clear_errors(pt_ctx *ctx, State &S);
-inline unsigned *order_buckets(State &S) { return static_cast<unsigned *>(S.counters.ptr) + 32; }
 int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n_aff, float theta,
          float softening, uint32_t flags, float *d_out);
 int run(pt_ctx *ctx, const float4 *d_aff, int n_aff, const float4 *d_src, int n_src, float theta, float softening,

@@ -149,9 +149,8 @@ __global__ void make_keys(const typename Prec<T>::V4 *__restrict__ bodies, int n
     if (hist) atomicAdd(&hist[(i / tile) * 256 + (int(k >> shift) & 255)], 1u);
 }
 
-// The walk's counters (counters + 4 ints) and its buckets of groups start from zero.
+// The walk's counters (counters + 4 ints) start from zero.
 __device__ __forceinline__ void clear_stats(int *counters, int i) {
-    if (i < ORDER_WORDS) counters[32 + i] = 0;
     if (i < WALK_STATS) (reinterpret_cast<unsigned long long *>(counters) + 2)[i] = 0ull;
 }
 

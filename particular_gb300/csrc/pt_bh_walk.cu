@@ -126,12 +126,6 @@ __device__ __forceinline__ void scale_cursor_walk(float cx, float cy, float cz, 
     }
 }
 
-// Two octaves of the scale (positive, or infinite) to a bucket, the largest first.
-static_assert(ORDER_BUCKETS == 128, "a float's sign and upper exponent bits");
-__device__ __forceinline__ int order_bucket(float scale) {
-    return ORDER_BUCKETS - 1 - ((__float_as_int(scale) & 0x7fffffff) >> 24);
-}
-
 // One thread per group: the group's box, then the cursor walk from its centre. (One
 // warp per group walking with a range stack, one node per lane and pop, was slower at
 // N = 4M: the walk phase, which includes this kernel, went from 5.68 to 5.85 ms. Its
@@ -141,15 +135,13 @@ __device__ __forceinline__ int order_bucket(float scale) {
 // own octant holds most of the visits. Four lanes per group popping up to four ranges
 // of a shared-memory stack per step took 0.18 ms: a walk from one point keeps few
 // ranges open, so the steps stayed nearly as many and each cost more.)
-// buckets: null, or counts the groups by order_bucket.
 __global__ void __launch_bounds__(128)
     bh_group_scale(const float4 *__restrict__ tbody, int n_aff, const float4 *__restrict__ nodeA,
                    const int4 *__restrict__ nodeB, const int *__restrict__ counters, float eps2, float alpha,
-                   float *__restrict__ gscale, unsigned *__restrict__ buckets) {
+                   float *__restrict__ gscale) {
     after_previous();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int g0 = g * GW_GROUP;
-    const unsigned active = __ballot_sync(0xffffffffu, g0 < n_aff);
     if (g0 >= n_aff) return;
     const int g1 = min(n_aff, g0 + GW_GROUP);
     float4 p = tbody[g0];
@@ -163,54 +155,105 @@ __global__ void __launch_bounds__(128)
     scale_cursor_walk(0.5f * (mn0 + mx0), 0.5f * (mn1 + mx1), 0.5f * (mn2 + mx2), nodeA, nodeB, counters[1], eps2,
                       ax, ay, az);
     const float a = sqrtf(fmaf(ax, ax, fmaf(ay, ay, az * az)));
-    const float s = 1.f / (alpha * fmaxf(a, 1e-30f));
-    gscale[g] = s;
-    if (!buckets) return;
-    __syncwarp(active);
-    const int b = order_bucket(s);
-    const unsigned peers = __match_any_sync(active, b);
-    if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(buckets + b, __popc(peers));
+    gscale[g] = 1.f / (alpha * fmaxf(a, 1e-30f));
+}
+
+// Two octaves of the scale (positive, or infinite) to a bucket, the largest first.
+constexpr int ORDER_BUCKETS = 128;  // a float's upper seven exponent bits
+__device__ __forceinline__ int order_bucket(float scale) {
+    return ORDER_BUCKETS - 1 - ((__float_as_int(scale) & 0x7fffffff) >> 24);
 }
 
 // The groups by descending key, for the walk to take them in: one that opens many cells and
 // starts last holds up the call. In the error-bound walk the key is the group's scale: one whose
 // error bound is small next to its forces opens the most (rank correlation with its walk 0.75).
-// Within a bucket they stay about in tree order, so that neighbours still share what they read.
-// Whole error-bound call in tree order and so ordered, us: N = 262144
-// 974 / 872, 524288 1513 / 1209, 1048576 1824 / 1825, 2097152 3880 / 3290, 4194304 6008 / 6020.
-// While all groups start at once there is nothing to order.
-__global__ void __launch_bounds__(256)
-    bh_group_order(const float *__restrict__ gscale, int groups, unsigned *__restrict__ buckets,
-                   int *__restrict__ gorder) {
+// Within a bucket they stay in tree order: neighbours still share what they read, and the order
+// is the same every time, which the masked walk needs, for it halves the groups that come last
+// and that shows in the rounding of their sums. A stable counting sort by one block, a warp to
+// each 32nd of the groups: 5.1 us for the 4096 groups of N = 262144, 10.5 for 16384 and 25 for
+// 65536. (Many blocks with a counter per bucket, so in no fixed order, took 3.8 to 4.8 us;
+// but in tree order the walk at N = 4M takes 5.08 ms, 5.2 in theirs.) Whole error-bound call
+// in tree order alone and by key, us: N = 262144 974 / 872, 524288 1513 / 1209, 1048576 1824 /
+// 1825, 2097152 3880 / 3290, 4194304 6008 / 5998.
+constexpr int ORDER_WARPS = 32, ORDER_BATCH = 8;
+
+__global__ void __launch_bounds__(32 * ORDER_WARPS)
+    bh_group_order(const float *__restrict__ key, int groups, int *__restrict__ gorder) {
     after_previous();
-    __shared__ unsigned first[ORDER_BUCKETS], wsum[4];
-    const int t = threadIdx.x, lane = t & 31, i = blockIdx.x * blockDim.x + t;
-    unsigned c = 0, incl = 0;
-    if (t < ORDER_BUCKETS) {
-        c = incl = buckets[t];
+    constexpr int PER = ORDER_BUCKETS / ORDER_WARPS;  // buckets a warp scans
+    __shared__ unsigned place[ORDER_WARPS][ORDER_BUCKETS + 1], first[ORDER_BUCKETS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int per = (groups + 32 * ORDER_WARPS - 1) / (32 * ORDER_WARPS) * 32;
+    const int g0 = min(groups, warp * per), g1 = min(groups, g0 + per);
+    int bucket[ORDER_BATCH];  // of the groups i0 + 32 r + lane
+    auto load = [&](int i0) {
+#pragma unroll
+        for (int r = 0; r < ORDER_BATCH; ++r) {
+            const int i = i0 + 32 * r + lane;
+            bucket[r] = i < g1 ? order_bucket(key[i]) : -1;
+        }
+    };
+    for (int b = lane; b < ORDER_BUCKETS; b += 32) place[warp][b] = 0;
+    load(g0);
+    __syncwarp();
+    for (int i0 = g0;;) {
+#pragma unroll
+        for (int r = 0; r < ORDER_BATCH; ++r)
+            if (bucket[r] >= 0) atomicAdd(&place[warp][bucket[r]], 1u);
+        if ((i0 += 32 * ORDER_BATCH) >= g1) break;
+        load(i0);
+    }
+    __syncthreads();
+    // where each warp's groups of a bucket go: lane w holds warp w's count
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int b = PER * warp + k;
+        const unsigned c = place[lane][b];
+        unsigned incl = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += u;
         }
-        if (lane == 31) wsum[t >> 5] = incl;
+        place[lane][b] = incl - c;
+        if (lane == 31) first[b] = incl;
     }
     __syncthreads();
-    if (t < ORDER_BUCKETS) {
-        for (int w = 0; w < t >> 5; ++w) incl += wsum[w];
-        first[t] = incl - c;
+    if (warp == 0) {  // the buckets' starts, PER to a lane
+        unsigned c[PER], sum = 0;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            c[k] = sum;
+            sum += first[PER * lane + k];
+        }
+        unsigned incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+#pragma unroll
+        for (int k = 0; k < PER; ++k) first[PER * lane + k] = incl - sum + c[k];
     }
     __syncthreads();
-    const unsigned active = __ballot_sync(0xffffffffu, i < groups);
-    if (i >= groups) return;
-    const int b = order_bucket(gscale[i]);
-    const unsigned peers = __match_any_sync(active, b);
-    const int leader = __ffs(peers) - 1;
-    unsigned at = 0;
-    if (lane == leader) at = atomicAdd(buckets + ORDER_BUCKETS + b, __popc(peers));
-    at = __shfl_sync(peers, at, leader);
-    const unsigned pos = first[b] + at + __popc(peers & ((1u << lane) - 1u));
-    if (pos < unsigned(groups)) gorder[pos] = i;  // (always: the buckets are cleared before they count)
+    if (per > 32 * ORDER_BATCH) load(g0);  // else the buckets are still there
+    for (int i0 = g0;;) {
+#pragma unroll
+        for (int r = 0; r < ORDER_BATCH; ++r) {
+            if (i0 + 32 * r >= g1) break;
+            const int b = bucket[r];
+            const unsigned peers = __match_any_sync(0xffffffffu, b), below = peers & ((1u << lane) - 1u);
+            const unsigned at = b >= 0 ? place[warp][b] : 0u;
+            __syncwarp();
+            if (b >= 0) {
+                gorder[first[b] + at + __popc(below)] = i0 + 32 * r + lane;
+                if (below == 0u) place[warp][b] = at + __popc(peers);
+            }
+            __syncwarp();
+        }
+        if ((i0 += 32 * ORDER_BATCH) >= g1) break;
+        load(i0);
+    }
 }
 
 // The key of the walks by opening angle: a group's squared width over its squared distance from
@@ -222,11 +265,8 @@ __global__ void __launch_bounds__(256)
 // 1825 -> 1739, 4M 6015 -> 6127.)
 __global__ void __launch_bounds__(256)
     bh_group_width(const float4 *__restrict__ tbody, int n_aff, int groups, int size,
-                   const float4 *__restrict__ nodeA, float *__restrict__ ratio, unsigned *__restrict__ buckets) {
+                   const float4 *__restrict__ nodeA, float *__restrict__ ratio) {
     after_previous();
-    __shared__ unsigned cnt[ORDER_BUCKETS];
-    for (int i = threadIdx.x; i < ORDER_BUCKETS; i += blockDim.x) cnt[i] = 0;
-    __syncthreads();
     const int lanes = min(32, size);  // a power of two
     const float4 root = nodeA[0];
     const int step = gridDim.x * blockDim.x / lanes;
@@ -256,14 +296,9 @@ __global__ void __launch_bounds__(256)
             const float s = fmaf(w0, w0, fmaf(w1, w1, w2 * w2)) / fmaf(d0, d0, fmaf(d1, d1, d2 * d2));
             // two buckets an octave from 2^-20 to 2^12, as order_bucket takes two octaves
             const float q = fminf(fmaxf(s, 9.5367431640625e-7f), 4096.f);
-            const float key = __int_as_float(((__float_as_int(q) - 0x35800000) >> 22) << 24);
-            ratio[g] = key;
-            atomicAdd(&cnt[order_bucket(key)], 1u);
+            ratio[g] = __int_as_float(((__float_as_int(q) - 0x35800000) >> 22) << 24);
         }
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < ORDER_BUCKETS; i += blockDim.x)
-        if (cnt[i]) atomicAdd(buckets + i, cnt[i]);
 }
 
 // ---- masked group walk: the reference's rule, per body, with shared traversal ----
@@ -1119,11 +1154,10 @@ int clear_errors(pt_ctx *ctx, State &S) {
     return PT_OK;
 }
 
-// The order of the groups whose keys are in S.gscale and counted in the buckets.
+// The order of the groups whose keys are in S.gscale.
 static int place_groups(pt_ctx *ctx, State &S, int groups, const int **order) {
     PT_TRY(ensure_buf(ctx, S.gorder, sizeof(int) * size_t(groups)));
-    launch_next(bh_group_order, blocks(groups), 256, 0, ctx->stream, as<float>(S.gscale), groups, order_buckets(S),
-                as<int>(S.gorder));
+    launch_next(bh_group_order, 1, 32 * ORDER_WARPS, 0, ctx->stream, as<float>(S.gscale), groups, as<int>(S.gorder));
     *order = as<int>(S.gorder);
     return check_launch(ctx, "bh_group_order");
 }
@@ -1137,7 +1171,7 @@ static int order_groups(pt_ctx *ctx, State &S, const float4 *tbody, int n_aff, i
     if (groups <= 24 * sms) return PT_OK;
     PT_TRY(ensure_buf(ctx, S.gscale, sizeof(float) * size_t(groups)));
     launch_next(bh_group_width, std::min(2 * sms, blocks(groups * std::min(32, size))), 256, 0, ctx->stream, tbody,
-                n_aff, groups, size, as<float4>(S.nodeA), as<float>(S.gscale), order_buckets(S));
+                n_aff, groups, size, as<float4>(S.nodeA), as<float>(S.gscale));
     PT_TRY(check_launch(ctx, "bh_group_width"));
     return place_groups(ctx, S, groups, order);
 }
@@ -1251,8 +1285,7 @@ int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n
             PT_TRY(ensure_buf(ctx, S.gscale, sizeof(float) * size_t(groups)));
             const bool ordered = groups > 20 * std::max(1, ctx->sm_count);  // more than start at once
             launch_next(bh_group_scale, blocks(groups, 128), 128, 0, st, tbody, n_aff, as<float4>(S.nodeA),
-                        as<int4>(S.nodeB), as<int>(S.counters), eps2, S.rel_alpha, as<float>(S.gscale),
-                        ordered ? order_buckets(S) : nullptr);
+                        as<int4>(S.nodeB), as<int>(S.counters), eps2, S.rel_alpha, as<float>(S.gscale));
             PT_TRY(check_launch(ctx, "bh_group_scale"));
             gscale = as<float>(S.gscale);
             if (ordered) PT_TRY(place_groups(ctx, S, groups, &gorder));

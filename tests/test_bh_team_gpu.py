@@ -88,3 +88,35 @@ def test_order_of_the_masked_walk_does_not_show(res, quadrupole):
         # the same nodes, added in another order: compensated sums
         scale = np.linalg.norm(want, axis=1) + np.median(np.linalg.norm(want, axis=1))
         assert (np.linalg.norm(got - want, axis=1) <= 2e-6 * scale).all()
+
+
+@pytest.mark.parametrize("quadrupole", [False, True])
+@pytest.mark.parametrize("turn", [24 * 32, 110 * 32])
+def test_ordered_walks_repeat_to_the_bit(res, quadrupole, turn):
+    """The reference's rule with its groups (of 32 bodies, of 64) taken in order and the last
+    ones halved: a call gives the same bits every time, and graph-replayed steps those of eager
+    ones."""
+    import torch
+    from particular_gb300 import _native as N
+    L, n = N.lib(), turn * res.sm_count + 31
+    r = np.random.RandomState(7)
+    x = r.normal(size=(n, 3)) * r.uniform(0.1, 1, (n, 1))
+    b = torch.from_numpy(np.concatenate([x, np.full((n, 1), 1 / n)], 1).astype(np.float32)).cuda()
+    fl = N.PT_BH_QUADRUPOLE if quadrupole else 0
+    outs = [torch.empty((n, 3), device="cuda") for _ in range(4)]
+    torch.cuda.synchronize()
+    for o in outs:
+        N.check(L.pt_bh_accel_f32_device(res.handle, b.data_ptr(), n, b.data_ptr(), n, 0.9, 0.01, fl, o.data_ptr()))
+    res.synchronize()
+    assert all(torch.equal(outs[0].view(torch.int32), o.view(torch.int32)) for o in outs[1:])
+    end = []
+    for use_graph in (0, 1):
+        p, v, a = b.clone(), torch.zeros((n, 4), device="cuda"), outs[0].clone()
+        torch.cuda.synchronize()
+        for _ in range(2):
+            N.check(L.pt_leapfrog_device(res.handle, p.data_ptr(), v.data_ptr(), a.data_ptr(), n, 1e-3, 2,
+                                         N.PT_METHOD_BARNES_HUT, 0.9, 0.01, fl, use_graph))
+        res.synchronize()
+        end.append((p, v, a))
+    for e, g in zip(*end):
+        assert torch.equal(e.view(torch.int32), g.view(torch.int32))
