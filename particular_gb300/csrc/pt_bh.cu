@@ -31,11 +31,6 @@ int validate(const char *fn, size_t n_aff, size_t n_src, uint32_t flags) {
     return PT_OK;
 }
 
-static int sort_error(const char *fn, int err) {
-    if (err & ERR_SORT_BARRIER) return set_error(PT_ERR_TIMEOUT, "%s: a grid barrier of the sort gave up", fn);
-    return PT_OK;
-}
-
 }  // namespace bh
 }  // namespace pt
 
@@ -175,7 +170,6 @@ int pt_bh_accel_f32(pt_ctx *ctx, const float *aff, size_t n_aff, const float *sr
     int err = 0;
     if (n_src) PT_TRY(copies.to_host(&err, static_cast<int *>(S->counters.ptr) + 3, sizeof(int)));
     PT_TRY(copies.finish());
-    PT_TRY(bh::sort_error("pt_bh_accel_f32", err));
     if (err & 2)
         return set_error(PT_ERR_CAPACITY, "pt_bh_accel_f32: learned-correction records overflowed");
     return PT_OK;
@@ -226,7 +220,6 @@ int pt_bh_accel_dvec3(pt_ctx *ctx, const double *aff, size_t n_aff, const double
     int err = 0;
     if (n_src) PT_TRY(copies.to_host(&err, static_cast<int *>(S->counters.ptr) + 3, sizeof(int)));
     PT_TRY(copies.finish());
-    PT_TRY(bh::sort_error("pt_bh_accel_dvec3", err));
     if (err & 1) return set_error(PT_ERR_CAPACITY, "pt_bh_accel_dvec3: a warp's stack ran out; its bodies are NaN");
     return PT_OK;
 }
@@ -437,7 +430,6 @@ int pt_bh_walk(pt_ctx *ctx, const float *aff, size_t n_aff, float theta, float s
     int err = 0;
     PT_TRY(copies.to_host(&err, static_cast<int *>(S->counters.ptr) + 3, sizeof(int)));
     PT_TRY(copies.finish());
-    PT_TRY(bh::sort_error("pt_bh_walk", err));
     if (err & 2) return set_error(PT_ERR_CAPACITY, "pt_bh_walk: learned-correction records overflowed");
     return PT_OK;
 }

@@ -1063,8 +1063,7 @@ int build_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_src, int n) {
     launch_next(make_keys<T>, blocks(n), 256, 0, st, d_src, n, as<T>(S.box),
                 rf.keys ? rf.keys : as<uint64_t>(S.keys), rf.hist, rf.shift, rf.tile);
     PT_TRY(check_launch(ctx, "make_keys"));
-    PT_TRY(radix_sort_u64(ctx, S.prims, as<uint64_t>(S.keys), as<uint32_t>(S.idx), n, 3 * LEVELS,
-                          counters + 3));
+    PT_TRY(radix_sort_u64(ctx, S.prims, as<uint64_t>(S.keys), as<uint32_t>(S.idx), n, 3 * LEVELS));
     PT_TRY(scan_generated(ctx, S.prims, UnitHead{as<uint64_t>(S.keys)},
                           UnitFill{as<uint64_t>(S.keys), n, as<uint64_t>(S.ukey), as<uint32_t>(S.ufirst), counters}, n));
     const int nstages = stages(n), span_blocks = stage_first(n, nstages + 1);
@@ -1124,8 +1123,7 @@ int sort_targets_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_aff, int
     launch_next(make_keys<T>, blocks(n), 256, 0, st, d_aff, n, as<T>(S.box),
                 rf.keys ? rf.keys : as<uint64_t>(S.tkeys), rf.hist, rf.shift, rf.tile);
     PT_TRY(check_launch(ctx, "make_keys(targets)"));
-    PT_TRY(radix_sort_u64(ctx, S.prims, as<uint64_t>(S.tkeys), as<uint32_t>(S.tidx), n, 3 * LEVELS,
-                          as<int>(S.counters) + 3));
+    PT_TRY(radix_sort_u64(ctx, S.prims, as<uint64_t>(S.tkeys), as<uint32_t>(S.tidx), n, 3 * LEVELS));
     launch_next(gather_bodies<V4>, blocks(n), 256, 0, st, d_aff, as<uint32_t>(S.tidx), n, as<V4>(tb), as<int>(S.counters));
     return check_launch(ctx, "gather_bodies(targets)");
 }

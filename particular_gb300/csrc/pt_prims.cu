@@ -1,9 +1,10 @@
 // Stable radix sort of 63-bit keys and their bodies' indices, written for the Barnes-Hut build.
 //
-// The upper HEAD_BITS bits are sorted by LSD passes of 8-bit digits; bodies that share them
-// are few and next to each other then, and rs_finish orders each such run by the whole key.
-// Where a run is longer than RUN_LIMIT (a cluster far smaller than 2^-13 of the box), it
-// raises a flag and rs_all, launched in any case, sorts everything by all eight digits.
+// The upper bits (see head_shift) are sorted by LSD passes of 8-bit digits; bodies that share
+// them are few and next to each other then, and rs_finish orders each such run by the whole
+// key. The runs that are too long for it (a cluster far smaller than 2^-13 of the box) it puts
+// on a list; rs_runs, launched in any case, sorts these by their lower digits, a block or a
+// cluster of blocks to a run. Nothing in a sort waits on a block that may not be running.
 //
 // A pass ranks keys stably inside a tile (each warp its own run of keys, with warp
 // match/popc), so equal digits keep their input order, stages the tile in shared memory in
@@ -12,6 +13,8 @@
 // the next pass as it writes. Above, a histogram pass (per-tile counts) and a row scan (one
 // block per digit value over the tiles) come before the scatter.
 #include "pt_prims.cuh"
+
+#include <cooperative_groups.h>
 
 #include <algorithm>
 
@@ -129,7 +132,7 @@ struct ScatterShared {
 // between rounds); one scan over the warps per digit then orders the warps, so equal digits
 // keep their input order. gstart(t): where digit t's keys of this tile go. vin null: a key's
 // value is its index. next: null, or the digit counts by tile of the pass at next_shift. (All
-// reads go to L2: within rs_all other blocks have written what an earlier pass read.)
+// reads go to L2: within rs_runs other blocks have written what an earlier pass read.)
 template <int ROUNDS, class Start>
 __device__ __forceinline__ void scatter_tile(ScatterShared<ROUNDS> &S, const uint64_t *kin, const uint32_t *vin,
                                              uint64_t *kout, uint32_t *vout, int n, int shift, int b,
@@ -247,126 +250,133 @@ __global__ void __launch_bounds__(RS_THREADS)
 }
 
 // Orders every run of keys with the same upper bits (key >> shift) by the whole key, stably:
-// each key counts those of its run that come before it. Raises *redo (and leaves the output
-// to rs_all) where a run reaches further than RUN_LIMIT keys to one side.
-constexpr int RUN_LIMIT = 48;
+// each key counts those of its run that come before it. A run of more than RUN_LIMIT + 1 keys is
+// left to rs_runs: its first key puts it on the list of those for a block, or of those longer than
+// BLOCK_RUN, for a cluster. (Builds at limits of 48 / 128 / 256, us: N = 262144 in knots of
+// some 60 bodies 531 / 377 / 378, 100 477 / 397 / 388, 200 451 / 477 / 432, 400 399 / 425 / 462.)
+constexpr int RUN_LIMIT = 128;
+constexpr int BLOCK_RUN = 2 * RS_TILE;
+
+struct RunLists {  // the first keys of the long runs; count: [0] those for a block, [1] for a cluster
+    int *count, *block, *cluster;
+};
 
 __global__ void __launch_bounds__(256)
     rs_finish(const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin, int n, int shift,
-              uint64_t *__restrict__ kout, uint32_t *__restrict__ vout, int *__restrict__ redo) {
+              uint64_t *__restrict__ kout, uint32_t *__restrict__ vout, RunLists runs) {
     after_previous();
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= n) return;
     const uint64_t k = kin[i], h = k >> shift;
-    int lo = i, hi = i, before = 0;
-    while (lo > 0 && i - lo < RUN_LIMIT) {
-        const uint64_t x = kin[lo - 1];
-        if ((x >> shift) != h) break;
-        --lo;
-        before += x <= k;
+    const auto same = [&](int j) { return j >= 0 && j < n && (kin[j] >> shift) == h; };
+    int lo = i, before = 0;
+    const bool below = same(i - 1), above = same(i + 1);
+    if (below || above) {
+        if (same(i - RUN_LIMIT)) return;  // in a long run
+        if (same(i + RUN_LIMIT)) {
+            if (!below) {  // its first key
+                const bool big = same(i + BLOCK_RUN);
+                (big ? runs.cluster : runs.block)[atomicAdd(runs.count + big, 1)] = i;
+            }
+            return;
+        }
+        for (; same(lo - 1); --lo) before += kin[lo - 1] <= k;  // (ends within RUN_LIMIT)
+        for (int hi = i; same(hi + 1); ++hi) before += kin[hi + 1] < k;
     }
-    while (hi + 1 < n && hi - i < RUN_LIMIT) {
-        const uint64_t x = kin[hi + 1];
-        if ((x >> shift) != h) break;
-        ++hi;
-        before += x < k;
-    }
-    if (i - lo >= RUN_LIMIT || hi - i >= RUN_LIMIT) *redo = 1;
-    const int pos = lo + before;  // in [lo, hi]
+    const int pos = lo + before;  // in the run
     kout[pos] = k;
     vout[pos] = vin[i];
 }
 
-// A barrier over the grid of a cooperative launch: ctrl[0] arrivals, ctrl[1] generation. It
-// gives up after SPIN_LIMIT waits (all blocks then leave): returns false.
-constexpr int SPIN_LIMIT = 1 << 24;
-__device__ bool grid_barrier(unsigned *ctrl, volatile unsigned *failed) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned *gen = ctrl + 1;
-        const unsigned g = *gen;
-        __threadfence();
-        if (atomicAdd(ctrl, 1u) == gridDim.x - 1) {
-            atomicExch(ctrl, 0u);
-            __threadfence();
-            atomicAdd(ctrl + 1, 1u);
-        } else {
-            int it = 0;
-            while (*gen == g) {
-                if (++it > SPIN_LIMIT || *failed) {
-                    *failed = 1u;
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-        ok = *failed == 0u;
+// The long runs of (kb, vb) go sorted to (ka, va): three LSD passes over the bits below those
+// that a run's keys share, kb -> ka -> kb -> ka within the run's range. A block, or each
+// block of a cluster, takes neighbouring tiles and ranks them one after the other; where a
+// digit's keys of a block start it knows from the digit counts of the cluster's blocks
+// (distributed shared memory). A cluster's blocks run together by themselves, so its barrier
+// needs no room on the chip beyond eight blocks and no limit.
+constexpr int RUN_CLUSTER = 8, RUN_PASSES = 3;
+
+struct RunShared {
+    ScatterShared<RS_ROUNDS> tile;
+    uint32_t cnt[256];
+};
+
+// The first key behind the run that starts at `start` (which holds start + RUN_LIMIT); `end`: a
+// bound of it. Every thread of the block must call it.
+__device__ __forceinline__ int run_end(const uint64_t *keys, int start, int end, int shift) {
+    const uint64_t h = __ldcg(keys + start) >> shift;
+    int lo = start + RUN_LIMIT, hi = end;  // lo is in the run, hi is not
+    while (hi - lo > 1) {
+        const int step = (hi - lo + RS_THREADS - 1) / RS_THREADS;
+        const long long i = lo + (long long)(threadIdx.x + 1) * step;
+        const int in = __syncthreads_count(i < hi && (__ldcg(keys + i) >> shift) == h);
+        hi = int(min((long long)hi, lo + (long long)(in + 1) * step));
+        lo += in * step;
     }
-    __syncthreads();
-    return ok;
+    return hi;
 }
 
-// When *redo is set: sorts (kb, vb) by all eight digits into (ka, va), one cooperative launch.
-// ctrl: arrivals, generation, failed; a barrier that gave up is told in *err. When *redo is
-// not set every block leaves at once.
-__global__ void __launch_bounds__(RS_THREADS)
-    rs_all(uint64_t *ka, uint32_t *va, uint64_t *kb, uint32_t *vb, int n, int passes, uint32_t *hist, uint32_t *offs,
-           uint32_t *rowsum, int nblocks, const int *redo, unsigned *ctrl, int *err) {
-    if (*redo == 0) return;
-    auto barrier = [&]() {
-        const bool ok = grid_barrier(ctrl, ctrl + 2);
-        if (!ok && threadIdx.x == 0) atomicOr(err, ERR_SORT_BARRIER);
-        return ok;
-    };
-    __shared__ ScatterShared<RS_ROUNDS> S;
-    uint64_t *kin = kb, *kout = ka;
-    uint32_t *vin = vb, *vout = va;
-    const bool few = nblocks <= 64;  // the blocks add up the tiles' counts themselves: few blocks
-                                     // would each scan many rows
-    for (int p = 0; p < passes; ++p) {
-        for (int b = blockIdx.x; b < nblocks; b += gridDim.x) {
-            hist_tile(kin, n, 8 * p, hist, nblocks, b, S.tstart);
-            __syncthreads();
-        }
-        if (!barrier()) return;
-        if (!few) {
-            for (int d = blockIdx.x; d < 256; d += gridDim.x) scan_row(hist, offs, rowsum, nblocks, d, S.wsum);
-            if (!barrier()) return;
-        }
-        for (int b = blockIdx.x; b < nblocks; b += gridDim.x) {
-            scatter_tile(S, kin, vin, kout, vout, n, 8 * p, b,
-                         [&](int t) {
-                             if (few) {
-                                 uint32_t before = 0, total = 0;
+template <class Cluster>
+__device__ __forceinline__ void sort_run(RunShared &S, uint64_t *ka, uint32_t *va, uint64_t *kb, uint32_t *vb,
+                                         int len, const Cluster &cluster) {
+    const int t = threadIdx.x, rank = cluster.rank();
+    const int tiles = (len + RS_TILE - 1) / RS_TILE, per = (tiles + cluster.size() - 1) / cluster.size();
+    const int t0 = min(tiles, rank * per), t1 = min(tiles, t0 + per);
+    for (int p = 0; p < RUN_PASSES; ++p) {
+        const uint64_t *kin = p & 1 ? ka : kb;
+        const uint32_t *vin = p & 1 ? va : vb;
+        S.cnt[t] = 0;
+        __syncthreads();
+        const int end = min(len, t1 * RS_TILE);
 #pragma unroll 8
-                                 for (int j = 0; j < nblocks; ++j) {
-                                     const uint32_t h = __ldcg(hist + t * nblocks + j);
-                                     if (j < b) before += h;
-                                     total += h;
-                                 }
-                                 return block_excl_scan(total, S.wsum, nullptr) + before;
-                             }
-                             return block_excl_scan(__ldcg(rowsum + t), S.wsum, nullptr) +
-                                    __ldcg(offs + size_t(t) * nblocks + b);
-                         },
+        for (int i = t0 * RS_TILE + t; i < end; i += RS_THREADS) atomicAdd(&S.cnt[digit_of(__ldcg(kin + i), 8 * p)], 1u);
+        cluster.sync();
+        uint32_t before = 0, total = 0;
+        for (int r = 0; r < cluster.size(); ++r) {
+            const uint32_t c = cluster.count(&S.cnt[t], r);
+            if (r < rank) before += c;
+            total += c;
+        }
+        uint32_t start = block_excl_scan(total, S.tile.wsum, nullptr) + before;
+        for (int b = t0; b < t1; ++b) {
+            scatter_tile(S.tile, kin, vin, p & 1 ? kb : ka, p & 1 ? vb : va, len, 8 * p, b, [&](int) { return start; },
                          nullptr, 0);
+            const uint32_t next = t < 255 ? S.tile.tstart[t + 1] : uint32_t(min(RS_TILE, len - b * RS_TILE));
+            start += next - S.tile.tstart[t];
             __syncthreads();
         }
-        if (!barrier()) return;
-        uint64_t *tk = kin;
-        kin = kout;
-        kout = tk;
-        uint32_t *tv = vin;
-        vin = vout;
-        vout = tv;
+        cluster.sync();  // the pass is written and the counts are read
     }
-    if (kin == kb)  // the last pass wrote the other pair
-        for (int i = blockIdx.x * RS_THREADS + threadIdx.x; i < n; i += gridDim.x * RS_THREADS) {
-            ka[i] = __ldcg(kb + i);
-            va[i] = __ldcg(vb + i);
-        }
+}
+
+struct OneBlock {
+    __device__ int rank() const { return 0; }
+    __device__ int size() const { return 1; }
+    __device__ void sync() const { __syncthreads(); }
+    __device__ uint32_t count(const uint32_t *c, int) const { return *c; }
+};
+struct BlockCluster {
+    cooperative_groups::cluster_group group = cooperative_groups::this_cluster();
+    __device__ int rank() const { return int(group.block_rank()); }
+    __device__ int size() const { return RUN_CLUSTER; }
+    __device__ void sync() const { group.sync(); }
+    __device__ uint32_t count(uint32_t *c, int r) const { return *group.map_shared_rank(c, r); }
+};
+
+__global__ void __cluster_dims__(RUN_CLUSTER, 1, 1) __launch_bounds__(RS_THREADS)
+    rs_runs(uint64_t *ka, uint32_t *va, uint64_t *kb, uint32_t *vb, int n, int shift, RunLists runs) {
+    after_previous();
+    __shared__ RunShared S;
+    const int few = runs.count[0], many = runs.count[1];
+    const BlockCluster cluster;
+    for (int r = blockIdx.x / RUN_CLUSTER; r < many; r += gridDim.x / RUN_CLUSTER) {
+        const int i = runs.cluster[r], end = run_end(kb, i, n, shift);
+        sort_run(S, ka + i, va + i, kb + i, vb + i, end - i, cluster);
+    }
+    for (int r = blockIdx.x; r < few; r += gridDim.x) {
+        const int i = runs.block[r], end = run_end(kb, i, min(n, i + BLOCK_RUN), shift);
+        sort_run(S, ka + i, va + i, kb + i, vb + i, end - i, OneBlock{});
+    }
 }
 
 }  // namespace prims
@@ -374,6 +384,7 @@ __global__ void __launch_bounds__(RS_THREADS)
 // The first sorted bit of n keys: five digits from the top (13 octree levels and a bit) leave
 // runs of a few bodies at 4M bulge+disk; a sixth from 8M on.
 static int head_shift(int n, int bits) { return std::max(0, bits - 8 * (n >= (1 << 23) ? 6 : 5)); }
+static_assert(63 - 8 * 5 <= 8 * prims::RUN_PASSES, "the runs' passes sort all lower bits");
 
 namespace prims {
 // How a sort of n keys is laid out: tiles of the direct passes (rounds = 0: three launches a
@@ -389,9 +400,9 @@ struct SortPlan {
           tiles((n + tile - 1) / tile),
           blocks((n + RS_TILE - 1) / RS_TILE),
           nhist(256 * size_t(blocks)) {
-        // counts per pass of the direct passes; counts, offsets and row sums; then the redo
-        // flag and the barrier of rs_all
-        words = std::max(rounds ? size_t(passes) * 256 * tiles : 0, 2 * nhist + 256) + 64;
+        // counts per pass of the direct passes, or counts, offsets and row sums; where these
+        // were, the lists of long runs; then the lengths of the lists
+        words = (rounds ? size_t(passes) * 256 * tiles : 2 * nhist + 256) + 64;
     }
 };
 }  // namespace prims
@@ -413,13 +424,11 @@ int radix_sort_prepare(pt_ctx *ctx, PrimScratch &s, int n, int bits, RadixFirst 
     return PT_OK;
 }
 
-int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, int n, int bits, int *err) {
+int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, int n, int bits) {
     using namespace prims;
     const SortPlan sp(n, bits);
     const int nblocks = sp.blocks, shift0 = sp.shift, passes = sp.passes;
     uint32_t *hist = static_cast<uint32_t *>(s.hist.ptr);
-    int *redo = reinterpret_cast<int *>(hist + (sp.words - 64));
-    unsigned *ctrl = reinterpret_cast<unsigned *>(redo + 16);
     uint32_t *offs = hist + sp.nhist, *rowsum = offs + sp.nhist;
     uint64_t *kb = static_cast<uint64_t *>(s.keys2.ptr), *k[2] = {keys, kb};
     uint32_t *vb = static_cast<uint32_t *>(s.vals2.ptr), *v[2] = {vals, vb};
@@ -447,17 +456,16 @@ int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, 
                     nblocks);
         PT_TRY(check_launch(ctx, "rs_scatter"));
     }
-    launch_next(rs_finish, (n + 255) / 256, 256, 0, st, kb, vb, n, shift0, keys, vals, redo);
+    int *lists = reinterpret_cast<int *>(hist);  // the passes' counts are read
+    const RunLists runs{reinterpret_cast<int *>(hist + (sp.words - 64)), lists,
+                        lists + n / (RUN_LIMIT + 1) + 1};
+    launch_next(rs_finish, (n + 255) / 256, 256, 0, st, kb, vb, n, shift0, keys, vals, runs);
     PT_TRY(check_launch(ctx, "rs_finish"));
-    int all = (bits + 7) / 8, nb = nblocks;
-    void *args[] = {&keys, &vals, &kb, &vb, &n, &all, &hist, &offs, &rowsum, &nb, &redo, &ctrl, &err};
-    static const int per_sm = [] {  // blocks that are resident together
-        int b = 0;
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rs_all, RS_THREADS, 0) == cudaSuccess ? std::max(1, b) : 1;
-    }();
-    const int grid = std::min(nblocks, per_sm * std::max(1, ctx->sm_count));
-    PT_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(rs_all), dim3(grid), dim3(RS_THREADS), args, 0, st));
-    return check_launch(ctx, "rs_all");
+    // runs for a block are shorter than two tiles and longer than half a block's threads: one
+    // block to 256 keys, up to four an SM
+    const int grid = std::min(n / 256, 4 * std::max(1, ctx->sm_count)) / RUN_CLUSTER * RUN_CLUSTER;
+    launch_next(rs_runs, std::max(RUN_CLUSTER, grid), RS_THREADS, 0, st, keys, vals, kb, vb, n, shift0, runs);
+    return check_launch(ctx, "rs_runs");
 }
 
 void prim_free(pt_ctx *ctx, PrimScratch &s) {

@@ -19,8 +19,7 @@ struct PrimScratch {
 // for small n, to count their first digits: hist[(i / tile) * 256 + (key >> shift & 255)]
 // for key i where hist is not null. radix_sort_u64 then leaves the keys ascending by
 // their low `bits` bits in keys, equal ones in the order of their index, and their indices in
-// vals. *err (device) gets ERR_SORT_BARRIER where a grid barrier of the general path gave up.
-constexpr int ERR_SORT_BARRIER = 4;
+// vals.
 struct RadixFirst {
     uint64_t *keys;
     uint32_t *hist;
@@ -29,7 +28,7 @@ struct RadixFirst {
     int zero_words;
 };
 int radix_sort_prepare(pt_ctx *ctx, PrimScratch &s, int n, int bits, RadixFirst *first);
-int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, int n, int bits, int *err);
+int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, int n, int bits);
 
 void prim_free(pt_ctx *ctx, PrimScratch &s);
 

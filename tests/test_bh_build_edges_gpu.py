@@ -104,3 +104,29 @@ def test_bodies_are_in_key_order(res, n, kind):
     assert np.array_equal(count, np.unique(key, return_counts=True)[1])
     single = count == 1
     assert np.array_equal(g["com_mass"][~leaves][single], b[order[first[single]]])
+
+
+# runs of bodies that share the bits the sort's passes sort, of lengths about those where
+# another kernel takes the run: a thread per body, a block, a cluster of blocks, one and
+# several tiles
+@pytest.mark.parametrize("seed,long", [(0, 0), (1, 20000), (2, 70001), (3, 300000)])
+def test_long_runs_of_close_bodies_are_in_key_order(res, seed, long):
+    r = np.random.RandomState(seed)
+    lengths = np.array([1, 2, 127, 128, 129, 130, 255, 256, 257, 2047, 2048, 2049, 4095, 4096, 4097, 4098, 16384, 16385,
+                        1 + long])
+    lengths = r.permutation(np.concatenate([lengths, r.randint(1, 400, 60)]))
+    cell = 2.0 ** -13  # the box is [-1, 1]: cells of the 14th level
+    knot = (r.randint(-8000, 8000, (len(lengths), 3)) + 0.5) * cell
+    x = np.repeat(knot, lengths, axis=0) + r.uniform(-0.12, 0.12, (lengths.sum(), 3)) * cell
+    x = np.concatenate([x, [[-1, -1, -1], [1, 1, 1]]])[r.permutation(lengths.sum() + 2)]
+    b = np.concatenate([x, np.ones((len(x), 1))], 1).astype(np.float32)
+    order, key = reference_order(b)
+    runs = np.unique(key >> np.uint64(23), return_counts=True)[1]
+    assert np.isin([128, 129, 130, 4096, 4097], runs).all() and runs.max() >= max(16385, long)
+    g = tree_of(res, b)
+    leaves = g["links"][:, 2] < 0
+    first, count = g["links"][~leaves, 2], g["links"][~leaves, 3]
+    assert count.sum() == len(b) and np.array_equal(first, np.cumsum(count) - count)
+    assert np.array_equal(count, np.unique(key, return_counts=True)[1])
+    single = count == 1
+    assert np.array_equal(g["com_mass"][~leaves][single], b[order[first[single]]])
