@@ -133,20 +133,66 @@ __device__ __forceinline__ uint64_t key_of(T px, T py, T pz, const T *box) {
     return key;
 }
 
-// hist (small n): the counts of the sort's first digit by tile of keys.
+// Sets *deep where the bodies crowd into cells that the sort's upper bits (key >> shift) do not
+// tell apart, some CROWD of them or more to a cell. SAMPLES bodies are looked at: of these,
+// SAMPLES^2 / 2 x (the mean run) / n share their cell with an earlier one. One block; it costs the
+// smallest call that has it 4 us and larger ones, where it ends before the other blocks, nothing.
+// CROWD: runs of a thread per key (up to 129) cost less than the three passes of the whole
+// chip, longer ones more (N = 1M in knots of some 60 bodies, below the line, 654 us, of some
+// 200, above it, 647, which took 962 without the passes).
+constexpr int SAMPLES = 1024, CROWD = 100;
+
 template <class T>
-__global__ void make_keys(const typename Prec<T>::V4 *__restrict__ bodies, int n, const T *__restrict__ box_g,
-                          uint64_t *__restrict__ keys, uint32_t *__restrict__ hist, int shift, int tile) {
+__device__ __forceinline__ void sample_keys(const typename Prec<T>::V4 *__restrict__ bodies, int n, const T *box,
+                                            int shift, int *deep) {
+    constexpr unsigned long long EMPTY = ~0ull;
+    __shared__ unsigned long long seen[2 * SAMPLES];
+    __shared__ int shared;
+    for (int i = threadIdx.x; i < 2 * SAMPLES; i += blockDim.x) seen[i] = EMPTY;
+    if (threadIdx.x == 0) shared = 0;
+    __syncthreads();
+    unsigned long long h[SAMPLES / 256];
+#pragma unroll
+    for (int s = 0; s < SAMPLES / 256; ++s) {
+        const typename Prec<T>::V4 p = bodies[(long long)(256 * s + threadIdx.x) * n / SAMPLES];
+        h[s] = key_of<T>(p.x, p.y, p.z, box) >> shift;
+    }
+#pragma unroll
+    for (int s = 0; s < SAMPLES / 256; ++s)
+        for (unsigned at = unsigned((h[s] * 0x9e3779b97f4a7c15ull) >> 32);; ++at) {
+            const unsigned long long was = atomicCAS(&seen[at % (2 * SAMPLES)], EMPTY, h[s]);
+            if (was == h[s]) atomicAdd(&shared, 1);
+            if (was == EMPTY || was == h[s]) break;
+        }
+    __syncthreads();
+    if (threadIdx.x == 0 && (long long)shared * n >= (long long)CROWD * SAMPLES * SAMPLES / 2) *deep = 1;
+}
+
+// hist (small n): the counts of the sort's first digit by tile of keys. SAMPLE (large n): the
+// first block samples instead.
+template <class T, bool SAMPLE>
+__global__ void __launch_bounds__(256)
+    make_keys(const typename Prec<T>::V4 *__restrict__ bodies, int n, const T *__restrict__ box_g,
+              uint64_t *__restrict__ keys, uint32_t *__restrict__ hist, int shift, int tile, int *deep) {
     after_previous();
     __shared__ T box[6];
     if (threadIdx.x < 6) box[threadIdx.x] = box_g[threadIdx.x];
     __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (SAMPLE && blockIdx.x == 0) return sample_keys<T>(bodies, n, box, shift, deep);
+    const int i = (blockIdx.x - SAMPLE) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const typename Prec<T>::V4 p = bodies[i];
     const uint64_t k = key_of<T>(p.x, p.y, p.z, box);
     keys[i] = k;
     if (hist) atomicAdd(&hist[(i / tile) * 256 + (int(k >> shift) & 255)], 1u);
+}
+
+template <class T>
+static int launch_make_keys(pt_ctx *ctx, const typename Prec<T>::V4 *bodies, int n, const T *box, uint64_t *keys,
+                            const RadixFirst &rf) {
+    launch_next(rf.deep ? make_keys<T, true> : make_keys<T, false>, blocks(n) + (rf.deep ? 1 : 0), 256, 0, ctx->stream,
+                bodies, n, box, rf.keys ? rf.keys : keys, rf.hist, rf.shift, rf.tile, rf.deep);
+    return check_launch(ctx, "make_keys");
 }
 
 // The walk's counters (counters + 4 ints) start from zero.
@@ -1060,9 +1106,7 @@ int build_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_src, int n) {
     launch_next(root_box<T>, nb, 256, 0, st, d_src, n, as<T>(S.box_part), as<T>(S.box), rf.zero, rf.zero_words,
                 ctx->keep_errors ? nullptr : counters + 3, reinterpret_cast<unsigned *>(counters) + ROOT_BOX_DONE);
     PT_TRY(check_launch(ctx, "root_box"));
-    launch_next(make_keys<T>, blocks(n), 256, 0, st, d_src, n, as<T>(S.box),
-                rf.keys ? rf.keys : as<uint64_t>(S.keys), rf.hist, rf.shift, rf.tile);
-    PT_TRY(check_launch(ctx, "make_keys"));
+    PT_TRY(launch_make_keys<T>(ctx, d_src, n, as<T>(S.box), as<uint64_t>(S.keys), rf));
     PT_TRY(radix_sort_u64(ctx, S.prims, as<uint64_t>(S.keys), as<uint32_t>(S.idx), n, 3 * LEVELS));
     PT_TRY(scan_generated(ctx, S.prims, UnitHead{as<uint64_t>(S.keys)},
                           UnitFill{as<uint64_t>(S.keys), n, as<uint64_t>(S.ukey), as<uint32_t>(S.ufirst), counters}, n));
@@ -1120,9 +1164,7 @@ int sort_targets_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_aff, int
     RadixFirst rf{};
     PT_TRY(radix_sort_prepare(ctx, S.prims, n, 3 * LEVELS, &rf));
     PT_CUDA(cudaMemsetAsync(rf.zero, 0, sizeof(uint32_t) * size_t(rf.zero_words), st));
-    launch_next(make_keys<T>, blocks(n), 256, 0, st, d_aff, n, as<T>(S.box),
-                rf.keys ? rf.keys : as<uint64_t>(S.tkeys), rf.hist, rf.shift, rf.tile);
-    PT_TRY(check_launch(ctx, "make_keys(targets)"));
+    PT_TRY(launch_make_keys<T>(ctx, d_aff, n, as<T>(S.box), as<uint64_t>(S.tkeys), rf));
     PT_TRY(radix_sort_u64(ctx, S.prims, as<uint64_t>(S.tkeys), as<uint32_t>(S.tidx), n, 3 * LEVELS));
     launch_next(gather_bodies<V4>, blocks(n), 256, 0, st, d_aff, as<uint32_t>(S.tidx), n, as<V4>(tb), as<int>(S.counters));
     return check_launch(ctx, "gather_bodies(targets)");

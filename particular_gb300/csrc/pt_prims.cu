@@ -4,7 +4,9 @@
 // them are few and next to each other then, and rs_finish orders each such run by the whole
 // key. The runs that are too long for it (a cluster far smaller than 2^-13 of the box) it puts
 // on a list; rs_runs, launched in any case, sorts these by their lower digits, a block or a
-// cluster of blocks to a run. Nothing in a sort waits on a block that may not be running.
+// cluster of blocks to a run. Where much of a large input is in such runs (a sample of the keys
+// tells) three passes over the lower bits come first instead. Nothing in a sort waits on a
+// block that may not be running.
 //
 // A pass ranks keys stably inside a tile (each warp its own run of keys, with warp
 // match/popc), so equal digits keep their input order, stages the tile in shared memory in
@@ -81,11 +83,28 @@ __device__ __forceinline__ void hist_tile(const uint64_t *__restrict__ keys, int
     hist[size_t(threadIdx.x) * nblocks + b] = cnt[threadIdx.x];
 }
 
-__global__ void __launch_bounds__(RS_THREADS)
-    rs_hist(const uint64_t *__restrict__ keys, int n, int shift, uint32_t *__restrict__ hist, int nblocks) {
+// Where bodies crowd (*deep), LOW_PASSES over the lower bits come before the passes of three
+// launches over the upper ones, which then start from the other pair of buffers. (In long runs
+// for a few clusters of blocks a large tree's bodies take longer than in the passes that the whole
+// chip makes: builds without and with them, us, N = 1M in two knots 1e-5 of the box wide 1018 /
+// 499, a Plummer sphere with one body 2e4 away 887 / 444; 4M 3387 / 1268 and 3160 / 1452. The
+// launches that find nothing to do cost every other build above 262144 bodies 8 us, of 190 and more.)
+constexpr int LOW_PASSES = 3;
+
+// A pass of three launches, from pair `in` of the buffers (the other if *deep) to the other.
+// first: unless *deep, a key's value is its index.
+struct Pass {
+    uint64_t *k0, *k1;
+    uint32_t *v0, *v1;
+    const int *deep;
+    int shift, in;
+    bool first;
+};
+
+__global__ void __launch_bounds__(RS_THREADS) rs_hist(Pass p, int n, uint32_t *__restrict__ hist, int nblocks) {
     after_previous();
     __shared__ uint32_t cnt[256];
-    hist_tile(keys, n, shift, hist, nblocks, blockIdx.x, cnt);
+    hist_tile(p.in ^ *p.deep ? p.k1 : p.k0, n, p.shift, hist, nblocks, blockIdx.x, cnt);
 }
 
 // Digit d: offs[d * nblocks + b] = count of digit d in tiles before b, rowsum[d] = count of
@@ -199,16 +218,71 @@ __device__ __forceinline__ void scatter_tile(ScatterShared<ROUNDS> &S, const uin
 }
 
 __global__ void __launch_bounds__(RS_THREADS)
-    rs_scatter(const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin, uint64_t *__restrict__ kout,
-               uint32_t *__restrict__ vout, int n, int shift, const uint32_t *__restrict__ offs,
-               const uint32_t *__restrict__ rowsum, int nblocks) {
+    rs_scatter(Pass p, int n, const uint32_t *__restrict__ offs, const uint32_t *__restrict__ rowsum, int nblocks) {
     after_previous();
     __shared__ ScatterShared<RS_ROUNDS> S;
-    const int b = blockIdx.x;
+    const int b = blockIdx.x, deep = *p.deep, in = p.in ^ deep;
+    const uint32_t *vin = p.first && !deep ? nullptr : in ? p.v1 : p.v0;
     // all smaller digits, then earlier tiles
-    scatter_tile(S, kin, vin, kout, vout, n, shift, b,
+    scatter_tile(S, in ? p.k1 : p.k0, vin, in ? p.k0 : p.k1, in ? p.v0 : p.v1, n, p.shift, b,
                  [&](int t) { return block_excl_scan(rowsum[t], S.wsum, nullptr) + offs[size_t(t) * nblocks + b]; },
                  nullptr, 0);
+}
+
+// The passes over the lower bits take two launches: counts by tile and by span of tiles, then
+// every block adds up the spans and the tiles of its own span. Most calls need none of them, so
+// they are few, with few blocks, and leave at once.
+struct LowPass {
+    const uint64_t *kin;
+    const uint32_t *vin;
+    uint64_t *kout;
+    uint32_t *vout;
+    const int *deep;
+    int n, shift, tiles, span;
+    uint32_t *cnt, *sum;  // [tile][256], [span][256] (zero)
+};
+
+__global__ void __launch_bounds__(RS_THREADS) rs_low_count(LowPass p) {
+    after_previous();
+    if (!*p.deep) return;
+    __shared__ uint32_t cnt[256];
+    const int t = threadIdx.x;
+    for (int b = blockIdx.x; b < p.tiles; b += gridDim.x) {
+        cnt[t] = 0;
+        __syncthreads();
+        const size_t end = min(size_t(p.n), size_t(b + 1) * RS_TILE);
+#pragma unroll 4
+        for (size_t i = size_t(b) * RS_TILE + t; i < end; i += RS_THREADS)
+            atomicAdd(&cnt[digit_of(__ldcg(p.kin + i), p.shift)], 1u);
+        __syncthreads();
+        const uint32_t c = cnt[t];
+        p.cnt[size_t(b) * 256 + t] = c;
+        if (c) atomicAdd(&p.sum[size_t(b / p.span) * 256 + t], c);
+    }
+}
+
+__global__ void __launch_bounds__(RS_THREADS) rs_low_scatter(LowPass p) {
+    after_previous();
+    if (!*p.deep) return;
+    __shared__ ScatterShared<RS_ROUNDS> S;
+    for (int b = blockIdx.x; b < p.tiles; b += gridDim.x) {
+        scatter_tile(S, p.kin, p.vin, p.kout, p.vout, p.n, p.shift, b,
+                     [&](int t) {
+                         const int mine = b / p.span, spans = (p.tiles + p.span - 1) / p.span;
+                         uint32_t before = 0, total = 0;
+#pragma unroll 8
+                         for (int j = 0; j < spans; ++j) {
+                             const uint32_t c = p.sum[size_t(j) * 256 + t];
+                             if (j < mine) before += c;
+                             total += c;
+                         }
+#pragma unroll 8
+                         for (int j = mine * p.span; j < b; ++j) before += p.cnt[size_t(j) * 256 + t];
+                         return block_excl_scan(total, S.wsum, nullptr) + before;
+                     },
+                     nullptr, 0);
+        __syncthreads();
+    }
 }
 
 // One pass in one launch: hist[b * 256 + d] holds the tiles' digit counts.
@@ -263,8 +337,9 @@ struct RunLists {  // the first keys of the long runs; count: [0] those for a bl
 
 __global__ void __launch_bounds__(256)
     rs_finish(const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin, int n, int shift,
-              uint64_t *__restrict__ kout, uint32_t *__restrict__ vout, RunLists runs) {
+              uint64_t *__restrict__ kout, uint32_t *__restrict__ vout, const int *__restrict__ deep, RunLists runs) {
     after_previous();
+    if (deep && *deep) return;  // sorted by all bits, and in (kout, vout)
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= n) return;
     const uint64_t k = kin[i], h = k >> shift;
@@ -384,14 +459,16 @@ __global__ void __cluster_dims__(RUN_CLUSTER, 1, 1) __launch_bounds__(RS_THREADS
 // The first sorted bit of n keys: five digits from the top (13 octree levels and a bit) leave
 // runs of a few bodies at 4M bulge+disk; a sixth from 8M on.
 static int head_shift(int n, int bits) { return std::max(0, bits - 8 * (n >= (1 << 23) ? 6 : 5)); }
-static_assert(63 - 8 * 5 <= 8 * prims::RUN_PASSES, "the runs' passes sort all lower bits");
+static_assert(63 - 8 * 5 <= 8 * prims::RUN_PASSES && 63 - 8 * 5 <= 8 * prims::LOW_PASSES, "all lower bits are sorted");
+static_assert(prims::LOW_PASSES % 2 == 1, "the upper passes then start from the other pair");
 
 namespace prims {
 // How a sort of n keys is laid out: tiles of the direct passes (rounds = 0: three launches a
 // pass) and words of histograms.
 struct SortPlan {
     int shift, passes, rounds, tile, tiles, blocks;
-    size_t nhist, words;
+    int span, spans;  // tiles to a span of the low passes
+    size_t nhist, sums, words;  // words: those of the low passes' spans from sums on, then the flags
     SortPlan(int n, int bits)
         : shift(head_shift(n, bits)),
           passes((bits - shift + 7) / 8),
@@ -399,10 +476,13 @@ struct SortPlan {
           tile(RS_THREADS * (rounds ? rounds : RS_ROUNDS)),
           tiles((n + tile - 1) / tile),
           blocks((n + RS_TILE - 1) / RS_TILE),
+          span(blocks <= 4096 ? 64 : 512),
+          spans((blocks + span - 1) / span),
           nhist(256 * size_t(blocks)) {
         // counts per pass of the direct passes, or counts, offsets and row sums; where these
-        // were, the lists of long runs; then the lengths of the lists
-        words = (rounds ? size_t(passes) * 256 * tiles : 2 * nhist + 256) + 64;
+        // were, the lists of long runs; then the lengths of the lists and the deep flag
+        sums = rounds ? size_t(passes) * 256 * tiles : 2 * nhist + 256;
+        words = sums + (rounds ? 0 : LOW_PASSES * 256 * size_t(spans)) + 64;
     }
 };
 }  // namespace prims
@@ -414,13 +494,14 @@ int radix_sort_prepare(pt_ctx *ctx, PrimScratch &s, int n, int bits, RadixFirst 
     PT_TRY(ensure_buf(ctx, s.vals2, sizeof(uint32_t) * size_t(n)));
     PT_TRY(ensure_buf(ctx, s.hist, sizeof(uint32_t) * p.words));
     uint32_t *hist = static_cast<uint32_t *>(s.hist.ptr);
-    first->zero = p.rounds ? hist : hist + (p.words - 64);
-    first->zero_words = p.rounds ? int(p.words) : 64;
+    first->zero = p.rounds ? hist : hist + p.sums;
+    first->zero_words = int(p.rounds ? p.words : p.words - p.sums);
     // an odd number of passes ends in the pair that the finishing pass reads
     first->keys = (p.passes & 1) ? nullptr : static_cast<uint64_t *>(s.keys2.ptr);
     first->hist = p.rounds ? hist : nullptr;
     first->shift = p.shift;
     first->tile = p.tile;
+    first->deep = p.rounds ? nullptr : reinterpret_cast<int *>(hist + (p.words - 64)) + 2;
     return PT_OK;
 }
 
@@ -433,33 +514,52 @@ int radix_sort_u64(pt_ctx *ctx, PrimScratch &s, uint64_t *keys, uint32_t *vals, 
     uint64_t *kb = static_cast<uint64_t *>(s.keys2.ptr), *k[2] = {keys, kb};
     uint32_t *vb = static_cast<uint32_t *>(s.vals2.ptr), *v[2] = {vals, vb};
     cudaStream_t st = ctx->stream;
-    int in = (passes & 1) ? 0 : 1;  // the passes end in (kb, vb)
-    for (int p = 0; p < passes; ++p, in ^= 1) {
-        const int shift = shift0 + 8 * p;
-        const uint32_t *vin = p == 0 ? nullptr : v[in];
-        if (sp.rounds) {
+    int *flags = reinterpret_cast<int *>(hist + (sp.words - 64));
+    const int in0 = (passes & 1) ? 0 : 1;  // the passes end in (kb, vb)
+    if (sp.rounds) {
+        for (int p = 0, in = in0; p < passes; ++p, in ^= 1) {
+            const int shift = shift0 + 8 * p;
             const size_t direct = 256 * size_t(sp.tiles);
             uint32_t *next = p + 1 < passes ? hist + (p + 1) * direct : nullptr;
             launch_next(sp.rounds == 1   ? rs_pass<1>
                         : sp.rounds == 4 ? rs_pass<4>
                                          : rs_pass<8>,
-                        sp.tiles, RS_THREADS, 0, st, k[in], vin, k[in ^ 1], v[in ^ 1], n, shift, hist + p * direct,
-                        sp.tiles, next, shift + 8);
+                        sp.tiles, RS_THREADS, 0, st, k[in], p == 0 ? nullptr : v[in], k[in ^ 1], v[in ^ 1], n, shift,
+                        hist + p * direct, sp.tiles, next, shift + 8);
             PT_TRY(check_launch(ctx, "rs_pass"));
-            continue;
         }
-        launch_next(rs_hist, nblocks, RS_THREADS, 0, st, k[in], n, shift, hist, nblocks);
-        PT_TRY(check_launch(ctx, "rs_hist"));
-        launch_next(rs_rowscan, 256, RS_THREADS, 0, st, hist, offs, rowsum, nblocks);
-        PT_TRY(check_launch(ctx, "rs_rowscan"));
-        launch_next(rs_scatter, nblocks, RS_THREADS, 0, st, k[in], vin, k[in ^ 1], v[in ^ 1], n, shift, offs, rowsum,
-                    nblocks);
-        PT_TRY(check_launch(ctx, "rs_scatter"));
+    } else {
+        const int few = std::min(nblocks, 4 * std::max(1, ctx->sm_count));
+        for (int p = 0, in = in0; p < LOW_PASSES; ++p, in ^= 1) {
+            // the lowest bits, the middle ones and those up to shift0, overlapping
+            const LowPass q{k[in],     p == 0 ? nullptr : v[in],
+                            k[in ^ 1], v[in ^ 1],
+                            flags + 2, n,
+                            p * (shift0 - 8) / (LOW_PASSES - 1), nblocks,
+                            sp.span,   hist,
+                            hist + sp.sums + p * 256 * size_t(sp.spans)};
+            launch_next(rs_low_count, few, RS_THREADS, 0, st, q);
+            PT_TRY(check_launch(ctx, "rs_low_count"));
+            launch_next(rs_low_scatter, few, RS_THREADS, 0, st, q);
+            PT_TRY(check_launch(ctx, "rs_low_scatter"));
+        }
+        Pass q{k[0], k[1], v[0], v[1], flags + 2};
+        for (int p = 0; p < passes; ++p) {
+            q.shift = shift0 + 8 * p;
+            q.in = in0 ^ (p & 1);
+            q.first = p == 0;
+            launch_next(rs_hist, nblocks, RS_THREADS, 0, st, q, n, hist, nblocks);
+            PT_TRY(check_launch(ctx, "rs_hist"));
+            launch_next(rs_rowscan, 256, RS_THREADS, 0, st, hist, offs, rowsum, nblocks);
+            PT_TRY(check_launch(ctx, "rs_rowscan"));
+            launch_next(rs_scatter, nblocks, RS_THREADS, 0, st, q, n, offs, rowsum, nblocks);
+            PT_TRY(check_launch(ctx, "rs_scatter"));
+        }
     }
     int *lists = reinterpret_cast<int *>(hist);  // the passes' counts are read
-    const RunLists runs{reinterpret_cast<int *>(hist + (sp.words - 64)), lists,
-                        lists + n / (RUN_LIMIT + 1) + 1};
-    launch_next(rs_finish, (n + 255) / 256, 256, 0, st, kb, vb, n, shift0, keys, vals, runs);
+    const RunLists runs{flags, lists, lists + n / (RUN_LIMIT + 1) + 1};
+    launch_next(rs_finish, (n + 255) / 256, 256, 0, st, kb, vb, n, shift0, keys, vals,
+                sp.rounds ? nullptr : flags + 2, runs);
     PT_TRY(check_launch(ctx, "rs_finish"));
     // runs for a block are shorter than two tiles and longer than half a block's threads: one
     // block to 256 keys, up to four an SM

@@ -24,6 +24,8 @@ struct RadixFirst {
     uint64_t *keys;
     uint32_t *hist;
     int shift, tile;
+    // n large, else null: the producer sets it where many keys share their bits from shift on
+    int *deep;
     uint32_t *zero;  // words that have to be zero before the keys are produced
     int zero_words;
 };

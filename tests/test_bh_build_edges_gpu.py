@@ -130,3 +130,32 @@ def test_long_runs_of_close_bodies_are_in_key_order(res, seed, long):
     assert np.array_equal(count, np.unique(key, return_counts=True)[1])
     single = count == 1
     assert np.array_equal(g["com_mass"][~leaves][single], b[order[first[single]]])
+
+
+# three launches a pass from 262145 bodies on: where many share the upper bits the lower ones are
+# sorted first; where few do, the few long runs are sorted by themselves
+@pytest.mark.parametrize("spread,crowded", [(300000, False), (0, True), (150000, True)])
+def test_large_trees_with_long_runs_are_in_key_order(res, spread, crowded):
+    r = np.random.RandomState(spread + 1)
+    lengths = np.concatenate([[127, 128, 129, 130, 2048, 2049, 4096, 4097, 6000], r.randint(1, 400, 20)])
+    if crowded:
+        lengths = np.concatenate([lengths, r.randint(50, 3000, 200)])
+    cell = 2.0 ** -13
+    knot = (r.randint(-8000, 8000, (len(lengths), 3)) + 0.5) * cell
+    x = np.repeat(knot, lengths, axis=0) + r.uniform(-0.12, 0.12, (lengths.sum(), 3)) * cell
+    x = np.concatenate([x, r.uniform(-1, 1, (spread, 3)), [[-1, -1, -1], [1, 1, 1]]])
+    x = x[r.permutation(len(x))]
+    assert len(x) > 262144
+    b = np.concatenate([x, np.ones((len(x), 1))], 1).astype(np.float32)
+    order, key = reference_order(b)
+    # of 1024 bodies, how many share their cell with an earlier one: far from the turn
+    some = key[np.arange(1024) * len(b) // 1024] >> np.uint64(23)
+    shared = 1024 - len(np.unique(some))
+    assert shared * len(b) > 2 * 52428800 if crowded else shared * len(b) < 52428800 / 2
+    g = tree_of(res, b)
+    leaves = g["links"][:, 2] < 0
+    first, count = g["links"][~leaves, 2], g["links"][~leaves, 3]
+    assert count.sum() == len(b) and np.array_equal(first, np.cumsum(count) - count)
+    assert np.array_equal(count, np.unique(key, return_counts=True)[1])
+    single = count == 1
+    assert np.array_equal(g["com_mass"][~leaves][single], b[order[first[single]]])
