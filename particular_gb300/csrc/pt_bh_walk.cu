@@ -655,11 +655,15 @@ __device__ __forceinline__ void
                 unsigned q0 = b0, q1 = b1;
                 // A body does not meet itself in the leaf: only one in the group's box can be at
                 // a body of the group. (Voting on every leaf body: 1M bodies, all but 20 within
-                // 1e-5 of the box, 14.5 ms a walk, and 8.9 like this.)
+                // 1e-5 of the box, 14.5 ms a walk, and 8.9 like this.) With softening it may: it
+                // adds 0 times a factor that is finite for eps >= 1e-6 and masses up to 1e20. (With
+                // the votes and without, us a walk: 524288 bodies in two knots 1e-5 of the box wide
+                // 1014 / 968, 1M 1985 / 1875, 1M in knots of some 200 718 / 644.)
                 const float e0 = fmaxf(fmaxf(mn0 - q.x, q.x - mx0), 0.0f);
                 const float e1 = fmaxf(fmaxf(mn1 - q.y, q.y - mx1), 0.0f);
                 const float e2b = fmaxf(fmaxf(mn2 - q.z, q.z - mx2), 0.0f);
-                unsigned vote = __ballot_sync(0xffffffffu, lane < n && !(fmaf(e0, e0, fmaf(e1, e1, e2b * e2b)) > 0.0f));
+                const bool in_box = lane < n && !(fmaf(e0, e0, fmaf(e1, e1, e2b * e2b)) > 0.0f);
+                unsigned vote = eps2 >= 1e-12f ? 0u : __ballot_sync(0xffffffffu, in_box);
                 while (vote) {
                     const int j = __ffs(vote) - 1;
                     vote &= vote - 1;

@@ -38,3 +38,32 @@ def test_sizes_agree_with_the_oracle(res, oracle, quad):
     if not quad:
         d = np.linalg.norm(want - ref, axis=1) / np.linalg.norm(ref, axis=1)
         assert np.median(d) < 1e-5
+
+
+# leaves of several bodies, at one place or closer than their keys tell apart, softened enough
+# that a body may meet itself in its leaf, and not; theta = 0 adds up every body by itself
+@pytest.mark.parametrize("soft", [0.0, 1e-20, 9e-7, 1.1e-6, 0.01])
+@pytest.mark.parametrize("n", [600, 40000, 130000])
+def test_bodies_of_a_shared_leaf(res, oracle, soft, n):
+    from particular_gb300 import AccelerationSoftened
+    r = np.random.RandomState(9)
+    x = r.normal(size=(n // 10, 3))
+    b = np.concatenate([np.repeat(x, 10, axis=0), r.uniform(0.5, 1.5, (n, 1))], 1).astype(np.float32)
+    near = r.uniform(-1, 1, (n, 3)) * (r.uniform(0, 1, (n, 1)) < 0.5)  # half of them at one place
+    b[:, :3] += (near * 2e-7).astype(np.float32)
+    m = cuda.BarnesHut(0.0, res, AccelerationSoftened(soft) if soft else Acceleration.checked())
+    got = m.compute(b)
+    g = m.export_tree()
+    shared = (g["links"][:, 2] < 0) | (g["links"][:, 3] > 1)
+    assert ((g["links"][:, 2] >= 0) & shared).sum() > n // 20
+    # a node whose centre of mass is a body's place is skipped whole for it, as the reference does
+    centres = {tuple(c) for c in g["com_mass"][shared, :3]}
+    pick = np.array([i for i in np.linspace(0, n - 1, 200).astype(int) if tuple(b[i, :3]) not in centres])
+    assert len(pick) > 100
+    want = oracle.bf_f64(b[pick], b, soft, True)
+    d = b[None, :, :3].astype(np.float64) - b[pick, None, :3].astype(np.float64)
+    r2 = (d * d).sum(-1)
+    scale = (b[None, :, 3] * np.sqrt(r2) / np.where(r2 > 0, r2 + float(np.float32(soft)) ** 2, 1.0) ** 1.5).sum(1)
+    # per pair 3 rsqrt factors (2^-22 each); a list's 128 entries in two packed halves
+    assert np.isfinite(got).all()
+    assert (np.abs(got[pick] - want).max(1) <= 1e-5 * scale).all()
