@@ -112,7 +112,7 @@ __device__ __forceinline__ void stage_tile(SoaTile &T, const float4 (&pre)[TILE 
 // N = 65536, the rest lost to operand reads and the two-sum folds). What else a call paid
 // for, and no longer does: the launch that laid the sources out, the coincidence test's
 // selects on every pair, and a scalar loop over the sources of a last, shorter tile
-// (1000003 targets x 3001 sources: unsoftened 1424 -> 1203 us, softened 1251 -> 1196; N =
+// (1000003 targets x 3001 sources: unsoftened 1424 -> 1229 us, softened 1251 -> 1200; N =
 // 4999 45 -> 38 us).
 
 // Four sources against a thread's K targets, in packed lo/hi partials.
@@ -138,47 +138,92 @@ __device__ __forceinline__ void tile_quad(const SoaTile &T, int q, const f2 (&xi
                    e2, ax, ay, az);
 }
 
+// One target's sum over a whole tile with the test for coincidence, by all lanes of a warp, eight
+// sources to a lane: every lane gets it.
+__device__ __forceinline__ void warp_tile(const SoaTile &T, float x, float y, float z, f2 e2, float &tx, float &ty,
+                                          float &tz) {
+    const f2 zero2 = pk2(0.f, 0.f);
+    const f2 xi[1] = {pk2(x, x)}, yi[1] = {pk2(y, y)}, zi[1] = {pk2(z, z)};
+    f2 ax[1] = {zero2}, ay[1] = {zero2}, az[1] = {zero2};
+#pragma unroll
+    for (int q = 0; q < TILE / 4; q += 32) tile_quad<1, true>(T, q + (threadIdx.x & 31), xi, yi, zi, e2, ax, ay, az);
+    float l, h;
+    upk2(ax[0], l, h);
+    tx = l + h;
+    upk2(ay[0], l, h);
+    ty = l + h;
+    upk2(az[0], l, h);
+    tz = l + h;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        tx += __shfl_xor_sync(0xffffffffu, tx, o);
+        ty += __shfl_xor_sync(0xffffffffu, ty, o);
+        tz += __shfl_xor_sync(0xffffffffu, tz, o);
+    }
+}
+
 // Adds a whole tile's partials to the targets' compensated sums and zeroes them.
 // GUARD (checked, eps == 0): tiles are evaluated without the test for coincidence, which
 // costs two selects per pair. A coincident pair then always makes the tile's sum NaN
 // (0 times an infinite s, or 0 times NaN), so only a tile whose sum is not finite is done
-// again with the test, by the threads that met it: one tile per target that is its own
-// source. A sum that is not finite for another reason comes out the same again.
+// again with the test. Where targets and sources have the same order, a warp's targets meet
+// themselves in one tile, and do it again side by side; where they do not, each meets itself in
+// another one, and up to ALONE of them are done one after the other, by the whole warp. A sum
+// that is not finite for another reason comes out so again. (Checked sums over the targets
+// in another order, us, side by side always / now, with the selects on every pair: N = 8192 79 /
+// AAA, 57.6; 16384 214 / BBB, 138; 131072 7351 / CCC, 7047.)
+constexpr int ALONE = 16;
+
 template <int K, bool GUARD>
 __device__ __forceinline__ void fold_tile(const SoaTile &T, const f2 (&xi)[K], const f2 (&yi)[K],
-                                         const f2 (&zi)[K], f2 e2, f2 (&ax)[K], f2 (&ay)[K], f2 (&az)[K],
-                                         float (&sx)[K], float (&sy)[K], float (&sz)[K], float (&cx)[K],
-                                         float (&cy)[K], float (&cz)[K]) {
+                                          const f2 (&zi)[K], f2 e2, f2 (&ax)[K], f2 (&ay)[K], f2 (&az)[K],
+                                          float (&sx)[K], float (&sy)[K], float (&sz)[K], float (&cx)[K],
+                                          float (&cy)[K], float (&cz)[K]) {
     const f2 zero2 = pk2(0.f, 0.f);
     float tx[K], ty[K], tz[K];
+    auto halves = [&]() {
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        float l, h;
-        upk2(ax[k], l, h);
-        tx[k] = l + h;
-        upk2(ay[k], l, h);
-        ty[k] = l + h;
-        upk2(az[k], l, h);
-        tz[k] = l + h;
-    }
+        for (int k = 0; k < K; ++k) {
+            float l, h;
+            upk2(ax[k], l, h);
+            tx[k] = l + h;
+            upk2(ay[k], l, h);
+            ty[k] = l + h;
+            upk2(az[k], l, h);
+            tz[k] = l + h;
+        }
+    };
+    halves();
     if (GUARD) {
-        bool redo = false;
+        unsigned met[K], any = 0;
 #pragma unroll
-        for (int k = 0; k < K; ++k) redo |= !(fabsf(tx[k]) + fabsf(ty[k]) + fabsf(tz[k]) <= FLT_MAX);
-        if (redo) {
+        for (int k = 0; k < K; ++k) {
+            met[k] = __ballot_sync(0xffffffffu, !(fabsf(tx[k]) + fabsf(ty[k]) + fabsf(tz[k]) <= FLT_MAX));
+            any |= met[k];
+        }
+        if (__popc(any) > ALONE) {
+            if ((any >> (threadIdx.x & 31)) & 1u) {
 #pragma unroll
-            for (int k = 0; k < K; ++k) ax[k] = ay[k] = az[k] = zero2;
+                for (int k = 0; k < K; ++k) ax[k] = ay[k] = az[k] = zero2;
 #pragma unroll 1
-            for (int q = 0; q < TILE / 4; ++q) tile_quad<K, true>(T, q, xi, yi, zi, e2, ax, ay, az);
+                for (int q = 0; q < TILE / 4; ++q) tile_quad<K, true>(T, q, xi, yi, zi, e2, ax, ay, az);
+                halves();
+            }
+        } else if (any) {
 #pragma unroll
             for (int k = 0; k < K; ++k) {
-                float l, h;
-                upk2(ax[k], l, h);
-                tx[k] = l + h;
-                upk2(ay[k], l, h);
-                ty[k] = l + h;
-                upk2(az[k], l, h);
-                tz[k] = l + h;
+                float x, y, z, unused;
+                upk2(xi[k], x, unused);
+                upk2(yi[k], y, unused);
+                upk2(zi[k], z, unused);
+#pragma unroll 1
+                for (unsigned m = met[k]; m; m &= m - 1) {
+                    const int j = __ffs(m) - 1;
+                    float ux, uy, uz;
+                    warp_tile(T, __shfl_sync(0xffffffffu, x, j), __shfl_sync(0xffffffffu, y, j),
+                              __shfl_sync(0xffffffffu, z, j), e2, ux, uy, uz);
+                    if (int(threadIdx.x & 31) == j) tx[k] = ux, ty[k] = uy, tz[k] = uz;
+                }
             }
         }
     }
@@ -203,7 +248,7 @@ __device__ __forceinline__ void two_sum_acc2(f2 &s, f2 &c, f2 t) {
 // packed sums, one half of which goes on from the targets' sums. Four sources a step, for a
 // short call waits on the steps' latency (5003 targets x 317 sources 7.2 us, two a step 7.7).
 // In plain runs of eight, only the runs' errors kept, 1000003 x 3001 took 1107 us where it
-// takes 1203, but the rms error was up to 0.9 % higher at 257 to 511 sources.
+// takes 1200, but the rms error was up to 0.9 % higher at 257 to 511 sources.
 template <int K, bool GUARD>
 __device__ __forceinline__ void each_source(const SoaTile &T, int cnt, const f2 (&xi)[K], const f2 (&yi)[K],
                                             const f2 (&zi)[K], f2 e2, float (&sx)[K], float (&sy)[K], float (&sz)[K],
@@ -271,7 +316,10 @@ __global__ void bf_fixup(const float4 *__restrict__ part, int n_aff, int slices,
 // Sources are read as rows and transposed on their way into shared memory, one tile ahead:
 // the next tile's rows are in registers while this tile is evaluated.
 // part (when non-null): [gridDim.y][2][n_aff] float4 = per-slice (sum, compensation).
-// NEXT: launched by launch_next (small calls: the wait at the start costs the compiled inner
+// NEXT: small calls. Their warps have few tiles to spread a second one over, so they test
+// every pair for coincidence (checked N = 512, same order / another, us: tiles done again 13.4 /
+// 17.6, selects 9.0 / 9.0; 1024 13.1 / 13.2, 8.6 / 8.6; 4096 27.7 / 28.8, 20.3 / 20.3). And they
+// are launched by launch_next (the wait at the start costs the compiled inner
 // loop some registers' worth of order, 127 -> 140 us at N = 16384, but a short call 2-3 us
 // less, 12.3 -> 9.4 at N = 1024).
 template <int K, bool GUARD, bool NEXT>
@@ -314,8 +362,8 @@ __global__ void __launch_bounds__(THREADS, K == 1 ? 8 : 1)
         const float4 *Z = reinterpret_cast<const float4 *>(T.c[2]);
         const float4 *M = reinterpret_cast<const float4 *>(T.c[3]);
 #pragma unroll 2
-        for (int q = 0; q < TILE / 4; ++q) quad<K, false>(X[q], Y[q], Z[q], M[q], xi2, yi2, zi2, e2, ax, ay, az);
-        fold_tile<K, GUARD>(T, xi2, yi2, zi2, e2, ax, ay, az, sx, sy, sz, cx, cy, cz);
+        for (int q = 0; q < TILE / 4; ++q) quad<K, GUARD && NEXT>(X[q], Y[q], Z[q], M[q], xi2, yi2, zi2, e2, ax, ay, az);
+        fold_tile<K, GUARD && !NEXT>(T, xi2, yi2, zi2, e2, ax, ay, az, sx, sy, sz, cx, cy, cz);
     }
     if (whole < ntiles) {  // the last, shorter tile
         SoaTile &T = tiles[whole & 1];

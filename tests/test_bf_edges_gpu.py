@@ -126,3 +126,35 @@ def test_no_source_behind_the_last_one(res, oracle, n_src, at):
     scale = np.linalg.norm(want[rest], axis=1)
     # one sum of at most 256 terms' rounding, rsqrt factors of 2^-22
     assert (np.linalg.norm(got[rest] - want[rest], axis=1) <= 1e-4 * scale + 1e-5 * n_src).all()
+
+
+# A target that is a source, anywhere in a warp and in any tile: few to a tile, so that a warp does
+# them one after the other, half a warp and more, and a warp's targets one by one in all tiles. Calls of
+# up to 4096 x 4096 pairs (more = 37) test every pair.
+@pytest.mark.parametrize("more", [37, 14037])
+@pytest.mark.parametrize("targets_per_thread", [1, 2, 4])
+@pytest.mark.parametrize("per_warp", [1, 15, 16, 17, 31, 32])
+def test_targets_meet_themselves_in_any_order(res, native_lib, oracle, targets_per_thread, per_warp, more):
+    from particular_gb300 import _native as N
+
+    src = bodies(1280, 5)
+    r = np.random.RandomState(per_warp)
+    spread = src[r.permutation(len(src))]  # a warp's targets in all five tiles
+    close = bodies(640, 6)
+    for w in range(0, 640, 32):  # some of a warp's targets in one tile
+        close[w + r.permutation(32)[:per_warp]] = src[256 * (w // 32 % 5) + r.permutation(256)[:per_warp]]
+    aff = np.concatenate([close, spread, bodies(more, 7)])
+    aff[3], src[1279, 3] = src[1279], 0.0  # and a massless one
+    try:
+        N.check(native_lib.pt_bf_set_plan(res.handle, targets_per_thread, 1))
+        got = cuda.BruteForce(res, Acceleration.checked()).compute(Between(aff, src))
+    finally:
+        N.check(native_lib.pt_bf_set_plan(res.handle, 0, 0))
+    assert np.isfinite(got).all()
+    aff, got = aff[:1957], got[:1957]
+    want = oracle.bf_f64(aff, src, 0.0, True)
+    d = src[None, :, :3].astype(np.float64) - aff[:, None, :3].astype(np.float64)
+    r2 = (d * d).sum(-1)
+    scale = (src[None, :, 3] * np.sqrt(r2) / np.where(r2 > 0, r2, 1.0) ** 1.5).sum(1)
+    # as above: 3 rsqrt factors a pair, at most 128 terms into each packed half
+    assert (np.abs(got - want).max(1) <= 1e-5 * scale).all()
