@@ -1069,7 +1069,8 @@ int build_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_src, int n) {
     DevBuf &nG = F64 ? S.nodeG64 : S.nodeG;
     cudaStream_t st = ctx->stream;
     const size_t N = size_t(n);
-    PT_TRY(ensure_buf(ctx, S.box_part, sizeof(T) * 6 * 1024));
+    const int nb = std::min(1024, blocks(n));  // of root_box
+    PT_TRY(ensure_buf(ctx, S.box_part, sizeof(T) * 6 * size_t(nb)));
     PT_TRY(ensure_buf(ctx, S.box, sizeof(T) * 8));
     PT_TRY(ensure_buf(ctx, S.keys, sizeof(uint64_t) * N));
     PT_TRY(ensure_buf(ctx, S.idx, sizeof(uint32_t) * N));
@@ -1101,7 +1102,6 @@ int build_t(pt_ctx *ctx, State &S, const typename Prec<T>::V4 *d_src, int n) {
 
     RadixFirst rf{};
     PT_TRY(radix_sort_prepare(ctx, S.prims, n, 3 * LEVELS, &rf));
-    const int nb = std::min(1024, blocks(n));
     int *counters = as<int>(S.counters);
     launch_next(root_box<T>, nb, 256, 0, st, d_src, n, as<T>(S.box_part), as<T>(S.box), rf.zero, rf.zero_words,
                 ctx->keep_errors ? nullptr : counters + 3, reinterpret_cast<unsigned *>(counters) + ROOT_BOX_DONE);

@@ -40,11 +40,13 @@ int ensure_buf(pt_ctx *ctx, DevBuf &b, size_t bytes) {
     if (bytes <= b.cap) return PT_OK;
     if (ctx->capturing)
         return set_error(PT_ERR_INVALID, "a buffer would grow during CUDA graph capture (%zu bytes)", bytes);
-    // Grow by 1/8 extra so slowly growing sizes do not reallocate every call.
+    // Grow by 1/8 extra so slowly growing sizes do not reallocate every call; under a capacity
+    // limit up to half of it only, so that the extra of a call's first buffers does not take the
+    // room of its last ones.
     size_t want = bytes + bytes / 8;
     want = (want + 255) & ~size_t(255);
     size_t after = ctx->bytes_held - b.cap + want;
-    if (ctx->capacity_limit && after > ctx->capacity_limit) {
+    if (ctx->capacity_limit && after > ctx->capacity_limit / 2) {
         want = bytes;
         after = ctx->bytes_held - b.cap + want;
         if (after > ctx->capacity_limit)

@@ -159,3 +159,27 @@ def test_large_trees_with_long_runs_are_in_key_order(res, spread, crowded):
     assert np.array_equal(count, np.unique(key, return_counts=True)[1])
     single = count == 1
     assert np.array_equal(g["com_mass"][~leaves][single], b[order[first[single]]])
+
+
+# bytes that an earlier build of the tree found enough, for bodies that are their own targets and
+# for separate targets
+@pytest.mark.parametrize("f64,separate,n,limit", [
+    (False, False, 1, 36700), (False, True, 1, 37100), (False, False, 513, 350600), (False, False, 16384, 9000000),
+    (True, False, 1, 64200), (True, True, 100, 138200), (True, False, 513, 403300), (True, True, 1000, 802100),
+    (True, False, 5000, 3225300), (True, True, 5000, 3754300), (True, False, 16384, 10821000),
+    (True, False, 65536, 43107700), (True, True, 65536, 48457900)])
+def test_a_call_fits_the_capacity_it_did(native_lib, f64, separate, n, limit):
+    from particular_gb300 import Between, CudaResources
+    r = np.random.RandomState(n)
+    b = np.concatenate([r.uniform(-1, 1, (n, 3)), np.ones((n, 1))], 1).astype(np.float64 if f64 else np.float32)
+    with CudaResources(0) as res:
+        m = cuda.BarnesHut(0.7, res, AccelerationSoftened(0.01), dvec3=f64)
+        want = m.compute(Between(b.copy(), b) if separate else b)
+    with CudaResources(0) as res:
+        res.set_capacity_limit(limit)
+        m = cuda.BarnesHut(0.7, res, AccelerationSoftened(0.01), dvec3=f64)
+        got = m.compute(Between(b.copy(), b) if separate else b)
+        assert native_lib.pt_ctx_device_bytes(res.handle) <= limit
+        # and again: nothing is left to grow
+        assert np.array_equal(got, m.compute(Between(b.copy(), b) if separate else b))
+    assert np.array_equal(got, want)
