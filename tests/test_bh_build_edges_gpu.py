@@ -183,3 +183,51 @@ def test_a_call_fits_the_capacity_it_did(native_lib, f64, separate, n, limit):
         # and again: nothing is left to grow
         assert np.array_equal(got, m.compute(Between(b.copy(), b) if separate else b))
     assert np.array_equal(got, want)
+
+
+# past 2^23 bodies, where the sort makes another pass, and past 2048 scan tiles of 4096: evenly
+# spread, and in knots that share the sorted bits
+@pytest.mark.parametrize("kind", ["cube", "knots"])
+def test_largest_trees_are_in_key_order(native_lib, kind):
+    import ctypes
+    import torch
+    from particular_gb300 import CudaResources, _native as N
+    n = (1 << 23) + 4097
+    g = torch.Generator(device="cuda")
+    g.manual_seed(8)
+    def rand(*shape):
+        return torch.rand(*shape, generator=g, device="cuda") * 2 - 1
+    b = torch.cat([rand(n, 3), (rand(n, 1) * 0.25 + 1) / n], 1)
+    if kind == "knots":  # of some 300 bodies, a quarter of a cell of the 16th level wide
+        k = torch.floor(rand(n // 300, 3) * 32000)[torch.randint(0, n // 300, (n,), generator=g, device="cuda")]
+        b[:, :3] = (k + 0.5) * 2.0 ** -15 + rand(n, 3) * 2.0 ** -18
+    b[0, :3], b[1, :3] = -1, 1  # the root box
+    lo, hi = torch.full((n, 3), -1.0, device="cuda"), torch.full((n, 3), 1.0, device="cuda")
+    key = torch.zeros(n, dtype=torch.int64, device="cuda")
+    for _ in range(21):  # the build's subdivision in its f32 ops
+        c = (lo + hi) * 0.5
+        left = b[:, :3] < c
+        hi, lo = torch.where(left, c, hi), torch.where(left, lo, c)
+        key = key * 8 + 7 - (left.long() * torch.tensor([1, 2, 4], device="cuda")).sum(1)
+    del lo, hi, c, left
+    order = torch.sort(key, stable=True)[1]
+    unique, counts = torch.unique_consecutive(key[order], return_counts=True)
+    torch.cuda.synchronize()
+    with CudaResources(0) as res:
+        N.check(native_lib.pt_bh_build_device(res.handle, b.data_ptr(), n, None))
+        res.synchronize()
+        st = N.BhStats()
+        N.check(native_lib.pt_bh_last_stats(res.handle, ctypes.byref(st)))
+        assert st.leaves == len(unique)
+        cm, ln = np.zeros((st.nodes, 4), np.float32), np.zeros((st.nodes, 4), np.int32)
+        N.check(native_lib.pt_bh_export_tree(res.handle, cm.ctypes.data, ln.ctypes.data, None, st.nodes))
+    leaves = ln[:, 2] >= 0
+    first, count = ln[leaves, 2].astype(np.int64), ln[leaves, 3].astype(np.int64)
+    assert np.array_equal(count, counts.cpu().numpy()) and np.array_equal(first, np.cumsum(count) - count)
+    single = count == 1
+    rows = b[order].cpu().numpy()[first[single]]
+    assert np.array_equal(cm[leaves][single], rows)
+    x = b.double()
+    M = x[:, 3].sum().item()
+    com = ((x[:, :3] * x[:, 3:]).sum(0) / M).cpu().numpy()
+    assert ln[0, 1] == st.nodes and abs(cm[0, 3] - M) <= 1e-6 * M and np.abs(cm[0, :3] - com).max() <= 1e-6
