@@ -485,6 +485,18 @@ static_assert(GW_FLAT >= 0 && GW_FLAT <= 1023, "flattened subtree size");
 #ifndef PT_GW_MINB
 #define PT_GW_MINB (GW_TPL == 1 ? 6 : 5)  // 4-warp CTAs per SM the register budget is set for
 #endif
+// A team's warps read the cells that they vote on from slots of their own; one warp alone from the
+// stack's free slots.
+template <int W>
+struct VoteSlots {
+    float4 vote[32];
+    __device__ __forceinline__ float4 *slots(int2 *) { return vote; }
+};
+template <>
+struct VoteSlots<1> {
+    __device__ __forceinline__ float4 *slots(int2 *free) { return reinterpret_cast<float4 *>(free); }
+};
+
 template <bool QUAD, bool GUARD, bool LEARNED, bool LOCAL, bool REL, int W>
 __global__ void __launch_bounds__(32 * W, (LOCAL ? PT_GW_LMINB : PT_GW_MINB) * 4 / W)
     bh_walk_group(const float4 *__restrict__ tbody, const uint32_t *__restrict__ tidx, int n_aff,
@@ -512,14 +524,19 @@ __global__ void __launch_bounds__(32 * W, (LOCAL ? PT_GW_LMINB : PT_GW_MINB) * 4
     // (W > 1: the warps have vote slots of their own.)
     constexpr int VOTE_SLACK = W > 1 ? 0 : 18;
     stack_cap = min(stack_cap, STK);
-    struct Shared {
+    struct Shared : VoteSlots<W> {
         CellList cells;
         BodyList bodies;
         float lx[LOCAL ? 19 : 1][32];
         float sums[QUAD && LOCAL ? 6 * GW_TPL : 1][32];
         int far[LOCAL ? 64 : 1];
-        float4 vote[W > 1 ? 32 : 1];
     };
+    // 20 warps per SM by shared memory too: 228 KB, of which a block takes 1 KB more than it
+    // declares, in steps of 128 bytes (16 bytes more, and 19 are resident: a whole call with the
+    // error bound at N = 4M takes 6040 us, and 5999 with 20)
+    static_assert(!(QUAD && LOCAL && W == 1) ||
+                      20 * ((sizeof(Shared) + sizeof(int2) * (STK + VOTE_SLACK) + 1024 + 127) / 128 * 128) <= 228 * 1024,
+                  "shared memory for 20 warps per SM");
     __shared__ __align__(16) int2 stack[STK + VOTE_SLACK];
     __shared__ __align__(16) Shared s_warp[W];
     __shared__ int s_push[W];
@@ -693,7 +710,7 @@ __global__ void __launch_bounds__(32 * W, (LOCAL ? PT_GW_LMINB : PT_GW_MINB) * 4
         bool marginal = false;
         // the cells to vote on are read back from the stack's free slots, two each
         unsigned amb = __ballot_sync(0xffffffffu, maybe && !sure);
-        float4 *voted = W > 1 ? my.vote : reinterpret_cast<float4 *>(stack + ((S + 1) & ~1));
+        float4 *voted = my.slots(stack + ((S + 1) & ~1));
         if (maybe && !sure) voted[__popc(amb & lt)] = make_float4(A.x, A.y, A.z, w * w);
         __syncwarp();
         for (int v = 0; amb; ++v) {
