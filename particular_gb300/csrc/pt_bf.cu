@@ -869,7 +869,9 @@ static void launch_fast(const Plan &p, bool guard, cudaStream_t st, const float4
 // Below this many targets the terms and the sum run in different warps (bf_ordered); from
 // here on a thread per target fills the chip and saves the trip through shared memory
 // (N = 50000: 4916 us ordered, 6233 a thread per target; N = 65535: 8238 and 9007; N =
-// 131071: 35452 and 25940).
+// 131071: 35452 and 25940). f64 sums, which the FP64 pipe bounds, are ordered at any size
+// (ordered / a thread per target, ms: N = 6007 2.24 / 7.50, 20000 25.0 / 46.8, 65536 259 /
+// 308, 100000 607 / 706).
 constexpr int ORD_MAX_AFF = 65536;
 
 template <class T, bool VEC3A>
@@ -1111,8 +1113,8 @@ int pt_bf_accel_dvec3(pt_ctx *ctx, const double *aff, size_t n_aff, const double
 }  // extern "C"
 
 // ---- allocation-free brute force ------------------------------------------
-// pt_bf_accel_f32_noalloc runs the same kernels as pt_bf_accel_f32_device
-// (bf_to_soa -> bf_fast -> bf_fixup) but takes its scratch from one file-scope
+// pt_bf_accel_f32_noalloc runs the same kernels as pt_bf_accel_f32_device (bf_fast, or
+// bf_to_soa -> bf_fast_ring, then bf_fixup) but takes its scratch from one file-scope
 // device array instead of context buffers, so a call never allocates device
 // memory. It serves callers that cannot call cudaMalloc: host programs that own
 // every byte of device memory through their own pool or fixed budget, and

@@ -2,7 +2,7 @@
 //
 // The tree is the reference's orthtree (particular/src/tree/mod.rs:91-138) built in
 // parallel instead of recursively:
-//  1. bbox_*   : the square root box of BoundingBox::square_with
+//  1. root_box : the square root box of BoundingBox::square_with
 //                (particular/src/tree/partition.rs:274-292), in the same f32 ops.
 //  2. make_keys: each body replays the reference's subdivision for 21 levels
 //                (centre = (min+max)/2, child bit = pos < centre, tree/mod.rs:116-124,

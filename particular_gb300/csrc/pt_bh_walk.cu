@@ -1104,7 +1104,11 @@ static GroupKernel group_kernel(bool quad, bool guard, bool learned, bool local,
 
 // Warps per group of the group walk. A group alone waits on its own loads and votes, so while
 // there are few groups several warps share each; once every SM has its 20 warps the team's
-// barriers only cost. Whole call at 1 / 2 / 4 / 8 / 16 warps, us: 79 groups (5003 probes of a
+// barriers only cost. The lines lie where calls of bodies that are their own targets turn (8 / 4
+// warps at 300, 340, 360 and 380 groups 218 / 241, 246 / 255, 265 / 260 and 258 / 252; 4 / 1 at 1563,
+// 1672 and 1673 546 / 534, 545 / 592 and 561 / 536; theta 0.6, quadrupoles); far-flung probes would
+// take the larger team for longer (8 / 4 at 381 groups 463 / 733, 4 / 1 at 1673 797 / 1241).
+// Whole call at 1 / 2 / 4 / 8 / 16 warps, us: 79 groups (5003 probes of a
 // 1M tree, theta 0.6, quadrupoles) 2141 / 1459 / 880 / 612 / 523; 157 groups (N = 10000) 329
 // / 296 / 260 / 244 / 235; 469 groups (N = 30000) 370 / 345 / 309 / 328 / 392; 1563 groups
 // (100003 probes) 1113 / 844 / 753 / 1001 / 1446; 2048 groups (N = 131072, theta 0.6) 678 /
@@ -1166,9 +1170,10 @@ static int place_groups(pt_ctx *ctx, State &S, int groups, const int **order) {
     return check_launch(ctx, "bh_group_order");
 }
 
-// The order of groups of `size` bodies by width over distance, or null while all start at once:
-// from 24 a SM on (20 or 24 are resident; N = 50000, 3125 groups of 16, took 237 us without and
-// 240 with it, N = 65536, 4096 groups, 266 and 265).
+// The order of groups of `size` bodies by width over distance, or null up to 24 a SM: 20 or 24
+// groups of one warp are resident (N = 50000, 3125 groups of 16, took 237 us without and 240 with
+// it, N = 65536, 4096 groups, 266 and 265). Groups walked by teams stay below the line and are not
+// ordered, although few teams start at once.
 static int order_groups(pt_ctx *ctx, State &S, const float4 *tbody, int n_aff, int size, const int **order) {
     const int sms = std::max(1, ctx->sm_count), groups = (n_aff + size - 1) / size;
     *order = nullptr;
@@ -1209,7 +1214,8 @@ int run(pt_ctx *ctx, const float4 *d_aff, int n_aff, const float4 *d_src, int n_
 
 // Lanes that share a body in bh_walk64. A warp of a small call is bound by its own FP64 latency,
 // so as many lanes, up to 16, as keep every warp resident at once (20 per SM by registers); once
-// the chip is full more lanes repeat the traversal but end more evenly. Whole host call, us, at
+// the chip is full more lanes repeat the traversal but end more evenly: which of the two counts
+// for more at a size depends on theta, by 1 to 4 % about the lines. Whole host call, us, at
 // 1 / 2 / 4 / 8 / 16 lanes: N = 2000 theta 0.6 - / - / 445 / 373 / 329, 5000 1206 / 787 / 589 /
 // 500 / 462, 10000 1462 / 895 / 712 / 651 / 693, 20000 1806 / 1258 / 1101 / 1132 / 1204; N = 50021
 // theta 0.5 3918 / 3413 / 3370, theta 0.9 1423 / 1395 / 1416; N = 100000 theta 0.5 7258 / 6923 /
@@ -1287,7 +1293,7 @@ int walk(pt_ctx *ctx, State &S, const float4 *tbody, const uint32_t *tidx, int n
         const int *gorder = nullptr;
         if (flags & PT_BH_RELATIVE) {
             PT_TRY(ensure_buf(ctx, S.gscale, sizeof(float) * size_t(groups)));
-            const bool ordered = groups > 20 * std::max(1, ctx->sm_count);  // more than start at once
+            const bool ordered = groups > 20 * std::max(1, ctx->sm_count);  // more than start at once by single warps
             launch_next(bh_group_scale, blocks(groups, 128), 128, 0, st, tbody, n_aff, as<float4>(S.nodeA),
                         as<int4>(S.nodeB), as<int>(S.counters), eps2, S.rel_alpha, as<float>(S.gscale));
             PT_TRY(check_launch(ctx, "bh_group_scale"));
